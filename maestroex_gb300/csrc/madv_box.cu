@@ -15,8 +15,8 @@ struct PPMBoxArgs {
     FabView s, u, T, F, DV, Ip, Im;
     int sc, uc, lo_ext, hi_ext, domlo, domhi;
     long long epsb;
-    double dt, dxd;
-    RecipC r6;
+    double dt;
+    RecipC rdx, r6;
 };
 
 __device__ __forceinline__ bool box_ijk(const RegionBox& r, int& i, int& j, int& k) {
@@ -46,7 +46,7 @@ __global__ void k_box_trace(PPMBoxArgs a) {
     int i, j, k;
     if (!box_ijk(a.r, i, j, k)) return;
     double A, B;
-    trace_coeffs(at(a.u, i, j, k, a.uc), a.dt, a.dxd, A, B);
+    trace_coeffs(at(a.u, i, j, k, a.uc), a.dt, a.rdx, A, B);
     at(a.T, i, j, k, 0) = A;
     at(a.T, i, j, k, 1) = B;
 }
@@ -193,7 +193,7 @@ int ppm_box_run(const madv_params& P, const madv_box* bx, const madv_fab* s, int
         a.hi_ext = hi_ext;
         a.domlo = P.dom_lo[d];
         a.domhi = P.dom_hi[d];
-        a.dxd = P.dx[d];
+        a.rdx = make_recip(P.dx[d]);
         a.u = view_of(*vel[d]);
         a.uc = 0;
         long t = 1;

@@ -18,6 +18,14 @@
 //    quotient is the correctly rounded one.  It holds while no intermediate underflows or
 //    overflows; zeros and |a| outside [2^-959, 2^977) take the IEEE division instead.
 //    Cost: 1 DMUL + 3 DFMA.
+//    By 6 the first step is already the quotient (div_6): with a = A 2^e the quotient is
+//    A/3 2^(e-1), and a third of an integer is never closer than 1/6 ulp to a rounding
+//    boundary, while a*zh + RN(a*zl) is off by 2^-106.  Cost: 1 DMUL + 1 DFMA.
+//
+// |x| and -x as plain expressions on the bit pattern are recognised by the compiler and
+// turned back into FP64 instructions (DADD 0 + |x|): k_dsvl ran 6 DADD per cell for its 3
+// differences.  dmag and dflip split the double into its two words with a mov, so that the
+// sign is handled on the integer pipe (64 instructions issue there for one FP64 instruction).
 #pragma once
 #include <cstdint>
 
@@ -27,6 +35,50 @@ constexpr long long SIGN_BIT = (long long)0x8000000000000000ULL;
 constexpr long long ABS_MASK = 0x7fffffffffffffffLL;
 
 __device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
+// the two words of x, and back
+__device__ __forceinline__ void dsplit(double x, int& hi, int& lo) {
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
+}
+__device__ __forceinline__ double djoin(int hi, int lo) {
+    double r;
+    asm("mov.b64 %0, {%1, %2};" : "=d"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ int dhigh(double x) {
+    int hi, lo;
+    dsplit(x, hi, lo);
+    return hi;
+}
+// bits of |x|
+__device__ __forceinline__ long long dmag(double x) {
+    int hi, lo;
+    dsplit(x, hi, lo);
+    long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi & 0x7fffffff));
+    return r;
+}
+// -x, and -x where f
+__device__ __forceinline__ double dflip(double x, bool f = true) {
+    int hi, lo;
+    dsplit(x, hi, lo);
+    return djoin(f ? hi ^ (int)0x80000000 : hi, lo);
+}
+__device__ __forceinline__ double dabs(double x) {
+    int hi, lo;
+    dsplit(x, hi, lo);
+    return djoin(hi & 0x7fffffff, lo);
+}
+// copysign(m, x) for m >= 0
+__device__ __forceinline__ double dsigned(double m, double x) {
+    int hi, lo;
+    dsplit(m, hi, lo);
+    return djoin(hi | (dhigh(x) & (int)0x80000000), lo);
+}
+// An integer that orders like x (both zeros 0; x not NaN): the magnitude, negated below 0.
+__device__ __forceinline__ long long dkey(double x) {
+    const long long s = (long long)(dhigh(x) >> 31);
+    return (dmag(x) ^ s) - s;
+}
 __host__ inline long long dbits_host(double x) {
     long long b;
     __builtin_memcpy(&b, &x, sizeof(b));
@@ -36,15 +88,15 @@ __host__ inline long long dbits_host(double x) {
 // x > 0.0
 __device__ __forceinline__ bool gt0(double x) { return dbits(x) > 0; }
 // x < 0.0 (-0 is not below 0): the pattern of -x is positive
-__device__ __forceinline__ bool lt0(double x) { return (dbits(x) ^ SIGN_BIT) > 0; }
+__device__ __forceinline__ bool lt0(double x) { return dbits(dflip(x)) > 0; }
 // |x| > 0.0
-__device__ __forceinline__ bool nz(double x) { return (dbits(x) & ABS_MASK) != 0; }
+__device__ __forceinline__ bool nz(double x) { return dmag(x) != 0; }
 // x > t, with tb = bits(t), t >= +0
 __device__ __forceinline__ bool gt_t(double x, long long tb) { return dbits(x) > tb; }
 // x < -t, with tb = bits(t), t >= +0
-__device__ __forceinline__ bool lt_negt(double x, long long tb) { return (dbits(x) ^ SIGN_BIT) > tb; }
+__device__ __forceinline__ bool lt_negt(double x, long long tb) { return dbits(dflip(x)) > tb; }
 // |x| > t, with tb = bits(t), t >= +0
-__device__ __forceinline__ bool abs_gt_t(double x, long long tb) { return (dbits(x) & ABS_MASK) > tb; }
+__device__ __forceinline__ bool abs_gt_t(double x, long long tb) { return dmag(x) > tb; }
 
 
 // 3. Scaling by 2 and by 1/2 on the bit pattern, equal to the FP multiply (round to nearest
@@ -53,28 +105,33 @@ __device__ __forceinline__ bool abs_gt_t(double x, long long tb) { return (dbits
 //    pattern 2a and x/2 the pattern RN(a/2); 2x past the largest finite double is infinity.
 //    Infinities and NaNs pass through.  No FP64 instruction is issued.
 __device__ __forceinline__ double twice(double x) {
-    const long long b = dbits(x), a = b & ABS_MASK, sg = b & SIGN_BIT;
+    int hi, lo;
+    dsplit(x, hi, lo);
+    const unsigned m = (unsigned)hi & 0x7fffffffu;
+    if (m - 0x00100000u < 0x7fd00000u) return djoin(hi + 0x00100000, lo);  // normal, and normal result
+    const long long b = dbits(x), a = dmag(x), sg = b & SIGN_BIT;
     long long r;
     if (a < (1LL << 52)) r = sg | (a << 1);                  // zero or subnormal
-    else if (a < (0x7feLL << 52)) r = b + (1LL << 52);       // normal result
     else if (a < (0x7ffLL << 52)) r = sg | (0x7ffLL << 52);  // overflow
     else r = b;                                              // infinity, NaN
     return __longlong_as_double(r);
 }
 __device__ __forceinline__ double half(double x) {
-    const long long b = dbits(x), a = b & ABS_MASK, sg = b & SIGN_BIT;
+    int hi, lo;
+    dsplit(x, hi, lo);
+    const unsigned m = (unsigned)hi & 0x7fffffffu;
+    if (m - 0x00200000u < 0x7fd00000u) return djoin(hi - 0x00100000, lo);  // normal result
+    const long long b = dbits(x), a = dmag(x), sg = b & SIGN_BIT;
     long long r;
-    if (a >= (0x7ffLL << 52)) r = b;                              // infinity, NaN
-    else if (a >= (2LL << 52)) r = b - (1LL << 52);               // normal result
-    else r = sg | ((a >> 1) + (a & (a >> 1) & 1));                // subnormal result, ties to even
+    if (a >= (0x7ffLL << 52)) r = b;                  // infinity, NaN
+    else r = sg | ((a >> 1) + (a & (a >> 1) & 1));    // subnormal result, ties to even
     return __longlong_as_double(r);
 }
 
 // Riemann upwinding of the reference:  v = (u > 0) ? l : r;  v = (|u| > t) ? v : (l+r)/2
 // (0.5 * x as half(x): the same bits, no FP64 multiply)
 __device__ __forceinline__ double upwind(double u, double l, double r, long long tb) {
-    const long long ub = dbits(u);
-    if ((ub & ABS_MASK) > tb) return ub > 0 ? l : r;
+    if (dmag(u) > tb) return dhigh(u) >= 0 ? l : r;
     return half(l + r);
 }
 
@@ -86,11 +143,12 @@ __device__ __forceinline__ double upwind(double u, double l, double r, long long
 //    case, decided by the signs alone); the rest compare the 106-bit significand product.
 //    Operands are not NaN.
 __device__ __forceinline__ bool prod_gt0(double x, double y) {
-    const long long bx = dbits(x), by = dbits(y);
-    const long long ax = bx & ABS_MASK, ay = by & ABS_MASK;
-    if ((bx ^ by) < 0 || ax == 0 || ay == 0) return false;
-    const int ex = (int)(ax >> 52), ey = (int)(ay >> 52);
+    const int hx = dhigh(x), hy = dhigh(y);
+    if ((hx ^ hy) < 0) return false;
+    const int ex = (int)(((unsigned)hx >> 20) & 0x7ff), ey = (int)(((unsigned)hy >> 20) & 0x7ff);
     if (ex >= 1 && ey >= 1 && ex + ey >= 972) return true;
+    const long long ax = dmag(x), ay = dmag(y);
+    if (ax == 0 || ay == 0) return false;
     if (ex == 0x7ff || ey == 0x7ff) return true;  // an infinity times a non-zero
     const unsigned long long mx = ex ? (unsigned long long)((ax & 0x000fffffffffffffLL) | (1LL << 52)) : ax;
     const unsigned long long my = ey ? (unsigned long long)((ay & 0x000fffffffffffffLL) | (1LL << 52)) : ay;
@@ -120,11 +178,55 @@ __host__ inline RecipC make_recip(double y) {
 }
 
 __device__ __forceinline__ double div_c(double a, const RecipC& r) {
-    const int ex = (int)((dbits(a) & ABS_MASK) >> 52);
+    const unsigned ex = ((unsigned)dhigh(a) >> 20) & 0x7ff;
     if (ex < 64 || ex >= 2000) return a / r.y;
     const double q0 = __fma_rn(a, r.zh, a * r.zl);
     const double rem = __fma_rn(-q0, r.y, a);
     return __fma_rn(rem, r.zh, q0);
+}
+
+// Division by a value y that several numerators share, formed on the device: the same
+// sequence with zh = RN(1/y) by the division and zl = RN(e zh), e = 1 - zh y exact (FMA), which
+// is 1/y - zh to a relative 2^-52.  ok: y is in a range where nothing under- or overflows.
+struct RecipV {
+    RecipC r;
+    bool ok;
+};
+__device__ __forceinline__ RecipV recip_v(double y) {
+    RecipV v;
+    const unsigned ex = ((unsigned)dhigh(y) >> 20) & 0x7ff;
+    v.ok = ex >= 823 && ex < 1223;  // 2^-200 .. 2^200
+    v.r.y = y;
+    v.r.zh = 1.0 / y;
+    v.r.zl = __fma_rn(-v.r.zh, y, 1.0) * v.r.zh;
+    return v;
+}
+__device__ __forceinline__ double div_v(double a, const RecipV& v) {
+    const unsigned ex = ((unsigned)dhigh(a) >> 20) & 0x7ff;
+    if (!v.ok || ex < 323 || ex >= 1723) return a / v.r.y;  // |a| outside 2^-700 .. 2^700
+    const double q0 = __fma_rn(a, v.r.zh, a * v.r.zl);
+    const double rem = __fma_rn(-q0, v.r.y, a);
+    return __fma_rn(rem, v.r.zh, q0);
+}
+
+// a / 6 with r6 = make_recip(6): exact for zeros too (zl > 0 keeps their sign)
+__device__ __forceinline__ double div_6(double a, const RecipC& r6) {
+    const unsigned ex = ((unsigned)dhigh(a) >> 20) & 0x7ff;
+    if ((ex < 64 && nz(a)) || ex >= 2000) return a / 6.0;
+    return __fma_rn(a, r6.zh, a * r6.zl);
+}
+
+// std::min(std::max(v, std::min(a, b)), std::max(a, b)) of the PPM interface clamp, the four
+// comparisons on integer keys: 3 keys and 4 comparisons cost about 35 integer instructions,
+// 4 FP64 comparisons the issue slots of 256.  v is an FP64 result of a and b: NaN if either
+// is, and passed on then.
+__device__ __forceinline__ double clamp_between(double v, double a, double b) {
+    if ((dhigh(v) & 0x7fffffff) > 0x7ff00000) return v;
+    const long long ka = dkey(a), kb = dkey(b), kv = dkey(v);
+    const bool ba = kb < ka, ab = ka < kb;
+    const double lo = ba ? b : a, hi = ab ? b : a;
+    const long long klo = ba ? kb : ka, khi = ab ? kb : ka;
+    return kv < klo ? lo : (khi < kv ? hi : v);
 }
 
 }  // namespace madv

@@ -266,10 +266,10 @@ __global__ void k_ppm_face(KARGS, int fs, int sc, int ff, int lo_ext, int hi_ext
 // (the reference forms them per component, cell and direction).
 // Face-centred velocity (the is_umac case): one (A, B) per D-face.
 template <int D>
-__global__ void k_trace_face(KARGS, int fu, int fout, double dt, double dxd) {
+__global__ void k_trace_face(KARGS, int fu, int fout, double dt, RecipC rdx) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     double A, B;
-    trace_coeffs(at(VW(fu), i, j, k), dt, dxd, A, B);
+    trace_coeffs(at(VW(fu), i, j, k), dt, rdx, A, B);
     const FabView o = VW(fout);
     at(o, i, j, k, 0) = A;
     at(o, i, j, k, 1) = B;
@@ -277,10 +277,10 @@ __global__ void k_trace_face(KARGS, int fu, int fout, double dt, double dxd) {
 
 // Cell-centred velocity (the velocity predictions): (A, B) per cell for each direction d,
 // from component d of the tracing velocity.
-__global__ void k_trace_cell(KARGS, int fu, double dt, double dx0, double dx1, double dx2) {
+__global__ void k_trace_cell(KARGS, int fu, double dt, RecipC dx0, RecipC dx1, RecipC dx2) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView u = VW(fu), o = VW(F_TRC);
-    const double dx[3] = {dx0, dx1, dx2};
+    const RecipC dx[3] = {dx0, dx1, dx2};
     for (int d = 0; d < 3; ++d) {
         double A, B;
         trace_coeffs(at(u, i, j, k, d), dt, dx[d], A, B);
@@ -510,9 +510,9 @@ void ppm_faces(Ctx& c, int d, int fs, int sc, int faces) {
 // tracing coefficients of the face velocity fields umac0..2 (or utrans0..2)
 static void trace_coeffs_faces(Ctx& c, int fu0) {
     // faces lo-1 .. hi+2 along d, cells lo-1 .. hi+1 across
-    launch(c, region(c, 1, 1, 1, 1, 1, 1, 0), 1, k_trace_face<0>, c.V(), fu0, F_TRA0, c.P.dt, c.P.dx[0]);
-    launch(c, region(c, 1, 1, 1, 1, 1, 1, 1), 1, k_trace_face<1>, c.V(), fu0 + 1, F_TRA1, c.P.dt, c.P.dx[1]);
-    launch(c, region(c, 1, 1, 1, 1, 1, 1, 2), 1, k_trace_face<2>, c.V(), fu0 + 2, F_TRA2, c.P.dt, c.P.dx[2]);
+    launch(c, region(c, 1, 1, 1, 1, 1, 1, 0), 1, k_trace_face<0>, c.V(), fu0, F_TRA0, c.P.dt, make_recip(c.P.dx[0]));
+    launch(c, region(c, 1, 1, 1, 1, 1, 1, 1), 1, k_trace_face<1>, c.V(), fu0 + 1, F_TRA1, c.P.dt, make_recip(c.P.dx[1]));
+    launch(c, region(c, 1, 1, 1, 1, 1, 1, 2), 1, k_trace_face<2>, c.V(), fu0 + 2, F_TRA2, c.P.dt, make_recip(c.P.dx[2]));
 }
 
 static void slope_any(Ctx& c, int d, int fs, int sc, int fout, int oc, int ncomp, const BCRecD* bcs_d, int bc_c0) {
@@ -611,7 +611,8 @@ void make_utrans(Ctx& c) {
     if (c.ndim == 2) return make_utrans_2d_entry(c);
     const double dt2 = 0.5 * c.P.dt;
     if (c.P.ppm_type != 0)
-        launch(c, rg_grow(c, 1), 1, k_trace_cell, c.V(), F_UFULL, c.P.dt, c.P.dx[0], c.P.dx[1], c.P.dx[2]);
+        launch(c, rg_grow(c, 1), 1, k_trace_cell, c.V(), F_UFULL, c.P.dt, make_recip(c.P.dx[0]),
+               make_recip(c.P.dx[1]), make_recip(c.P.dx[2]));
     for (int d = 0; d < 3; ++d) {
         if (c.P.ppm_type == 0) {
             slope_any(c, d, F_UTILDE, d, F_SLOPE, 0, 1, bcs_dev(c, BCS_U), d);
@@ -978,12 +979,20 @@ __global__ void k_es_simh(KARGS, int comp, int bclo, int bchi, int domlo, int do
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     constexpr int di = D == 0, dj = D == 1, dk = D == 2;
     const int I = D == 0 ? i : (D == 1 ? j : k);
-    double l = at(VW(F_IPC0), i - di, j - dj, k - dk, D), r = at(VW(F_IMC0), i, j, k, D);
-    if (I == domlo || I == domhi + 1) {
-        const FabView sc = VW(F_SOLD);
-        es_pred_bc(I, bclo, bchi, domlo, domhi, vclamp, at(sc, i - di, j - dj, k - dk, comp), at(sc, i, j, k, comp), l, r);
+    const double u = at(VW(F_UMAC0 + D), i, j, k);
+    const bool bnd = I == domlo || I == domhi + 1;
+    double v;
+    if (!bnd && nz(u)) {  // the one state that is taken
+        v = dhigh(u) >= 0 ? at(VW(F_IPC0), i - di, j - dj, k - dk, D) : at(VW(F_IMC0), i, j, k, D);
+    } else {
+        double l = at(VW(F_IPC0), i - di, j - dj, k - dk, D), r = at(VW(F_IMC0), i, j, k, D);
+        if (bnd) {
+            const FabView sc = VW(F_SOLD);
+            es_pred_bc(I, bclo, bchi, domlo, domhi, vclamp, at(sc, i - di, j - dj, k - dk, comp), at(sc, i, j, k, comp), l, r);
+        }
+        v = upwind(u, l, r, 0);  // tie test |u| > 0
     }
-    at(VW(F_SIMH0 + D), i, j, k) = upwind(at(VW(F_UMAC0 + D), i, j, k), l, r, 0);  // tie test |u| > 0
+    at(VW(F_SIMH0 + D), i, j, k) = v;
 }
 
 // MakeEdgeScalTransverse, 3-D (Source/MaestroMakeEdgeScalars.cpp:865-1359): D-faces
@@ -1000,6 +1009,25 @@ __global__ void __launch_bounds__(TPB, CONS ? 4 : 6) k_es_transverse(KARGS, int 
     const int il = i - di, jl = j - dj, kl = k - dk;
     const FabView st = VW(F_SIMH0 + T), sc = VW(F_SOLD), ut = VW(F_UMAC0 + T);
     auto simh = [&](int a, int bb, int cc) -> double { return at(st, a, bb, cc); };
+    const double ud = at(VW(F_UMAC0 + D), i, j, k);
+    if (I != domlo && I != domhi + 1 && dmag(ud) > epsb) {
+        // only the upwind side's state is taken: form that one (the other side's corrections,
+        // half of the FP64 work, are needed on domain faces and where |u| <= rel_eps alone)
+        const bool left = dhigh(ud) >= 0;
+        const int ci = left ? il : i, cj = left ? jl : j, ck = left ? kl : k;
+        double q;
+        if (INL) q = left ? at(VW(F_IPC0), ci, cj, ck, D) : at(VW(F_IMC0), ci, cj, ck, D);
+        else q = left ? at(VW(F_SL0 + D), i, j, k) : at(VW(F_SR0 + D), i, j, k);
+        if (CONS) {
+            const double s0 = at(sc, ci, cj, ck, comp), up = at(ut, ci + ti, cj + tj, ck + tk), um = at(ut, ci, cj, ck);
+            q = q - dt3h * (simh(ci + ti, cj + tj, ck + tk) * up - simh(ci, cj, ck) * um) -
+                dt3 * s0 * at(VW(F_DIVU), ci, cj, ck) + dt3h * s0 * (up - um);
+        } else {
+            q = q - at(VW(F_TCOEF), ci, cj, ck, T) * (simh(ci + ti, cj + tj, ck + tk) - simh(ci, cj, ck));
+        }
+        at(VW(Q_FIELD(D, T)), i, j, k) = q;
+        return;
+    }
     double sl, sr;
     if (INL) {
         es_pred_lr<D>(VW(F_IPC0), VW(F_IMC0), bclo, bchi, domlo, domhi, vclamp, i, j, k, sl, sr);
@@ -1046,7 +1074,7 @@ __global__ void __launch_bounds__(TPB, CONS ? 4 : 6) k_es_transverse(KARGS, int 
             rq = 0.0;
         }
     }
-    at(VW(Q_FIELD(D, T)), i, j, k) = upwind(at(VW(F_UMAC0 + D), i, j, k), lq, rq, epsb);
+    at(VW(Q_FIELD(D, T)), i, j, k) = upwind(ud, lq, rq, epsb);
 }
 
 // MakeEdgeScalEdges, 3-D (Source/MaestroMakeEdgeScalars.cpp:1361-1667).  Advective form:
@@ -1066,6 +1094,33 @@ __global__ void k_es_edges(KARGS, int comp, int force_zero, double dt2, double d
     const FabView q1 = VW(Q_FIELD(T1, T2)), q2 = VW(Q_FIELD(T2, T1));
     const FabView udf = VW(F_UMAC0 + D);
     const FabView sc = VW(F_SOLD);
+    const double ud = at(udf, i, j, k);
+    if (I != domlo && I != domhi + 1 && dmag(ud) > epsb) {  // the upwind side alone (see k_es_transverse)
+        const bool left = dhigh(ud) >= 0;
+        const int ci = left ? il : i, cj = left ? jl : j, ck = left ? kl : k;
+        double v;
+        if (INL) v = left ? at(VW(F_IPC0), ci, cj, ck, D) : at(VW(F_IMC0), ci, cj, ck, D);
+        else v = left ? at(VW(F_SL0 + D), i, j, k) : at(VW(F_SR0 + D), i, j, k);
+        const double q1p = at(q1, ci + a1i, cj + a1j, ck + a1k), q1m = at(q1, ci, cj, ck);
+        const double q2p = at(q2, ci + a2i, cj + a2j, ck + a2k), q2m = at(q2, ci, cj, ck);
+        double f = 0.0;
+        if (!force_zero) {
+            if (ptf) f = left ? at(VW(F_IPF), ci, cj, ck, D) : at(VW(F_IMF), ci, cj, ck, D);
+            else f = at(VW(F_SCALFORCE), ci, cj, ck, comp);
+        }
+        if (CONS) {
+            const FabView u1 = VW(F_UMAC0 + T1), u2 = VW(F_UMAC0 + T2);
+            v = v - dt2h1 * (q1p * at(u1, ci + a1i, cj + a1j, ck + a1k) - q1m * at(u1, ci, cj, ck)) -
+                dt2h2 * (q2p * at(u2, ci + a2i, cj + a2j, ck + a2k) - q2m * at(u2, ci, cj, ck)) -
+                dt2hd * at(sc, ci, cj, ck, comp) * (at(udf, ci + di, cj + dj, ck + dk) - at(udf, ci, cj, ck)) + dt2 * f;
+        } else {
+            const FabView tc = VW(F_TCOEF);
+            v = v - at(tc, ci, cj, ck, 3 + T1) * (q1p - q1m) - at(tc, ci, cj, ck, 3 + T2) * (q2p - q2m);
+            if (!force_zero) v = v + dt2 * f;
+        }
+        at(VW(F_SEDGE0 + D), i, j, k, oc) = v;
+        return;
+    }
     double sl, sr;
     if (INL) {
         es_pred_lr<D>(VW(F_IPC0), VW(F_IMC0), bclo, bchi, domlo, domhi, vclamp, i, j, k, sl, sr);
@@ -1102,7 +1157,7 @@ __global__ void k_es_edges(KARGS, int comp, int force_zero, double dt2, double d
             rq = rq + dt2 * (ptf ? at(VW(F_IMF), i, j, k, D) : at(f, i, j, k, comp));
         }
     }
-    double v = upwind(at(udf, i, j, k), lq, rq, epsb);
+    double v = upwind(ud, lq, rq, epsb);
     if (I == domlo) {
         if (bclo == BC_EXT_DIR) v = at(sc, il, jl, kl, comp);
         else if (bclo == BC_FOEXTRAP || bclo == BC_HOEXTRAP) v = vclamp ? mn(rq, 0.0) : rq;
@@ -1336,9 +1391,13 @@ void put_in_pert_form(Ctx& c, const double* d_s0, int comp, int flag) {
 __global__ void k_rhox_to_x(KARGS, int c0, int nc, int flag) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView s = VW(F_SOLD);
-    for (int comp = c0; comp < c0 + nc; ++comp) {
-        if (flag) at(s, i, j, k, comp) = at(s, i, j, k, comp) / at(s, i, j, k, RHO);
-        else at(s, i, j, k, comp) = at(s, i, j, k, comp) * at(s, i, j, k, RHO);
+    const double rho = at(s, i, j, k, RHO);
+    if (flag) {
+        // every species over the same rho: its reciprocal once, then 4 FP64 instructions each
+        const RecipV r = recip_v(rho);
+        for (int comp = c0; comp < c0 + nc; ++comp) at(s, i, j, k, comp) = div_v(at(s, i, j, k, comp), r);
+    } else {
+        for (int comp = c0; comp < c0 + nc; ++comp) at(s, i, j, k, comp) = at(s, i, j, k, comp) * rho;
     }
 }
 
@@ -1742,7 +1801,8 @@ __global__ void k_utrans_2dy(KARGS, int ppm_type, double dt2dy, int bclo, int bc
 static void make_utrans_2d(Ctx& c) {
     const double dt2 = 0.5 * c.P.dt;
     if (c.P.ppm_type != 0)
-        launch(c, rg2(c, 1), 1, k_trace_cell, c.V(), F_UFULL, c.P.dt, c.P.dx[0], c.P.dx[1], c.P.dx[2]);
+        launch(c, rg2(c, 1), 1, k_trace_cell, c.V(), F_UFULL, c.P.dt, make_recip(c.P.dx[0]),
+               make_recip(c.P.dx[1]), make_recip(c.P.dx[2]));
     for (int d = 0; d < 2; ++d) {
         if (c.P.ppm_type == 0) slope_any(c, d, F_UTILDE, d, F_SLOPE, 0, 1, bcs_dev(c, BCS_U), d);
         else ppm_any(c, d, F_UTILDE, d, c.bcs_u[d], F_UFULL, d, 0, F_IPC0 + d, F_IMC0 + d);
@@ -2024,8 +2084,8 @@ static void make_edge_scal_2d(Ctx& c, int start_comp, int num_comp, int which_bc
     const BCRecD* bh = bcs_host(c, which_bcs);
     const double dt2 = 0.5 * c.P.dt, dt4 = 0.25 * c.P.dt;
     if (c.P.ppm_type != 0) {
-        launch(c, region(c, 1, 1, 0, 1, 1, 0, 0), 1, k_trace_face<0>, c.V(), F_UMAC0, F_TRA0, c.P.dt, c.P.dx[0]);
-        launch(c, region(c, 1, 1, 0, 1, 1, 0, 1), 1, k_trace_face<1>, c.V(), F_UMAC1, F_TRA1, c.P.dt, c.P.dx[1]);
+        launch(c, region(c, 1, 1, 0, 1, 1, 0, 0), 1, k_trace_face<0>, c.V(), F_UMAC0, F_TRA0, c.P.dt, make_recip(c.P.dx[0]));
+        launch(c, region(c, 1, 1, 0, 1, 1, 0, 1), 1, k_trace_face<1>, c.V(), F_UMAC1, F_TRA1, c.P.dt, make_recip(c.P.dx[1]));
     }
     for (int comp = start_comp; comp < start_comp + num_comp; ++comp) {
         const BCRecD& bc = bh[comp];
@@ -2255,7 +2315,8 @@ void make_utrans_2d_entry(Ctx& c) { make_utrans_2d(c); }
 void vel_pred_prep(Ctx& c) {
     if (c.P.ppm_type == 0) return;
     const RegionTable& rt = c.ndim == 2 ? rg2(c, 1) : rg_grow(c, 1);
-    launch(c, rt, 1, k_trace_cell, c.V(), F_UFULL, c.P.dt, c.P.dx[0], c.P.dx[1], c.P.dx[2]);
+    launch(c, rt, 1, k_trace_cell, c.V(), F_UFULL, c.P.dt, make_recip(c.P.dx[0]),
+               make_recip(c.P.dx[1]), make_recip(c.P.dx[2]));
     for (int d = 0; d < c.ndim; ++d) ppm_any(c, d, F_UTILDE, d, c.bcs_u[d], F_UFULL, d, 0, F_IPC0 + d, F_IMC0 + d);
 }
 void vel_pred_2d_entry(Ctx& c) { vel_pred_2d(c); }

@@ -11,22 +11,23 @@ namespace madv {
 // S(m): the field at cell (index + m) along direction D.
 #define SHIFT_S(s, sc) [&](int m) -> double { return at(s, i + m * di, j + m * dj, k + m * dk, sc); }
 
+// Van Leer slope from the differences c = s(1) - s(-1), l = s(0) - s(-1), r = s(1) - s(0)
+// (Source/MaestroPPM.cpp:37-73): dsc = c/2, dsl = 2l, dsr = 2r, and if (dsl*dsr > 0)
+// copysign(1, dsc) * min(|dsc|, min(|dsl|, |dsr|)).  The minimum of non-negative (finite)
+// doubles is the minimum of their bit patterns, and copysign(1, dsc) * m with m >= 0 is m
+// with the sign of dsc.  No FP64 instruction.
+__device__ __forceinline__ double vl_slope(double c, double l, double r) {
+    const double dsl = twice(l), dsr = twice(r);
+    if (!prod_gt0(dsl, dsr)) return 0.0;
+    return dsigned(__longlong_as_double(min(dmag(half(c)), min(dmag(dsl), dmag(dsr)))), c);
+}
+
 // Van Leer slope of cell (i,j,k) along D (Source/MaestroPPM.cpp:37-73).
 template <int D>
 __device__ __forceinline__ double ppm_dsvl(const FabView& s, int sc, int i, int j, int k) {
     constexpr int di = D == 0, dj = D == 1, dk = D == 2;
     auto S = SHIFT_S(s, sc);
-    const double dsc = half(S(1) - S(-1));
-    const double dsl = twice(S(0) - S(-1));
-    const double dsr = twice(S(1) - S(0));
-    // reference: if (dsl*dsr > 0) dsvl = copysign(1,dsc) * min(|dsc|, min(|dsl|, |dsr|)).
-    // The minimum of non-negative (finite) doubles is the minimum of their bit patterns, and
-    // copysign(1, dsc) * m with m >= 0 is m with the sign of dsc.
-    if (!prod_gt0(dsl, dsr)) return 0.0;
-    long long m = dbits(dsc) & ABS_MASK;
-    m = min(m, dbits(dsl) & ABS_MASK);
-    m = min(m, dbits(dsr) & ABS_MASK);
-    return __longlong_as_double(m | (dbits(dsc) & SIGN_BIT));
+    return vl_slope(S(1) - S(-1), S(0) - S(-1), S(1) - S(0));
 }
 
 // Interior fourth-order limited face value (ppm_type 2), face between cells c+m-1 and c+m.
@@ -39,13 +40,16 @@ __device__ __forceinline__ double ppm2_face_regular(const FabView& s, int sc, in
     double se = (7.0 / 12.0) * (S(m - 1) + S(m)) - (1.0 / 12.0) * (S(m - 2) + S(m + 1));
     // reference: (se - s(m-1)) * (s(m) - se) < 0, i.e. the product of (se - s(m-1)) and
     // -(s(m) - se) = se - s(m) (exact) is positive
-    if (prod_gt0(se - S(m - 1), se - S(m))) {
-        double D2 = 3.0 * (S(m - 1) - 2.0 * se + S(m));
-        double D2L = S(m - 2) - 2.0 * S(m - 1) + S(m);
-        double D2R = S(m - 1) - 2.0 * S(m) + S(m + 1);
-        double sgn = copysign(1.0, D2);
-        double D2LIM = sgn * mx(mn(C * sgn * D2L, mn(C * sgn * D2R, sgn * D2)), 0.0);
-        se = half(S(m - 1) + S(m)) - div_c(D2LIM, r6);
+    // the differences have the sign of the comparison (on integer keys, no FP64 instruction);
+    // equal signs -- se outside its two cells -- are rare, and only then the product is looked at
+    const long long ks = dkey(se), ka = dkey(S(m - 1)), kb = dkey(S(m));
+    if (((ks > ka && ks > kb) || (ks < ka && ks < kb)) && prod_gt0(se - S(m - 1), se - S(m))) {
+        double D2 = 3.0 * (S(m - 1) - twice(se) + S(m));
+        double D2L = S(m - 2) - twice(S(m - 1)) + S(m);
+        double D2R = S(m - 1) - twice(S(m)) + S(m + 1);
+        const bool neg = dhigh(D2) < 0;  // sgn = copysign(1, D2): sgn * x is x or -x
+        double D2LIM = dflip(mx(mn(C * dflip(D2L, neg), mn(C * dflip(D2R, neg), dabs(D2))), 0.0), neg);
+        se = half(S(m - 1) + S(m)) - div_6(D2LIM, r6);
     }
     return se;
 }
@@ -76,9 +80,7 @@ __device__ __forceinline__ double ppm_face_value(const FabView& s, int sc, const
     } else if (PPMT == 1) {
         const double dvl = at(dv, i - di, j - dj, k - dk);
         const double dvr = at(dv, i, j, k);
-        v = half(S(0) + S(-1)) - div_c(dvr - dvl, r6);
-        v = mx(v, mn(S(0), S(-1)));
-        v = mn(v, mx(S(0), S(-1)));
+        v = clamp_between(half(S(0) + S(-1)) - div_6(dvr - dvl, r6), S(0), S(-1));
     } else {
         v = ppm2_face_regular<D>(s, sc, i, j, k, 0, r6);
     }
@@ -87,10 +89,14 @@ __device__ __forceinline__ double ppm_face_value(const FabView& s, int sc, const
 
 // Characteristic-tracing coefficients (Source/MaestroPPM.cpp:209-251):
 // sigma = |u| dt / dx, A = 0.5 sigma, B = 1 - 2/3 sigma.
-__device__ __forceinline__ void trace_coeffs(double u, double dt, double dxd, double& A, double& B) {
-    const double sigma = fabs(u) * dt / dxd;
-    A = 0.5 * sigma;
+__device__ __forceinline__ void trace_coeffs(double u, double dt, const RecipC& rdx, double& A, double& B) {
+    const double sigma = div_c(dabs(u) * dt, rdx);
+    A = half(sigma);
     B = 1.0 - 2.0 / 3.0 * sigma;
+}
+
+__device__ __forceinline__ bool finite2(double a, double b) {
+    return (dhigh(a) & 0x7ff00000) != 0x7ff00000 && (dhigh(b) & 0x7ff00000) != 0x7ff00000;
 }
 
 // Edge values sm, sp of cell (i,j,k) along D from the face values F (quadratic limiter
@@ -115,9 +121,7 @@ __device__ __forceinline__ void ppm_cell_edges(const FabView& s, int sc, const F
             if (PPMT == 2) return ppm2_face_regular<D>(s, sc, i, j, k, m, r6);
             const double dvl = at(dv, i + (m - 1) * di, j + (m - 1) * dj, k + (m - 1) * dk);
             const double dvr = at(dv, i + m * di, j + m * dj, k + m * dk);
-            double v = half(S(m) + S(m - 1)) - div_c(dvr - dvl, r6);
-            v = mx(v, mn(S(m), S(m - 1)));
-            return mn(v, mx(S(m), S(m - 1)));
+            return clamp_between(half(S(m) + S(m - 1)) - div_6(dvr - dvl, r6), S(m), S(m - 1));
         }
         return at(F, i + m * di, j + m * dj, k + m * dk);
     };
@@ -130,13 +134,18 @@ __device__ __forceinline__ void ppm_cell_edges(const FabView& s, int sc, const F
             // reference: (sp-s0)*(s0-sm) <= 0;  |sp-s0| >= 2|sm-s0|;  |sm-s0| >= 2|sp-s0|.
             // sm-s0 = -(s0-sm) exactly; non-negative doubles compare like their bit patterns.
             const double a = sp - s0, q = s0 - sm;
+            const long long ma = dmag(a), mq = dmag(q);
             if (!prod_gt0(a, q)) {
                 sp = s0;
                 sm = s0;
-            } else if ((dbits(a) & ABS_MASK) >= (dbits(twice(q)) & ABS_MASK)) {
-                sp = 3.0 * s0 - twice(sm);
-            } else if ((dbits(q) & ABS_MASK) >= (dbits(twice(a)) & ABS_MASK)) {
-                sm = 3.0 * s0 - twice(sp);
+            } else {
+                // the two cases as one expression, so that a warp with both issues it once
+                const bool up = ma >= dmag(twice(q)), dn = mq >= dmag(twice(a));
+                if (up || dn) {
+                    const double v = 3.0 * s0 - twice(up ? sm : sp);
+                    if (up) sp = v;
+                    else sm = v;
+                }
             }
         }
     } else {
@@ -155,61 +164,51 @@ __device__ __forceinline__ void ppm_cell_edges(const FabView& s, int sc, const F
             double alpham = sedge - s0;
             // |alphap| > 2|alpham| and |alpham| > 2|alphap| on magnitudes' bit patterns;
             // alpham * alphap >= 0 is "not (alpham * -alphap > 0)"
-            const bool bigp = (dbits(alphap) & ABS_MASK) > (dbits(twice(alpham)) & ABS_MASK);
-            const bool bigm = (dbits(alpham) & ABS_MASK) > (dbits(twice(alphap)) & ABS_MASK);
+            const long long mp = dmag(alphap), mm = dmag(alpham);
+            const bool bigp = mp > dmag(twice(alpham));
+            const bool bigm = mm > dmag(twice(alphap));
             bool extremum = false;
-            if (!prod_gt0(alpham, -alphap)) {
+            if (!prod_gt0(alpham, dflip(alphap))) {
                 extremum = true;
             } else if (bigp || bigm) {
                 double dafacem = sedge - sedgel;
                 double dafacep = sedgerr - sedger;
                 double dabarm = s0 - S(-1);
                 double dabarp = S(1) - s0;
-                double dafacemin = mn(fabs(dafacem), fabs(dafacep));
-                double dabarmin = mn(fabs(dabarm), fabs(dabarp));
-                double dachkm, dachkp;
-                if (dafacemin >= dabarmin) {
-                    dachkm = dafacem;
-                    dachkp = dafacep;
-                } else {
-                    dachkm = dabarm;
-                    dachkp = dabarp;
-                }
-                extremum = !prod_gt0(dachkm, dachkp);
+                const bool face = min(dmag(dafacem), dmag(dafacep)) >= min(dmag(dabarm), dmag(dabarp));
+                extremum = !prod_gt0(face ? dafacem : dabarm, face ? dafacep : dabarp);
             }
             if (extremum) {
                 double D2 = 6.0 * (alpham + alphap);
-                double D2L = S(-2) - 2.0 * S(-1) + s0;
-                double D2R = s0 - 2.0 * S(1) + S(2);
-                double D2C = S(-1) - 2.0 * s0 + S(1);
-                double sgn = copysign(1.0, D2);
-                double D2LIM = mx(mn(sgn * D2, mn(C * sgn * D2L, mn(C * sgn * D2R, C * sgn * D2C))), 0.0);
-                double D2ABS = mx(fabs(D2), 1.e-10);
-                alpham = alpham * D2LIM / D2ABS;
-                alphap = alphap * D2LIM / D2ABS;
-            } else {
-                if (bigp) {
-                    double sgn = copysign(1.0, alpham);
-                    double amax = -alphap * alphap / (4.0 * (alpham + alphap));
-                    double delam = S(-1) - s0;
-                    if (sgn * amax >= sgn * delam) {
-                        if (sgn * (delam - alpham) >= 1.e-10) {
-                            alphap = -2.0 * delam - 2.0 * sgn * sqrt(delam * delam - delam * alpham);
-                        } else {
-                            alphap = -2.0 * alpham;
-                        }
-                    }
+                double D2L = S(-2) - twice(S(-1)) + s0;
+                double D2R = s0 - twice(S(1)) + S(2);
+                double D2C = S(-1) - twice(s0) + S(1);
+                const bool neg = dhigh(D2) < 0;  // sgn = copysign(1, D2)
+                double D2LIM = mx(mn(dabs(D2), mn(C * dflip(D2L, neg), mn(C * dflip(D2R, neg), C * dflip(D2C, neg)))), 0.0);
+                if (nz(D2LIM) || !finite2(alpham, alphap)) {
+                    double D2ABS = mx(dabs(D2), 1.e-10);
+                    alpham = alpham * D2LIM / D2ABS;
+                    alphap = alphap * D2LIM / D2ABS;
+                } else {  // a finite alpha times 0 over a positive number: the zero of its sign
+                    alpham = dsigned(0.0, alpham);
+                    alphap = dsigned(0.0, alphap);
                 }
-                if (bigm) {
-                    double sgn = copysign(1.0, alphap);
-                    double amax = -alpham * alpham / (4.0 * (alpham + alphap));
-                    double delap = S(1) - s0;
-                    if (sgn * amax >= sgn * delap) {
-                        if (sgn * (delap - alphap) >= bigm_tol) {
-                            alpham = (-2.0 * delap - 2.0 * sgn * sqrt(delap * delap - delap * alphap));
-                        } else {
-                            alpham = -2.0 * alphap;
-                        }
+            } else {
+                // |alphap| > 2|alpham| and |alpham| > 2|alphap| exclude each other: the two
+                // one-sided rewrites as one, on (a, b) = (alpham, alphap) or (alphap, alpham), so
+                // that a warp with both issues the division and the square root once
+                if (bigp || bigm) {
+                    const double a = bigp ? alpham : alphap, b = bigp ? alphap : alpham;
+                    const bool neg = dhigh(a) < 0;  // sgn = copysign(1, a)
+                    const double tol = bigp ? 1.e-10 : bigm_tol;
+                    const double amax = dflip(b) * b / twice(twice(alpham + alphap));
+                    const double del = (bigp ? S(-1) : S(1)) - s0;
+                    if (dflip(amax, neg) >= dflip(del, neg)) {
+                        double v = dflip(twice(a));
+                        if (dflip(del - a, neg) >= tol)
+                            v = dflip(twice(del)) - dflip(twice(sqrt(del * del - del * a)), neg);
+                        if (bigp) alphap = v;
+                        else alpham = v;
                     }
                 }
             }
@@ -219,15 +218,27 @@ __device__ __forceinline__ void ppm_cell_edges(const FabView& s, int sc, const F
     }
 }
 
+__device__ __forceinline__ double trace_side(double sm, double sp, double d, double s6, double A, double B, bool p) {
+    return (p ? sp : sm) + dflip(A * (d + dflip(B * s6, p)), p);
+}
+
 // Characteristic tracing of one cell: Ip from the velocity at the high face (coefficients
 // Ap, Bp), Im from the low face (Am, Bm); tb = bits(rel_eps).
 __device__ __forceinline__ void ppm_trace(double s0, double sm, double sp, double up, double um, double Ap, double Bp,
                                           double Am, double Bm, long long tb, double& ip, double& im) {
-    const double s6 = 6.0 * s0 - 3.0 * (sm + sp);
+    // ip = sp - Ap (sp - sm - Bp s6) where up > rel_eps, im = sm + Am (sp - sm + Bm s6) where
+    // um < -rel_eps; x - y is x + (-y), so both are one expression up to signs, issued once
+    // for a warp whose lanes need the one or the other (a cell that needs both -- flow out
+    // through both faces -- takes a second turn)
     ip = s0;
     im = s0;
-    if (gt_t(up, tb)) ip = sp - Ap * (sp - sm - Bp * s6);
-    if (lt_negt(um, tb)) im = sm + Am * (sp - sm + Bm * s6);
+    const bool p = gt_t(up, tb), m = lt_negt(um, tb);
+    if (!p && !m) return;
+    const double s6 = 6.0 * s0 - 3.0 * (sm + sp), d = sp - sm;
+    const double v = trace_side(sm, sp, d, s6, p ? Ap : Am, p ? Bp : Bm, p);
+    if (p) ip = v;
+    else im = v;
+    if (p && m) im = trace_side(sm, sp, d, s6, Am, Bm, false);
 }
 
 }  // namespace madv

@@ -64,7 +64,7 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
 
 // Random doubles with exponents spread over [2^-1000, 2^1000], both signs, plus
 // zeros, subnormals and values next to powers of two; each checked bit for bit.
-__global__ void k_selftest(unsigned long long n, unsigned long long seed, RecipC r, double thr,
+__global__ void k_selftest(unsigned long long n, unsigned long long seed, RecipC r, RecipC r6, double thr,
                            unsigned long long* fails) {
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -113,6 +113,21 @@ __global__ void k_selftest(unsigned long long n, unsigned long long seed, RecipC
         if (ey > 2046) ey = 2046;
         const double yv = __longlong_as_double((long long)((h2 & 0x800fffffffffffffULL) | ((unsigned long long)ey << 52)));
         if (prod_gt0(e, yv) != (e * yv > 0.0)) ++local;
+        // division by 6 and by a run-time value, signs and magnitudes, the ordering key and
+        // the interface clamp (b next to a, or of its own; c between them or outside)
+        if (dbits(div_6(e, r6)) != dbits(e / 6.0)) ++local;
+        if (yv != 0.0 && dbits(div_v(e, recip_v(yv))) != dbits(e / yv)) ++local;
+        const double y1 = __longlong_as_double((dbits(yv) & ~(0x7ffLL << 52)) | ((1000LL + (ey & 63)) << 52));
+        const double e1 = __longlong_as_double((dbits(e) & ~(0x7ffLL << 52)) | ((1000LL + (ex & 63)) << 52));
+        if (dbits(div_v(e1, recip_v(y1))) != dbits(e1 / y1)) ++local;
+        if (dbits(dflip(e)) != dbits(-e) || dbits(dabs(e)) != dbits(fabs(e))) ++local;
+        if (dbits(dsigned(fabs(e), yv)) != dbits(copysign(e, yv))) ++local;
+        const double b = (h2 & 0x400000) ? yv : __longlong_as_double(dbits(e) ^ (long long)((h2 >> 40) & 3));
+        const double c = (h2 & 0x800000) ? 0.5 * e + 0.5 * b : a;
+        if ((dkey(e) < dkey(b)) != (e < b) || (dkey(b) < dkey(c)) != (b < c)) ++local;
+        const double lo = (b < e) ? b : e, hi = (e < b) ? b : e;
+        const double m1 = (c < lo) ? lo : c, m2 = (hi < m1) ? hi : m1;
+        if (dbits(clamp_between(c, e, b)) != dbits(m2)) ++local;
     }
     if (local) atomicAdd(fails, local);
 }
@@ -128,7 +143,8 @@ extern "C" int madv_selftest_exact(double y, double threshold, long long n, long
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    madv::k_selftest<<<nsm * 8, 256, 0, s>>>((unsigned long long)n, 0x1234567ULL, madv::make_recip(y), threshold, d);
+    madv::k_selftest<<<nsm * 8, 256, 0, s>>>((unsigned long long)n, 0x1234567ULL, madv::make_recip(y), madv::make_recip(6.0),
+                                               threshold, d);
     unsigned long long h = 0;
     cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, s);
     cudaStreamSynchronize(s);
