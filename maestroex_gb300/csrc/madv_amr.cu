@@ -194,11 +194,7 @@ static const RegionTable& shell_table(Ctx& c, int ng, int nodal) {
         }
     }
     t.total = start;
-    if (!t.h.empty()) {
-        if (cudaMalloc(&t.d, sizeof(RegionBox) * t.h.size()) != cudaSuccess ||
-            cudaMemcpy(t.d, t.h.data(), sizeof(RegionBox) * t.h.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-            throw Fail{MADV_ERR_CUDA};
-    }
+    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -236,11 +232,7 @@ static const RegionTable& down_table(Ctx& cf, const Ctx& cc, int nodal) {
         }
     }
     t.total = start;
-    if (!t.h.empty()) {
-        if (cudaMalloc(&t.d, sizeof(RegionBox) * t.h.size()) != cudaSuccess ||
-            cudaMemcpy(t.d, t.h.data(), sizeof(RegionBox) * t.h.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-            throw Fail{MADV_ERR_CUDA};
-    }
+    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -375,10 +367,7 @@ static const RegionTable& reg_table(Ctx& cf, int o) {
         t.h.push_back(r);
     }
     t.total = start;
-    if (!cuda_ok(cudaMalloc(&t.d, sizeof(RegionBox) * t.h.size()), "cudaMalloc(register table)") ||
-        !cuda_ok(cudaMemcpy(t.d, t.h.data(), sizeof(RegionBox) * t.h.size(), cudaMemcpyHostToDevice),
-                 "cudaMemcpy(register table)"))
-        throw Fail{MADV_ERR_CUDA};
+    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
     return t;
 }
 

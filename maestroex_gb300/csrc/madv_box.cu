@@ -122,6 +122,7 @@ static RegionBox rbox(const int lo[3], const int hi[3]) {
         r.lo[d] = lo[d];
         r.n[d] = hi[d] - lo[d] + 1;
     }
+    r.dv = piece_div(r.n);
     return r;
 }
 

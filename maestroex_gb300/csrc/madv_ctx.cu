@@ -77,11 +77,7 @@ const RegionTable& region(Ctx& c, int glo0, int glo1, int glo2, int ghi0, int gh
         }
     }
     t.total = start;
-    if (!t.h.empty()) {
-        if (cudaMalloc(&t.d, sizeof(RegionBox) * t.h.size()) != cudaSuccess ||
-            cudaMemcpy(t.d, t.h.data(), sizeof(RegionBox) * t.h.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-            throw Fail{MADV_ERR_CUDA};
-    }
+    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -188,11 +184,7 @@ const CopyTable& copy_table(Ctx& c, int ng, int nodal) {
         }
     }
     t.total = start;
-    if (!t.h.empty()) {
-        if (cudaMalloc(&t.d, sizeof(CopyDesc) * t.h.size()) != cudaSuccess ||
-            cudaMemcpy(t.d, t.h.data(), sizeof(CopyDesc) * t.h.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-            throw Fail{MADV_ERR_CUDA};
-    }
+    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, COPY_HINT);
     return t;
 }
 

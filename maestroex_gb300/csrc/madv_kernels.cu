@@ -71,20 +71,9 @@ __global__ void k_fill_boundary(const CopyDesc* __restrict__ D, int nd, long tot
                                 int nb, int f, int c0, int nc) {
     const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= total) return;
-    int lo = 0, hi = nd - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (D[mid].start <= gid) lo = mid;
-        else hi = mid - 1;
-    }
-    const CopyDesc& cd = D[lo];
-    long l = gid - cd.start;
-    const long nx = cd.n[0], ny = cd.n[1];
-    const long q = l / nx;
-    const int i = cd.lo[0] + (int)(l - q * nx);
-    const long q2 = q / ny;
-    const int j = cd.lo[1] + (int)(q - q2 * ny);
-    const int k = cd.lo[2] + (int)q2;
+    const CopyDesc& cd = D[find_piece<COPY_HINT>(D, nd, gid)];
+    int i, j, k;
+    piece_ijk(cd.lo, cd.n, cd.dv, gid - cd.start, i, j, k);
     const FabView dst = V[f * nb + cd.dst_b];
     const FabView src = V[f * nb + cd.src_b];
     for (int n = c0; n < c0 + nc; ++n)

@@ -49,6 +49,7 @@ extern "C" int madv_probe_fp64_peak(double* tflops, void* stream) {
     return MADV_OK;
 }
 
+#include "madv_core.cuh"
 #include "madv_exact.cuh"
 
 namespace madv {
@@ -128,6 +129,18 @@ __global__ void k_selftest(unsigned long long n, unsigned long long seed, RecipC
         const double lo = (b < e) ? b : e, hi = (e < b) ? b : e;
         const double m1 = (c < lo) ? lo : c, m2 = (hi < m1) ? hi : m1;
         if (dbits(clamp_between(c, e, b)) != dbits(m2)) ++local;
+        // a piece's extents by their reciprocals: small, even, prime and long extents, and elements
+        // at and next to the multiples of each
+        const int lim = 1 << (1 + (int)((h2 >> 44) & 9));
+        const int pn[3] = {1 + (int)(h % lim), 1 + (int)((h2 >> 17) % (unsigned)lim), 1 + (int)((h >> 33) & 3)};
+        const long tot = (long)pn[0] * pn[1] * pn[2];
+        long l = (long)((h ^ h2) % (unsigned long long)tot);
+        if (h2 & 0x1000000) l = l / pn[0] * pn[0];
+        if (h2 & 0x2000000) l = tot - 1;
+        const int plo[3] = {-3, 5, 0};
+        int pi, pj, pk;
+        piece_ijk(plo, pn, piece_div(pn), l, pi, pj, pk);
+        if (pi != -3 + (int)(l % pn[0]) || pj != 5 + (int)(l / pn[0] % pn[1]) || pk != (int)(l / pn[0] / pn[1])) ++local;
     }
     if (local) atomicAdd(fails, local);
 }
