@@ -816,11 +816,13 @@ __global__ void k_adj_dsvl(KARGS, int fs, int sc, int ts, int tcomp) {
 // its adjoint is added there and cleared.
 __global__ void k_adj_fill_boundary(const CopyDesc* __restrict__ D, int nd, long total, const FabView* __restrict__ V,
                                     int nb, int f, int nc) {
+    MADV_LET_NEXT();
     const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= total) return;
     const CopyDesc& cd = D[find_piece<COPY_HINT>(D, nd, gid)];
     int i, j, k;
     piece_ijk(cd.lo, cd.n, cd.dv, gid - cd.start, i, j, k);
+    MADV_WAIT();
     const FabView dst = V[f * nb + cd.dst_b], src = V[f * nb + cd.src_b];
     for (int n = 0; n < nc; ++n) {
         double& g = at(dst, i, j, k, n);
@@ -1173,7 +1175,8 @@ void adj_fill_boundary(Ctx& c, int slot, int nc, int ng, int nodal) {
     const CopyTable& ct = copy_table(c, ng, nodal);
     if (ct.total == 0 || c.dry) return;
     unsigned grid = (unsigned)((ct.total + TPB - 1) / TPB);
-    k_adj_fill_boundary<<<grid, TPB, 0, c.stream>>>(ct.d, (int)ct.h.size(), ct.total, c.V(), c.nb, F_USER + slot, nc);
+    launch_next(c, grid, TPB, k_adj_fill_boundary, (const CopyDesc*)ct.d, (int)ct.h.size(), ct.total, c.V(), c.nb,
+                F_USER + slot, nc);
     c.launches++;
 }
 

@@ -112,14 +112,23 @@ __device__ __forceinline__ void region_ijk(const RegionBox& r, long l, int& i, i
     piece_ijk(r.lo, r.n, r.dv, l, i, j, k);
 }
 
-// Common launch prologue: returns false for threads past the range.
+// Programmatic dependent launch: a kernel lets the next one of its stream start at once (its
+// blocks take the places that drain, find their elements in the constant tables) and itself
+// waits here until everything before it is complete and visible.  Nothing but those
+// tables may be read before MADV_WAIT, and every kernel that launch_next starts has it.
+#define MADV_LET_NEXT() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
+#define MADV_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
+
+// Common launch prologue: returns for threads past the range.
 #define MADV_ELEMENT(R, ne, g0, g1, b, i, j, k)                            \
+    MADV_LET_NEXT();                                                      \
     const long gid_ = (g0) + (long)blockIdx.x * blockDim.x + threadIdx.x; \
     if (gid_ >= (g1)) return;                                             \
     const int e_ = find_box((R), (ne), gid_);                             \
     const int b = (R)[e_].b;                                              \
     int i, j, k;                                                          \
-    region_ijk((R)[e_], gid_ - (R)[e_].start, i, j, k)
+    region_ijk((R)[e_], gid_ - (R)[e_].start, i, j, k);                   \
+    MADV_WAIT()
 
 // amrex::min / amrex::max (std::min / std::max semantics).  (An integer-key form measured
 // slower: the FP64 min/max instruction is not the costly part of the FP64 pipe.)

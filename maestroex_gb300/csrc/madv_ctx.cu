@@ -1107,6 +1107,7 @@ static int finish(Hier& H) {
 static void set_mode(Hier& H, cudaStream_t st, int per_box, bool dry) {
     for (auto* c : H.L) {
         c->stream = st;
+        c->capturing = false;
         c->per_box = per_box;
         c->dry = dry;
     }
@@ -1818,8 +1819,12 @@ static int stage_forward_h(madv_ctx* h, int mode, int nlev, const madv_multifab*
                 reset_launches(H);
                 cudaGraph_t g;
                 CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-                for (auto* lc : H.L) upload_user_views(*lc);
+                for (auto* lc : H.L) {
+                    lc->capturing = true;
+                    upload_user_views(*lc);
+                }
                 stage_body(H, io);
+                for (auto* lc : H.L) lc->capturing = false;
                 CK(cudaStreamEndCapture(cs, &g));
                 CK(cudaGraphInstantiate(&c.graph_exec, g, 0));
                 cudaGraphDestroy(g);

@@ -169,6 +169,7 @@ struct Ctx {
     cudaStream_t stream = nullptr;
     int per_box = 0;      // launch mode: 0 batched, 1 one launch per box
     bool dry = false;     // build region / copy tables only, launch nothing
+    bool capturing = false;  // the stage is being captured: kernels in plain order (launch_next)
     // per-kernel timing (madv_profile): events around every launch
     bool profiling = false;
     struct ProfRec {

@@ -69,11 +69,13 @@ void put1d(Ctx& c, int fid, const double* d_s0, int outcomp, int edge, int vec) 
 // ============================================================ ghost fills
 __global__ void k_fill_boundary(const CopyDesc* __restrict__ D, int nd, long total, const FabView* __restrict__ V,
                                 int nb, int f, int c0, int nc) {
+    MADV_LET_NEXT();
     const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= total) return;
     const CopyDesc& cd = D[find_piece<COPY_HINT>(D, nd, gid)];
     int i, j, k;
     piece_ijk(cd.lo, cd.n, cd.dv, gid - cd.start, i, j, k);
+    MADV_WAIT();
     const FabView dst = V[f * nb + cd.dst_b];
     const FabView src = V[f * nb + cd.src_b];
     for (int n = c0; n < c0 + nc; ++n)
@@ -85,7 +87,8 @@ void fill_boundary(Ctx& c, int fid, int c0, int nc) {
     const CopyTable& ct = copy_table(c, s.ng, s.nodal);
     if (ct.total == 0 || c.dry) return;
     unsigned grid = (unsigned)((ct.total + TPB - 1) / TPB);
-    k_fill_boundary<<<grid, TPB, 0, c.stream>>>(ct.d, (int)ct.h.size(), ct.total, c.V(), c.nb, fid, c0, nc);
+    launch_next(c, grid, TPB, k_fill_boundary, (const CopyDesc*)ct.d, (int)ct.h.size(), ct.total, c.V(), c.nb, fid,
+                c0, nc);
     c.launches++;
 }
 
@@ -1666,6 +1669,8 @@ void update_vel(Ctx& c, int fu, int fsponge) {
 // w0m: spherical with uniform bins and an evolving base state, the face w0mac averaged to the
 // cell (Source/MaestroDt.cpp:313-334); other spherical cases add 0.5 (0 + 0)
 __global__ void k_dt_maxima(KARGS, int sph, int nd, int w0m, unsigned long long* out) {
+    MADV_LET_NEXT();
+    MADV_WAIT();
     const long gid = g0 + (long)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long m[7] = {0ULL, 0ULL, 0ULL, 0ULL, 0ULL, 0ULL, 0ULL};
     if (gid < g1) {
