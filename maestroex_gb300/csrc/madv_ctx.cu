@@ -1791,21 +1791,21 @@ static int stage_forward_h(madv_ctx* h, int mode, int nlev, const madv_multifab*
         for (int l = 0; l < nlev; ++l)
             side_views(H[l], H[l].dviews == H[l].dviews_alias ? H[l].hviews_alias : H[l].hviews_pinned);
         if (mode == MADV_MODE_GRAPH) {
+            // What a captured stage depends on: which FABs the call passes, which of them the
+            // stage works in, and the view table it reads.  Not the FABs themselves: every
+            // kernel reaches them through the tables, which each call uploads.  (With the
+            // descriptors' addresses in the key, a caller that built them anew for each call
+            // had the stage captured again each time.)
             std::vector<const void*> key;
             for (int l = 0; l < nlev; ++l) {
+                intptr_t has = 0;
+                for (const madv_multifab* m : {io[l].gpi, io[l].thermal, io[l].snew, io[l].umac, io[l].sedge,
+                                               io[l].sflux, io[l].eta, io[l].sold_out ? io[l].sold : nullptr})
+                    has = 2 * has + (m != nullptr);
                 key.push_back((const void*)(intptr_t)io[l].alias);
-                const madv_multifab* all[] = {io[l].uold, io[l].sold, io[l].gpi, io[l].thermal, io[l].snew, io[l].eta};
-                for (auto m : all) {
-                    key.push_back(m);
-                    if (m)
-                        for (int b = 0; b < m->nfab; ++b) key.push_back(m->fab[b].p);
-                }
-                for (auto m3 : {io[l].umac, io[l].sedge, io[l].sflux}) {
-                    key.push_back(m3);
-                    if (m3)
-                        for (int d = 0; d < H[l].ndim; ++d)
-                            for (int b = 0; b < m3[d].nfab; ++b) key.push_back(m3[d].fab[b].p);
-                }
+                key.push_back((const void*)has);
+                key.push_back(H[l].dviews);
+                key.push_back(H[l].side_mirror);
             }
             if (!c.graph_exec || key != c.graph_key) {
                 drop_graph(h);
