@@ -54,6 +54,7 @@ struct RegionBox {
     int pad;
     long start;
     PieceDiv dv;
+    int ext, len;  // march regions: cells along the march, and of one chunk
 };
 
 __host__ __device__ inline PieceDiv piece_div(const int* n) {
@@ -120,9 +121,11 @@ __device__ __forceinline__ void region_ijk(const RegionBox& r, long l, int& i, i
 #define MADV_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
 
 // Common launch prologue: returns for threads past the range.
-#define MADV_ELEMENT(R, ne, g0, g1, b, i, j, k)                            \
+// MADV_ELEMENT_OF: the element of block bx (kernels that put components into the block index).
+#define MADV_ELEMENT(R, ne, g0, g1, b, i, j, k) MADV_ELEMENT_OF(blockIdx.x, R, ne, g0, g1, b, i, j, k)
+#define MADV_ELEMENT_OF(bx, R, ne, g0, g1, b, i, j, k)                     \
     MADV_LET_NEXT();                                                      \
-    const long gid_ = (g0) + (long)blockIdx.x * blockDim.x + threadIdx.x; \
+    const long gid_ = (g0) + (long)(bx) * blockDim.x + threadIdx.x;        \
     if (gid_ >= (g1)) return;                                             \
     const int e_ = find_box((R), (ne), gid_);                             \
     const int b = (R)[e_].b;                                              \

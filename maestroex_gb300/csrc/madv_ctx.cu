@@ -2539,7 +2539,7 @@ static bool is_ppm_kernel(Ctx& c, const void* fn) {
     bool yes = false;
     if (cudaFuncGetName(&nm, fn) == cudaSuccess && nm)
         yes = std::strstr(nm, "k_dsvl") || std::strstr(nm, "k_ppm_face") || std::strstr(nm, "k_ppm_cell") ||
-              std::strstr(nm, "k_ppm_sweep");
+              std::strstr(nm, "k_ppm_sweep") || std::strstr(nm, "k_ppm_march") || std::strstr(nm, "k_ppm_rows");
     return c.is_ppm_fn[fn] = yes;
 }
 

@@ -267,6 +267,10 @@ bool cuda_ok(cudaError_t e, const char* what);
 bool ppm_sweep(Ctx& c, int D, int fs, int sc, int fu, int uc, int umac, int fip, int fim, int lo_ext, int hi_ext);
 void sweep_free(Ctx& c);
 
+// ---- PPM marched along each direction, edge states from the upwind cell (madv_march.cu) ----
+void ppm_march_comps(Ctx& c, int dirs, int fs, int sc0, int nq, const BCRecD* bc, int fu, int umac, int fip, int fim);
+void edge_scal_ctu(Ctx& c, int comp0, int nq, const BCRecD* bc, int oc0, int force_zero, int is_vel);
+
 // ---- kernel launch wrappers (madv_kernels.cu) ----
 void fill_boundary(Ctx& c, int fid, int c0, int nc);
 void phys_fill(Ctx& c, int fid, int c0, int nc, const BCRecD* bcs_dev, int bc_c0, int is_vel,

@@ -474,7 +474,12 @@ static void ppm_dir(Ctx& c, int fs, int sc, const BCRecD& bc, int fu, int uc, in
     }
 }
 
+// The PPM sweeps run marched (madv_march.cu) unless the staged form is asked for.
+static bool ppm_marches(const Ctx& c) { return c.P.ppm_type != 0 && !c.staged_ppm; }
+
 static void ppm_any(Ctx& c, int d, int fs, int sc, const BCRecD& bc, int fu, int uc, int umac, int fip, int fim) {
+    if (ppm_marches(c) && !c.edge_tape_begin)
+        return ppm_march_comps(c, 1 << d, fs, sc, 1, &bc, umac ? fu - d : fu, umac, fip, fim);
     if (d == 0) ppm_dir<0>(c, fs, sc, bc, fu, uc, umac, fip, fim);
     else if (d == 1) ppm_dir<1>(c, fs, sc, bc, fu, uc, umac, fip, fim);
     else ppm_dir<2>(c, fs, sc, bc, fu, uc, umac, fip, fim);
@@ -605,10 +610,14 @@ void make_utrans(Ctx& c) {
     if (c.P.ppm_type != 0)
         launch(c, rg_grow(c, 1), 1, k_trace_cell, c.V(), F_UFULL, c.P.dt, make_recip(c.P.dx[0]),
                make_recip(c.P.dx[1]), make_recip(c.P.dx[2]));
+    // every sweep of the velocity at once: those of component d along d are read here, the
+    // others by vel_pred
+    const bool march = ppm_marches(c);
+    if (march) ppm_march_comps(c, 7, F_UTILDE, 0, 3, c.bcs_u, F_UFULL, 0, F_IPC0, F_IMC0);
     for (int d = 0; d < 3; ++d) {
         if (c.P.ppm_type == 0) {
             slope_any(c, d, F_UTILDE, d, F_SLOPE, 0, 1, bcs_dev(c, BCS_U), d);
-        } else {
+        } else if (!march) {
             ppm_any(c, d, F_UTILDE, d, c.bcs_u[d], F_UFULL, d, 0, F_IPC0 + d, F_IMC0 + d);
         }
         const RegionTable& rt = rg_grow(c, 0, d);
@@ -855,8 +864,9 @@ void vel_pred(Ctx& c) {
         slope_any(c, 1, F_UTILDE, 0, F_IMC1, 0, 3, bcs_dev(c, BCS_U), 0);  // slopey -> Imv
         slope_any(c, 2, F_UTILDE, 0, F_IMC2, 0, 3, bcs_dev(c, BCS_U), 0);  // slopez -> Imw
     } else {
-        // the sweeps of component d along d were done by make_utrans (same inputs)
-        for (int cc = 0; cc < 3; ++cc)
+        // the sweeps of component d along d (marched: all of them) were done by make_utrans (same
+        // inputs)
+        for (int cc = 0; cc < 3 && !ppm_marches(c); ++cc)
             for (int d = 0; d < 3; ++d)
                 if (cc != d) ppm_any(c, d, F_UTILDE, cc, c.bcs_u[cc], F_UFULL, d, 0, F_IPC0 + cc, F_IMC0 + cc);
         // ppm_trace_forces: force component d traced along d, the direction VelPredVelocities
@@ -1255,6 +1265,18 @@ void make_edge_scal(Ctx& c, int start_comp, int num_comp, int which_bcs, int is_
         cudaEventRecord(c.ev_fork, main_stream);
         cudaStreamWaitEvent(c.side, c.ev_fork, 0);
     }
+    // marched PPM and edge states from the upwind cell, up to three components a launch (their Ip
+    // / Im in the velocity predictor's fields, free here)
+    const bool ctu = ppm_marches(c) && c.es_inline && !c.edge_tape_begin && !is_cons;
+    const int batch = two || c.P.ppm_trace_forces ? 1 : 3;
+    for (int comp = start_comp; ctu && !two && comp < start_comp + num_comp; comp += batch) {
+        const int nq = std::min(batch, start_comp + num_comp - comp);
+        ppm_march_comps(c, 7, F_SOLD, comp, nq, bh + comp, F_UMAC0, 1, F_IPC0, F_IMC0);
+        if (c.P.ppm_trace_forces && !force_zero)
+            ppm_march_comps(c, 7, F_SCALFORCE, comp, 1, bh + comp, F_UMAC0, 1, F_IPF, F_IMF);
+        edge_scal_ctu(c, comp, nq, bh + comp, slot >= 0 ? slot : comp, force_zero, is_vel);
+    }
+    if (ctu && !two) return;
     for (int comp = start_comp; comp < start_comp + num_comp; ++comp) {
         const bool alt = two && ((comp - start_comp) & 1);
         c.stream = alt ? c.side : main_stream;
@@ -1275,6 +1297,10 @@ void make_edge_scal(Ctx& c, int start_comp, int num_comp, int which_bcs, int is_
         // kernels form them themselves and only the upwind state is stored (the full
         // predictor runs where the adjoint's tape keeps its fields)
         const bool inl = c.es_inline && c.P.ppm_type != 0 && !c.edge_tape_begin;
+        if (ctu) {
+            edge_scal_ctu(c, comp, 1, &bc, slot >= 0 ? slot : comp, force_zero, is_vel);
+            continue;
+        }
         if (inl) {
             es_simh_launch<0>(c, comp, bc, v0);
             es_simh_launch<1>(c, comp, bc, v1);
@@ -2311,6 +2337,7 @@ void vel_pred_prep(Ctx& c) {
     const RegionTable& rt = c.ndim == 2 ? rg2(c, 1) : rg_grow(c, 1);
     launch(c, rt, 1, k_trace_cell, c.V(), F_UFULL, c.P.dt, make_recip(c.P.dx[0]),
                make_recip(c.P.dx[1]), make_recip(c.P.dx[2]));
+    if (c.ndim == 3 && ppm_marches(c)) return ppm_march_comps(c, 7, F_UTILDE, 0, 3, c.bcs_u, F_UFULL, 0, F_IPC0, F_IMC0);
     for (int d = 0; d < c.ndim; ++d) ppm_any(c, d, F_UTILDE, d, c.bcs_u[d], F_UFULL, d, 0, F_IPC0 + d, F_IMC0 + d);
 }
 void vel_pred_2d_entry(Ctx& c) { vel_pred_2d(c); }

@@ -32,20 +32,26 @@ static inline void launch_next(const Ctx& c, dim3 grid, int tpb, void (*kern)(P.
 // One launch over every box (batched), or one launch per region piece (per-box mode, the
 // MFIter + ParallelFor form of the reference).  Kernel arguments after the region are
 // (V, nb, ...).  Threads per block: the kernel's autotuned value on this level.
+// per_warp > 0: kernels whose warps advance by that many elements instead of 32.
+// gq components are interleaved in the block index, so that the blocks of one place run together
+// and share what they read.
 template <typename Kern, typename... Args>
-static inline void launch(Ctx& c, const RegionTable& rt, int gy, Kern kern, const FabView* V, Args... args) {
+static inline void launch(Ctx& c, const RegionTable& rt, int gq, Kern kern, int per_warp, const FabView* V, Args... args) {
     const int tpb = c.tpb_of((const void*)kern);  // before a dry return: no attribute query while capturing
     if (rt.total == 0 || c.dry) return;
     const int ne = (int)rt.h.size();
+    auto grid = [&](long n) {
+        const long threads = per_warp ? (n + per_warp - 1) / per_warp * 32 : n;
+        return dim3((unsigned)((threads + tpb - 1) / tpb * gq));
+    };
     if (!c.per_box) {
-        dim3 grid((unsigned)((rt.total + tpb - 1) / tpb), gy);
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         if (c.profiling) {
             e0 = c.next_event();
             e1 = c.next_event();
             cudaEventRecord(e0, c.stream);
         }
-        launch_next(c, grid, tpb, kern, (const RegionBox*)rt.d, ne, 0L, rt.total, V, c.nb, args...);
+        launch_next(c, grid(rt.total), tpb, kern, (const RegionBox*)rt.d, ne, 0L, rt.total, V, c.nb, args...);
         if (c.profiling) {
             cudaEventRecord(e1, c.stream);
             c.prof.push_back({(const void*)kern, e0, e1});
@@ -56,11 +62,14 @@ static inline void launch(Ctx& c, const RegionTable& rt, int gy, Kern kern, cons
             long s0 = rt.h[e].start;
             long s1 = (e + 1 < ne) ? rt.h[e + 1].start : rt.total;
             if (s1 <= s0) continue;
-            dim3 grid((unsigned)((s1 - s0 + tpb - 1) / tpb), gy);
-            launch_next(c, grid, tpb, kern, (const RegionBox*)rt.d, ne, s0, s1, V, c.nb, args...);
+            launch_next(c, grid(s1 - s0), tpb, kern, (const RegionBox*)rt.d, ne, s0, s1, V, c.nb, args...);
             c.launches++;
         }
     }
+}
+template <typename Kern, typename... Args>
+static inline void launch(Ctx& c, const RegionTable& rt, int gq, Kern kern, const FabView* V, Args... args) {
+    launch(c, rt, gq, kern, 0, V, args...);
 }
 
 // Region helpers: the valid box grown by g, and face boxes.

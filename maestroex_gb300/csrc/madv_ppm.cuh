@@ -30,12 +30,10 @@ __device__ __forceinline__ double ppm_dsvl(const FabView& s, int sc, int i, int 
     return vl_slope(S(1) - S(-1), S(0) - S(-1), S(1) - S(0));
 }
 
-// Interior fourth-order limited face value (ppm_type 2), face between cells c+m-1 and c+m.
-template <int D>
-__device__ __forceinline__ double ppm2_face_regular(const FabView& s, int sc, int i, int j, int k, int m,
-                                                    const RecipC& r6) {
-    constexpr int di = D == 0, dj = D == 1, dk = D == 2;
-    auto S = SHIFT_S(s, sc);
+// Interior fourth-order limited face value (ppm_type 2), face between cells m-1 and m of S,
+// S(q) the field q cells along D.
+template <typename SF>
+__device__ __forceinline__ double ppm2_face_regular(SF S, int m, const RecipC& r6) {
     const double C = 1.25;
     double se = (7.0 / 12.0) * (S(m - 1) + S(m)) - (1.0 / 12.0) * (S(m - 2) + S(m + 1));
     // reference: (se - s(m-1)) * (s(m) - se) < 0, i.e. the product of (se - s(m-1)) and
@@ -54,37 +52,52 @@ __device__ __forceinline__ double ppm2_face_regular(const FabView& s, int sc, in
     return se;
 }
 
-// Limited interface value of the face (i,j,k) between cells f-1 and f along D
+// Van Leer slope of the cell m of S, and the interior interface value between cells m-1 and m
+// (ppm_type 1).
+template <typename SF>
+__device__ __forceinline__ double vl_at(SF S, int m) {
+    return vl_slope(S(m + 1) - S(m - 1), S(m) - S(m - 1), S(m + 1) - S(m));
+}
+__device__ __forceinline__ double ppm1_face_regular(double sl, double sr, double dvl, double dvr, const RecipC& r6) {
+    return clamp_between(half(sr + sl) - div_6(dvr - dvl, r6), sr, sl);
+}
+
+// Limited interface value of the face of index f along D, between cells m-1 and m of S
 // (ppm_type 1 :37-111, ppm_type 2 :257-335; the boundary stencils of :131-205 / :443-700
 // are the values the reference assigns to the faces next to an ext_dir/hoextrap
-// boundary).  dv: van Leer slopes per cell (ppm_type 1).
+// boundary).  DV(m): van Leer slope of cell m (ppm_type 1).
+template <int PPMT, typename SF, typename DF>
+__device__ __forceinline__ double ppm_face_any(SF S, DF DV, int m, int f, int lo_ext, int hi_ext, int domlo, int domhi,
+                                               const RecipC& r6) {
+    double v;
+    if (lo_ext && f == domlo) {
+        v = S(m - 1);
+    } else if (hi_ext && f == domhi + 1) {
+        v = S(m);
+    } else if (lo_ext && f == domlo + 1) {
+        v = -0.2 * S(m - 2) + 0.75 * S(m - 1) + 0.5 * S(m) - 0.05 * S(m + 1);
+        v = mx(v, mn(S(m), S(m - 1)));
+        v = mn(v, mx(S(m), S(m - 1)));
+    } else if (hi_ext && f == domhi) {
+        v = -0.2 * S(m + 1) + 0.75 * S(m) + 0.5 * S(m - 1) - 0.05 * S(m - 2);
+        v = mx(v, mn(S(m - 1), S(m)));
+        v = mn(v, mx(S(m - 1), S(m)));
+    } else if (PPMT == 1) {
+        v = ppm1_face_regular(S(m - 1), S(m), DV(m - 1), DV(m), r6);
+    } else {
+        v = ppm2_face_regular(S, m, r6);
+    }
+    return v;
+}
+
+// The same for the face (i,j,k) of a field with its van Leer slopes stored per cell.
 template <int D, int PPMT>
 __device__ __forceinline__ double ppm_face_value(const FabView& s, int sc, const FabView& dv, int i, int j, int k,
                                                  int lo_ext, int hi_ext, int domlo, int domhi, const RecipC& r6) {
     constexpr int di = D == 0, dj = D == 1, dk = D == 2;
     auto S = SHIFT_S(s, sc);
-    const int I = D == 0 ? i : (D == 1 ? j : k);
-    double v;
-    if (lo_ext && I == domlo) {
-        v = S(-1);
-    } else if (hi_ext && I == domhi + 1) {
-        v = S(0);
-    } else if (lo_ext && I == domlo + 1) {
-        v = -0.2 * S(-2) + 0.75 * S(-1) + 0.5 * S(0) - 0.05 * S(1);
-        v = mx(v, mn(S(0), S(-1)));
-        v = mn(v, mx(S(0), S(-1)));
-    } else if (hi_ext && I == domhi) {
-        v = -0.2 * S(1) + 0.75 * S(0) + 0.5 * S(-1) - 0.05 * S(-2);
-        v = mx(v, mn(S(-1), S(0)));
-        v = mn(v, mx(S(-1), S(0)));
-    } else if (PPMT == 1) {
-        const double dvl = at(dv, i - di, j - dj, k - dk);
-        const double dvr = at(dv, i, j, k);
-        v = clamp_between(half(S(0) + S(-1)) - div_6(dvr - dvl, r6), S(0), S(-1));
-    } else {
-        v = ppm2_face_regular<D>(s, sc, i, j, k, 0, r6);
-    }
-    return v;
+    auto DV = SHIFT_S(dv, 0);
+    return ppm_face_any<PPMT>(S, DV, 0, D == 0 ? i : (D == 1 ? j : k), lo_ext, hi_ext, domlo, domhi, r6);
 }
 
 // Characteristic-tracing coefficients (Source/MaestroPPM.cpp:209-251):
@@ -99,31 +112,24 @@ __device__ __forceinline__ bool finite2(double a, double b) {
     return (dhigh(a) & 0x7ff00000) != 0x7ff00000 && (dhigh(b) & 0x7ff00000) != 0x7ff00000;
 }
 
-// Edge values sm, sp of cell (i,j,k) along D from the face values F (quadratic limiter
+// Edge values sm, sp of the cell of index I along D from the face values F (quadratic limiter
 // :117-128 for ppm_type 1, Colella-2008 limiter :337-434 for ppm_type 2, with the
-// boundary re-limiting of :131-205 / :443-700).
+// boundary re-limiting of :131-205 / :443-700).  S(m): the field m cells along D; F(m): the
+// interface value between cells m-1 and m.
 //
 // F holds, on the two faces next to an ext_dir/hoextrap boundary, the values the reference
 // assigns for the first interior cells.  Cells outside the domain (ghost cells of a grown
 // box) are not re-limited by the reference and see the regular interpolants on those faces,
-// which are recomputed here (dv: van Leer slopes, ppm_type 1).
-template <int D, int PPMT>
-__device__ __forceinline__ void ppm_cell_edges(const FabView& s, int sc, const FabView& F, const FabView& dv, int i,
-                                               int j, int k, int lo_ext, int hi_ext, int domlo, int domhi,
-                                               const RecipC& r6, double& sm, double& sp) {
-    constexpr int di = D == 0, dj = D == 1, dk = D == 2;
-    auto S = SHIFT_S(s, sc);
-    const int I = D == 0 ? i : (D == 1 ? j : k);
+// FR(m).
+template <int D, int PPMT, typename SF, typename FF, typename RF>
+__device__ __forceinline__ void ppm_cell_any(SF S, FF F, RF FR, int I, int lo_ext, int hi_ext, int domlo, int domhi,
+                                             double& sm, double& sp) {
     const bool outside = (lo_ext && I < domlo) || (hi_ext && I > domhi);
     auto Fc = [&](int m) -> double {
         const int f = I + m;
-        if (outside && ((lo_ext && (f == domlo || f == domlo + 1)) || (hi_ext && (f == domhi || f == domhi + 1)))) {
-            if (PPMT == 2) return ppm2_face_regular<D>(s, sc, i, j, k, m, r6);
-            const double dvl = at(dv, i + (m - 1) * di, j + (m - 1) * dj, k + (m - 1) * dk);
-            const double dvr = at(dv, i + m * di, j + m * dj, k + m * dk);
-            return clamp_between(half(S(m) + S(m - 1)) - div_6(dvr - dvl, r6), S(m), S(m - 1));
-        }
-        return at(F, i + m * di, j + m * dj, k + m * dk);
+        if (outside && ((lo_ext && (f == domlo || f == domlo + 1)) || (hi_ext && (f == domhi || f == domhi + 1))))
+            return FR(m);
+        return F(m);
     };
     const double s0 = S(0);
     if (PPMT == 1) {
@@ -151,7 +157,7 @@ __device__ __forceinline__ void ppm_cell_edges(const FabView& s, int sc, const F
     } else {
         const double C = 1.25;
         double sedgel = Fc(-1), sedge = Fc(0), sedger = Fc(1), sedgerr = Fc(2);
-        if (D == 0 && hi_ext && I == domhi - 1) sedgerr = ppm2_face_regular<D>(s, sc, i, j, k, 2, r6);
+        if (D == 0 && hi_ext && I == domhi - 1) sedgerr = FR(2);
         if (lo_ext && I == domlo) {
             sm = sedge;
             sp = sedger;
@@ -216,6 +222,21 @@ __device__ __forceinline__ void ppm_cell_edges(const FabView& s, int sc, const F
             sp = s0 + alphap;
         }
     }
+}
+
+// The same for cell (i,j,k) of a field with stored interface values F and slopes dv.
+template <int D, int PPMT>
+__device__ __forceinline__ void ppm_cell_edges(const FabView& s, int sc, const FabView& F, const FabView& dv, int i,
+                                               int j, int k, int lo_ext, int hi_ext, int domlo, int domhi,
+                                               const RecipC& r6, double& sm, double& sp) {
+    constexpr int di = D == 0, dj = D == 1, dk = D == 2;
+    auto S = SHIFT_S(s, sc);
+    auto FS = SHIFT_S(F, 0);
+    auto DV = SHIFT_S(dv, 0);
+    auto FR = [&](int m) -> double {
+        return PPMT == 2 ? ppm2_face_regular(S, m, r6) : ppm1_face_regular(S(m - 1), S(m), DV(m - 1), DV(m), r6);
+    };
+    ppm_cell_any<D, PPMT>(S, FS, FR, D == 0 ? i : (D == 1 ? j : k), lo_ext, hi_ext, domlo, domhi, sm, sp);
 }
 
 __device__ __forceinline__ double trace_side(double sm, double sp, double d, double s6, double A, double B, bool p) {
