@@ -10,8 +10,11 @@
 //                   in registers: 20 FP64 instructions a cell (ppm_type 1) against 23 in three
 //                   launches, one load of the state instead of nine.
 //   k_ppm_rows      x: lanes along the row, slopes and interface values passed to the
-//                   neighbour lane by shuffles, the warps overlapping by 2 (ppm_type 2: 3)
-//                   lanes.  A march across lanes would read 32 rows at once.
+//                   neighbour lane by shuffles, the warps overlapping by 2 lanes.  A march across lanes would read 32 rows at once.
+//   k_ppm_march2, k_ppm_rows2  the same for ppm_type 2, the limited faces and cells listed and
+//                   finished 32 at a time (madv_march.cuh): three components at 128^3 0.26 ms a
+//                   direction, 0.47 ms with the limiter in place (the velocity's sweeps 0.43
+//                   against 0.72 to 1.08 ms).
 //   k_es_cinc       the transverse increment c_T of each cell, (dt/6/h_T) (u_T sum) times the
 //                   difference of the upwind states on its T-faces: each is used by the two
 //                   other directions and by both sides of a face, where the transverse
@@ -92,13 +95,62 @@ __global__ void __launch_bounds__(256) k_ppm_rows(KARGS, int fs, int sc0, int fu
     at(VW(fim + q), i, j, k, 0) = imv;
 }
 
+// ============================================================ ppm_type 2
+template <int D, int UMAC>
+__global__ void __launch_bounds__(32 * P2_WARPS) k_ppm_march2(KARGS, int fs, int sc0, int fu, int fip, int fim,
+                                                               unsigned lo_mask, unsigned hi_mask, int domlo, int domhi,
+                                                               long long epsb, RecipC r6, unsigned nq) {
+    __shared__ P2Column sh[P2_WARPS];
+    MADV_LET_NEXT();
+    const unsigned bx = blockIdx.x / nq, q = blockIdx.x - bx * nq;
+    const long gid = g0 + (long)bx * blockDim.x + threadIdx.x, gc = gid < g1 ? gid : g1 - 1;
+    const int e = find_box(R, ne, gc), b = R[e].b, lo = R[e].lo[D];
+    int i, j, k;
+    region_ijk(R[e], gc - R[e].start, i, j, k);
+    const int I0 = lo + ((D == 1 ? j : k) - lo) * R[e].len, n = gid < g1 ? min(R[e].len, lo + R[e].ext - I0) : 0;
+    if (D == 1) j = I0;
+    else k = I0;
+    MADV_WAIT();
+    const FabView s = VW(fs), ip = VW(fip + q), im = VW(fim + q), u = VW(fu), T = UMAC ? VW(F_TRA0 + D) : VW(F_TRC);
+    auto st = [](const FabView& f) { return D == 1 ? f.sj : (int)f.sk; };
+    const P2Cell c{&at(s, i, j, k, sc0 + q), &at(u, i, j, k, UMAC ? 0 : D), &at(T, i, j, k, UMAC ? 0 : 2 * D),
+                   &at(T, i, j, k, UMAC ? 1 : 2 * D + 1), &at(ip, i, j, k, D), &at(im, i, j, k, D), st(s), st(u), st(T)};
+    const MarchBC bc{(int)(lo_mask >> q) & 1, (int)(hi_mask >> q) & 1, domlo, domhi};
+    ppm2_column<D, UMAC, false>(sh[threadIdx.x >> 5], c, st(ip), I0, n, bc, 0.0, r6, epsb, r6);
+}
+
+template <int UMAC>
+__global__ void __launch_bounds__(32 * P2_WARPS) k_ppm_rows2(KARGS, int fs, int sc0, int fu, int fip, int fim,
+                                                              unsigned lo_mask, unsigned hi_mask, int domlo, int domhi,
+                                                              long long epsb, RecipC r6, unsigned nq, int np) {
+    __shared__ P2Row sh[P2_WARPS];
+    MADV_LET_NEXT();
+    const unsigned bx = blockIdx.x / nq, q = blockIdx.x - bx * nq;
+    const long t0 = g0 + (((long)bx * blockDim.x + threadIdx.x) >> 5) * (np - 3) - 1;
+    MADV_WAIT();
+    auto at_pos = [&](int p, P2Cell& x, int& i) -> bool {
+        const long t = t0 + p, tc = t < g0 ? g0 : (t >= g1 ? g1 - 1 : t);  // past the ends: a copy
+        const int e = find_box(R, ne, tc), b = R[e].b;
+        int j, k;
+        region_ijk(R[e], tc - R[e].start, i, j, k);
+        const FabView s = VW(fs), u = VW(fu), T = UMAC ? VW(F_TRA0) : VW(F_TRC);
+        x = P2Cell{&at(s, i, j, k, sc0 + q), &at(u, i, j, k, 0), &at(T, i, j, k, 0), &at(T, i, j, k, 1),
+                   &at(VW(fip + q), i, j, k, 0), &at(VW(fim + q), i, j, k, 0), 1, 1, 1};
+        const int r = i - R[e].lo[0];
+        return t == tc && r >= 1 && r <= R[e].ext;
+    };
+    const MarchBC bc{(int)(lo_mask >> q) & 1, (int)(hi_mask >> q) & 1, domlo, domhi};
+    ppm2_rows<UMAC, false>(sh[threadIdx.x >> 5], np, at_pos, bc, 0.0, r6, epsb, r6);
+}
+
 // Cells a thread marches over: chunks short enough that the columns of the level fill the
 // chip (about 2^16 threads: 430 a SM), at most 24 cells (a chunk forms two slopes and an
 // interface value of its neighbour again: 2% at 24, 6% at 8 cells).
+// (ppm_type 2: at most P2_CHUNK, the interface values held in shared memory.)
 static int march_len(const Ctx& c) {
     long cells = 0;
     for (const HBox& v : c.ba) cells += (long)(v.hi[0] - v.lo[0] + 3) * (v.hi[1] - v.lo[1] + 3) * (v.hi[2] - v.lo[2] + 3);
-    return (int)std::min(24L, std::max(2L, cells >> 16));
+    return (int)std::min(c.P.ppm_type == 2 ? (long)P2_CHUNK : 24L, std::max(2L, cells >> 16));
 }
 
 static const RegionTable& march_region(Ctx& c, int D) {
@@ -143,12 +195,20 @@ static void march_dir(Ctx& c, int fs, int sc0, int nq, const BCRecD* bc, int fu,
     const long long eb = dbits_host(c.P.rel_eps);
     const int dl = c.P.dom_lo[D], dh = c.P.dom_hi[D];
     const RecipC r6 = make_recip(6.0);
-    if constexpr (D == 0)
-        launch(c, rt, nq, k_ppm_rows<PPMT, UMAC>, row_out(PPMT), c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6,
-               (unsigned)nq);
-    else
-        launch(c, rt, nq, k_ppm_march<D, PPMT, UMAC>, 0, c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6,
-               (unsigned)nq);
+    const unsigned n = (unsigned)nq;
+    if constexpr (PPMT == 2 && D == 0) {
+        // positions of a warp: 512 (three components at 128^3: 0.26 ms; 0.35 at 128, where the lists
+        // of a warp fill a third of a turn; 3 positions overlap the next warp), fewer where the
+        // level has too few rows for 16 warps a SM
+        const int np = (int)std::min((long)P2_ROW, std::max(32L, rt.total / (152 * 16) / 32 * 32));
+        launch(c, rt, nq, k_ppm_rows2<UMAC>, np - 3, c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6, n, np);
+    } else if constexpr (PPMT == 2) {
+        launch(c, rt, nq, k_ppm_march2<D, UMAC>, 0, c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6, n);
+    } else if constexpr (D == 0) {
+        launch(c, rt, nq, k_ppm_rows<PPMT, UMAC>, row_out(PPMT), c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6, n);
+    } else {
+        launch(c, rt, nq, k_ppm_march<D, PPMT, UMAC>, 0, c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6, n);
+    }
 }
 
 // PPM of components sc0 .. sc0 + nq - 1 (nq <= 3) of field fs, boundary records bc[0 .. nq-1],

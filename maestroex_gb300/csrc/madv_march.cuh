@@ -191,4 +191,220 @@ __device__ __forceinline__ void ppm_row(const double* __restrict__ ps, const dou
     ppm_trace(s0, sm, sp, up, um, Ap, Bp, Am, Bm, epsb, ipv, imv);
 }
 
+// ---- ppm_type 2, limited cells apart
+// The Colella limiter changes few faces and cells -- 1-7% of the faces, 2-12% of the cells of
+// the smooth fields the stage advects -- but 27-100% of the warps hold one, and its division,
+// square root and curvature tests then cost the whole warp: 39-82 FP64 instructions a cell were
+// issued for 20 that a lane executed.  So a warp forms the unlimited interface values of its chunk (in
+// shared memory), lists the ones outside their cells and limits them 32 at a time, traces the
+// cells the limiter leaves alone, lists the others and finishes those 32 at a time.
+constexpr int P2_WARPS = 4;   // warps of a block
+constexpr int P2_CHUNK = 21;  // cells of a column chunk at most
+constexpr int P2_ROW = 512;   // positions of a row segment at most
+
+struct P2Column {
+    double f[P2_CHUNK + 3][32];
+    unsigned short list[(P2_CHUNK + 3) * 32];
+};
+struct P2Row {
+    double f[P2_ROW];
+    unsigned short list[P2_ROW];
+};
+
+// lane's place in a list the warp appends to
+__device__ __forceinline__ void warp_push(unsigned short* list, int& n, bool yes, int item) {
+    const unsigned m = __ballot_sync(0xffffffffu, yes);
+    if (yes) list[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1))] = (unsigned short)item;
+    n += __popc(m);
+}
+template <typename T>
+__device__ __forceinline__ T* lane_ptr(T* p, int lane) {
+    return reinterpret_cast<T*>(__shfl_sync(0xffffffffu, (unsigned long long)p, lane));
+}
+
+// A cell of the column or row: the fields at it and at its low face
+struct P2Cell {
+    const double *s, *u, *A, *B;
+    double *ip, *im;
+    int ss, su, sT;  // strides along the direction
+};
+
+// Ip, Im from the limited edge values
+template <int UMAC, bool INL>
+__device__ __forceinline__ void p2_trace(const P2Cell& c, double s0, double sm, double sp, double dt, const RecipC& rdx,
+                                         long long epsb) {
+    double up, um, Ap, Bp, Am, Bm;
+    um = c.u[0];
+    if (UMAC) {
+        up = c.u[c.su];
+        if (INL) {
+            trace_coeffs(up, dt, rdx, Ap, Bp);
+            trace_coeffs(um, dt, rdx, Am, Bm);
+        } else {
+            Ap = c.A[c.sT], Bp = c.B[c.sT], Am = c.A[0], Bm = c.B[0];
+        }
+    } else {
+        up = um;
+        if (INL) {
+            trace_coeffs(up, dt, rdx, Ap, Bp);
+        } else {
+            Ap = c.A[0], Bp = c.B[0];
+        }
+        Am = Ap, Bm = Bp;
+    }
+    double ipv, imv;
+    ppm_trace(s0, sm, sp, up, um, Ap, Bp, Am, Bm, epsb, ipv, imv);
+    *c.ip = ipv;
+    *c.im = imv;
+}
+
+// a listed cell of index I: the limiter in full
+template <int D, int UMAC, bool INL, typename FF>
+__device__ __forceinline__ void p2_limited(const P2Cell& c, FF F, int I, const MarchBC& bc, double dt, const RecipC& rdx,
+                                           long long epsb, const RecipC& r6) {
+    double sm, sp;
+    const double* ps = c.s;
+    const long st = c.ss;
+    if (bc.touches(I)) {
+        const double2 v = ppm_cell_bnd<D, 2>(ps, st, I, bc, r6);
+        sm = v.x, sp = v.y;
+    } else {
+        auto S = [=](int m) -> double { return ps[m * st]; };
+        auto none = [](int) -> double { return 0.0; };
+        ppm_cell_any<D, 2>(S, F, none, I, 0, 0, 0, 0, sm, sp);
+    }
+    p2_trace<UMAC, INL>(c, *ps, sm, sp, dt, rdx, epsb);
+}
+
+// Ip, Im of the n cells from I0 of a column (n <= P2_CHUNK, 0: none; lanes may differ); c: the
+// first cell.  Every lane of the warp calls.
+template <int D, int UMAC, bool INL>
+__device__ __forceinline__ void ppm2_column(P2Column& w, P2Cell c, int so, int I0, int n, const MarchBC& bc, double dt,
+                                            const RecipC& rdx, long long epsb, const RecipC& r6) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int nmax = __reduce_max_sync(ALL, n);
+    // interface values I0 - 1 .. I0 + n + 1
+    int nl = 0;
+    {
+        const long st = c.ss;
+        const int nf = n ? n + 3 : 0;
+        const double* p = c.s;
+        double a = 0, b = 0, cc = 0, d = 0;
+        if (n) a = p[-3 * st], b = p[-2 * st], cc = p[-st], d = p[0];
+        for (int t = 0; t < nmax + 3; ++t) {
+            const bool in = t < nf;
+            double nx = 0;
+            if (t + 1 < nf) nx = p[(t + 1) * st];
+            bool out = false;
+            if (in) {
+                auto S = [&](int m) -> double { return m == -2 ? a : m == -1 ? b : m == 0 ? cc : d; };
+                const double se = ppm2_face_raw(S, 0);
+                w.f[t][lane] = se;
+                out = ppm2_face_out(se, b, cc);
+            }
+            warp_push(w.list, nl, out, t << 5 | lane);
+            a = b, b = cc, cc = d, d = nx;
+        }
+    }
+    __syncwarp();
+    for (int q0 = 0; q0 < nl; q0 += 32) {
+        const int it = w.list[min(q0 + lane, nl - 1)], ol = it & 31, t = it >> 5;
+        const double* p = lane_ptr(c.s, ol);
+        const long st = __shfl_sync(ALL, c.ss, ol);
+        if (q0 + lane < nl) {
+            p += (t - 1) * st;
+            auto S = [=](int m) -> double { return p[m * st]; };
+            w.f[t][ol] = ppm2_face_limit(S, 0, w.f[t][ol], r6);
+        }
+    }
+    __syncwarp();
+    // the cells the limiter leaves alone
+    nl = 0;
+    for (int t = 0; t < nmax; ++t) {
+        bool listed = false;
+        if (t < n) {
+            const P2Cell x{c.s + (long)t * c.ss, c.u + (long)t * c.su, c.A + (long)t * c.sT, c.B + (long)t * c.sT,
+                           c.ip + (long)t * so, c.im + (long)t * so, c.ss, c.su, c.sT};
+            const double s0 = *x.s, am = w.f[t + 1][lane] - s0, ap = w.f[t + 2][lane] - s0;
+            listed = bc.touches(I0 + t) || !ppm2_cell_plain(am, ap);
+            if (!listed) p2_trace<UMAC, INL>(x, s0, s0 + am, s0 + ap, dt, rdx, epsb);
+        }
+        warp_push(w.list, nl, listed, t << 5 | lane);
+    }
+    __syncwarp();
+    for (int q0 = 0; q0 < nl; q0 += 32) {
+        const int it = w.list[min(q0 + lane, nl - 1)], ol = it & 31, t = it >> 5;
+        P2Cell x;
+        x.ss = __shfl_sync(ALL, c.ss, ol), x.su = __shfl_sync(ALL, c.su, ol), x.sT = __shfl_sync(ALL, c.sT, ol);
+        const int o = __shfl_sync(ALL, so, ol), i0 = __shfl_sync(ALL, I0, ol);
+        x.s = lane_ptr(c.s, ol) + (long)t * x.ss;
+        x.u = lane_ptr(c.u, ol) + (long)t * x.su;
+        x.A = lane_ptr(c.A, ol) + (long)t * x.sT;
+        x.B = lane_ptr(c.B, ol) + (long)t * x.sT;
+        x.ip = lane_ptr(c.ip, ol) + (long)t * o;
+        x.im = lane_ptr(c.im, ol) + (long)t * o;
+        if (q0 + lane < nl) {
+            auto F = [&](int m) -> double { return w.f[t + 1 + m][ol]; };
+            p2_limited<D, UMAC, INL>(x, F, i0 + t, bc, dt, rdx, epsb, r6);
+        }
+    }
+}
+
+// Ip, Im of np positions of the rows (a multiple of 32, <= P2_ROW), the first and the last two of
+// which only pass interface values on.  at(p, x, i): position p's cell x and index i; false if p
+// passes values on (its state is there all the same).  Every lane calls.
+template <int UMAC, bool INL, typename AT>
+__device__ __forceinline__ void ppm2_rows(P2Row& w, int np, AT at, const MarchBC& bc, double dt, const RecipC& rdx,
+                                          long long epsb, const RecipC& r6) {
+    const int lane = threadIdx.x & 31;
+    int nl = 0;
+    for (int p0 = 0; p0 < np; p0 += 32) {
+        const int p = p0 + lane;
+        P2Cell x;
+        int i;
+        at(p, x, i);
+        const double a = x.s[-2], b = x.s[-1], cc = x.s[0], d = x.s[1];
+        auto S = [&](int m) -> double { return m == -2 ? a : m == -1 ? b : m == 0 ? cc : d; };
+        const double se = ppm2_face_raw(S, 0);
+        w.f[p] = se;
+        warp_push(w.list, nl, ppm2_face_out(se, b, cc), p);
+    }
+    __syncwarp();
+    for (int q0 = 0; q0 < nl; q0 += 32)
+        if (q0 + lane < nl) {
+            const int p = w.list[q0 + lane];
+            P2Cell x;
+            int i;
+            at(p, x, i);
+            const double* ps = x.s;
+            auto S = [=](int m) -> double { return ps[m]; };
+            w.f[p] = ppm2_face_limit(S, 0, w.f[p], r6);
+        }
+    __syncwarp();
+    nl = 0;
+    for (int p0 = 0; p0 < np; p0 += 32) {
+        const int p = p0 + lane;
+        P2Cell x;
+        int i;
+        bool listed = false;
+        if (at(p, x, i) && p >= 1 && p <= np - 3) {
+            const double s0 = *x.s, am = w.f[p] - s0, ap = w.f[p + 1] - s0;
+            listed = bc.touches(i) || !ppm2_cell_plain(am, ap);
+            if (!listed) p2_trace<UMAC, INL>(x, s0, s0 + am, s0 + ap, dt, rdx, epsb);
+        }
+        warp_push(w.list, nl, listed, p);
+    }
+    __syncwarp();
+    for (int q0 = 0; q0 < nl; q0 += 32)
+        if (q0 + lane < nl) {
+            const int p = w.list[q0 + lane];
+            P2Cell x;
+            int i;
+            at(p, x, i);
+            auto F = [&](int m) -> double { return w.f[p + m]; };
+            p2_limited<0, UMAC, INL>(x, F, i, bc, dt, rdx, epsb, r6);
+        }
+}
+
 }  // namespace madv

@@ -30,18 +30,24 @@ __device__ __forceinline__ double ppm_dsvl(const FabView& s, int sc, int i, int 
     return vl_slope(S(1) - S(-1), S(0) - S(-1), S(1) - S(0));
 }
 
-// Interior fourth-order limited face value (ppm_type 2), face between cells m-1 and m of S,
-// S(q) the field q cells along D.
+// Fourth-order interface value (ppm_type 2) of the face between cells m-1 and m of S, S(q) the
+// field q cells along D, before it is limited.
 template <typename SF>
-__device__ __forceinline__ double ppm2_face_regular(SF S, int m, const RecipC& r6) {
+__device__ __forceinline__ double ppm2_face_raw(SF S, int m) {
+    return (7.0 / 12.0) * (S(m - 1) + S(m)) - (1.0 / 12.0) * (S(m - 2) + S(m + 1));
+}
+// Whether it may lie outside its two cells a, b.  reference: (se - s(m-1)) * (s(m) - se) < 0, i.e.
+// the product of (se - s(m-1)) and -(s(m) - se) = se - s(m) (exact) is positive.  The
+// differences have the sign of the comparison (on integer keys, no FP64 instruction).
+__device__ __forceinline__ bool ppm2_face_out(double se, double a, double b) {
+    const long long ks = dkey(se), ka = dkey(a), kb = dkey(b);
+    return (ks > ka && ks > kb) || (ks < ka && ks < kb);
+}
+// the limited value of one that does
+template <typename SF>
+__device__ __forceinline__ double ppm2_face_limit(SF S, int m, double se, const RecipC& r6) {
     const double C = 1.25;
-    double se = (7.0 / 12.0) * (S(m - 1) + S(m)) - (1.0 / 12.0) * (S(m - 2) + S(m + 1));
-    // reference: (se - s(m-1)) * (s(m) - se) < 0, i.e. the product of (se - s(m-1)) and
-    // -(s(m) - se) = se - s(m) (exact) is positive
-    // the differences have the sign of the comparison (on integer keys, no FP64 instruction);
-    // equal signs -- se outside its two cells -- are rare, and only then the product is looked at
-    const long long ks = dkey(se), ka = dkey(S(m - 1)), kb = dkey(S(m));
-    if (((ks > ka && ks > kb) || (ks < ka && ks < kb)) && prod_gt0(se - S(m - 1), se - S(m))) {
+    if (prod_gt0(se - S(m - 1), se - S(m))) {
         double D2 = 3.0 * (S(m - 1) - twice(se) + S(m));
         double D2L = S(m - 2) - twice(S(m - 1)) + S(m);
         double D2R = S(m - 1) - twice(S(m)) + S(m + 1);
@@ -50,6 +56,18 @@ __device__ __forceinline__ double ppm2_face_regular(SF S, int m, const RecipC& r
         se = half(S(m - 1) + S(m)) - div_6(D2LIM, r6);
     }
     return se;
+}
+// Interior fourth-order limited face value (ppm_type 2).
+template <typename SF>
+__device__ __forceinline__ double ppm2_face_regular(SF S, int m, const RecipC& r6) {
+    const double se = ppm2_face_raw(S, m);
+    return ppm2_face_out(se, S(m - 1), S(m)) ? ppm2_face_limit(S, m, se, r6) : se;
+}
+// Whether the cell limiter leaves alpham = f0 - s0, alphap = f1 - s0 as they are: neither an
+// extremum (alpham * alphap >= 0) nor one more than twice the other.
+__device__ __forceinline__ bool ppm2_cell_plain(double alpham, double alphap) {
+    return prod_gt0(alpham, dflip(alphap)) && !(dmag(alphap) > dmag(twice(alpham))) &&
+           !(dmag(alpham) > dmag(twice(alphap)));
 }
 
 // Van Leer slope of the cell m of S, and the interior interface value between cells m-1 and m
