@@ -19,6 +19,7 @@
 // singular: the rhs is made mean-free, as MLMG does, and phi is returned mean-free.
 #include <cstring>
 
+#include "madv_exact.cuh"
 #include "madv_launch.cuh"
 
 namespace madv {
@@ -40,6 +41,7 @@ struct MGGrid {
     // the operator's weights, formed once per solve (k_mg_prep): W_d = B_d / h_d^2 on every
     // face, and per cell the diagonal and its reciprocal (0 where the diagonal is 0)
     double *W[3], *diag, *idiag;
+    PieceDiv dv, dvh;  // cells of the grid, and of one colour (rows of n[0] / 2)
 };
 struct MGBC {
     int lo[3], hi[3];
@@ -110,33 +112,28 @@ __device__ __forceinline__ void mg_apply(const MGGrid& g, const MGBC& bc, int i,
 #undef MG_TERM
 }
 
-// sum_f W_f phi_nb over the faces of cell (i,j,k) with a neighbour (interior and periodic
-// faces), in mg_apply's order, from the stored weights
-__device__ __forceinline__ double mg_off(const MGGrid& g, const MGBC& bc, const double* __restrict__ phi, int i,
-                                         int j, int k) {
-    double off = 0.0;
-    const int idx[3] = {i, j, k};
-#pragma unroll
-    for (int D = 0; D < 3; ++D)
-#pragma unroll
-        for (int hi = 0; hi < 2; ++hi) {
-            const int m = idx[D], n = g.n[D];
-            const bool edge = hi ? (m == n - 1) : (m == 0);
-            int b[3] = {i, j, k};
-            if (!edge) {
-                b[D] = hi ? m + 1 : m - 1;
-            } else if ((hi ? bc.hi[D] : bc.lo[D]) == MG_PER) {
-                b[D] = hi ? 0 : n - 1;
-            } else {
-                continue;
-            }
-            int a[3] = {i, j, k};
-            a[D] = hi ? m + 1 : m;
-            const long f = D == 0 ? mg_face<0>(g, a[0], a[1], a[2])
-                                  : (D == 1 ? mg_face<1>(g, a[0], a[1], a[2]) : mg_face<2>(g, a[0], a[1], a[2]));
-            off += g.W[D][f] * phi[mg_cell(g, b[0], b[1], b[2])];
-        }
-    return off;
+// init + sum_f W_f phi_nb over the faces of cell (i,j,k) with a neighbour (interior and periodic
+// faces), in mg_apply's order, from the stored weights, one fused multiply-add a face: FP64 issue
+// bounds the sweeps, and product and sum apart took twice the instructions (256^3, 17 cycles: 77.7
+// ms, with the residual below 38.1 ms).  A face without a
+// neighbour adds 0 times the cell itself.  (Grids have fewer than 2^31 cells: 32-bit offsets.)
+__device__ __forceinline__ double mg_sum(const MGGrid& g, const MGBC& bc, const double* __restrict__ phi, int i, int j,
+                                         int k, double init) {
+    const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2], p = n0 * n1;
+    const int row = j + n1 * k, c = i + n0 * row;
+    double s = init;
+    auto term = [&](double w, bool edge, int nb, int type, int wrap) {
+        const bool no = edge && type != MG_PER;
+        s = __fma_rn(no ? 0.0 : w, phi[no ? c : (edge ? wrap : nb)], s);
+    };
+    const double *wx = g.W[0] + c + row, *wy = g.W[1] + c + n0 * k, *wz = g.W[2] + c;
+    term(wx[0], i == 0, c - 1, bc.lo[0], c + n0 - 1);
+    term(wx[1], i == n0 - 1, c + 1, bc.hi[0], c - n0 + 1);
+    term(wy[0], j == 0, c - n0, bc.lo[1], c + p - n0);
+    term(wy[n0], j == n1 - 1, c + n0, bc.hi[1], c - p + n0);
+    term(wz[0], k == 0, c - p, bc.lo[2], c + p * (n2 - 1));
+    term(wz[p], k == n2 - 1, c + p, bc.hi[2], c - p * (n2 - 1));
+    return s;
 }
 
 // W_d = B_d / h_d^2 on the faces of direction D
@@ -161,49 +158,69 @@ __global__ void k_mg_prep_diag(MGGrid g, MGBC bc) {
 
 // Gauss-Seidel update of cell (i,j,k), from the stored weights
 __device__ __forceinline__ void mg_smooth_cell(const MGGrid& g, const MGBC& bc, int i, int j, int k) {
-    const long c = mg_cell(g, i, j, k);
+    const int c = i + g.n[0] * (j + g.n[1] * k);
     const double id = g.idiag[c];
-    if (id > 0.0) g.phi[c] = (g.rhs[c] + mg_off(g, bc, g.phi, i, j, k)) * id;
+    if (id > 0.0) g.phi[c] = mg_sum(g, bc, g.phi, i, j, k, g.rhs[c]) * id;
 }
-__device__ __forceinline__ void mg_resid_cell(const MGGrid& g, const MGBC& bc, int i, int j, int k) {
-    const long c = mg_cell(g, i, j, k);
-    g.res[c] = g.rhs[c] - (g.diag[c] * g.phi[c] - mg_off(g, bc, g.phi, i, j, k));
+// rhs - A phi
+__device__ __forceinline__ double mg_resid_cell(const MGGrid& g, const MGBC& bc, int i, int j, int k) {
+    const int c = i + g.n[0] * (j + g.n[1] * k);
+    return mg_sum(g, bc, g.phi, i, j, k, __fma_rn(-g.diag[c], g.phi[c], g.rhs[c]));
 }
-__device__ __forceinline__ void mg_restrict_cell(const MGGrid& f, const MGGrid& cg, int I, int J, int K) {
+// Coarse rhs = mean of the 8 fine residuals.  The sweeps before it end with colour 1, whose cells
+// then satisfy their equation, so the residual of the 4 children of colour 0 is the sum.
+// The coarse phi is 0 but for its first half sweep -- colour 0, all neighbours 0 --, done here.
+__device__ __forceinline__ void mg_restrict_cell(const MGGrid& f, const MGBC& bc, const MGGrid& cg, int I, int J, int K) {
     double s = 0.0;
-    for (int q = 0; q < 8; ++q) s += f.res[mg_cell(f, 2 * I + (q & 1), 2 * J + ((q >> 1) & 1), 2 * K + (q >> 2))];
-    const long c = mg_cell(cg, I, J, K);
-    cg.rhs[c] = 0.125 * s;
-    cg.phi[c] = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int dj = q & 1, dk = q >> 1;
+        s += mg_resid_cell(f, bc, 2 * I + (dj ^ dk), 2 * J + dj, 2 * K + dk);
+    }
+    const int c = I + cg.n[0] * (J + cg.n[1] * K);
+    const double r = 0.125 * s, id = cg.idiag[c];
+    cg.rhs[c] = r;
+    cg.phi[c] = ((I + J + K) & 1) == 0 && id > 0.0 ? r * id : 0.0;
 }
 
 // Gauss-Seidel on the cells of one colour ((i + j + k) % 2 == color)
 __global__ void k_mg_smooth(MGGrid g, MGBC bc, int color) {
-    const long half = (long)g.n[0] * g.n[1] * g.n[2] / 2;
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= half) return;
+    MADV_LET_NEXT();
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (t >= g.n[0] / 2 * g.n[1] * g.n[2]) return;
     // the t-th cell of the colour: rows of n[0] cells hold n[0]/2 of each colour
-    const long row = t / (g.n[0] / 2);
-    const int jj = (int)(row % g.n[1]), kk = (int)(row / g.n[1]);
-    mg_smooth_cell(g, bc, 2 * (int)(t % (g.n[0] / 2)) + ((jj + kk + color) & 1), jj, kk);
-}
-
-// res = rhs - A phi
-__global__ void k_mg_resid(MGGrid g, MGBC bc) {
-    const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= (long)g.n[0] * g.n[1] * g.n[2]) return;
+    const int lo[3] = {0, 0, 0}, nh[3] = {g.n[0] / 2, g.n[1], g.n[2]};
     int i, j, k;
-    mg_ijk(g, c, i, j, k);
-    mg_resid_cell(g, bc, i, j, k);
+    piece_ijk(lo, nh, g.dvh, t, i, j, k);
+    MADV_WAIT();
+    mg_smooth_cell(g, bc, 2 * i + ((j + k + color) & 1), j, k);
 }
 
-// coarse rhs = mean of the 8 fine residuals; coarse phi = 0
-__global__ void k_mg_restrict(MGGrid f, MGGrid cg) {
-    const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= (long)cg.n[0] * cg.n[1] * cg.n[2]) return;
+// max |rhs - A phi| (bit pattern of a non-negative double)
+__global__ void k_mg_resid_max(MGGrid g, MGBC bc, unsigned long long* out_max) {
+    MADV_LET_NEXT();
+    MADV_WAIT();
+    const int n = g.n[0] * g.n[1] * g.n[2];
+    const int lo[3] = {0, 0, 0};
+    long long m = 0;
+    for (int c = (int)(blockIdx.x * blockDim.x + threadIdx.x); c < n; c += gridDim.x * blockDim.x) {
+        int i, j, k;
+        piece_ijk(lo, g.n, g.dv, c, i, j, k);
+        m = max(m, dmag(mg_resid_cell(g, bc, i, j, k)));
+    }
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(out_max, (unsigned long long)m);
+}
+
+__global__ void k_mg_restrict(MGGrid f, MGBC bc, MGGrid cg) {
+    MADV_LET_NEXT();
+    const int c = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (c >= cg.n[0] * cg.n[1] * cg.n[2]) return;
+    const int lo[3] = {0, 0, 0};
     int I, J, K;
-    mg_ijk(cg, c, I, J, K);
-    mg_restrict_cell(f, cg, I, J, K);
+    piece_ijk(lo, cg.n, cg.dv, c, I, J, K);
+    MADV_WAIT();
+    mg_restrict_cell(f, bc, cg, I, J, K);
 }
 
 // coarse face coefficient = mean of the 4 fine faces it covers
@@ -228,68 +245,128 @@ __global__ void k_mg_coarsen_b(MGGrid f, MGGrid cg) {
     cg.B[D][c] = 0.25 * s;
 }
 
-// fine phi += coarse phi (piecewise constant)
-__device__ __forceinline__ void mg_prolong_cell(const MGGrid& cg, const MGGrid& f, int i, int j, int k) {
-    f.phi[mg_cell(f, i, j, k)] += cg.phi[mg_cell(cg, i / 2, j / 2, k / 2)];
+// fine phi += coarse phi (piecewise constant), on the cells of colour 0: the next sweep begins
+// with colour 1, which reads those and replaces its own.  The t-th cell of the colour.
+__device__ __forceinline__ void mg_prolong_cell(const MGGrid& cg, const MGGrid& f, int t) {
+    const int lo[3] = {0, 0, 0}, nh[3] = {f.n[0] / 2, f.n[1], f.n[2]};
+    int h, j, k;
+    piece_ijk(lo, nh, f.dvh, t, h, j, k);
+    const int i = 2 * h + ((j + k) & 1);
+    f.phi[i + f.n[0] * (j + f.n[1] * k)] += cg.phi[h + cg.n[0] * (j / 2 + cg.n[1] * (k / 2))];
 }
 __global__ void k_mg_prolong(MGGrid cg, MGGrid f) {
-    const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= (long)f.n[0] * f.n[1] * f.n[2]) return;
-    int i, j, k;
-    mg_ijk(f, c, i, j, k);
-    mg_prolong_cell(cg, f, i, j, k);
+    MADV_LET_NEXT();
+    MADV_WAIT();
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (t < f.n[0] / 2 * f.n[1] * f.n[2]) mg_prolong_cell(cg, f, t);
 }
 
 // The V-cycle from a grid of at most MG_BLOCK_CELLS cells down, in one thread block: the
-// same per-cell smoothing, residual, restriction and prolongation as the launches of
+// same per-cell smoothing, restriction and prolongation as the launches of
 // mg_vcycle, in the same order (a colour's update reads only the other colour, so the order
 // within a sweep does not matter), with the block synchronised between steps.  The result
-// is bitwise that of one launch per step; the coarse levels' ~170 launches of a few cells
-// each become one.
+// is bitwise that of one launch per step; the coarse levels' launches of a few cells
+// each become one.  The coarsest grid's sweeps to convergence (64 at least) run in one warp on
+// shared memory where it holds at most 64 cells: a block-wide sweep of 4 cells took 1.5 us.
 constexpr long MG_BLOCK_CELLS = 4096;
 constexpr int MG_BLOCK_LEVELS = 12;
 constexpr int MG_BLOCK_THREADS = 1024;
+constexpr int MG_WARP_CELLS = 64;
 struct MGStack {
     MGGrid g[MG_BLOCK_LEVELS];
     int n;
 };
 
-__device__ void mgb_smooth(const MGGrid& g, const MGBC& bc, int color) {
-    const int nh = g.n[0] / 2, tot = nh * g.n[1] * g.n[2];
+__device__ __forceinline__ void mgb_smooth(const MGGrid& g, const MGBC& bc, int color) {
+    const int lo[3] = {0, 0, 0}, nh[3] = {g.n[0] / 2, g.n[1], g.n[2]};
+    const int tot = nh[0] * nh[1] * nh[2];
     for (int t = threadIdx.x; t < tot; t += blockDim.x) {
-        const int row = t / nh, jj = row % g.n[1], kk = row / g.n[1];
-        mg_smooth_cell(g, bc, 2 * (t % nh) + ((jj + kk + color) & 1), jj, kk);
+        int i, j, k;
+        piece_ijk(lo, nh, g.dvh, t, i, j, k);
+        mg_smooth_cell(g, bc, 2 * i + ((j + k + color) & 1), j, k);
     }
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(MG_BLOCK_THREADS) k_mg_block_cycle(MGStack S, MGBC bc, int nu, int bottom) {
+// `sweeps` sweeps of a grid of at most MG_WARP_CELLS cells by one warp: mg_smooth_cell's update
+// with the cells' weights, neighbours and values in shared memory
+struct MGWarpGrid {
+    double w[6][MG_WARP_CELLS], rhs[MG_WARP_CELLS], id[MG_WARP_CELLS], phi[MG_WARP_CELLS];
+    int nb[6][MG_WARP_CELLS];
+};
+__device__ __forceinline__ void mgw_smooth(MGWarpGrid& s, const MGGrid& g, const MGBC& bc, int sweeps) {
+    const int lane = threadIdx.x & 31, n0 = g.n[0], n1 = g.n[1], n2 = g.n[2], p = n0 * n1, n = p * n2;
+    for (int c = lane; c < n; c += 32) {
+        const int i = c % n0, j = c / n0 % n1, k = c / p, row = j + n1 * k;
+        const double* W[6] = {g.W[0] + c + row, g.W[0] + c + row + 1, g.W[1] + c + n0 * k, g.W[1] + c + n0 * k + n0,
+                              g.W[2] + c, g.W[2] + c + p};
+        const int x[3] = {i, j, k}, st[3] = {1, n0, p};
+        for (int q = 0; q < 6; ++q) {
+            const int d = q >> 1, hi = q & 1;
+            const bool edge = x[d] == (hi ? g.n[d] - 1 : 0);
+            const bool no = edge && (hi ? bc.hi[d] : bc.lo[d]) != MG_PER;
+            const int step = edge ? (hi ? 1 - g.n[d] : g.n[d] - 1) : (hi ? 1 : -1);
+            s.w[q][c] = no ? 0.0 : *W[q];
+            s.nb[q][c] = no ? c : c + step * st[d];
+        }
+        s.rhs[c] = g.rhs[c];
+        s.id[c] = g.idiag[c];
+        s.phi[c] = g.phi[c];
+    }
+    __syncwarp();
+    const int half = n / 2, nh = n0 / 2;
+    for (int h = 0; h < 2 * sweeps; ++h) {
+        const int color = h & 1;
+        for (int t = lane; t < half; t += 32) {
+            const int row = t / nh, j = row % n1, k = row / n1, c = 2 * (t % nh) + ((j + k + color) & 1) + n0 * row;
+            const double id = s.id[c];
+            if (id > 0.0) {
+                double v = s.rhs[c];
+#pragma unroll
+                for (int q = 0; q < 6; ++q) v = __fma_rn(s.w[q][c], s.phi[s.nb[q][c]], v);
+                s.phi[c] = v * id;
+            }
+        }
+        __syncwarp();
+    }
+    for (int c = lane; c < n; c += 32) g.phi[c] = s.phi[c];
+}
+
+// started: the first grid's first half sweep was done by the restriction onto it
+__global__ void __launch_bounds__(MG_BLOCK_THREADS) k_mg_block_cycle(MGStack S, MGBC bc, int nu, int bottom, int started) {
+    __shared__ MGWarpGrid ws;
+    MADV_LET_NEXT();
+    MADV_WAIT();
     const int last = S.n - 1;
     for (int l = 0; l < last; ++l) {
         const MGGrid& g = S.g[l];
         const MGGrid& cg = S.g[l + 1];
         for (int s = 0; s < nu; ++s) {
-            mgb_smooth(g, bc, 0);
+            if (s || !(l || started)) mgb_smooth(g, bc, 0);
             mgb_smooth(g, bc, 1);
         }
-        const int n = g.n[0] * g.n[1] * g.n[2];
-        for (int c = threadIdx.x; c < n; c += blockDim.x)
-            mg_resid_cell(g, bc, c % g.n[0], (c / g.n[0]) % g.n[1], c / (g.n[0] * g.n[1]));
-        __syncthreads();
-        const int nc = cg.n[0] * cg.n[1] * cg.n[2];
-        for (int c = threadIdx.x; c < nc; c += blockDim.x)
-            mg_restrict_cell(g, cg, c % cg.n[0], (c / cg.n[0]) % cg.n[1], c / (cg.n[0] * cg.n[1]));
+        const int nc = cg.n[0] * cg.n[1] * cg.n[2], lo[3] = {0, 0, 0};
+        for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+            int I, J, K;
+            piece_ijk(lo, cg.n, cg.dv, c, I, J, K);
+            mg_restrict_cell(g, bc, cg, I, J, K);
+        }
         __syncthreads();
     }
-    for (int s = 0; s < bottom; ++s) {
-        mgb_smooth(S.g[last], bc, 0);
-        mgb_smooth(S.g[last], bc, 1);
+    const MGGrid& gb = S.g[last];
+    if (gb.n[0] * gb.n[1] * gb.n[2] <= MG_WARP_CELLS) {
+        if (threadIdx.x < 32) mgw_smooth(ws, gb, bc, bottom);
+        __syncthreads();
+    } else {
+        for (int s = 0; s < bottom; ++s) {
+            mgb_smooth(gb, bc, 0);
+            mgb_smooth(gb, bc, 1);
+        }
     }
     for (int l = last - 1; l >= 0; --l) {
         const MGGrid& g = S.g[l];
-        const int n = g.n[0] * g.n[1] * g.n[2];
-        for (int c = threadIdx.x; c < n; c += blockDim.x)
-            mg_prolong_cell(S.g[l + 1], g, c % g.n[0], (c / g.n[0]) % g.n[1], c / (g.n[0] * g.n[1]));
+        const int n = g.n[0] / 2 * g.n[1] * g.n[2];
+        for (int t = threadIdx.x; t < n; t += blockDim.x) mg_prolong_cell(S.g[l + 1], g, t);
         __syncthreads();
         for (int s = 0; s < nu; ++s) {
             mgb_smooth(g, bc, 1);
@@ -298,24 +375,26 @@ __global__ void __launch_bounds__(MG_BLOCK_THREADS) k_mg_block_cycle(MGStack S, 
     }
 }
 
-// out_max = max |x| (bit pattern of a non-negative double); part[block] = the block's sum of
-// x.  Every partial sum is formed in a fixed order (grid-stride per thread, a shuffle tree
+// out_max = max |x| (bit pattern of a non-negative double, compared as such); part[block] = the
+// block's sum of x (null: no sum).  Every partial sum is formed in a fixed order (grid-stride per thread, a shuffle tree
 // per warp, warps in order per block), so the sum does not depend on scheduling.
 __global__ void k_mg_norms(const double* __restrict__ x, long n, unsigned long long* out_max, double* part) {
     __shared__ double ws[32];
-    double m = 0.0, s = 0.0;
+    long long m = 0;
+    double s = 0.0;
     for (long c = (long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long)gridDim.x * blockDim.x) {
-        m = fmax(m, fabs(x[c]));
-        s += x[c];
+        m = max(m, dmag(x[c]));
+        if (part) s += x[c];
     }
     for (int o = 16; o > 0; o >>= 1) {
-        m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-        s += __shfl_down_sync(0xffffffffu, s, o);
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (part) s += __shfl_down_sync(0xffffffffu, s, o);
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(out_max, (unsigned long long)__double_as_longlong(m));
+        atomicMax(out_max, (unsigned long long)m);
         ws[threadIdx.x >> 5] = s;
     }
+    if (!part) return;
     __syncthreads();
     if (threadIdx.x == 0) {
         double b = 0.0;
@@ -362,7 +441,7 @@ __global__ void k_mp_beta_faces(KARGS, MGGrid g, double* __restrict__ out, int l
 // Valid cells: rho into g.res (read by the coefficient kernels), the solver rhs
 // macrhs - div(beta0 umac) (ComputeMACSolverRHS after MultFacesByBeta0 or, spherical, the
 // product with beta0mac), phi = 0.
-__global__ void k_mp_gather(KARGS, MGGrid g, int srhs, int srho, MPBeta be, double dx0, double dx1, double dx2, int l0,
+__global__ void k_mp_gather(KARGS, MGGrid g, int srhs, int srho, MPBeta be, RecipC dx0, RecipC dx1, RecipC dx2, int l0,
                             int l1, int l2) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView u = VW(F_UMAC0), v = VW(F_UMAC1), w = VW(F_UMAC2);
@@ -370,9 +449,9 @@ __global__ void k_mp_gather(KARGS, MGGrid g, int srhs, int srho, MPBeta be, doub
     const long c = mg_cell(g, a0, a1, kr);
     g.res[c] = at(VW(F_USER + srho), i, j, k);
     g.rhs[c] = at(VW(F_USER + srhs), i, j, k) -
-               ((at(u, i + 1, j, k) * mp_beta<0>(be, g, a0 + 1, a1, kr) - at(u, i, j, k) * mp_beta<0>(be, g, a0, a1, kr)) / dx0 +
-                (at(v, i, j + 1, k) * mp_beta<1>(be, g, a0, a1 + 1, kr) - at(v, i, j, k) * mp_beta<1>(be, g, a0, a1, kr)) / dx1 +
-                (at(w, i, j, k + 1) * mp_beta<2>(be, g, a0, a1, kr + 1) - at(w, i, j, k) * mp_beta<2>(be, g, a0, a1, kr)) / dx2);
+               (div_c(at(u, i + 1, j, k) * mp_beta<0>(be, g, a0 + 1, a1, kr) - at(u, i, j, k) * mp_beta<0>(be, g, a0, a1, kr), dx0) +
+                div_c(at(v, i, j + 1, k) * mp_beta<1>(be, g, a0, a1 + 1, kr) - at(v, i, j, k) * mp_beta<1>(be, g, a0, a1, kr), dx1) +
+                div_c(at(w, i, j, k + 1) * mp_beta<2>(be, g, a0, a1, kr + 1) - at(w, i, j, k) * mp_beta<2>(be, g, a0, a1, kr), dx2));
     g.phi[c] = 0.0;
 }
 
@@ -443,7 +522,7 @@ __global__ void k_pcg_apply(MGGrid g, MGBC bc, const double* __restrict__ p, dou
     if (c >= (long)g.n[0] * g.n[1] * g.n[2]) return;
     int i, j, k;
     mg_ijk(g, c, i, j, k);
-    q[c] = g.diag[c] * p[c] - mg_off(g, bc, p, i, j, k);
+    q[c] = __fma_rn(g.diag[c], p[c], -mg_sum(g, bc, p, i, j, k, 0.0));
 }
 
 // part[block] = the block's sum of x * y, in a fixed order (as k_mg_norms)
@@ -556,6 +635,9 @@ static int mac_hierarchy(Ctx& c, const int n0[3], int nr) {
             g.ih2[d] = 1.0 / h2[d];
         }
         const long nc = (long)n[0] * n[1] * n[2];
+        const int nh[3] = {n[0] / 2, n[1], n[2]};
+        g.dv = piece_div(n);
+        g.dvh = piece_div(nh);
         g.phi = alloc(nc);
         g.rhs = alloc(nc);
         g.res = alloc(nc);
@@ -602,13 +684,22 @@ static int mac_hierarchy(Ctx& c, const int n0[3], int nr) {
 }
 
 static void mg_smooth(Ctx& c, const MGGrid& g, const MGBC& bc, int color) {
-    k_mg_smooth<<<blocks_of(ncell(g) / 2), TPB, 0, c.stream>>>(g, bc, color);
+    launch_next(c, blocks_of(ncell(g) / 2), TPB, k_mg_smooth, g, bc, color);
     c.launches++;
 }
 
-static void mg_resid(Ctx& c, const MGGrid& g, const MGBC& bc) {
-    k_mg_resid<<<blocks_of(ncell(g)), TPB, 0, c.stream>>>(g, bc);
+// max |rhs - A phi|, read back (the stream is synchronised)
+static int mg_resid_max(Ctx& c, const MGGrid& g, const MGBC& bc, double& amax) {
+    MacMG& M = *c.mac;
+    MP_CK(cudaMemsetAsync(M.d_max, 0, sizeof(unsigned long long), c.stream));
+    const unsigned nb = (unsigned)std::min<long>((ncell(g) + TPB - 1) / TPB, NORM_BLOCKS);
+    launch_next(c, dim3(nb), TPB, k_mg_resid_max, g, bc, M.d_max);
     c.launches++;
+    unsigned long long bits = 0;
+    MP_CK(cudaMemcpyAsync(&bits, M.d_max, sizeof(bits), cudaMemcpyDeviceToHost, c.stream));
+    MP_CK(cudaStreamSynchronize(c.stream));
+    std::memcpy(&amax, &bits, sizeof(double));
+    return MADV_OK;
 }
 
 static int mg_bottom_sweeps(const MGGrid& g) {  // the coarsest grid: to convergence
@@ -625,7 +716,7 @@ static void mg_vcycle(Ctx& c, const MGBC& bc, int l) {
         MGStack S{};
         S.n = nrest;
         for (int q = 0; q < nrest; ++q) S.g[q] = M.lev[l + q];
-        k_mg_block_cycle<<<1, MG_BLOCK_THREADS, 0, c.stream>>>(S, bc, nu, mg_bottom_sweeps(M.lev.back()));
+        launch_next(c, dim3(1), MG_BLOCK_THREADS, k_mg_block_cycle, S, bc, nu, mg_bottom_sweeps(M.lev.back()), (int)(l > 0));
         c.launches++;
         return;
     }
@@ -637,15 +728,14 @@ static void mg_vcycle(Ctx& c, const MGBC& bc, int l) {
         return;
     }
     for (int s = 0; s < nu; ++s) {
-        mg_smooth(c, g, bc, 0);
+        if (s || l == 0) mg_smooth(c, g, bc, 0);  // below the finest grid the restriction does the first
         mg_smooth(c, g, bc, 1);
     }
     const MGGrid& cg = M.lev[l + 1];
-    mg_resid(c, g, bc);
-    k_mg_restrict<<<blocks_of(ncell(cg)), TPB, 0, c.stream>>>(g, cg);
+    launch_next(c, blocks_of(ncell(cg)), TPB, k_mg_restrict, g, bc, cg);
     c.launches++;
     mg_vcycle(c, bc, l + 1);
-    k_mg_prolong<<<blocks_of(ncell(g)), TPB, 0, c.stream>>>(cg, g);
+    launch_next(c, blocks_of(ncell(g) / 2), TPB, k_mg_prolong, cg, g);
     c.launches++;
     for (int s = 0; s < nu; ++s) {  // the reverse colour order keeps the cycle symmetric
         mg_smooth(c, g, bc, 1);
@@ -658,14 +748,15 @@ static int mg_norms(Ctx& c, const double* x, long n, double& amax, double* sum_o
     MacMG& M = *c.mac;
     MP_CK(cudaMemsetAsync(M.d_max, 0, sizeof(unsigned long long), c.stream));
     const unsigned nb = (unsigned)std::min<long>((n + TPB - 1) / TPB, NORM_BLOCKS);
-    k_mg_norms<<<nb, TPB, 0, c.stream>>>(x, n, M.d_max, M.d_part);
-    k_mg_sum_parts<<<1, 1, 0, c.stream>>>(M.d_part, (int)nb, M.d_sum);
-    c.launches += 2;
+    const bool sum = sum_out || device_sum_only;
+    k_mg_norms<<<nb, TPB, 0, c.stream>>>(x, n, M.d_max, sum ? M.d_part : nullptr);
+    if (sum) k_mg_sum_parts<<<1, 1, 0, c.stream>>>(M.d_part, (int)nb, M.d_sum);
+    c.launches += 1 + sum;
     if (device_sum_only) return MADV_OK;
     unsigned long long bits = 0;
     double s = 0.0;
     MP_CK(cudaMemcpyAsync(&bits, M.d_max, sizeof(bits), cudaMemcpyDeviceToHost, c.stream));
-    MP_CK(cudaMemcpyAsync(&s, M.d_sum, sizeof(s), cudaMemcpyDeviceToHost, c.stream));
+    if (sum) MP_CK(cudaMemcpyAsync(&s, M.d_sum, sizeof(s), cudaMemcpyDeviceToHost, c.stream));
     MP_CK(cudaStreamSynchronize(c.stream));
     std::memcpy(&amax, &bits, sizeof(double));
     if (sum_out) *sum_out = s;
@@ -777,8 +868,8 @@ int mac_project_level(Ctx& c, int srhs, int srho, int sphi, const double* beta0,
         MP_CK(cudaMemcpyAsync(M.d_beta, beta0, sizeof(double) * nr, cudaMemcpyHostToDevice, c.stream));
         MP_CK(cudaMemcpyAsync(M.d_beta + nr, beta0_edge, sizeof(double) * (nr + 1), cudaMemcpyHostToDevice, c.stream));
     }
-    launch(c, rg_grow(c, 0), 1, k_mp_gather, c.V(), g, srhs, srho, be, c.P.dx[0], c.P.dx[1], c.P.dx[2], l[0], l[1],
-           l[2]);
+    launch(c, rg_grow(c, 0), 1, k_mp_gather, c.V(), g, srhs, srho, be, make_recip(c.P.dx[0]),
+           make_recip(c.P.dx[1]), make_recip(c.P.dx[2]), l[0], l[1], l[2]);
     auto faces = [&](long n, int d) { return n / g.n[d] * (g.n[d] + 1); };
     k_mp_bcoef<0><<<blocks_of(faces(ncell(g), 0)), TPB, 0, c.stream>>>(g, bc, be);
     k_mp_bcoef<1><<<blocks_of(faces(ncell(g), 1)), TPB, 0, c.stream>>>(g, bc, be);
@@ -814,8 +905,7 @@ int mac_project_level(Ctx& c, int srhs, int srho, int sphi, const double* beta0,
     double res_max = 0.0;
     if (!c.sph) {  // V-cycles on the residual equation until the reference's stopping test holds
         while (true) {
-            mg_resid(c, g, bc);
-            if ((rc = mg_norms(c, g.res, n, res_max, nullptr))) return rc;
+            if ((rc = mg_resid_max(c, g, bc, res_max))) return rc;
             if (res_max <= target || it >= max_iter) break;
             mg_vcycle(c, bc, 0);
             ++it;
