@@ -351,6 +351,29 @@ static void cell_to_edge_chunk(const std::vector<double>& cc, std::vector<double
     }
 }
 
+// A radial array as the device holds it.  A bin-centred array of uniform spherical bins is followed
+// by what the quadratic interpolation around bin i needs and no cell changes: the divided
+// differences (y1 - y0) / (x1 - x0) and ((y2 - y1) / (x2 - x1) - that) / (x2 - x0) of the points
+// i - 1, i, i + 1, and the largest and smallest of their values, nr + 1 doubles each.
+static size_t radial_table_max(const Ctx& c) { return (size_t)(c.nr + 1) * (c.sph && !c.geo.exact ? 5 : 1); }
+static std::vector<double> radial_table(const Ctx& c, const std::vector<double>& y) {
+    std::vector<double> t(y);
+    const size_t q = (size_t)c.nr + 1;
+    auto rc = c.h1.find("r_cc_loc");
+    if (!c.sph || c.geo.exact || (int)y.size() != c.nr || rc == c.h1.end()) return t;
+    const std::vector<double>& x = rc->second;
+    t.resize(5 * q, 0.0);
+    for (int i = 1; i + 1 < c.nr; ++i) {
+        const double x0 = x[i - 1], x1 = x[i], x2 = x[i + 1], y0 = y[i - 1], y1 = y[i], y2 = y[i + 1];
+        t[q + i] = (y1 - y0) / (x1 - x0);
+        t[2 * q + i] = ((y2 - y1) / (x2 - x1) - (y1 - y0) / (x1 - x0)) / (x2 - x0);
+        const double m12 = y1 > y2 ? y1 : y2, n12 = y1 < y2 ? y1 : y2;
+        t[3 * q + i] = y0 > m12 ? y0 : m12;
+        t[4 * q + i] = y0 < n12 ? y0 : n12;
+    }
+    return t;
+}
+
 // ------------------------------------------------------------------ user FAB binding
 struct Binding {
     int slot;
@@ -1180,6 +1203,7 @@ struct madv_ctx {
 static void sph_radial_grid(Ctx& c, double dxf, int nfine) {
     c.geo.dxf = dxf;
     c.geo.drf = dxf / (c.P.drdxfac > 0 ? c.P.drdxfac : 1);
+    c.geo.rdrf = make_recip(c.geo.drf);
     if (c.geo.exact) {
         const double domhi = nfine;
         c.nr = int((3.0 * (domhi / 2 - 0.5) * (domhi / 2 - 0.5) - 0.75) / 2.0) + 1;
@@ -1724,8 +1748,9 @@ int madv_set_base_state_levels(madv_ctx* h, int nlev, const madv_base_state* bsl
         Ctx& c = H[l];
         for (auto& kv : c.h1) {
             double*& d = c.d1[kv.first];
-            if (!d && !cuda_ok(cudaMalloc(&d, sizeof(double) * (c.nr + 1)), "cudaMalloc(base)")) return MADV_ERR_CUDA;
-            if (!cuda_ok(cudaMemcpy(d, kv.second.data(), sizeof(double) * kv.second.size(), cudaMemcpyHostToDevice),
+            const std::vector<double> v = radial_table(c, kv.second);
+            if (!d && !cuda_ok(cudaMalloc(&d, sizeof(double) * radial_table_max(c)), "cudaMalloc(base)")) return MADV_ERR_CUDA;
+            if (!cuda_ok(cudaMemcpy(d, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice),
                          "cudaMemcpy(base)"))
                 return MADV_ERR_CUDA;
         }
@@ -2298,8 +2323,9 @@ int madv_mac_project(madv_ctx* h, const madv_multifab* umac, const madv_multifab
             std::vector<double>& b = c.h1["beta0_mac"];
             b.assign(beta0, beta0 + c.nr);
             double*& d = c.d1["beta0_mac"];
-            if (!d && !cuda_ok(cudaMalloc(&d, sizeof(double) * (c.nr + 1)), "cudaMalloc(beta0)")) return MADV_ERR_CUDA;
-            if (!cuda_ok(cudaMemcpyAsync(d, b.data(), sizeof(double) * c.nr, cudaMemcpyHostToDevice, c.stream),
+            const std::vector<double> v = radial_table(c, b);
+            if (!d && !cuda_ok(cudaMalloc(&d, sizeof(double) * radial_table_max(c)), "cudaMalloc(beta0)")) return MADV_ERR_CUDA;
+            if (!cuda_ok(cudaMemcpyAsync(d, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice, c.stream),
                          "cudaMemcpyAsync(beta0)"))
                 return MADV_ERR_CUDA;
             make_s0mac_h(H, "beta0_mac", F_S0MAC0);

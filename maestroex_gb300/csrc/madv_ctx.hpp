@@ -11,6 +11,7 @@
 
 #include "../../include/maestro_adv.h"
 #include "madv_core.cuh"
+#include "madv_exact.cuh"
 
 namespace madv {
 
@@ -29,6 +30,7 @@ struct SphGeo {
     double plo[3], dx[3], ctr[3];
     double dxf;  // cell size of the finest level, which sets the radial grid
     double drf;  // base_geom.dr_fine
+    RecipC rdrf;  // division by it
     int exact;   // use_exact_base_state
     int nr;      // nr_fine
     int w0i, w0maci, s0i, s0maci;  // w0_interp_type, w0mac_interp_type, s0_interp_type, s0mac_interp_type

@@ -9,18 +9,23 @@
 //
 // 2. Division by a constant y from a precomputed double-word reciprocal zh + zl
 //    (zh = RN(1/y), zl = RN(1/y - zh)):
-//        q0 = RN(a*zh + RN(a*zl))            faithful (error <= 1/2 ulp + 2^-104 rel.)
+//        q0 = RN(a*zh + RN(a*zl))            within 2^-52 ulp of a/y before its last rounding
+//    q0 is RN(a/y) unless a/y lies that close to a rounding boundary.  With integer significands
+//    X, Y in [2^52, 2^53) that needs |2^s X - (2m+1) Y| < 4 (s = 53 where X >= Y, 54 below), which
+//    at most a few X solve, found once from the residues of X modulo Y (multiplication by an
+//    arbitrary-precision constant: N. Brisebarre, J.-M. Muller, IEEE Trans. Comput. 57(2),
+//    2008); the significands that do round wrongly are kept (none where Y ends in two zero
+//    bits) and take the IEEE division, as do zeros and |a| outside [2^-959, 2^977).
+//    Cost: 1 DMUL + 1 DFMA.
+//    By 6 there are none: with a = A 2^e the quotient is A/3 2^(e-1), and a third of an integer
+//    is never closer than 1/6 ulp to a rounding boundary.
+//    By a value known on the device only (recip_v, div_v) the quotient is corrected:
 //        r  = RN(a - q0*y)                   exact (FMA; the remainder is representable)
 //        q  = RN(q0 + r*zh)                  = RN(a/y)
 //    The last step is Markstein's theorem (P. Markstein, IBM J. Res. Dev. 34(1), 1990;
 //    see also N. Brisebarre, J.-M. Muller, S. K. Raina, IEEE Trans. Comput. 53(8),
 //    2004): with zh the correctly rounded reciprocal and q0 faithful, the corrected
-//    quotient is the correctly rounded one.  It holds while no intermediate underflows or
-//    overflows; zeros and |a| outside [2^-959, 2^977) take the IEEE division instead.
-//    Cost: 1 DMUL + 3 DFMA.
-//    By 6 the first step is already the quotient (div_6): with a = A 2^e the quotient is
-//    A/3 2^(e-1), and a third of an integer is never closer than 1/6 ulp to a rounding
-//    boundary, while a*zh + RN(a*zl) is off by 2^-106.  Cost: 1 DMUL + 1 DFMA.
+//    quotient is the correctly rounded one.  Cost: 1 DMUL + 3 DFMA.
 //
 // |x| and -x as plain expressions on the bit pattern are recognised by the compiler and
 // turned back into FP64 instructions (DADD 0 + |x|): k_dsvl ran 6 DADD per cell for its 3
@@ -165,7 +170,30 @@ __device__ __forceinline__ bool prod_gt0(double x, double y) {
 
 struct RecipC {
     double y, zh, zl;
+    unsigned bad[4];  // low words of the significands that the two-step quotient misrounds
+    int nbad;         // -1: more than 4 (or y not normal), the quotient is corrected
 };
+
+// The integer significands X in [2^52, 2^53) whose quotient by Y (the same range) comes within
+// 2^-52 ulp of a rounding boundary: at most 16 (out holds them).
+__host__ inline int hard_significands(unsigned long long Y, unsigned long long out[16]) {
+    const unsigned long long lo = 1ULL << 52, hi = 1ULL << 53;
+    const int v = (Y & 1) ? 0 : (Y & 2) ? 1 : 2;
+    if (v == 2) return 0;  // 2^v divides 2^s X - (2m+1) Y, which is not 0: at least 4
+    const unsigned long long Y0 = Y >> v, inv2 = (Y0 + 1) / 2;
+    int n = 0;
+    for (int s = 53; s <= 54; ++s) {
+        unsigned long long inv = 1 % Y0;  // of 2^(s-v) modulo Y0
+        for (int q = 0; q < s - v; ++q) inv = (unsigned long long)((unsigned __int128)inv * inv2 % Y0);
+        for (int N = -3; N <= 3; ++N) {  // the difference over 2^v
+            if (N % 2 == 0 || (v == 1 && (N == 3 || N == -3))) continue;
+            const unsigned long long r = N > 0 ? (unsigned long long)N % Y0 : (Y0 - (unsigned long long)(-N) % Y0) % Y0;
+            for (unsigned long long X = (unsigned long long)((unsigned __int128)r * inv % Y0); X < hi; X += Y0)
+                if (X >= lo && (X >= Y) == (s == 53) && n < 16) out[n++] = X;
+        }
+    }
+    return n;
+}
 
 __host__ inline RecipC make_recip(double y) {
     RecipC r;
@@ -174,15 +202,44 @@ __host__ inline RecipC make_recip(double y) {
     // 1/y - zh = (1 - zh*y)/y; the residual 1 - zh*y is exact with an FMA
     const double e = __builtin_fma(-r.zh, y, 1.0);
     r.zl = e / y;
+    r.nbad = 0;
+    const long long b = dbits_host(y);
+    const int ex = (int)(b >> 52) & 0x7ff;
+    if (ex < 64 || ex > 1983) {  // the reciprocal's words could under- or overflow
+        r.nbad = -1;
+        return r;
+    }
+    unsigned long long X[16];
+    const int n = hard_significands((unsigned long long)(b & 0x000fffffffffffffLL) | (1ULL << 52), X);
+    for (int q = 0; q < n; ++q) {
+        const double a = (double)X[q];
+        if (__builtin_fma(a, r.zh, a * r.zl) == a / y) continue;
+        if (r.nbad == 4) {
+            r.nbad = -1;
+            return r;
+        }
+        r.bad[r.nbad++] = (unsigned)X[q];
+    }
+    for (int q = r.nbad; q < 4; ++q) r.bad[q] = r.nbad ? r.bad[0] : 0;
     return r;
 }
 
-__device__ __forceinline__ double div_c(double a, const RecipC& r) {
-    const unsigned ex = ((unsigned)dhigh(a) >> 20) & 0x7ff;
-    if (ex < 64 || ex >= 2000) return a / r.y;
+__device__ __forceinline__ double div_corrected(double a, const RecipC& r) {
     const double q0 = __fma_rn(a, r.zh, a * r.zl);
     const double rem = __fma_rn(-q0, r.y, a);
     return __fma_rn(rem, r.zh, q0);
+}
+__device__ __forceinline__ double div_c(double a, const RecipC& r) {
+    int hi, lo;
+    dsplit(a, hi, lo);
+    const unsigned ex = ((unsigned)hi >> 20) & 0x7ff;
+    if (ex < 64 || ex >= 2000) return a / r.y;
+    if (r.nbad != 0) {
+        if (r.nbad < 0) return div_corrected(a, r);
+        const unsigned l = (unsigned)lo;
+        if (l == r.bad[0] || l == r.bad[1] || l == r.bad[2] || l == r.bad[3]) return a / r.y;
+    }
+    return __fma_rn(a, r.zh, a * r.zl);
 }
 
 // Division by a value y that several numerators share, formed on the device: the same
@@ -204,9 +261,7 @@ __device__ __forceinline__ RecipV recip_v(double y) {
 __device__ __forceinline__ double div_v(double a, const RecipV& v) {
     const unsigned ex = ((unsigned)dhigh(a) >> 20) & 0x7ff;
     if (!v.ok || ex < 323 || ex >= 1723) return a / v.r.y;  // |a| outside 2^-700 .. 2^700
-    const double q0 = __fma_rn(a, v.r.zh, a * v.r.zl);
-    const double rem = __fma_rn(-q0, v.r.y, a);
-    return __fma_rn(rem, v.r.zh, q0);
+    return div_corrected(a, v.r);
 }
 
 // a / 6 with r6 = make_recip(6): exact for zeros too (zl > 0 keeps their sign)

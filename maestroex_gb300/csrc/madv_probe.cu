@@ -2,6 +2,8 @@
 // probe used as the roofline ceiling of the FP64-bound stage kernels.
 #include <cuda_runtime.h>
 
+#include <cstring>
+
 #include "../../include/maestro_adv.h"
 
 namespace madv {
@@ -65,7 +67,11 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
 
 // Random doubles with exponents spread over [2^-1000, 2^1000], both signs, plus
 // zeros, subnormals and values next to powers of two; each checked bit for bit.
-__global__ void k_selftest(unsigned long long n, unsigned long long seed, RecipC r, RecipC r6, double thr,
+struct HardX {
+    unsigned long long x[16];
+    int n;
+};
+__global__ void k_selftest(unsigned long long n, unsigned long long seed, RecipC r, RecipC r6, HardX hx, double thr,
                            unsigned long long* fails) {
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -85,6 +91,12 @@ __global__ void k_selftest(unsigned long long n, unsigned long long seed, RecipC
             unsigned long long bits = (ex << 52) | (kind == 2 ? 0ULL : (kind == 3 ? 0x000fffffffffffffULL : mant));
             if (h & 32) bits |= 0x8000000000000000ULL;
             a = __longlong_as_double((long long)bits);
+        }
+        // the significands next to a rounding boundary of the quotient, and one off them
+        if (hx.n && kind == 4) {
+            unsigned long long X = hx.x[(h >> 40) % hx.n] + ((h >> 50) & 1 ? 0 : (h >> 51) % 3 - 1);
+            a = __longlong_as_double((long long)((X & 0x000fffffffffffffULL) | ((100 + (h >> 20) % 1800) << 52)));
+            if (h & 32) a = -a;
         }
         const double q = div_c(a, r);
         const double qi = a / r.y;
@@ -156,8 +168,14 @@ extern "C" int madv_selftest_exact(double y, double threshold, long long n, long
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    madv::HardX hx{};
+    {
+        long long b;
+        memcpy(&b, &y, sizeof(b));
+        hx.n = madv::hard_significands((unsigned long long)(b & 0x000fffffffffffffLL) | (1ULL << 52), hx.x);
+    }
     madv::k_selftest<<<nsm * 8, 256, 0, s>>>((unsigned long long)n, 0x1234567ULL, madv::make_recip(y), madv::make_recip(6.0),
-                                               threshold, d);
+                                               hx, threshold, d);
     unsigned long long h = 0;
     cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, s);
     cudaStreamSynchronize(s);

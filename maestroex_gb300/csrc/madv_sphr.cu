@@ -5,8 +5,8 @@
 // spherical branches of Put1dArrayOnCart, MakeW0mac, MakeS0mac, Addw0, MakeVelForce,
 // ModifyScalForce, MakeRhoHForce, PutInPertForm, MakeRhoXFlux and MakeRhoHFlux.  The
 // MakeUtrans / VelPred Riemann solves with w0mac are flags of their kernels in
-// madv_kernels.cu.  Divisions by dx and radii are IEEE divisions, as the reference writes
-// them; `sqrt` is the correctly rounded square root.
+// madv_kernels.cu.  Divisions by dx and radii are correctly rounded, as the reference writes
+// them (div_c, div_v); `sqrt` is the correctly rounded square root.
 #include "madv_exact.cuh"
 #include "madv_launch.cuh"
 
@@ -52,7 +52,7 @@ __device__ __forceinline__ double sph_edge_value(const SphGeo& g, const double* 
         if (index < nr) rfac = (radius - redge[index + 1]) / (rcc[index + 1] - rcc[index]);
         else rfac = (radius - redge[index + 1]) / (rcc[index] - rcc[index - 1]);
     } else {
-        rfac = (radius - double(index) * g.drf) / g.drf;
+        rfac = div_c(radius - double(index) * g.drf, g.rdrf);
     }
     if (t == 1) return rfac > 0.5 ? s0[index + 1] : s0[index];
     if (t == 2) return index < nr ? rfac * s0[index + 1] + (1.0 - rfac) * s0[index] : s0[nr];
@@ -70,21 +70,31 @@ __device__ __forceinline__ double sph_edge_value(const SphGeo& g, const double* 
 __device__ __forceinline__ double sph_cell_value(const SphGeo& g, const double* __restrict__ s0,
                                                  const double* __restrict__ rcc, double radius, int t) {
     const int nr = g.nr;
-    const double drf = g.drf;
-    int index = int(radius / drf);
+    int index = int(div_c(radius, g.rdrf));
     if (t == 1) return s0[index];
     if (t == 2) {
         if (index > nr - 1) return s0[nr - 1];
         if (radius >= rcc[index]) {
             if (index >= nr - 1) return s0[nr - 1];
-            return s0[index + 1] * (radius - rcc[index]) / drf + s0[index] * (rcc[index + 1] - radius) / drf;
+            return div_c(s0[index + 1] * (radius - rcc[index]), g.rdrf) +
+                   div_c(s0[index] * (rcc[index + 1] - radius), g.rdrf);
         }
         if (index == 0) return s0[index];
-        return s0[index] * (radius - rcc[index - 1]) / drf + s0[index - 1] * (rcc[index] - radius) / drf;
+        return div_c(s0[index] * (radius - rcc[index - 1]), g.rdrf) +
+               div_c(s0[index - 1] * (rcc[index] - radius), g.rdrf);
     }
     if (index == 0) index = 1;
     else if (index >= nr - 1) index = nr - 2;
-    return quad_interp(radius, rcc[index - 1], rcc[index], rcc[index + 1], s0[index - 1], s0[index], s0[index + 1]);
+    // quad_interp with what depends on the bin alone -- the divided differences and the range of
+    // the three values -- from the array's table (radial_table): 7 FP64 instructions and no
+    // division, where the three divisions of each cell took 40
+    const int q = nr + 1;
+    const double dx = radius - rcc[index - 1];
+    double y = s0[index - 1] + s0[q + index] * dx + s0[2 * q + index] * dx * (radius - rcc[index]);
+    const double mx = s0[3 * q + index], mn = s0[4 * q + index];
+    if (y > mx) y = mx;
+    if (y < mn) y = mn;
+    return y;
 }
 
 // the value of a bin-centred array at cell (i, j, k): injected from the cell's bin (exact
@@ -108,16 +118,17 @@ __global__ void k_put1d_sph(KARGS, int f, const double* __restrict__ s0, int out
     const double radius = sqrt(x * x + y * y + z * z);
     double v;
     if (edge) {
-        const int index = g.exact ? sph_bin(g, i, j, k) : int(radius / g.drf);
+        const int index = g.exact ? sph_bin(g, i, j, k) : int(div_c(radius, g.rdrf));
         v = sph_edge_value(g, s0, rcc, redge, radius, index, g.w0i);
     } else {
         v = g.exact ? s0[sph_bin(g, i, j, k)] : sph_cell_value(g, s0, rcc, radius, g.s0i);
     }
     const FabView o = VW(f);
     if (vec) {
-        at(o, i, j, k, 0) = v * x / radius;
-        at(o, i, j, k, 1) = v * y / radius;
-        at(o, i, j, k, 2) = v * z / radius;
+        const RecipV r = recip_v(radius);
+        at(o, i, j, k, 0) = div_v(v * x, r);
+        at(o, i, j, k, 1) = div_v(v * y, r);
+        at(o, i, j, k, 2) = div_v(v * z, r);
     } else {
         at(o, i, j, k, outcomp) = v;
     }
@@ -155,8 +166,8 @@ __device__ __forceinline__ void sph_face_xyz(const SphGeo& g, int i, int j, int 
 
 // w0 interpolated linearly in uniform bins of drf (MakeW0mac types 2 and 4)
 __device__ __forceinline__ double w0_linear(const SphGeo& g, const double* __restrict__ w0, double radius) {
-    const int index = int(radius / g.drf);
-    const double rfac = (radius - double(index) * g.drf) / g.drf;
+    const int index = int(div_c(radius, g.rdrf));
+    const double rfac = div_c(radius - double(index) * g.drf, g.rdrf);
     return index < g.nr ? rfac * w0[index + 1] + (1.0 - rfac) * w0[index] : w0[g.nr];
 }
 
@@ -173,7 +184,7 @@ __global__ void k_w0mac_interp(KARGS, const double* __restrict__ w0, const doubl
     if (g.w0maci == 2) {
         v = w0_linear(g, w0, radius);
     } else {
-        int index = int(radius / g.drf);
+        int index = int(div_c(radius, g.rdrf));
         if (index <= 0) index = 0;
         else if (index >= g.nr - 1) index = g.nr - 2;
         else if (radius - redge[index] < redge[index + 1]) index--;
@@ -197,9 +208,10 @@ __global__ void k_w0_nodal(KARGS, const double* __restrict__ w0, SphGeo g) {
     if (radius == 0.0) {
         for (int n = 0; n < 3; ++n) at(o, i, j, k, n) = v;
     } else {
-        at(o, i, j, k, 0) = v * x / radius;
-        at(o, i, j, k, 1) = v * y / radius;
-        at(o, i, j, k, 2) = v * z / radius;
+        const RecipV r = recip_v(radius);
+        at(o, i, j, k, 0) = div_v(v * x, r);
+        at(o, i, j, k, 1) = div_v(v * y, r);
+        at(o, i, j, k, 2) = div_v(v * z, r);
     }
 }
 
@@ -298,15 +310,15 @@ void make_vel_force_sph(Ctx& c, int fe) {
 
 // ModifyScalForce, spherical (Source/MaestroForce.cpp:335-412); divu_cart is Put1dArrayOnCart
 // of divw0 (F_DIVW0, uniform bins), 0 with the exact base state (:283-302)
-__global__ void k_modify_scal_force_sph(KARGS, int comp, int s0cart, int fullform, double dx0, double dx1, double dx2,
+__global__ void k_modify_scal_force_sph(KARGS, int comp, int s0cart, int fullform, RecipC dx0, RecipC dx1, RecipC dx2,
                                         int lo0, int lo1, int lo2, int hi0, int hi1, int hi2, int exact) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView um = VW(F_UMAC0), vm = VW(F_UMAC1), wm = VW(F_UMAC2), s0a = VW(s0cart);
     const double divu_c = exact ? 0.0 : at(VW(F_DIVW0), i, j, k);
     const double scal = at(VW(F_SOLD), i, j, k, comp);
     double& force = at(VW(F_SCALFORCE), i, j, k, comp);
-    const double divumac = (at(um, i + 1, j, k) - at(um, i, j, k)) / dx0 + (at(vm, i, j + 1, k) - at(vm, i, j, k)) / dx1 +
-                           (at(wm, i, j, k + 1) - at(wm, i, j, k)) / dx2;
+    const double divumac = div_c(at(um, i + 1, j, k) - at(um, i, j, k), dx0) + div_c(at(vm, i, j + 1, k) - at(vm, i, j, k), dx1) +
+                           div_c(at(wm, i, j, k + 1) - at(wm, i, j, k), dx2);
     if (fullform == 1) {
         force -= scal * (divumac + divu_c);
     } else {
@@ -317,30 +329,30 @@ __global__ void k_modify_scal_force_sph(KARGS, int comp, int s0cart, int fullfor
         const double syl = j > lo1 ? half(s + at(s0a, i, j - 1, k)) : s;
         const double szh = k < hi2 ? half(s + at(s0a, i, j, k + 1)) : s;
         const double szl = k > lo2 ? half(s + at(s0a, i, j, k - 1)) : s;
-        const double divs0u = (at(um, i + 1, j, k) * sxh - at(um, i, j, k) * sxl) / dx0 +
-                              (at(vm, i, j + 1, k) * syh - at(vm, i, j, k) * syl) / dx1 +
-                              (at(wm, i, j, k + 1) * szh - at(wm, i, j, k) * szl) / dx2;
+        const double divs0u = div_c(at(um, i + 1, j, k) * sxh - at(um, i, j, k) * sxl, dx0) +
+                              div_c(at(vm, i, j + 1, k) * syh - at(vm, i, j, k) * syl, dx1) +
+                              div_c(at(wm, i, j, k + 1) * szh - at(wm, i, j, k) * szl, dx2);
         force += -divs0u - (scal - s) * (divumac + divu_c);
     }
 }
 
 void modify_scal_force_sph(Ctx& c, int comp, int s0cart_fid, int fullform) {
-    launch(c, rg_grow(c, 0), 1, k_modify_scal_force_sph, c.V(), comp, s0cart_fid, fullform, c.P.dx[0], c.P.dx[1],
-           c.P.dx[2], c.P.dom_lo[0], c.P.dom_lo[1], c.P.dom_lo[2], c.P.dom_hi[0], c.P.dom_hi[1], c.P.dom_hi[2],
+    launch(c, rg_grow(c, 0), 1, k_modify_scal_force_sph, c.V(), comp, s0cart_fid, fullform, make_recip(c.P.dx[0]),
+           make_recip(c.P.dx[1]), make_recip(c.P.dx[2]), c.P.dom_lo[0], c.P.dom_lo[1], c.P.dom_lo[2], c.P.dom_hi[0], c.P.dom_hi[1], c.P.dom_hi[2],
            c.geo.exact);
 }
 
 // MakeRhoHForce, spherical (Source/MaestroForce.cpp:637-670): u.grad p0 = div(u p0) - p0 div u,
 // p0 on faces in F_S0MAC0..2 (MakeS0mac of p0)
-__global__ void k_rhoh_force_sph(KARGS, int psi_in, int add_thermal, double dx0, double dx1, double dx2) {
+__global__ void k_rhoh_force_sph(KARGS, int psi_in, int add_thermal, RecipC dx0, RecipC dx1, RecipC dx2) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView um = VW(F_UMAC0), vm = VW(F_UMAC1), wm = VW(F_UMAC2);
     const FabView px = VW(F_S0MAC0), py = VW(F_S0MAC1), pz = VW(F_S0MAC2);
-    const double divup = (at(um, i + 1, j, k) * at(px, i + 1, j, k) - at(um, i, j, k) * at(px, i, j, k)) / dx0 +
-                         (at(vm, i, j + 1, k) * at(py, i, j + 1, k) - at(vm, i, j, k) * at(py, i, j, k)) / dx1 +
-                         (at(wm, i, j, k + 1) * at(pz, i, j, k + 1) - at(wm, i, j, k) * at(pz, i, j, k)) / dx2;
-    const double p0divu = ((at(um, i + 1, j, k) - at(um, i, j, k)) / dx0 + (at(vm, i, j + 1, k) - at(vm, i, j, k)) / dx1 +
-                           (at(wm, i, j, k + 1) - at(wm, i, j, k)) / dx2) *
+    const double divup = div_c(at(um, i + 1, j, k) * at(px, i + 1, j, k) - at(um, i, j, k) * at(px, i, j, k), dx0) +
+                         div_c(at(vm, i, j + 1, k) * at(py, i, j + 1, k) - at(vm, i, j, k) * at(py, i, j, k), dx1) +
+                         div_c(at(wm, i, j, k + 1) * at(pz, i, j, k + 1) - at(wm, i, j, k) * at(pz, i, j, k), dx2);
+    const double p0divu = (div_c(at(um, i + 1, j, k) - at(um, i, j, k), dx0) + div_c(at(vm, i, j + 1, k) - at(vm, i, j, k), dx1) +
+                           div_c(at(wm, i, j, k + 1) - at(wm, i, j, k), dx2)) *
                           at(VW(F_P0CART), i, j, k);
     double f = divup - p0divu;
     if (psi_in) f += at(VW(F_PSICART), i, j, k);
@@ -351,7 +363,8 @@ __global__ void k_rhoh_force_sph(KARGS, int psi_in, int add_thermal, double dx0,
 void make_rhoh_force_sph(Ctx& c, int is_prediction, int add_thermal) {
     const int ept = c.P.enthalpy_pred_type;
     const int psi_in = (is_prediction == 1 && ept == 2) || (is_prediction == 1 && ept == 0) || (is_prediction == 0);
-    launch(c, rg_grow(c, 0), 1, k_rhoh_force_sph, c.V(), psi_in, add_thermal, c.P.dx[0], c.P.dx[1], c.P.dx[2]);
+    launch(c, rg_grow(c, 0), 1, k_rhoh_force_sph, c.V(), psi_in, add_thermal, make_recip(c.P.dx[0]),
+           make_recip(c.P.dx[1]), make_recip(c.P.dx[2]));
 }
 
 // PutInPertForm with the spherical Put1dArrayOnCart (cell-centred s0 injected by bin, or
