@@ -1,80 +1,107 @@
 // Single-box entry points: Maestro::PPM on one box (Source/Maestro.H:1396,
 // Source/MaestroPPM.cpp:5-2262), the routine the reference calls once per box and per
-// traced component.  Scratch (interface values, van Leer slopes, tracing coefficients)
-// is owned by the context and grown on demand.
-#include <cstring>
-
+// traced component.
+//
+// One launch: the blocks are divided among the three directions, each running the sweep of
+// the level kernels (madv_march.cuh: columns marched along y and z, rows by shuffles, ppm_type
+// 2's limited cells listed) with the tracing coefficients formed where they are used.  No
+// scratch.  Twelve dependent launches with every intermediate in memory spent their time
+// between launches: 62 us for a 34^3 box against BOX_NOTE.
 #include "madv_ctx.hpp"
 #include "madv_exact.cuh"
-#include "madv_ppm.cuh"
+#include "madv_launch.cuh"
+#include "madv_march.cuh"
 
 namespace madv {
 
 struct PPMBoxArgs {
-    RegionBox r;  // lo, n; b and start unused
-    FabView s, u, T, F, DV, Ip, Im;
-    int sc, uc, lo_ext, hi_ext, domlo, domhi;
+    FabView s, u[3], ip, im;
+    RecipC rdx[3], r6;
+    MarchBC bc[3];
+    RegionBox r[3];   // x: rows with the lanes that pass values on; y, z: columns in chunks
+    long total[3];    // threads (x: positions)
+    unsigned first[3];  // first block of each direction
+    int sc, np;
     long long epsb;
     double dt;
-    RecipC rdx, r6;
 };
 
-__device__ __forceinline__ bool box_ijk(const RegionBox& r, int& i, int& j, int& k) {
-    const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (long)r.n[0] * r.n[1] * r.n[2]) return false;
-    region_ijk(r, gid, i, j, k);
-    return true;
-}
-
 template <int D>
-__global__ void k_box_dsvl(PPMBoxArgs a) {
-    int i, j, k;
-    if (!box_ijk(a.r, i, j, k)) return;
-    at(a.DV, i, j, k) = ppm_dsvl<D>(a.s, a.sc, i, j, k);
-}
-
-template <int D, int PPMT>
-__global__ void k_box_face(PPMBoxArgs a) {
-    int i, j, k;
-    if (!box_ijk(a.r, i, j, k)) return;
-    at(a.F, i, j, k) = ppm_face_value<D, PPMT>(a.s, a.sc, a.DV, i, j, k, a.lo_ext, a.hi_ext, a.domlo, a.domhi, a.r6);
-}
-
-// tracing coefficients: per face of the face velocity (umac) or per cell of component
-// uc of the cell velocity
-__global__ void k_box_trace(PPMBoxArgs a) {
-    int i, j, k;
-    if (!box_ijk(a.r, i, j, k)) return;
-    double A, B;
-    trace_coeffs(at(a.u, i, j, k, a.uc), a.dt, a.rdx, A, B);
-    at(a.T, i, j, k, 0) = A;
-    at(a.T, i, j, k, 1) = B;
-}
+__device__ __forceinline__ int stride_of(const FabView& f) { return D == 0 ? 1 : (D == 1 ? f.sj : (int)f.sk); }
 
 template <int D, int PPMT, int UMAC>
-__global__ void k_box_cell(PPMBoxArgs a) {
+__device__ __forceinline__ void box_column(const PPMBoxArgs& a, P2Column* sh) {
+    const long t = (long)(blockIdx.x - a.first[D]) * blockDim.x + threadIdx.x;
+    const bool in = t < a.total[D];
     int i, j, k;
-    if (!box_ijk(a.r, i, j, k)) return;
-    constexpr int di = D == 0, dj = D == 1, dk = D == 2;
-    double sm, sp;
-    ppm_cell_edges<D, PPMT>(a.s, a.sc, a.F, a.DV, i, j, k, a.lo_ext, a.hi_ext, a.domlo, a.domhi, a.r6, sm, sp);
-    double up, um, Ap, Bp, Am, Bm;
-    if (UMAC) {
-        up = at(a.u, i + di, j + dj, k + dk);
-        um = at(a.u, i, j, k);
-        Ap = at(a.T, i + di, j + dj, k + dk, 0);
-        Bp = at(a.T, i + di, j + dj, k + dk, 1);
-        Am = at(a.T, i, j, k, 0);
-        Bm = at(a.T, i, j, k, 1);
+    region_ijk(a.r[D], in ? t : a.total[D] - 1, i, j, k);
+    const int lo = a.r[D].lo[D], I0 = lo + ((D == 1 ? j : k) - lo) * a.r[D].len, I1 = min(I0 + a.r[D].len, lo + a.r[D].ext);
+    if (D == 1) j = I0;
+    else k = I0;
+    const FabView u = a.u[D];
+    const double* pu = &at(u, i, j, k);
+    double *ip = &at(a.ip, i, j, k, D), *im = &at(a.im, i, j, k, D);
+    const double* ps = &at(a.s, i, j, k, a.sc);
+    if (PPMT == 1) {
+        if (!in) return;
+        MarchCoef c;
+        c.u = pu, c.A = c.B = pu;
+        c.su = stride_of<D>(u), c.sT = 0;
+        c.dt = a.dt, c.rdx = a.rdx[D];
+        ppm_march<D, 1, UMAC, true>(ps, stride_of<D>(a.s), c, ip, im, stride_of<D>(a.ip), I0, I1, a.bc[D], a.epsb, a.r6);
     } else {
-        up = um = at(a.u, i, j, k, a.uc);
-        Ap = Am = at(a.T, i, j, k, 0);
-        Bp = Bm = at(a.T, i, j, k, 1);
+        const P2Cell c{ps, pu, pu, pu, ip, im, stride_of<D>(a.s), stride_of<D>(u), 0};
+        ppm2_column<D, UMAC, true>(sh[threadIdx.x >> 5], c, stride_of<D>(a.ip), I0, in ? I1 - I0 : 0, a.bc[D], a.dt,
+                                   a.rdx[D], a.epsb, a.r6);
     }
+}
+
+template <int UMAC>
+__device__ __forceinline__ void box_rows1(const PPMBoxArgs& a) {
+    const int lane = threadIdx.x & 31;
+    const long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long t = w * row_out(1) + lane - 1, tc = t < 0 ? 0 : (t >= a.total[0] ? a.total[0] - 1 : t);
+    int i, j, k;
+    region_ijk(a.r[0], tc, i, j, k);
+    const int r = i - a.r[0].lo[0];
+    const bool out = t == tc && lane >= 1 && lane <= row_out(1) && r >= 1 && r <= a.r[0].ext;
+    const double* pu = &at(a.u[0], i, j, k);
     double ip, im;
-    ppm_trace(at(a.s, i, j, k, a.sc), sm, sp, up, um, Ap, Bp, Am, Bm, a.epsb, ip, im);
-    at(a.Ip, i, j, k, D) = ip;
-    at(a.Im, i, j, k, D) = im;
+    ppm_row<1, UMAC, true>(&at(a.s, i, j, k, a.sc), pu, pu, pu, i, out, a.bc[0], a.epsb, a.r6, a.dt, a.rdx[0], ip, im);
+    if (!out) return;
+    at(a.ip, i, j, k, 0) = ip;
+    at(a.im, i, j, k, 0) = im;
+}
+
+template <int UMAC>
+__device__ __forceinline__ void box_rows2(const PPMBoxArgs& a, P2Row* sh) {
+    const long t0 = (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (a.np - 3) - 1;
+    auto at_pos = [&](int p, P2Cell& x, int& i) -> bool {
+        const long t = t0 + p, tc = t < 0 ? 0 : (t >= a.total[0] ? a.total[0] - 1 : t);
+        int j, k;
+        region_ijk(a.r[0], tc, i, j, k);
+        const double* pu = &at(a.u[0], i, j, k);
+        x = P2Cell{&at(a.s, i, j, k, a.sc), pu, pu, pu, &at(a.ip, i, j, k, 0), &at(a.im, i, j, k, 0), 1, 1, 0};
+        const int r = i - a.r[0].lo[0];
+        return t == tc && r >= 1 && r <= a.r[0].ext;
+    };
+    ppm2_rows<UMAC, true>(sh[threadIdx.x >> 5], a.np, at_pos, a.bc[0], a.dt, a.rdx[0], a.epsb, a.r6);
+}
+
+constexpr int BOX_TPB = 32 * P2_WARPS;
+
+template <int PPMT, int UMAC>
+__global__ void __launch_bounds__(BOX_TPB) k_ppm_box(PPMBoxArgs a) {
+    __shared__ union Sh {
+        P2Column c[PPMT == 2 ? P2_WARPS : 1];
+        P2Row r[PPMT == 2 ? P2_WARPS : 1];
+    } sh;
+    MADV_LET_NEXT();
+    MADV_WAIT();
+    if (blockIdx.x >= a.first[2]) box_column<2, PPMT, UMAC>(a, sh.c);
+    else if (blockIdx.x >= a.first[1]) box_column<1, PPMT, UMAC>(a, sh.c);
+    else if (PPMT == 1) box_rows1<UMAC>(a);
+    else box_rows2<UMAC>(a, sh.r);
 }
 
 static FabView view_of(const madv_fab& f) {
@@ -90,17 +117,6 @@ static FabView view_of(const madv_fab& f) {
     return v;
 }
 
-static FabView scratch_view(double* p, const int lo[3], const int hi[3]) {
-    madv_fab f{};
-    f.p = p;
-    for (int d = 0; d < 3; ++d) {
-        f.lo[d] = lo[d];
-        f.hi[d] = hi[d];
-    }
-    f.ncomp = 1;
-    return view_of(f);
-}
-
 static bool covers(const madv_fab* f, const int lo[3], const int hi[3], int ncomp) {
     if (!f || !f->p || f->ncomp < ncomp) return false;
     for (int d = 0; d < 3; ++d)
@@ -108,45 +124,11 @@ static bool covers(const madv_fab* f, const int lo[3], const int hi[3], int ncom
     return true;
 }
 
-static void launch_box(const RegionBox& r, cudaStream_t st, void (*kern)(PPMBoxArgs), PPMBoxArgs a, long& count) {
-    a.r = r;
-    const long n = (long)r.n[0] * r.n[1] * r.n[2];
-    if (n <= 0) return;
-    kern<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a);
-    ++count;
-}
-
-static RegionBox rbox(const int lo[3], const int hi[3]) {
-    RegionBox r{};
-    for (int d = 0; d < 3; ++d) {
-        r.lo[d] = lo[d];
-        r.n[d] = hi[d] - lo[d] + 1;
-    }
-    r.dv = piece_div(r.n);
-    return r;
-}
-
-// Scratch (doubles) that one PPM call on box extents n needs: per direction (reused)
-// an interface-value array (n_d + 4 faces), a van Leer slope array (n_d + 2 cells) and
-// two tracing-coefficient arrays (n_d + 1 faces), the transverse extents being n_t.
-long ppm_box_scratch_doubles(const int n[3]) {
-    long worst = 0;
-    for (int d = 0; d < 3; ++d) {
-        long t = 1;
-        for (int e = 0; e < 3; ++e)
-            if (e != d) t *= n[e];
-        const long need = t * ((n[d] + 4) + (n[d] + 2) + 2 * (n[d] + 1));
-        worst = need > worst ? need : worst;
-    }
-    return worst;
-}
-
-// Validates the arguments and runs the PPM of one box with the scratch at `scratch`
-// (at least ppm_box_scratch_doubles(n) doubles).  Returns a madv error code.
+// Validates the arguments and runs the PPM of one box.  Returns a madv error code.
 int ppm_box_run(const madv_params& P, const madv_box* bx, const madv_fab* s, int comp, const madv_fab* u,
                 const madv_fab* v, const madv_fab* w, int is_umac, const int* bc, const madv_fab* Ip,
-                const madv_fab* Im, double* scratch, cudaStream_t st, long& launches) {
-    if (!bx || !s || !u || !v || !w || !bc || !Ip || !Im || !scratch) return MADV_ERR_PARAM;
+                const madv_fab* Im, cudaStream_t st, long& launches) {
+    if (!bx || !s || !u || !v || !w || !bc || !Ip || !Im) return MADV_ERR_PARAM;
     if (P.ppm_type != 1 && P.ppm_type != 2) {
         set_error("madv_ppm: ppm_type must be 1 or 2 (ppm_type 0 uses the slopes)");
         return MADV_ERR_UNSUPPORTED;
@@ -182,73 +164,50 @@ int ppm_box_run(const madv_params& P, const madv_box* bx, const madv_fab* s, int
     PPMBoxArgs a{};
     a.s = view_of(*s);
     a.sc = comp;
-    a.Ip = view_of(*Ip);
-    a.Im = view_of(*Im);
+    a.ip = view_of(*Ip);
+    a.im = view_of(*Im);
     a.epsb = dbits_host(P.rel_eps);
     a.dt = P.dt;
     a.r6 = make_recip(6.0);
+    const long cells = (long)n[0] * n[1] * n[2];
+    // chunks of a column short enough for 2^14 threads a direction; a box this small is bound by
+    // latency, and the two slopes and the interface value a chunk repeats cost nothing
+    const int len = (int)std::min((long)P2_CHUNK, std::max(2L, cells >> 14));
+    unsigned blocks = 0;
     for (int d = 0; d < 3; ++d) {
-        const int lo_ext = (bc[d] == BC_EXT_DIR || bc[d] == BC_HOEXTRAP);
-        const int hi_ext = (bc[3 + d] == BC_EXT_DIR || bc[3 + d] == BC_HOEXTRAP);
-        a.lo_ext = lo_ext;
-        a.hi_ext = hi_ext;
-        a.domlo = P.dom_lo[d];
-        a.domhi = P.dom_hi[d];
-        a.rdx = make_recip(P.dx[d]);
-        a.u = view_of(*vel[d]);
-        a.uc = 0;
-        long t = 1;
-        for (int e = 0; e < 3; ++e)
-            if (e != d) t *= n[e];
-        double* pF = scratch;
-        double* pDV = pF + t * (n[d] + 4);
-        double* pT = pDV + t * (n[d] + 2);
-        // van Leer slopes: cells lo-1 .. hi+1 along d
-        int lo[3] = {bx->lo[0], bx->lo[1], bx->lo[2]}, hi[3] = {bx->hi[0], bx->hi[1], bx->hi[2]};
-        lo[d] -= 1;
-        hi[d] += 1;
-        a.DV = scratch_view(pDV, lo, hi);
-        // interface values: faces lo .. hi+1 (ppm_type 1) or lo-1 .. hi+2 (ppm_type 2)
-        int flo[3] = {bx->lo[0], bx->lo[1], bx->lo[2]}, fhi[3] = {bx->hi[0], bx->hi[1], bx->hi[2]};
-        flo[d] -= 2;
-        fhi[d] += 2;
-        a.F = scratch_view(pF, flo, fhi);
-        // tracing coefficients: faces lo .. hi+1 (umac) or cells lo .. hi; 2 comps
-        int tlo[3] = {bx->lo[0], bx->lo[1], bx->lo[2]}, thi[3] = {bx->hi[0], bx->hi[1], bx->hi[2]};
-        if (is_umac) thi[d] += 1;
-        {
-            madv_fab tf{};
-            tf.p = pT;
-            for (int e = 0; e < 3; ++e) {
-                tf.lo[e] = tlo[e];
-                tf.hi[e] = thi[e];
-            }
-            tf.ncomp = 2;
-            a.T = view_of(tf);
+        a.bc[d] = MarchBC{bc[d] == BC_EXT_DIR || bc[d] == BC_HOEXTRAP, bc[3 + d] == BC_EXT_DIR || bc[3 + d] == BC_HOEXTRAP,
+                          P.dom_lo[d], P.dom_hi[d]};
+        a.rdx[d] = make_recip(P.dx[d]);
+        a.u[d] = view_of(*vel[d]);
+        RegionBox& r = a.r[d];
+        for (int e = 0; e < 3; ++e) {
+            r.lo[e] = bx->lo[e];
+            r.n[e] = n[e];
         }
-        launch_box(rbox(tlo, thi), st, k_box_trace, a, launches);
-        int clo[3] = {bx->lo[0], bx->lo[1], bx->lo[2]}, chi[3] = {bx->hi[0], bx->hi[1], bx->hi[2]};
-        if (P.ppm_type == 1) {
-            launch_box(rbox(lo, hi), st, d == 0 ? k_box_dsvl<0> : (d == 1 ? k_box_dsvl<1> : k_box_dsvl<2>), a,
-                       launches);
-            int f1lo[3] = {bx->lo[0], bx->lo[1], bx->lo[2]}, f1hi[3] = {bx->hi[0], bx->hi[1], bx->hi[2]};
-            f1hi[d] += 1;
-            launch_box(rbox(f1lo, f1hi), st,
-                       d == 0 ? k_box_face<0, 1> : (d == 1 ? k_box_face<1, 1> : k_box_face<2, 1>), a, launches);
-            void (*kc)(PPMBoxArgs) = is_umac ? (d == 0 ? k_box_cell<0, 1, 1> : (d == 1 ? k_box_cell<1, 1, 1> : k_box_cell<2, 1, 1>))
-                                             : (d == 0 ? k_box_cell<0, 1, 0> : (d == 1 ? k_box_cell<1, 1, 0> : k_box_cell<2, 1, 0>));
-            launch_box(rbox(clo, chi), st, kc, a, launches);
+        r.ext = n[d];
+        if (d == 0) {
+            r.lo[0] -= 1;
+            r.n[0] += 32 - row_out(P.ppm_type);
         } else {
-            int f2lo[3] = {bx->lo[0], bx->lo[1], bx->lo[2]}, f2hi[3] = {bx->hi[0], bx->hi[1], bx->hi[2]};
-            f2lo[d] -= 1;
-            f2hi[d] += 2;
-            launch_box(rbox(f2lo, f2hi), st,
-                       d == 0 ? k_box_face<0, 2> : (d == 1 ? k_box_face<1, 2> : k_box_face<2, 2>), a, launches);
-            void (*kc)(PPMBoxArgs) = is_umac ? (d == 0 ? k_box_cell<0, 2, 1> : (d == 1 ? k_box_cell<1, 2, 1> : k_box_cell<2, 2, 1>))
-                                             : (d == 0 ? k_box_cell<0, 2, 0> : (d == 1 ? k_box_cell<1, 2, 0> : k_box_cell<2, 2, 0>));
-            launch_box(rbox(clo, chi), st, kc, a, launches);
+            const int nch = (n[d] + len - 1) / len;
+            r.len = (n[d] + nch - 1) / nch;
+            r.n[d] = (n[d] + r.len - 1) / r.len;
         }
+        r.dv = piece_div(r.n);
+        a.total[d] = (long)r.n[0] * r.n[1] * r.n[2];
+        a.first[d] = blocks;
+        long threads = a.total[d];
+        if (d == 0) {
+            a.np = (int)std::min((long)P2_ROW, std::max(32L, a.total[0] / (152 * 8) / 32 * 32));
+            const int out = P.ppm_type == 1 ? row_out(1) : a.np - 3;
+            threads = (a.total[0] + out - 1) / out * 32;
+        }
+        blocks += (unsigned)((threads + BOX_TPB - 1) / BOX_TPB);
     }
+    void (*kern)(PPMBoxArgs) = P.ppm_type == 1 ? (is_umac ? k_ppm_box<1, 1> : k_ppm_box<1, 0>)
+                                               : (is_umac ? k_ppm_box<2, 1> : k_ppm_box<2, 0>);
+    launch_on(st, false, dim3(blocks), BOX_TPB, kern, a);
+    ++launches;
     return cuda_ok(cudaGetLastError(), "madv_ppm launch") ? MADV_OK : MADV_ERR_CUDA;
 }
 

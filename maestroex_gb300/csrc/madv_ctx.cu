@@ -1275,8 +1275,6 @@ static void destroy_level(Ctx& c) {
     if (c.ev_join) cudaEventDestroy(c.ev_join);
     c.side = nullptr;
     c.ev_fork = c.ev_join = nullptr;
-    if (c.box_scratch) cudaFree(c.box_scratch);
-    c.box_scratch = nullptr;
     if (c.d_bcs) cudaFree(c.d_bcs);
     c.d_bcs = nullptr;
     if (c.d_flag) cudaFree(c.d_flag);
@@ -2523,18 +2521,8 @@ int madv_ppm(madv_ctx* h, const madv_box* bx, const madv_fab* s, int comp, const
         n[d] = bx->hi[d] - bx->lo[d] + 1;
         if (n[d] <= 0) return MADV_ERR_LAYOUT;
     }
-    const long need = ppm_box_scratch_doubles(n);
-    if (need > c.box_scratch_n) {
-        if (c.box_scratch) cudaFree(c.box_scratch);
-        c.box_scratch = nullptr;
-        c.box_scratch_n = 0;
-        if (!cuda_ok(cudaMalloc(&c.box_scratch, sizeof(double) * need), "cudaMalloc(madv_ppm scratch)"))
-            return MADV_ERR_CUDA;
-        c.box_scratch_n = need;
-    }
     c.launches = 0;
-    return ppm_box_run(c.P, bx, s, comp, u, v, w, is_umac, bc, Ip, Im, c.box_scratch, (cudaStream_t)stream,
-                       c.launches);
+    return ppm_box_run(c.P, bx, s, comp, u, v, w, is_umac, bc, Ip, Im, (cudaStream_t)stream, c.launches);
 }
 
 // ------------------------------------------------------------------ launch-shape autotuner

@@ -233,9 +233,6 @@ struct Ctx {
     FabView* dviews_side = nullptr;
     FabView* hviews_side = nullptr;
     const FabView* side_mirror = nullptr;
-    // scratch of the single-box entry points (madv_ppm), grown on demand
-    double* box_scratch = nullptr;
-    long box_scratch_n = 0;
 
     // coarse-fine data (hierarchies of more than one level)
     std::vector<int> h_owner;  // box owning each cell of the level's domain, -1 = none
@@ -316,10 +313,9 @@ void make_rhoh_flux(Ctx& c, const double* rh0_old, const double* rh0e_old, const
 void convert_rhoh_to_h(Ctx& c, int flag);  // valid region
 void h_force(Ctx& c);                      // scal_force(RhoH) /= sold(Rho), valid + 1 ghost
 void sum_species_edges(Ctx& c);
-long ppm_box_scratch_doubles(const int n[3]);
 int ppm_box_run(const madv_params& P, const madv_box* bx, const madv_fab* s, int comp, const madv_fab* u,
                 const madv_fab* v, const madv_fab* w, int is_umac, const int* bc, const madv_fab* Ip,
-                const madv_fab* Im, double* scratch, cudaStream_t st, long& launches);
+                const madv_fab* Im, cudaStream_t st, long& launches);
 void update_scal(Ctx& c, int start_comp);
 // UpdateScal of the species split for streaming: one species from its flux in F_SFLUX* comp
 // `slot`, then the density, floor and negative-species pass over all of them

@@ -16,17 +16,21 @@ static constexpr int TPB = 256;
 // elements the early start costs (4.7 against 3.5 us a kernel), so captured launches are
 // plain.
 template <typename... P, typename... Args>
-static inline void launch_next(const Ctx& c, dim3 grid, int tpb, void (*kern)(P...), Args... args) {
+static inline void launch_on(cudaStream_t st, bool plain, dim3 grid, int tpb, void (*kern)(P...), Args... args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)tpb);
-    cfg.stream = c.stream;
+    cfg.stream = st;
     cfg.attrs = &at;
-    cfg.numAttrs = c.capturing ? 0 : 1;
+    cfg.numAttrs = plain ? 0 : 1;
     cudaLaunchKernelEx(&cfg, kern, (P)args...);
+}
+template <typename... P, typename... Args>
+static inline void launch_next(const Ctx& c, dim3 grid, int tpb, void (*kern)(P...), Args... args) {
+    launch_on(c.stream, c.capturing, grid, tpb, kern, args...);
 }
 
 // One launch over every box (batched), or one launch per region piece (per-box mode, the
