@@ -414,10 +414,11 @@ int madv_autotune_apply(madv_ctx* ctx, const char* json);
  *                     the per-component scratch (allocated at first use: about 46 doubles per
  *                     cell); 0 (default): one stream -- the stage is FP64-issue bound and
  *                     the overlap measures 0.5% on GB300.
- *   "es_inline"       1 (default): with ppm_type 1 / 2, MakeEdgeScal's transverse and edge
- *                     kernels take the predictor's left / right states straight from the
- *                     traced Ip / Im, and only the upwind state is stored per face; 0: the
- *                     predictor stores all three (as the reference's slx / srx / simhx).
+ *   "es_inline"       1 (default): in 3-D, MakeEdgeScal forms only the side of each face that
+ *                     the wind comes from, transverse states included, in per-direction
+ *                     kernels that store three fields a component; 0: the predictor,
+ *                     transverse and edge states of both sides in kernels of their own, which
+ *                     store all of them (as the reference's slx / srx / simhx).
  *   "mg_block_cycle"  1 (default): the MAC projection's multigrid V-cycle, from its first
  *                     grid of at most 4096 cells down to the coarsest, runs in one thread
  *                     block with the same per-cell arithmetic (bitwise the same result);

@@ -6,7 +6,7 @@
 // the level kernels (madv_march.cuh: columns marched along y and z, rows by shuffles, ppm_type
 // 2's limited cells listed) with the tracing coefficients formed where they are used.  No
 // scratch.  Twelve dependent launches with every intermediate in memory spent their time
-// between launches: 62 us for a 34^3 box against BOX_NOTE.
+// between launches: 63 us a call for a 34^3 box, 27 us now with the caller's side of it.
 #include "madv_ctx.hpp"
 #include "madv_exact.cuh"
 #include "madv_launch.cuh"
@@ -48,7 +48,7 @@ __device__ __forceinline__ void box_column(const PPMBoxArgs& a, P2Column* sh) {
         c.u = pu, c.A = c.B = pu;
         c.su = stride_of<D>(u), c.sT = 0;
         c.dt = a.dt, c.rdx = a.rdx[D];
-        ppm_march<D, 1, UMAC, true>(ps, stride_of<D>(a.s), c, ip, im, stride_of<D>(a.ip), I0, I1, a.bc[D], a.epsb, a.r6);
+        ppm_march<D, UMAC, true>(ps, stride_of<D>(a.s), c, ip, im, stride_of<D>(a.ip), I0, I1, a.bc[D], a.epsb, a.r6);
     } else {
         const P2Cell c{ps, pu, pu, pu, ip, im, stride_of<D>(a.s), stride_of<D>(u), 0};
         ppm2_column<D, UMAC, true>(sh[threadIdx.x >> 5], c, stride_of<D>(a.ip), I0, in ? I1 - I0 : 0, a.bc[D], a.dt,
@@ -67,7 +67,7 @@ __device__ __forceinline__ void box_rows1(const PPMBoxArgs& a) {
     const bool out = t == tc && lane >= 1 && lane <= row_out(1) && r >= 1 && r <= a.r[0].ext;
     const double* pu = &at(a.u[0], i, j, k);
     double ip, im;
-    ppm_row<1, UMAC, true>(&at(a.s, i, j, k, a.sc), pu, pu, pu, i, out, a.bc[0], a.epsb, a.r6, a.dt, a.rdx[0], ip, im);
+    ppm_row<UMAC, true>(&at(a.s, i, j, k, a.sc), pu, pu, pu, i, out, a.bc[0], a.epsb, a.r6, a.dt, a.rdx[0], ip, im);
     if (!out) return;
     at(a.ip, i, j, k, 0) = ip;
     at(a.im, i, j, k, 0) = im;

@@ -221,8 +221,8 @@ struct Ctx {
     // side_mirror with those fields moved); built per stage call, used while dviews ==
     // side_mirror
     bool comp_streams = false;
-    // option "es_inline": MakeEdgeScal's edge kernels form the predictor's l / r from Ip / Im
-    // and only the upwind state is stored (ppm_type 1 / 2, outside the adjoint's tape)
+    // option "es_inline": MakeEdgeScal forms only each face's upwind side (madv_march.cu;
+    // outside the adjoint's tape, which keeps the separate kernels' fields)
     bool es_inline = true;
     // option "mg_block_cycle": the MAC multigrid's V-cycle from the first grid of at most 4096
     // cells down runs in one thread block (one launch per cycle instead of ~170)
@@ -268,7 +268,8 @@ void sweep_free(Ctx& c);
 
 // ---- PPM marched along each direction, edge states from the upwind cell (madv_march.cu) ----
 void ppm_march_comps(Ctx& c, int dirs, int fs, int sc0, int nq, const BCRecD* bc, int fu, int umac, int fip, int fim);
-void edge_scal_ctu(Ctx& c, int comp0, int nq, const BCRecD* bc, int oc0, int force_zero, int is_vel);
+void slope_states(Ctx& c, int sc0, int nq, const BCRecD* bc);
+void edge_scal_ctu(Ctx& c, int comp0, int nq, const BCRecD* bc, int oc0, int force_zero, int is_vel, int is_cons);
 
 // ---- kernel launch wrappers (madv_kernels.cu) ----
 void fill_boundary(Ctx& c, int fid, int c0, int nc);

@@ -19,6 +19,7 @@
 #include "madv_exact.cuh"
 #include "madv_launch.cuh"
 #include "madv_ppm.cuh"
+#include "madv_slope.cuh"
 
 namespace madv {
 
@@ -315,7 +316,7 @@ __global__ void k_ppm_cell(KARGS, int fs, int sc, int ff, int fu, int uc, int fi
 // Limited slopes for ppm_type 0 (Maestro::Slopex/y/z, Source/MaestroSlopes.cpp:6-600).
 template <int D>
 __global__ void k_slope(KARGS, int fs, int sc, int fout, int oc, int ncomp, const BCRecD* __restrict__ bcs, int bc_c0,
-                        int slope_order, int ilo, int ihi) {
+                        int slope_order, int ilo, int ihi, RecipC r6) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     constexpr int di = D == 0, dj = D == 1, dk = D == 2;
     const FabView s = VW(fs);
@@ -323,116 +324,7 @@ __global__ void k_slope(KARGS, int fs, int sc, int fout, int oc, int ncomp, cons
     const int I = D == 0 ? i : (D == 1 ? j : k);
     for (int n = 0; n < ncomp; ++n) {
         auto S = SHIFT_S(s, sc + n);
-        const int bclo = bcs[bc_c0 + n].lo[D], bchi = bcs[bc_c0 + n].hi[D];
-        const bool lo_ext = (bclo == BC_EXT_DIR || bclo == BC_HOEXTRAP);
-        const bool hi_ext = (bchi == BC_EXT_DIR || bchi == BC_HOEXTRAP);
-        double out = 0.0;
-        if (slope_order == 2) {
-            double del = half(S(1) - S(-1));
-            double dpls = 2.0 * (S(1) - S(0));
-            double dmin = 2.0 * (S(0) - S(-1));
-            double slim = mn(fabs(dpls), fabs(dmin));
-            slim = dpls * dmin > 0.0 ? slim : 0.0;
-            double sflag = copysign(1.0, del);
-            out = sflag * mn(slim, fabs(del));
-            if (lo_ext) {
-                if (I == ilo - 1) {
-                    out = 0.0;
-                } else if (I == ilo) {
-                    del = (S(1) + 3.0 * S(0) - 4.0 * S(-1)) / 3.0;
-                    dpls = 2.0 * (S(1) - S(0));
-                    dmin = 2.0 * (S(0) - S(-1));
-                    slim = mn(fabs(dpls), fabs(dmin));
-                    slim = dpls * dmin > 0.0 ? slim : 0.0;
-                    sflag = copysign(1.0, del);
-                    out = sflag * mn(slim, fabs(del));
-                }
-            }
-            if (hi_ext) {
-                if (I == ihi + 1) {
-                    out = 0.0;
-                } else if (I == ihi) {
-                    del = -(S(-1) + 3.0 * S(0) - 4.0 * S(1)) / 3.0;
-                    dpls = 2.0 * (S(0) - S(-1));
-                    dmin = 2.0 * (S(1) - S(0));
-                    slim = mn(fabs(dpls), fabs(dmin));
-                    slim = dpls * dmin > 0.0 ? slim : 0.0;
-                    sflag = copysign(1.0, del);
-                    out = sflag * mn(slim, fabs(del));
-                }
-            }
-        } else if (slope_order == 4) {
-            double dcen = half(S(0) - S(-2));
-            double dmin = 2.0 * (S(-1) - S(-2));
-            double dpls = 2.0 * (S(0) - S(-1));
-            double dlim = mn(fabs(dmin), fabs(dpls));
-            dlim = dpls * dmin > 0.0 ? dlim : 0.0;
-            double dflag = copysign(1.0, dcen);
-            double dxl = dflag * mn(dlim, fabs(dcen));
-            dcen = half(S(2) - S(0));
-            dmin = 2.0 * (S(1) - S(0));
-            dpls = 2.0 * (S(2) - S(1));
-            dlim = mn(fabs(dmin), fabs(dpls));
-            dlim = dpls * dmin > 0.0 ? dlim : 0.0;
-            dflag = copysign(1.0, dcen);
-            double dxr = dflag * mn(dlim, fabs(dcen));
-            dcen = half(S(1) - S(-1));
-            dmin = 2.0 * (S(0) - S(-1));
-            dpls = 2.0 * (S(1) - S(0));
-            dlim = mn(fabs(dmin), fabs(dpls));
-            dlim = dpls * dmin > 0.0 ? dlim : 0.0;
-            dflag = copysign(1.0, dcen);
-            double ds = 4.0 / 3.0 * dcen - (dxr + dxl) / 6.0;
-            out = dflag * mn(fabs(ds), dlim);
-            // the x sweep tests the centred dlim where y and z test the one-sided slim
-            if (lo_ext) {
-                if (I == ilo - 1) {
-                    out = 0.0;
-                } else if (I == ilo) {
-                    double del = -16.0 / 15.0 * S(-1) + 0.5 * S(0) + 2.0 / 3.0 * S(1) - 0.1 * S(2);
-                    dmin = 2.0 * (S(0) - S(-1));
-                    dpls = 2.0 * (S(1) - S(0));
-                    double slim = mn(fabs(dpls), fabs(dmin));
-                    slim = dpls * dmin > 0.0 ? (D == 0 ? dlim : slim) : 0.0;
-                    double sflag = copysign(1.0, del);
-                    out = sflag * mn(slim, fabs(del));
-                } else if (I == ilo + 1) {
-                    double del = -16.0 / 15.0 * S(-2) + 0.5 * S(-1) + 2.0 / 3.0 * S(0) - 0.1 * S(1);
-                    dmin = 2.0 * (S(-1) - S(-2));
-                    dpls = 2.0 * (S(0) - S(-1));
-                    double slim = mn(fabs(dpls), fabs(dmin));
-                    slim = dpls * dmin > 0.0 ? (D == 0 ? dlim : slim) : 0.0;
-                    double sflag = copysign(1.0, del);
-                    dxl = sflag * mn(slim, fabs(del));
-                    ds = 4.0 / 3.0 * dcen - (dxr + dxl) / 6.0;
-                    out = dflag * mn(fabs(ds), dlim);
-                }
-            }
-            if (hi_ext) {
-                if (I == ihi + 1) {
-                    out = 0.0;
-                } else if (I == ihi) {
-                    double del = -(-16.0 / 15.0 * S(1) + 0.5 * S(0) + 2.0 / 3.0 * S(-1) - 0.1 * S(-2));
-                    dmin = 2.0 * (S(0) - S(-1));
-                    dpls = 2.0 * (S(1) - S(0));
-                    double slim = mn(fabs(dpls), fabs(dmin));
-                    slim = dpls * dmin > 0.0 ? (D == 0 ? dlim : slim) : 0.0;
-                    double sflag = copysign(1.0, del);
-                    out = sflag * mn(slim, fabs(del));
-                } else if (I == ihi - 1) {
-                    double del = -(-16.0 / 15.0 * S(2) + 0.5 * S(1) + 2.0 / 3.0 * S(0) - 0.1 * S(-1));
-                    dmin = 2.0 * (S(1) - S(0));
-                    dpls = 2.0 * (S(2) - S(1));
-                    double slim = mn(fabs(dpls), fabs(dmin));
-                    slim = dpls * dmin > 0.0 ? (D == 0 ? dlim : slim) : 0.0;
-                    double sflag = copysign(1.0, del);
-                    dxr = sflag * mn(slim, fabs(del));
-                    ds = 4.0 / 3.0 * dcen - (dxl + dxr) / 6.0;
-                    out = dflag * mn(fabs(ds), dlim);
-                }
-            }
-        }
-        at(o, i, j, k, oc + n) = out;
+        at(o, i, j, k, oc + n) = limited_slope<D>(S, I, bcs[bc_c0 + n].lo[D], bcs[bc_c0 + n].hi[D], slope_order, ilo, ihi, r6);
     }
 }
 
@@ -515,9 +407,12 @@ static void trace_coeffs_faces(Ctx& c, int fu0) {
 static void slope_any(Ctx& c, int d, int fs, int sc, int fout, int oc, int ncomp, const BCRecD* bcs_d, int bc_c0) {
     const RegionTable& rc = rg_grow(c, 1);
     const int lo = c.P.dom_lo[d], hi = c.P.dom_hi[d], so = c.P.slope_order;
-    if (d == 0) launch(c, rc, 1, k_slope<0>, c.V(), fs, sc, fout, oc, ncomp, bcs_d, bc_c0, so, lo, hi);
-    else if (d == 1) launch(c, rc, 1, k_slope<1>, c.V(), fs, sc, fout, oc, ncomp, bcs_d, bc_c0, so, lo, hi);
-    else launch(c, rc, 1, k_slope<2>, c.V(), fs, sc, fout, oc, ncomp, bcs_d, bc_c0, so, lo, hi);
+    if (d == 0) launch(c, rc, 1, k_slope<0>, c.V(), fs, sc, fout, oc, ncomp, bcs_d, bc_c0, so, lo, hi,
+                       make_recip(6.0));
+    else if (d == 1) launch(c, rc, 1, k_slope<1>, c.V(), fs, sc, fout, oc, ncomp, bcs_d, bc_c0, so, lo, hi,
+                       make_recip(6.0));
+    else launch(c, rc, 1, k_slope<2>, c.V(), fs, sc, fout, oc, ncomp, bcs_d, bc_c0, so, lo, hi,
+                       make_recip(6.0));
 }
 
 // Transverse-correction coefficients of a face velocity field (u0..u2 = three D-face
@@ -929,25 +824,6 @@ __device__ __forceinline__ void es_pred_bc(int I, int bclo, int bchi, int domlo,
     }
 }
 
-// The predictor's states of the D-face (i,j,k) with ppm_type 1 / 2 as its consumers use them:
-// Ip of the cell below, Im of the cell above (F_IPC0 / F_IMC0 component D).  On a domain face
-// the consumers' own boundary rules (k_es_transverse, k_es_edges) overwrite both states for
-// ext_dir and reflect_odd, and the outside one (l below, r above) for foextrap, hoextrap and
-// reflect_even, so of the predictor's rules only the velocity clamp of the inside state is
-// left to apply here.  k_es_simh stores the upwind state with every rule.
-template <int D>
-__device__ __forceinline__ void es_pred_lr(const FabView& ip, const FabView& im, int bclo, int bchi, int domlo,
-                                           int domhi, int vclamp, int i, int j, int k, double& l, double& r) {
-    constexpr int di = D == 0, dj = D == 1, dk = D == 2;
-    const int I = D == 0 ? i : (D == 1 ? j : k);
-    l = at(ip, i - di, j - dj, k - dk, D);
-    r = at(im, i, j, k, D);
-    if (vclamp) {
-        if (I == domlo && (bclo == BC_FOEXTRAP || bclo == BC_HOEXTRAP)) r = mn(r, 0.0);
-        else if (I == domhi + 1 && (bchi == BC_FOEXTRAP || bchi == BC_HOEXTRAP)) l = mx(l, 0.0);
-    }
-}
-
 // MakeEdgeScalPredictor, 3-D (Source/MaestroMakeEdgeScalars.cpp:662-863)
 template <int D>
 __global__ void k_es_predictor(KARGS, int comp, int ppm_type, double dt, double hd, int bclo, int bchi, int domlo,
@@ -974,34 +850,11 @@ __global__ void k_es_predictor(KARGS, int comp, int ppm_type, double dt, double 
     at(VW(F_SIMH0 + D), i, j, k) = upwind(ud, l, r, 0);  // tie test |u| > 0
 }
 
-// The predictor's upwind state alone (ppm_type 1 / 2): the transverse kernels read it at
-// neighbouring faces, while the edge states' l and r are formed where they are used.
-template <int D>
-__global__ void k_es_simh(KARGS, int comp, int bclo, int bchi, int domlo, int domhi, int vclamp) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    constexpr int di = D == 0, dj = D == 1, dk = D == 2;
-    const int I = D == 0 ? i : (D == 1 ? j : k);
-    const double u = at(VW(F_UMAC0 + D), i, j, k);
-    const bool bnd = I == domlo || I == domhi + 1;
-    double v;
-    if (!bnd && nz(u)) {  // the one state that is taken
-        v = dhigh(u) >= 0 ? at(VW(F_IPC0), i - di, j - dj, k - dk, D) : at(VW(F_IMC0), i, j, k, D);
-    } else {
-        double l = at(VW(F_IPC0), i - di, j - dj, k - dk, D), r = at(VW(F_IMC0), i, j, k, D);
-        if (bnd) {
-            const FabView sc = VW(F_SOLD);
-            es_pred_bc(I, bclo, bchi, domlo, domhi, vclamp, at(sc, i - di, j - dj, k - dk, comp), at(sc, i, j, k, comp), l, r);
-        }
-        v = upwind(u, l, r, 0);  // tie test |u| > 0
-    }
-    at(VW(F_SIMH0 + D), i, j, k) = v;
-}
-
 // MakeEdgeScalTransverse, 3-D (Source/MaestroMakeEdgeScalars.cpp:865-1359): D-faces
 // corrected in direction T.  Advective form: F_TCOEF comp T = (dt6/h_T)*(u_T sum).
-// INL (ppm_type 1 / 2): the D-face's predictor states l and r are formed here from F_IPC0 /
-// F_IMC0 instead of read from F_SL0 / F_SR0 (the same values: Ip, Im and the boundary rules).
-template <int D, int T, bool CONS, bool INL>
+// The separate predictor, transverse and edge kernels serve the adjoint's taped forward, which
+// keeps their fields, and es_inline = 0; otherwise madv_march.cu forms the edge states.
+template <int D, int T, bool CONS>
 __global__ void __launch_bounds__(TPB, CONS ? 4 : 6) k_es_transverse(KARGS, int comp, double dt3, double dt3h, int bclo, int bchi, int domlo, int domhi,
                                 long long epsb, int vclamp) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
@@ -1017,9 +870,7 @@ __global__ void __launch_bounds__(TPB, CONS ? 4 : 6) k_es_transverse(KARGS, int 
         // half of the FP64 work, are needed on domain faces and where |u| <= rel_eps alone)
         const bool left = dhigh(ud) >= 0;
         const int ci = left ? il : i, cj = left ? jl : j, ck = left ? kl : k;
-        double q;
-        if (INL) q = left ? at(VW(F_IPC0), ci, cj, ck, D) : at(VW(F_IMC0), ci, cj, ck, D);
-        else q = left ? at(VW(F_SL0 + D), i, j, k) : at(VW(F_SR0 + D), i, j, k);
+        double q = left ? at(VW(F_SL0 + D), i, j, k) : at(VW(F_SR0 + D), i, j, k);
         if (CONS) {
             const double s0 = at(sc, ci, cj, ck, comp), up = at(ut, ci + ti, cj + tj, ck + tk), um = at(ut, ci, cj, ck);
             q = q - dt3h * (simh(ci + ti, cj + tj, ck + tk) * up - simh(ci, cj, ck) * um) -
@@ -1030,13 +881,7 @@ __global__ void __launch_bounds__(TPB, CONS ? 4 : 6) k_es_transverse(KARGS, int 
         at(VW(Q_FIELD(D, T)), i, j, k) = q;
         return;
     }
-    double sl, sr;
-    if (INL) {
-        es_pred_lr<D>(VW(F_IPC0), VW(F_IMC0), bclo, bchi, domlo, domhi, vclamp, i, j, k, sl, sr);
-    } else {
-        sl = at(VW(F_SL0 + D), i, j, k);
-        sr = at(VW(F_SR0 + D), i, j, k);
-    }
+    const double sl = at(VW(F_SL0 + D), i, j, k), sr = at(VW(F_SR0 + D), i, j, k);
     double lq, rq;
     if (CONS) {
         const FabView dv = VW(F_DIVU);
@@ -1082,8 +927,7 @@ __global__ void __launch_bounds__(TPB, CONS ? 4 : 6) k_es_transverse(KARGS, int 
 // MakeEdgeScalEdges, 3-D (Source/MaestroMakeEdgeScalars.cpp:1361-1667).  Advective form:
 // F_TCOEF comp 3+t = (dt4/h_t)*(u_t sum).  force_zero: the component's force is
 // identically zero (species), so the + dt/2*force term is skipped.
-// INL: the D-face's predictor states formed from F_IPC0 / F_IMC0 (as in k_es_transverse).
-template <int D, bool CONS, bool INL>
+template <int D, bool CONS>
 __global__ void k_es_edges(KARGS, int comp, int force_zero, double dt2, double dt2h1, double dt2h2, double dt2hd,
                            int bclo, int bchi, int domlo, int domhi, long long epsb, int vclamp, int ptf, int oc) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
@@ -1100,9 +944,7 @@ __global__ void k_es_edges(KARGS, int comp, int force_zero, double dt2, double d
     if (I != domlo && I != domhi + 1 && dmag(ud) > epsb) {  // the upwind side alone (see k_es_transverse)
         const bool left = dhigh(ud) >= 0;
         const int ci = left ? il : i, cj = left ? jl : j, ck = left ? kl : k;
-        double v;
-        if (INL) v = left ? at(VW(F_IPC0), ci, cj, ck, D) : at(VW(F_IMC0), ci, cj, ck, D);
-        else v = left ? at(VW(F_SL0 + D), i, j, k) : at(VW(F_SR0 + D), i, j, k);
+        double v = left ? at(VW(F_SL0 + D), i, j, k) : at(VW(F_SR0 + D), i, j, k);
         const double q1p = at(q1, ci + a1i, cj + a1j, ck + a1k), q1m = at(q1, ci, cj, ck);
         const double q2p = at(q2, ci + a2i, cj + a2j, ck + a2k), q2m = at(q2, ci, cj, ck);
         double f = 0.0;
@@ -1123,13 +965,7 @@ __global__ void k_es_edges(KARGS, int comp, int force_zero, double dt2, double d
         at(VW(F_SEDGE0 + D), i, j, k, oc) = v;
         return;
     }
-    double sl, sr;
-    if (INL) {
-        es_pred_lr<D>(VW(F_IPC0), VW(F_IMC0), bclo, bchi, domlo, domhi, vclamp, i, j, k, sl, sr);
-    } else {
-        sl = at(VW(F_SL0 + D), i, j, k);
-        sr = at(VW(F_SR0 + D), i, j, k);
-    }
+    const double sl = at(VW(F_SL0 + D), i, j, k), sr = at(VW(F_SR0 + D), i, j, k);
     double lq, rq;
     if (CONS) {
         // the traced force if ppm_trace_forces = 1 (Source/MaestroMakeEdgeScalars.cpp:1405-1408)
@@ -1185,59 +1021,28 @@ static void es_predictor_launch(Ctx& c, int comp, const BCRecD& bc, int vclamp) 
            c.P.dom_lo[D], c.P.dom_hi[D], vclamp);
 }
 
-template <int D>
-static void es_simh_launch(Ctx& c, int comp, const BCRecD& bc, int vclamp) {
-    int glo[3] = {1, 1, 1};
-    glo[D] = 0;
-    const RegionTable& rt = region(c, glo[0], glo[1], glo[2], 1, 1, 1, -1);
-    launch(c, rt, 1, k_es_simh<D>, c.V(), comp, bc.lo[D], bc.hi[D], c.P.dom_lo[D], c.P.dom_hi[D], vclamp);
-}
-
-template <int D, int T, bool INL>
-static void es_transverse_launch_t(Ctx& c, const RegionTable& rt, int comp, const BCRecD& bc, int is_cons,
-                                   int vclamp) {
-    const double dt3 = c.P.dt / 3.0;
-    if (is_cons)
-        launch(c, rt, 1, k_es_transverse<D, T, true, INL>, c.V(), comp, dt3, dt3 / c.P.dx[T], bc.lo[D], bc.hi[D],
-               c.P.dom_lo[D], c.P.dom_hi[D], dbits_host(c.P.rel_eps), vclamp);
-    else
-        launch(c, rt, 1, k_es_transverse<D, T, false, INL>, c.V(), comp, dt3, dt3 / c.P.dx[T], bc.lo[D], bc.hi[D],
-               c.P.dom_lo[D], c.P.dom_hi[D], dbits_host(c.P.rel_eps), vclamp);
-}
-
-// inl: the D-face's predictor states formed in the kernel
 template <int D, int T>
-static void es_transverse_launch(Ctx& c, int comp, const BCRecD& bc, int is_cons, int vclamp, bool inl) {
+static void es_transverse_launch(Ctx& c, int comp, const BCRecD& bc, int is_cons, int vclamp) {
     constexpr int O = 3 - D - T;
     int glo[3] = {0, 0, 0}, ghi[3] = {0, 0, 0};
     glo[O] = 1;
     ghi[O] = 1;
     ghi[D] = 1;
     const RegionTable& rt = region(c, glo[0], glo[1], glo[2], ghi[0], ghi[1], ghi[2], -1);
-    if (inl) es_transverse_launch_t<D, T, true>(c, rt, comp, bc, is_cons, vclamp);
-    else es_transverse_launch_t<D, T, false>(c, rt, comp, bc, is_cons, vclamp);
-}
-
-template <int D, bool INL>
-static void es_edges_launch_t(Ctx& c, int comp, const BCRecD& bc, int is_cons, int force_zero, int vclamp, int oc) {
-    constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
-    const double dt2 = 0.5 * c.P.dt;
-    const int ptf = c.P.ppm_trace_forces;
-    if (is_cons)
-        launch(c, rg_grow(c, 0, D), 1, k_es_edges<D, true, INL>, c.V(), comp, force_zero, dt2, dt2 / c.P.dx[T1],
-               dt2 / c.P.dx[T2], dt2 / c.P.dx[D], bc.lo[D], bc.hi[D], c.P.dom_lo[D], c.P.dom_hi[D],
-               dbits_host(c.P.rel_eps), vclamp, ptf, oc);
-    else
-        launch(c, rg_grow(c, 0, D), 1, k_es_edges<D, false, INL>, c.V(), comp, force_zero, dt2, dt2 / c.P.dx[T1],
-               dt2 / c.P.dx[T2], dt2 / c.P.dx[D], bc.lo[D], bc.hi[D], c.P.dom_lo[D], c.P.dom_hi[D],
-               dbits_host(c.P.rel_eps), vclamp, ptf, oc);
+    const double dt3 = c.P.dt / 3.0;
+    auto kern = is_cons ? k_es_transverse<D, T, true> : k_es_transverse<D, T, false>;
+    launch(c, rt, 1, kern, c.V(), comp, dt3, dt3 / c.P.dx[T], bc.lo[D], bc.hi[D], c.P.dom_lo[D], c.P.dom_hi[D],
+           dbits_host(c.P.rel_eps), vclamp);
 }
 
 template <int D>
-static void es_edges_launch(Ctx& c, int comp, const BCRecD& bc, int is_cons, int force_zero, int vclamp, int oc,
-                            bool inl) {
-    if (inl) es_edges_launch_t<D, true>(c, comp, bc, is_cons, force_zero, vclamp, oc);
-    else es_edges_launch_t<D, false>(c, comp, bc, is_cons, force_zero, vclamp, oc);
+static void es_edges_launch(Ctx& c, int comp, const BCRecD& bc, int is_cons, int force_zero, int vclamp, int oc) {
+    constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
+    const double dt2 = 0.5 * c.P.dt;
+    auto kern = is_cons ? k_es_edges<D, true> : k_es_edges<D, false>;
+    launch(c, rg_grow(c, 0, D), 1, kern, c.V(), comp, force_zero, dt2, dt2 / c.P.dx[T1], dt2 / c.P.dx[T2],
+           dt2 / c.P.dx[D], bc.lo[D], bc.hi[D], c.P.dom_lo[D], c.P.dom_hi[D], dbits_host(c.P.rel_eps), vclamp,
+           c.P.ppm_trace_forces, oc);
 }
 
 // velocity-only quantities shared by every component of a MakeEdgeScal call
@@ -1265,61 +1070,49 @@ void make_edge_scal(Ctx& c, int start_comp, int num_comp, int which_bcs, int is_
         cudaEventRecord(c.ev_fork, main_stream);
         cudaStreamWaitEvent(c.side, c.ev_fork, 0);
     }
-    // marched PPM and edge states from the upwind cell, up to three components a launch (their Ip
-    // / Im in the velocity predictor's fields, free here)
-    const bool ctu = ppm_marches(c) && c.es_inline && !c.edge_tape_begin && !is_cons;
-    const int batch = two || c.P.ppm_trace_forces ? 1 : 3;
-    for (int comp = start_comp; ctu && !two && comp < start_comp + num_comp; comp += batch) {
+    // marched PPM (ppm_type 0: the slopes' states) and edge states from the upwind cell, up to three
+    // components a launch (their Ip / Im in the velocity predictor's fields, free here); one
+    // where a component has fields of its own: the conservative form's terms, the traced force,
+    // the second stream's scratch, the staged sweep's output
+    const bool ctu = c.es_inline && !c.edge_tape_begin;
+    const bool marched = c.P.ppm_type == 0 || ppm_marches(c);
+    const int batch = !ctu || two || is_cons || c.P.ppm_trace_forces || !marched ? 1 : 3;
+    for (int comp = start_comp; comp < start_comp + num_comp; comp += batch) {
         const int nq = std::min(batch, start_comp + num_comp - comp);
-        ppm_march_comps(c, 7, F_SOLD, comp, nq, bh + comp, F_UMAC0, 1, F_IPC0, F_IMC0);
-        if (c.P.ppm_trace_forces && !force_zero)
-            ppm_march_comps(c, 7, F_SCALFORCE, comp, 1, bh + comp, F_UMAC0, 1, F_IPF, F_IMF);
-        edge_scal_ctu(c, comp, nq, bh + comp, slot >= 0 ? slot : comp, force_zero, is_vel);
-    }
-    if (ctu && !two) return;
-    for (int comp = start_comp; comp < start_comp + num_comp; ++comp) {
         const bool alt = two && ((comp - start_comp) & 1);
         c.stream = alt ? c.side : main_stream;
         c.dviews = alt ? c.dviews_side : main_views;
         if (c.edge_tape_begin) c.edge_tape_begin(comp);
         const BCRecD& bc = bh[comp];  // start_bccomp == start_scomp at every call site
         if (c.P.ppm_type == 0) {
-            for (int d = 0; d < 3; ++d) slope_any(c, d, F_SOLD, comp, F_SLOPE, d, 1, bcs_dev(c, which_bcs), comp);
+            if (ctu) slope_states(c, comp, nq, bh + comp);
+            else for (int d = 0; d < 3; ++d) slope_any(c, d, F_SOLD, comp, F_SLOPE, d, 1, bcs_dev(c, which_bcs), comp);
         } else {
-            for (int d = 0; d < 3; ++d) ppm_any(c, d, F_SOLD, comp, bc, F_UMAC0 + d, 0, 1, F_IPC0, F_IMC0);
+            if (ctu && marched) ppm_march_comps(c, 7, F_SOLD, comp, nq, bh + comp, F_UMAC0, 1, F_IPC0, F_IMC0);
+            else for (int d = 0; d < 3; ++d) ppm_any(c, d, F_SOLD, comp, bc, F_UMAC0 + d, 0, 1, F_IPC0, F_IMC0);
             // ppm_trace_forces: the component's force traced like it (Source/MaestroMakeEdgeScalars.cpp:
             // 137-141, 223-227); a force known to be zero traces to zero and is not read
             if (c.P.ppm_trace_forces && !force_zero)
                 for (int d = 0; d < 3; ++d) ppm_any(c, d, F_SCALFORCE, comp, bc, F_UMAC0 + d, 0, 1, F_IPF, F_IMF);
         }
-        const int v0 = is_vel && comp == 0, v1 = is_vel && comp == 1, v2 = is_vel && comp == 2;
-        // with PPM the predictor's l and r are Ip / Im passed on: the transverse and edge
-        // kernels form them themselves and only the upwind state is stored (the full
-        // predictor runs where the adjoint's tape keeps its fields)
-        const bool inl = c.es_inline && c.P.ppm_type != 0 && !c.edge_tape_begin;
+        const int oc = slot >= 0 ? slot : comp;
         if (ctu) {
-            edge_scal_ctu(c, comp, 1, &bc, slot >= 0 ? slot : comp, force_zero, is_vel);
+            edge_scal_ctu(c, comp, nq, bh + comp, oc, force_zero, is_vel, is_cons);
             continue;
         }
-        if (inl) {
-            es_simh_launch<0>(c, comp, bc, v0);
-            es_simh_launch<1>(c, comp, bc, v1);
-            es_simh_launch<2>(c, comp, bc, v2);
-        } else {
-            es_predictor_launch<0>(c, comp, bc, v0);
-            es_predictor_launch<1>(c, comp, bc, v1);
-            es_predictor_launch<2>(c, comp, bc, v2);
-        }
-        es_transverse_launch<0, 1>(c, comp, bc, is_cons, v0, inl);
-        es_transverse_launch<0, 2>(c, comp, bc, is_cons, v0, inl);
-        es_transverse_launch<1, 0>(c, comp, bc, is_cons, v1, inl);
-        es_transverse_launch<1, 2>(c, comp, bc, is_cons, v1, inl);
-        es_transverse_launch<2, 0>(c, comp, bc, is_cons, v2, inl);
-        es_transverse_launch<2, 1>(c, comp, bc, is_cons, v2, inl);
-        const int oc = slot >= 0 ? slot : comp;
-        es_edges_launch<0>(c, comp, bc, is_cons, force_zero, v0, oc, inl);
-        es_edges_launch<1>(c, comp, bc, is_cons, force_zero, v1, oc, inl);
-        es_edges_launch<2>(c, comp, bc, is_cons, force_zero, v2, oc, inl);
+        const int v0 = is_vel && comp == 0, v1 = is_vel && comp == 1, v2 = is_vel && comp == 2;
+        es_predictor_launch<0>(c, comp, bc, v0);
+        es_predictor_launch<1>(c, comp, bc, v1);
+        es_predictor_launch<2>(c, comp, bc, v2);
+        es_transverse_launch<0, 1>(c, comp, bc, is_cons, v0);
+        es_transverse_launch<0, 2>(c, comp, bc, is_cons, v0);
+        es_transverse_launch<1, 0>(c, comp, bc, is_cons, v1);
+        es_transverse_launch<1, 2>(c, comp, bc, is_cons, v1);
+        es_transverse_launch<2, 0>(c, comp, bc, is_cons, v2);
+        es_transverse_launch<2, 1>(c, comp, bc, is_cons, v2);
+        es_edges_launch<0>(c, comp, bc, is_cons, force_zero, v0, oc);
+        es_edges_launch<1>(c, comp, bc, is_cons, force_zero, v1, oc);
+        es_edges_launch<2>(c, comp, bc, is_cons, force_zero, v2, oc);
         if (c.edge_tape) c.edge_tape(comp);
     }
     c.stream = main_stream;

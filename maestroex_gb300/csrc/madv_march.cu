@@ -38,11 +38,12 @@
 #include "madv_launch.cuh"
 #include "madv_march.cuh"
 #include "madv_ppm.cuh"
+#include "madv_slope.cuh"
 
 namespace madv {
 
 // ============================================================ PPM along y or z
-template <int D, int PPMT, int UMAC>
+template <int D, int UMAC>
 __global__ void __launch_bounds__(256) k_ppm_march(KARGS, int fs, int sc0, int fu, int fip, int fim, unsigned lo_mask,
                                                     unsigned hi_mask, int domlo, int domhi, long long epsb, RecipC r6, unsigned nq) {
     const unsigned bx = blockIdx.x / nq, q = blockIdx.x - bx * nq;
@@ -60,21 +61,21 @@ __global__ void __launch_bounds__(256) k_ppm_march(KARGS, int fs, int sc0, int f
     c.B = &at(T, i, j, k, UMAC ? 1 : 2 * D + 1);
     c.sT = D == 1 ? T.sj : T.sk;
     const MarchBC bc{(int)(lo_mask >> q) & 1, (int)(hi_mask >> q) & 1, domlo, domhi};
-    ppm_march<D, PPMT, UMAC, false>(&at(s, i, j, k, sc0 + q), D == 1 ? s.sj : s.sk, c, &at(ip, i, j, k, D),
+    ppm_march<D, UMAC, false>(&at(s, i, j, k, sc0 + q), D == 1 ? s.sj : s.sk, c, &at(ip, i, j, k, D),
                                     &at(im, i, j, k, D), D == 1 ? ip.sj : ip.sk, I0, I1, bc, epsb, r6);
 }
 
 // ============================================================ PPM along x
 // Positions are the cells of the rows with the neighbours their interface values need; a
-// warp covers 32 of them and writes the inner ROW_OUT.
-template <int PPMT, int UMAC>
+// warp covers 32 of them and writes the inner 30.
+template <int UMAC>
 __global__ void __launch_bounds__(256) k_ppm_rows(KARGS, int fs, int sc0, int fu, int fip, int fim, unsigned lo_mask,
                                                    unsigned hi_mask, int domlo, int domhi, long long epsb, RecipC r6, unsigned nq) {
     MADV_LET_NEXT();
     const unsigned bx = blockIdx.x / nq, q = blockIdx.x - bx * nq;
     const int lane = threadIdx.x & 31;
     const long w = ((long)bx * blockDim.x + threadIdx.x) >> 5;
-    const long t = g0 + w * row_out(PPMT) + lane - 1;
+    const long t = g0 + w * row_out(1) + lane - 1;
     const long tc = t < g0 ? g0 : (t >= g1 ? g1 - 1 : t);  // lanes past the ends work on a copy
     const int e = find_box(R, ne, tc);
     const int b = R[e].b;
@@ -82,13 +83,13 @@ __global__ void __launch_bounds__(256) k_ppm_rows(KARGS, int fs, int sc0, int fu
     region_ijk(R[e], tc - R[e].start, i, j, k);
     const int r = i - R[e].lo[0];
     // a cell of the row proper, not one of the lanes that only pass values on
-    const bool out = t == tc && lane >= 1 && lane <= row_out(PPMT) && r >= 1 && r <= R[e].ext;
+    const bool out = t == tc && lane >= 1 && lane <= row_out(1) && r >= 1 && r <= R[e].ext;
     MADV_WAIT();
     const FabView s = VW(fs), u = VW(fu), T = UMAC ? VW(F_TRA0) : VW(F_TRC);
     const double* ps = &at(s, i, j, k, sc0 + q);
     const MarchBC bc{(int)(lo_mask >> q) & 1, (int)(hi_mask >> q) & 1, domlo, domhi};
     double ipv, imv;
-    ppm_row<PPMT, UMAC, false>(ps, &at(u, i, j, k, 0), &at(T, i, j, k, 0), &at(T, i, j, k, 1), i, out, bc, epsb, r6,
+    ppm_row<UMAC, false>(ps, &at(u, i, j, k, 0), &at(T, i, j, k, 0), &at(T, i, j, k, 1), i, out, bc, epsb, r6,
                                0.0, r6, ipv, imv);
     if (!out) return;
     at(VW(fip + q), i, j, k, 0) = ipv;
@@ -205,9 +206,9 @@ static void march_dir(Ctx& c, int fs, int sc0, int nq, const BCRecD* bc, int fu,
     } else if constexpr (PPMT == 2) {
         launch(c, rt, nq, k_ppm_march2<D, UMAC>, 0, c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6, n);
     } else if constexpr (D == 0) {
-        launch(c, rt, nq, k_ppm_rows<PPMT, UMAC>, row_out(PPMT), c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6, n);
+        launch(c, rt, nq, k_ppm_rows<UMAC>, row_out(1), c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6, n);
     } else {
-        launch(c, rt, nq, k_ppm_march<D, PPMT, UMAC>, 0, c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6, n);
+        launch(c, rt, nq, k_ppm_march<D, UMAC>, 0, c.V(), fs, sc0, fu, fip, fim, lo, hi, dl, dh, eb, r6, n);
     }
 }
 
@@ -230,6 +231,44 @@ void ppm_march_comps(Ctx& c, int dirs, int fs, int sc0, int nq, const BCRecD* bc
     if (dirs & 1) one(std::integral_constant<int, 0>{});
     if (dirs & 2) one(std::integral_constant<int, 1>{});
     if (dirs & 4) one(std::integral_constant<int, 2>{});
+}
+
+// ============================================================ ppm_type 0
+// The states of MakeEdgeScalPredictor without PPM (Source/MaestroMakeEdgeScalars.cpp:662-863) kept
+// per cell where PPM's Ip and Im are: above the cell s + (1 - dt u / h) / 2 slope, below it
+// s - (1 + dt u / h) / 2 slope, u on the cell's high and low face.
+struct SlopeBC {
+    int lo[3][3], hi[3][3];  // [component][direction]
+};
+template <int D>
+__device__ __forceinline__ void slope_state(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int sc, int q,
+                                            int bclo, int bchi, int so, int dlo, int dhi, double dt, const RecipC& rh,
+                                            const RecipC& r6) {
+    constexpr int di = D == 0, dj = D == 1, dk = D == 2;
+    const FabView s = VW(F_SOLD), u = VW(F_UMAC0 + D);
+    auto S = SHIFT_S(s, sc);
+    const double sl = limited_slope<D>(S, D == 0 ? i : (D == 1 ? j : k), bclo, bchi, so, dlo, dhi, r6);
+    const double up = at(u, i + di, j + dj, k + dk), um = at(u, i, j, k);
+    at(VW(F_IPC0 + q), i, j, k, D) = S(0) + half(1.0 - div_c(dt * up, rh)) * sl;
+    at(VW(F_IMC0 + q), i, j, k, D) = S(0) - half(1.0 + div_c(dt * um, rh)) * sl;
+}
+__global__ void __launch_bounds__(256) k_slope_states(KARGS, int sc0, unsigned nq, SlopeBC bc, int so, int dl0, int dl1,
+                                                       int dl2, int dh0, int dh1, int dh2, double dt, RecipC h0,
+                                                       RecipC h1, RecipC h2, RecipC r6) {
+    const unsigned bx = blockIdx.x / nq, q = blockIdx.x - bx * nq;
+    MADV_ELEMENT_OF(bx, R, ne, g0, g1, b, i, j, k);
+    slope_state<0>(V, nb, b, i, j, k, sc0 + q, q, bc.lo[q][0], bc.hi[q][0], so, dl0, dh0, dt, h0, r6);
+    slope_state<1>(V, nb, b, i, j, k, sc0 + q, q, bc.lo[q][1], bc.hi[q][1], so, dl1, dh1, dt, h1, r6);
+    slope_state<2>(V, nb, b, i, j, k, sc0 + q, q, bc.lo[q][2], bc.hi[q][2], so, dl2, dh2, dt, h2, r6);
+}
+
+void slope_states(Ctx& c, int sc0, int nq, const BCRecD* bc) {
+    SlopeBC sb{};
+    for (int q = 0; q < nq; ++q)
+        for (int d = 0; d < 3; ++d) sb.lo[q][d] = bc[q].lo[d], sb.hi[q][d] = bc[q].hi[d];
+    launch(c, rg_grow(c, 1), nq, k_slope_states, c.V(), sc0, (unsigned)nq, sb, c.P.slope_order, c.P.dom_lo[0],
+           c.P.dom_lo[1], c.P.dom_lo[2], c.P.dom_hi[0], c.P.dom_hi[1], c.P.dom_hi[2], c.P.dt, make_recip(c.P.dx[0]),
+           make_recip(c.P.dx[1]), make_recip(c.P.dx[2]), make_recip(6.0));
 }
 
 // ============================================================ edge states from Ip / Im
@@ -299,10 +338,17 @@ __device__ __forceinline__ EsBox es_box(const FabView* __restrict__ V, int nb, i
     return EsBox{p.p, p.sj, p.sk, p.sn, p.lo0, p.lo1, p.lo2};
 }
 
+// v less the transverse correction of the cell at o (components sn apart)
+template <bool CONS>
+__device__ __forceinline__ double es_less(double v, const double* c, long o, long sn) {
+    return CONS ? v - c[o] - c[o + sn] + c[o + 2 * sn] : v - c[o];
+}
+
 // The state of a boundary face by its rule: of the inside one of the cells at lo (below) and o
 // (above), less the increment inc of its cell (null: none).  ghost: the ext_dir state of the
 // cell outside.
-__device__ __noinline__ double es_bnd(const double* ip, const double* im, const double* inc, long lo, long o,
+template <bool CONS>
+__device__ __noinline__ double es_bnd(const double* ip, const double* im, const double* inc, long sn, long lo, long o,
                                       unsigned rule, const double* ghost) {
     const unsigned code = rule & 7;
     const bool below = rule & 8;
@@ -312,7 +358,7 @@ __device__ __noinline__ double es_bnd(const double* ip, const double* im, const 
     double v = (below ? ip : im)[oc];
     if (code == FR_CLAMP) v = clamp_out(v, below);
     if (inc) {
-        v = v - inc[oc];
+        v = es_less<CONS>(v, inc, oc, sn);
         if (code == FR_CLAMP) v = clamp_out(v, below);
     }
     return v;
@@ -339,12 +385,19 @@ __device__ __forceinline__ int trans_field(int a, int b) {
     k = klo + (k - klo) * len;                                              \
     const int k1 = min(k + len, klo + r.ext)
 
-// c_T = F_TCOEF_T * (upwind state above - below) of the cells (F_SIMH0 + T component q holds it)
-template <int T>
+// The conservative form's factors: dt/3/h_T, dt/2/h_T, dt/3
+struct EsCons {
+    double dt3h[3], dt2h[3], dt3;
+};
+
+// c_T = F_TCOEF_T * (upwind state above - below) of the cells (F_SIMH0 + T component q holds it).
+// CONS: the three terms of the correction, (dt/3/h) (s u above - s u below), (dt/3) s div u and
+// (dt/3/h) s (u above - u below), in components 0, 1, 2 (one component a launch).
+template <int T, bool CONS>
 __device__ __forceinline__ void es_cinc(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int k1, int comp,
-                                        int q, const EsRules& rules) {
+                                        int q, const EsRules& rules, const EsCons& ec) {
     const EsBox x = es_box(V, nb, b);
-    const FabView uv = VW(F_UMAC0 + T);
+    const FabView uv = VW(F_UMAC0 + T), sv = VW(F_SOLD), dvv = VW(F_DIVU);
     const double* pu = &at(uv, i, j, k);
     const long uk = uv.sk, us = T == 0 ? 1 : (T == 1 ? uv.sj : uv.sk);
     const long o = x.off(i, j, k), s = x.s<T>();
@@ -357,31 +410,39 @@ __device__ __forceinline__ void es_cinc(const FabView* __restrict__ V, int nb, i
             un = T == 2 ? up : pu[uk];
             uq = pu[uk + us];
         }
-        const double t = *tc;
+        const double t = CONS ? 0.0 : *tc;
         double vm = dhigh(um) >= 0 ? ip[-s] : im[0], vp = dhigh(up) >= 0 ? ip[0] : im[s];
         const int I = T == 0 ? i : (T == 1 ? j : k), bm = face_side<T>(rules, I), bp = face_side<T>(rules, I + 1);
         if (!nz(um)) vm = half(ip[-s] + im[0]);  // tie test |u| > 0
         if (!nz(up)) vp = half(ip[0] + im[s]);
         if (bm || bp) {
             const unsigned rm = bm ? face_rule<T>(rules, q, bm) : 0, rp = bp ? face_rule<T>(rules, q, bp) : 0;
-            if (rm) vm = es_bnd(ip, im, nullptr, -s, 0, rm, es_ghost(V, nb, b, i, j, k, T, rm & 8 ? 0 : -1, comp));
-            if (rp) vp = es_bnd(ip, im, nullptr, 0, s, rp, es_ghost(V, nb, b, i, j, k, T, rp & 8 ? 1 : 0, comp));
+            if (rm) vm = es_bnd<false>(ip, im, nullptr, 0, -s, 0, rm, es_ghost(V, nb, b, i, j, k, T, rm & 8 ? 0 : -1, comp));
+            if (rp) vp = es_bnd<false>(ip, im, nullptr, 0, 0, s, rp, es_ghost(V, nb, b, i, j, k, T, rp & 8 ? 1 : 0, comp));
         }
-        *out = t * (vp - vm);
+        if (CONS) {
+            const double s0 = at(sv, i, j, k, comp);
+            out[0] = ec.dt3h[T] * (vp * up - vm * um);
+            out[x.sn] = ec.dt3 * s0 * at(dvv, i, j, k);
+            out[2 * x.sn] = ec.dt3h[T] * s0 * (up - um);
+        } else {
+            *out = t * (vp - vm);
+        }
         um = un, up = uq;
         pu += uk, tc += x.s2, ip += x.s2, im += x.s2, out += x.s2;
     }
 }
-__global__ void __launch_bounds__(256) k_es_cinc(KARGS, int comp0, unsigned nq, EsRules rules) {
+template <bool CONS>
+__global__ void __launch_bounds__(256) k_es_cinc(KARGS, int comp0, unsigned nq, EsRules rules, EsCons ec) {
     MADV_ES_COLUMN();
-    if (dir == 0) es_cinc<0>(V, nb, b, i, j, k, k1, comp0 + q, q, rules);
-    else if (dir == 1) es_cinc<1>(V, nb, b, i, j, k, k1, comp0 + q, q, rules);
-    else es_cinc<2>(V, nb, b, i, j, k, k1, comp0 + q, q, rules);
+    if (dir == 0) es_cinc<0, CONS>(V, nb, b, i, j, k, k1, comp0 + q, q, rules, ec);
+    else if (dir == 1) es_cinc<1, CONS>(V, nb, b, i, j, k, k1, comp0 + q, q, rules, ec);
+    else es_cinc<2, CONS>(V, nb, b, i, j, k, k1, comp0 + q, q, rules, ec);
 }
 
 // Transverse states of A-faces, corrected along B where the face's cells lie in the box along B
 // (bi, bj: its cells in x, y; bk0 .. bk1: in z), and along C
-template <int A>
+template <int A, bool CONS>
 __device__ __forceinline__ void es_trans(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int k1, bool bi,
                                          bool bj, int bk0, int bk1, int comp, int q, const EsRules& rules,
                                          long long epsb) {
@@ -403,21 +464,21 @@ __device__ __forceinline__ void es_trans(const FabView* __restrict__ V, int nb, 
         const bool left = dhigh(u) >= 0;
         const long oc = left ? -s : 0;
         const double base = (left ? ip : im)[oc];
-        double vb = wantB ? cb[oc] : 0.0, vc = wantC ? cc[oc] : 0.0;
-        vb = base - vb;
-        vc = base - vc;
+        double vb = 0.0, vc = 0.0;
+        if (wantB) vb = es_less<CONS>(base, cb, oc, x.sn);
+        if (wantC) vc = es_less<CONS>(base, cc, oc, x.sn);
         if (dmag(u) <= epsb) {  // the mean of both sides' states
             const double l = ip[-s], rr = im[0];
-            if (wantB) vb = half((l - cb[-s]) + (rr - cb[0]));
-            if (wantC) vc = half((l - cc[-s]) + (rr - cc[0]));
+            if (wantB) vb = half(es_less<CONS>(l, cb, -s, x.sn) + es_less<CONS>(rr, cb, 0, x.sn));
+            if (wantC) vc = half(es_less<CONS>(l, cc, -s, x.sn) + es_less<CONS>(rr, cc, 0, x.sn));
         }
         const int side = face_side<A>(rules, A == 0 ? i : (A == 1 ? j : k));
         if (side) {
             const unsigned r = face_rule<A>(rules, q, side);
             if (r) {
                 const double* g = es_ghost(V, nb, b, i, j, k, A, r & 8 ? 0 : -1, comp);
-                if (wantB) vb = es_bnd(ip, im, cb, -s, 0, r, g);
-                if (wantC) vc = es_bnd(ip, im, cc, -s, 0, r, g);
+                if (wantB) vb = es_bnd<CONS>(ip, im, cb, x.sn, -s, 0, r, g);
+                if (wantC) vc = es_bnd<CONS>(ip, im, cc, x.sn, -s, 0, r, g);
             }
         }
         if (wantB) *qb = vb;
@@ -426,22 +487,22 @@ __device__ __forceinline__ void es_trans(const FabView* __restrict__ V, int nb, 
         pu += uk, ip += x.s2, im += x.s2, cb += x.s2, cc += x.s2, qb += x.s2, qc += x.s2;
     }
 }
+template <bool CONS>
 __global__ void __launch_bounds__(256) k_es_trans(KARGS, int comp0, unsigned nq, EsRules rules, long long epsb) {
     MADV_ES_COLUMN();
     // the region is grown by one across the direction: its inner cells lie in the box
     const bool bi = i > r.lo[0] && i < r.lo[0] + r.n[0] - 1, bj = j > r.lo[1] && j < r.lo[1] + r.n[1] - 1;
     const int bk0 = klo + 1, bk1 = klo + r.ext - 2;
-    if (dir == 0) es_trans<0>(V, nb, b, i, j, k, k1, bi, bj, bk0, bk1, comp0 + q, q, rules, epsb);
-    else if (dir == 1) es_trans<1>(V, nb, b, i, j, k, k1, bi, bj, bk0, bk1, comp0 + q, q, rules, epsb);
-    else es_trans<2>(V, nb, b, i, j, k, k1, bi, bj, bk0, bk1, comp0 + q, q, rules, epsb);
+    if (dir == 0) es_trans<0, CONS>(V, nb, b, i, j, k, k1, bi, bj, bk0, bk1, comp0 + q, q, rules, epsb);
+    else if (dir == 1) es_trans<1, CONS>(V, nb, b, i, j, k, k1, bi, bj, bk0, bk1, comp0 + q, q, rules, epsb);
+    else es_trans<2, CONS>(V, nb, b, i, j, k, k1, bi, bj, bk0, bk1, comp0 + q, q, rules, epsb);
 }
 
-// Edge states of D-faces, advective form (MakeEdgeScalEdges,
-// Source/MaestroMakeEdgeScalars.cpp:1361-1667).
-template <int D>
+// Edge states of D-faces (MakeEdgeScalEdges, Source/MaestroMakeEdgeScalars.cpp:1361-1667).
+template <int D, bool CONS>
 __device__ __forceinline__ void es_edge(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int k1, int comp,
                                         int oc0, int q, const EsRules& rules, int force_zero, int ptf, double dt2,
-                                        long long epsb) {
+                                        long long epsb, const EsCons& ec) {
     constexpr int A = D == 0 ? 1 : 0, B = D == 2 ? 1 : 2;
     constexpr int di = D == 0, dj = D == 1, dk = D == 2;
     const EsBox x = es_box(V, nb, b);
@@ -465,7 +526,17 @@ __device__ __forceinline__ void es_edge(const FabView* __restrict__ V, int nb, i
         const long c = below ? -s : 0;
         double v = (below ? ip : im)[c];
         if (code == FR_CLAMP) v = clamp_out(v, below);
-        v = v - ta[c] * (qa[c + sa] - qa[c]) - tb[c] * (qb[c + sb] - qb[c]);
+        if (CONS) {
+            const int m = below ? -1 : 0, ci = i + m * di, cj = j + m * dj, ck = k + m * dk;
+            const FabView ua = VW(F_UMAC0 + A), ub = VW(F_UMAC0 + B), sv = VW(F_SOLD);
+            const double a0 = at(ua, ci, cj, ck), a1 = at(ua, ci + (A == 0), cj + (A == 1), ck + (A == 2));
+            const double b0 = at(ub, ci, cj, ck), b1 = at(ub, ci + (B == 0), cj + (B == 1), ck + (B == 2));
+            const double d0 = at(uv, ci, cj, ck), d1 = at(uv, ci + di, cj + dj, ck + dk);
+            v = v - ec.dt2h[A] * (qa[c + sa] * a1 - qa[c] * a0) - ec.dt2h[B] * (qb[c + sb] * b1 - qb[c] * b0) -
+                ec.dt2h[D] * at(sv, ci, cj, ck, comp) * (d1 - d0);
+        } else {
+            v = v - ta[c] * (qa[c + sa] - qa[c]) - tb[c] * (qb[c + sb] - qb[c]);
+        }
         if (!force_zero) v = v + dt2 * (below ? fp[-fs] : fm[0]);
         if (code == FR_CLAMP) v = clamp_out(v, below);
         return v;
@@ -488,12 +559,13 @@ __device__ __forceinline__ void es_edge(const FabView* __restrict__ V, int nb, i
         out += e.sk;
     }
 }
+template <bool CONS>
 __global__ void __launch_bounds__(256) k_es_edge(KARGS, int comp0, int oc0, unsigned nq, EsRules rules, int force_zero,
-                                                  int ptf, double dt2, long long epsb) {
+                                                  int ptf, double dt2, long long epsb, EsCons ec) {
     MADV_ES_COLUMN();
-    if (dir == 0) es_edge<0>(V, nb, b, i, j, k, k1, comp0 + q, oc0, q, rules, force_zero, ptf, dt2, epsb);
-    else if (dir == 1) es_edge<1>(V, nb, b, i, j, k, k1, comp0 + q, oc0, q, rules, force_zero, ptf, dt2, epsb);
-    else es_edge<2>(V, nb, b, i, j, k, k1, comp0 + q, oc0, q, rules, force_zero, ptf, dt2, epsb);
+    if (dir == 0) es_edge<0, CONS>(V, nb, b, i, j, k, k1, comp0 + q, oc0, q, rules, force_zero, ptf, dt2, epsb, ec);
+    else if (dir == 1) es_edge<1, CONS>(V, nb, b, i, j, k, k1, comp0 + q, oc0, q, rules, force_zero, ptf, dt2, epsb, ec);
+    else es_edge<2, CONS>(V, nb, b, i, j, k, k1, comp0 + q, oc0, q, rules, force_zero, ptf, dt2, epsb, ec);
 }
 
 // Regions of the three directions one after the other (pad = D): the faces (nodal) or cells of
@@ -530,17 +602,29 @@ static const RegionTable& dirs_region(Ctx& c, bool nodal, int g) {
     return t;
 }
 
-// Edge states of components comp0 .. comp0 + nq - 1 (nq <= 3) of F_SOLD, advective form, 3-D,
-// ppm_type 1 / 2, into components oc0 .. of F_SEDGE*: Ip / Im in F_IPC0 + q / F_IMC0 + q, the
-// tracing and transverse coefficients of F_UMAC* in place (edge_scal_setup).
-void edge_scal_ctu(Ctx& c, int comp0, int nq, const BCRecD* bc, int oc0, int force_zero, int is_vel) {
-    const EsRules r = es_rules(c, bc, comp0, nq, is_vel);
+// Edge states of components comp0 .. comp0 + nq - 1 (nq <= 3; conservative form: 1) of F_SOLD, 3-D,
+// into components oc0 .. of F_SEDGE*: Ip / Im (slope_states, ppm_type 0) in F_IPC0 + q /
+// F_IMC0 + q, the tracing and transverse coefficients of F_UMAC* or div u in place
+// (edge_scal_setup).
+template <bool CONS>
+static void es_launch(Ctx& c, int comp0, int nq, const EsRules& r, int oc0, int force_zero) {
     const long long eb = dbits_host(c.P.rel_eps);
     const unsigned n = (unsigned)nq;
-    launch(c, dirs_region(c, false, 1), nq, k_es_cinc, c.V(), comp0, n, r);
-    launch(c, dirs_region(c, true, 1), nq, k_es_trans, c.V(), comp0, n, r, eb);
-    launch(c, dirs_region(c, true, 0), nq, k_es_edge, c.V(), comp0, oc0, n, r, force_zero, c.P.ppm_trace_forces,
-           0.5 * c.P.dt, eb);
+    EsCons ec{};
+    ec.dt3 = c.P.dt / 3.0;
+    for (int d = 0; d < 3; ++d) {
+        ec.dt3h[d] = ec.dt3 / c.P.dx[d];
+        ec.dt2h[d] = 0.5 * c.P.dt / c.P.dx[d];
+    }
+    launch(c, dirs_region(c, false, 1), nq, k_es_cinc<CONS>, c.V(), comp0, n, r, ec);
+    launch(c, dirs_region(c, true, 1), nq, k_es_trans<CONS>, c.V(), comp0, n, r, eb);
+    launch(c, dirs_region(c, true, 0), nq, k_es_edge<CONS>, c.V(), comp0, oc0, n, r, force_zero, c.P.ppm_trace_forces,
+           0.5 * c.P.dt, eb, ec);
+}
+void edge_scal_ctu(Ctx& c, int comp0, int nq, const BCRecD* bc, int oc0, int force_zero, int is_vel, int is_cons) {
+    const EsRules r = es_rules(c, bc, comp0, nq, is_vel);
+    if (is_cons) es_launch<true>(c, comp0, nq, r, oc0, force_zero);
+    else es_launch<false>(c, comp0, nq, r, oc0, force_zero);
 }
 
 }  // namespace madv

@@ -8,7 +8,7 @@
 namespace madv {
 
 // lanes of a warp that k_ppm_rows writes: a cell needs the slope below its low face and the
-// interface value above it (ppm_type 2: two above)
+// interface value above it (ppm_type 2: positions that only pass values on, one below, two above)
 __host__ __device__ constexpr int row_out(int ppm_type) { return ppm_type == 1 ? 30 : 29; }
 
 // ext_dir / hoextrap boundaries along the march
@@ -45,8 +45,8 @@ __device__ __noinline__ double2 ppm_cell_bnd(const double* ps, long st, int I, M
     return v;
 }
 
-// Ip, Im of the cells I0 .. I1 - 1 of a column; pointers at cell (low face) I0.
-template <int D, int PPMT, int UMAC, bool INL>
+// Ip, Im of the cells I0 .. I1 - 1 of a column (ppm_type 1); pointers at cell (low face) I0.
+template <int D, int UMAC, bool INL>
 __device__ __forceinline__ void ppm_march(const double* __restrict__ ps, long st, MarchCoef c, double* __restrict__ pip,
                                           double* __restrict__ pim, long so, int I0, int I1, const MarchBC& bc,
                                           long long epsb, const RecipC& r6) {
@@ -58,35 +58,22 @@ __device__ __forceinline__ void ppm_march(const double* __restrict__ ps, long st
             B = *c.B;
         }
     };
-    double um, Am, Bm, up, Ap, Bp;
+    double um = 0, Am = 0, Bm = 0, up, Ap, Bp;
     if (UMAC) {
         um = *c.u;
         coef(um, Am, Bm);
     }
-    double s0 = ps[0], sB = ps[-st], s1 = ps[st];
-    double d1 = s1 - s0;
-    double dv0 = 0, f0 = 0, fm = 0, f1 = 0, sA = 0, s2 = 0;
     auto none = [](int) -> double { return 0.0; };
-    if (PPMT == 1) {
-        const double sa = ps[-2 * st], dA = sB - sa, d0 = s0 - sB;
-        const double dvB = vl_slope(s0 - sa, dA, d0);
-        dv0 = vl_slope(s1 - sB, d0, d1);
-        f0 = ppm1_face_regular(sB, s0, dvB, dv0, r6);
-    } else {
-        sA = ps[-2 * st];
-        s2 = ps[2 * st];
-        auto S = [&](int m) -> double {
-            return m == -3 ? ps[-3 * st] : m == -2 ? sA : m == -1 ? sB : m == 0 ? s0 : m == 1 ? s1 : s2;
-        };
-        fm = ppm2_face_regular(S, -1, r6);
-        f0 = ppm2_face_regular(S, 0, r6);
-        f1 = ppm2_face_regular(S, 1, r6);
-    }
-    constexpr int AHEAD = PPMT == 1 ? 2 : 3;
-    double sN = ps[AHEAD * st];  // the state the next interface value needs
+    double s0 = ps[0], sB = ps[-st], s1 = ps[st];
+    const double sA = ps[-2 * st], dA = sB - sA, d0 = s0 - sB;
+    double d1 = s1 - s0;
+    const double dvB = vl_slope(s0 - sA, dA, d0);
+    double dv0 = vl_slope(s1 - sB, d0, d1);
+    double f0 = ppm1_face_regular(sB, s0, dvB, dv0, r6);
+    double sN = ps[2 * st];  // the state the next interface value needs
     for (int I = I0; I < I1; ++I) {
-        const double snext = sN;
-        if (I + 1 < I1) sN = ps[(AHEAD + 1) * st];
+        const double s2 = sN;
+        if (I + 1 < I1) sN = ps[3 * st];
         if (UMAC) {
             c.u += c.su;
             c.A += c.sT;
@@ -100,22 +87,15 @@ __device__ __forceinline__ void ppm_march(const double* __restrict__ ps, long st
             c.A += c.sT;
             c.B += c.sT;
         }
-        double sm, sp, f2 = 0, dv1 = 0, d2 = 0;
-        if (PPMT == 1) {
-            d2 = snext - s1;
-            dv1 = vl_slope(snext - s0, d1, d2);
-            f1 = ppm1_face_regular(s0, s1, dv0, dv1, r6);
-        } else {
-            auto S = [&](int m) -> double { return m == 0 ? s0 : m == 1 ? s1 : m == 2 ? s2 : snext; };
-            f2 = ppm2_face_regular(S, 2, r6);
-        }
+        const double d2 = s2 - s1, dv1 = vl_slope(s2 - s0, d1, d2), f1 = ppm1_face_regular(s0, s1, dv0, dv1, r6);
+        double sm, sp;
         if (bc.touches(I)) {
-            const double2 v = ppm_cell_bnd<D, PPMT>(ps, st, I, bc, r6);
+            const double2 v = ppm_cell_bnd<D, 1>(ps, st, I, bc, r6);
             sm = v.x, sp = v.y;
         } else {
-            auto S = [&](int m) -> double { return m == -2 ? sA : m == -1 ? sB : m == 0 ? s0 : m == 1 ? s1 : s2; };
-            auto F = [&](int m) -> double { return m == -1 ? fm : m == 0 ? f0 : m == 1 ? f1 : f2; };
-            ppm_cell_any<D, PPMT>(S, F, none, I, 0, 0, 0, 0, sm, sp);
+            auto S = [&](int) -> double { return s0; };
+            auto F = [&](int m) -> double { return m == 0 ? f0 : f1; };
+            ppm_cell_any<D, 1>(S, F, none, I, 0, 0, 0, 0, sm, sp);
         }
         double ipv, imv;
         ppm_trace(s0, sm, sp, up, um, Ap, Bp, Am, Bm, epsb, ipv, imv);
@@ -124,51 +104,36 @@ __device__ __forceinline__ void ppm_march(const double* __restrict__ ps, long st
         pip += so;
         pim += so;
         ps += st;
-        if (PPMT == 2) {
-            sA = sB, fm = f0, f0 = f1, f1 = f2;
-            sB = s0, s0 = s1, s1 = s2, s2 = snext;
-        } else {
-            f0 = f1, dv0 = dv1, d1 = d2;
-            sB = s0, s0 = s1, s1 = snext;
-        }
+        f0 = f1, dv0 = dv1, d1 = d2;
+        sB = s0, s0 = s1, s1 = s2;
         um = up, Am = Ap, Bm = Bp;
     }
 }
 
-// Ip, Im of the cell i of a row, one cell a lane: slopes and interface values come from the
-// neighbour lanes.  Every lane of the warp calls; the results are valid where `out`.
+// Ip, Im of the cell i of a row (ppm_type 1), one cell a lane: slopes and interface values come from
+// the neighbour lanes.  Every lane of the warp calls; the results are valid where `out`.
 // Pointers at the cell (its low face).
-template <int PPMT, int UMAC, bool INL>
+template <int UMAC, bool INL>
 __device__ __forceinline__ void ppm_row(const double* __restrict__ ps, const double* __restrict__ pu,
                                         const double* __restrict__ pA, const double* __restrict__ pB, int i, bool out,
                                         const MarchBC& bc, long long epsb, const RecipC& r6, double dt,
                                         const RecipC& rdx, double& ipv, double& imv) {
     constexpr unsigned ALL = 0xffffffffu;
     const double sB = ps[-1], s0 = ps[0], s1 = ps[1];
-    double fm = 0, f0, f1, f2 = 0;
-    if (PPMT == 1) {
-        const double dv = vl_slope(s1 - sB, s0 - sB, s1 - s0);
-        const double dvB = __shfl_up_sync(ALL, dv, 1);
-        f0 = ppm1_face_regular(sB, s0, dvB, dv, r6);
-        f1 = __shfl_down_sync(ALL, f0, 1);
-    } else {
-        const double sA = ps[-2];
-        auto S = [&](int m) -> double { return m == -2 ? sA : m == -1 ? sB : m == 0 ? s0 : s1; };
-        f0 = ppm2_face_regular(S, 0, r6);
-        fm = __shfl_up_sync(ALL, f0, 1);
-        f1 = __shfl_down_sync(ALL, f0, 1);
-        f2 = __shfl_down_sync(ALL, f0, 2);
-    }
+    const double dv = vl_slope(s1 - sB, s0 - sB, s1 - s0);
+    const double dvB = __shfl_up_sync(ALL, dv, 1);
+    const double f0 = ppm1_face_regular(sB, s0, dvB, dv, r6);
+    const double f1 = __shfl_down_sync(ALL, f0, 1);
     if (!out) return;
     double sm, sp;
     if (bc.touches(i)) {
-        const double2 v = ppm_cell_bnd<0, PPMT>(ps, 1, i, bc, r6);
+        const double2 v = ppm_cell_bnd<0, 1>(ps, 1, i, bc, r6);
         sm = v.x, sp = v.y;
     } else {
-        auto S = [&](int m) -> double { return m == 0 ? s0 : m == -1 ? sB : m == 1 ? s1 : ps[m]; };
-        auto F = [&](int m) -> double { return m == -1 ? fm : m == 0 ? f0 : m == 1 ? f1 : f2; };
+        auto S = [&](int) -> double { return s0; };
+        auto F = [&](int m) -> double { return m == 0 ? f0 : f1; };
         auto none = [](int) -> double { return 0.0; };
-        ppm_cell_any<0, PPMT>(S, F, none, i, 0, 0, 0, 0, sm, sp);
+        ppm_cell_any<0, 1>(S, F, none, i, 0, 0, 0, 0, sm, sp);
     }
     double up, um, Ap, Bp, Am, Bm;
     if (UMAC) {

@@ -1,7 +1,8 @@
-"""The marched PPM sweeps and the one-sided edge states (madv_march.cu: up to three components a
-launch, chunks of columns, rows by shuffles) against the oracle's MakeEdgeScal, bit for bit:
-boxes whose extents leave remainders in the chunks and rows, every scalar boundary rule, and MAC
-velocities with ties -- exactly zero and within rel_eps -- in one direction or all of them."""
+"""The marched PPM sweeps, the slopes' states and the one-sided edge states (madv_march.cu: up to
+three components a launch, chunks of columns, rows by shuffles; advective and conservative
+form) against the oracle's MakeEdgeScal, bit for bit: boxes whose extents leave remainders in the
+chunks and rows, every scalar boundary rule, and MAC velocities with ties -- exactly zero and
+within rel_eps -- in one direction or all of them."""
 import numpy as np
 import pytest
 import torch
@@ -26,11 +27,11 @@ def _built():
     build.build_library()
 
 
-@pytest.mark.parametrize("ppm_type", [1, 2])
+@pytest.mark.parametrize("ppm_type,cons", [(1, 0), (2, 0), (0, 0), (1, 1), (0, 1)])
 @pytest.mark.parametrize("shape", range(len(SHAPES)))
 @pytest.mark.parametrize("bc", range(len(BCS)))
 @pytest.mark.parametrize("ties", ["none", "x", "y", "z", "all"])
-def test_edge_states_match_oracle(ppm_type, shape, bc, ties):
+def test_edge_states_match_oracle(ppm_type, cons, shape, bc, ties):
     n, boxes = SHAPES[shape]
     cfg = configs.planar_config(n=n, nspec=4, ppm_type=ppm_type, boxes=boxes, bc_lo=BCS[bc][0], bc_hi=BCS[bc][1])
     inp = MemberInputs(cfg)
@@ -48,11 +49,11 @@ def test_edge_states_match_oracle(ppm_type, shape, bc, ties):
     state, umac, force = inp.fabs("state", g), inp.fabs("uface", 1), inp.fabs("scal_force", 1)
     out = [MultiFab(b, inp.nscal, 0, nodal=d) for d in range(3)]
     st.make_edge_scal(to_mf(state, b, g), out, [to_mf(umac[d], b, 1, d) for d in range(3)], to_mf(force, b, 1), 0,
-                      FIRSTSPEC, FIRSTSPEC, 4, 0)
+                      FIRSTSPEC, FIRSTSPEC, 4, cons)
     torch.cuda.synchronize()
     ref = [zeros_like(f) for f in inp.fabs("sedge", 0)]
     pyoracle.member(cfg, "make_edge_scal", {"state": state, "umac": umac, "force": force, "sedge": ref},
-                    start_comp=FIRSTSPEC, num_comp=4, is_conservative=0)
+                    start_comp=FIRSTSPEC, num_comp=4, is_conservative=cons)
     bad = []
     for d in range(3):
         worst, bitwise = compare(out[d], ref[d], range(FIRSTSPEC, FIRSTSPEC + 4), f"sedge {d}")
