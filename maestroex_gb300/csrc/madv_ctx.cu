@@ -81,6 +81,30 @@ const RegionTable& region(Ctx& c, int glo0, int glo1, int glo2, int ghi0, int gh
     return t;
 }
 
+const RegionTable& region_union(Ctx& c, const std::vector<RegionKey>& parts) {
+    std::vector<int> key;
+    for (const RegionKey& p : parts) key.insert(key.end(), p.begin(), p.end());
+    auto it = c.unions.find(key);
+    if (it != c.unions.end()) return it->second;
+    std::vector<RegionBox> h;
+    long total = 0;
+    for (size_t q = 0; q < parts.size(); ++q) {
+        const RegionKey& p = parts[q];
+        const RegionTable& r = region(c, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7]);
+        for (RegionBox e : r.h) {
+            e.start += total;
+            e.pad = (int)q;
+            h.push_back(e);
+        }
+        total += r.total;
+    }
+    RegionTable& t = c.unions[key];
+    t.h = h;
+    t.total = total;
+    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    return t;
+}
+
 // a minus b as up to six disjoint boxes appended to out
 static void box_minus(const HBox& a, const HBox& b, std::vector<HBox>& out) {
     for (int d = 0; d < 3; ++d)
@@ -184,6 +208,28 @@ const CopyTable& copy_table(Ctx& c, int ng, int nodal) {
         }
     }
     t.total = start;
+    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, COPY_HINT);
+    return t;
+}
+
+const CopyTable& copy_table_faces(Ctx& c, int ng) {
+    std::array<int, 3> key{ng, 0, 1};
+    auto it = c.copies.find(key);
+    if (it != c.copies.end()) return it->second;
+    std::vector<CopyDesc> h;
+    long total = 0;
+    for (int d = 0; d < 3; ++d) {
+        const CopyTable& one = copy_table(c, ng, d);
+        for (CopyDesc e : one.h) {
+            e.start += total;
+            e.df = d;
+            h.push_back(e);
+        }
+        total += one.total;
+    }
+    CopyTable& t = c.copies[key];
+    t.h = h;
+    t.total = total;
     if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, COPY_HINT);
     return t;
 }
@@ -302,6 +348,9 @@ static void free_layout(Ctx& c) {
     for (auto& kv : c.regions)
         if (kv.second.d) cudaFree(kv.second.d);
     c.regions.clear();
+    for (auto& kv : c.unions)
+        if (kv.second.d) cudaFree(kv.second.d);
+    c.unions.clear();
     for (auto& kv : c.copies)
         if (kv.second.d) cudaFree(kv.second.d);
     c.copies.clear();
@@ -444,6 +493,11 @@ static void fill_patch_h(Hier& H, int fid, int c0, int nc, int which_bcs, int bc
         fill_patch(H[l], fid, c0, nc, which_bcs, bc_c0, is_vel, state_c0);
     }
 }
+// the same for two component ranges of a field: one level fills both at once
+static void fill_patch_h(Hier& H, int fid, const FillRange& a, const FillRange& b) {
+    if (H.n() == 1) return fill_patch(H[0], fid, a, b);
+    for (const FillRange* r : {&a, &b}) fill_patch_h(H, fid, r->c0, r->nc, r->which_bcs, r->bc_c0, 0, r->c0);
+}
 // Maestro::AverageDown (Source/MaestroFillData.cpp:145-154)
 static void average_down_h(Hier& H, int fid, int comp, int ncomp) {
     for (int l = H.n() - 2; l >= 0; --l) average_down(H[l + 1], H[l], fid, comp, ncomp);
@@ -466,15 +520,32 @@ static void sync_faces_h(Hier& H, int f0) {
         fill_face_ghosts(H[l], f0);
     }
 }
-// Maestro::Put1dArrayOnCart, planar (Source/MaestroFill3dData.cpp:9-36)
+// Maestro::Put1dArrayOnCart (Source/MaestroFill3dData.cpp:9-36) of several arrays, each into its
+// own field
+struct Put1d {
+    int fid;
+    const char* s0;
+    int outcomp, nc, edge, which_bcs, bc_c0, is_vel, state_c0;
+};
+static void put1d_h(Hier& H, const std::vector<Put1d>& list) {
+    std::vector<Put1dJob> jobs;
+    for (const Put1d& p : list) {
+        if (H.n() == 1 && put1d_fills(H[0])) {
+            jobs.push_back({p.fid, H[0].b1(p.s0), p.outcomp, p.nc, p.edge, p.which_bcs, p.bc_c0});
+            continue;
+        }
+        for (auto* c : H.L) {
+            set_val(*c, p.fid, 0.0, 0, p.nc, c->F[p.fid].spec.ng);
+            put1d(*c, p.fid, c->b1(p.s0), p.outcomp, p.edge, p.nc == 3);
+        }
+        average_down_h(H, p.fid, 0, p.nc);
+        fill_patch_h(H, p.fid, 0, p.nc, p.which_bcs, p.bc_c0, p.is_vel, p.state_c0);
+    }
+    if (!jobs.empty()) put1d_filled(H[0], jobs);
+}
 static void put1d_h(Hier& H, int fid, const char* s0, int outcomp, int nc, int edge, int which_bcs, int bc_c0,
                     int is_vel, int state_c0) {
-    for (auto* c : H.L) {
-        set_val(*c, fid, 0.0, 0, nc, c->F[fid].spec.ng);
-        put1d(*c, fid, c->b1(s0), outcomp, edge, nc == 3);
-    }
-    average_down_h(H, fid, 0, nc);
-    fill_patch_h(H, fid, 0, nc, which_bcs, bc_c0, is_vel, state_c0);
+    put1d_h(H, {{fid, s0, outcomp, nc, edge, which_bcs, bc_c0, is_vel, state_c0}});
 }
 // Maestro::Addw0 (Source/MaestroFill3dData.cpp:357-462)
 static void addw0_h(Hier& H, int f0, double mult) {
@@ -499,13 +570,14 @@ static void make_s0mac_h(Hier& H, const char* s0, int dst0) {
 static void w0_carts(Hier& H) {
     const int nd = H[0].ndim;
     // Put1dArrayOnCart(w0, w0_cart, true, true, bcs_u, 0, 1)  (Source/MaestroAdvance.cpp:326)
-    put1d_h(H, F_W0CART, "w0", nd - 1, nd, 1, BCS_U, 0, 1, -1);
+    // and w0_force_cart (w0_force, false, true, bcs_f, 0) (:341), evolve_base_state only
+    std::vector<Put1d> list{{F_W0CART, "w0", nd - 1, nd, 1, BCS_U, 0, 1, -1}};
+    for (auto* c : H.L) set_val(*c, F_W0FCART, 0.0, 0, 3, 1);
+    if (H[0].P.evolve_base_state) list.push_back({F_W0FCART, "w0_force", nd - 1, nd, 0, BCS_F, 0, 0, -1});
+    put1d_h(H, list);
     // MakeW0mac (Source/MaestroAdvance.cpp:335-338)
     if (H[0].sph)
         for (auto* c : H.L) make_w0mac(*c);
-    // Put1dArrayOnCart(w0_force, w0_force_cart, false, true, bcs_f, 0) (:341), evolve_base_state only
-    for (auto* c : H.L) set_val(*c, F_W0FCART, 0.0, 0, 3, 1);
-    if (H[0].P.evolve_base_state) put1d_h(H, F_W0FCART, "w0_force", nd - 1, nd, 0, BCS_F, 0, 0, -1);
 }
 
 // Maestro::MakeVelForce, planar (Source/MaestroForce.cpp:6-259)
@@ -515,8 +587,8 @@ static void make_vel_force_h(Hier& H, int fe = F_UTRANS0, const char* rho0 = "rh
     const int nd = H[0].ndim;
     // spherical, uniform bins: dw0/dr on the cells (Source/MaestroForce.cpp:36-52)
     if (H[0].sph && !H[0].geo.exact) put1d_h(H, F_GRADW0, "gradw0", 0, 1, 0, BCS_U, 0, 1, -1);
-    put1d_h(H, F_GRAVCART, "grav_cell", nd - 1, nd, 0, BCS_F, 0, 0, -1);
-    put1d_h(H, F_RHO0CART, rho0, 0, 1, 0, BCS_S, RHO, 0, RHO);
+    put1d_h(H, {{F_GRAVCART, "grav_cell", nd - 1, nd, 0, BCS_F, 0, 0, -1},
+                {F_RHO0CART, rho0, 0, 1, 0, BCS_S, RHO, 0, RHO}});
     for (auto* c : H.L) make_vel_force(*c, fe);
     average_down_h(H, F_VELFORCE, 0, nd);
     fill_patch_h(H, F_VELFORCE, 0, nd, BCS_U, 0, 1, -1);
@@ -526,15 +598,15 @@ static void make_vel_force_h(Hier& H, int fe = F_UTRANS0, const char* rho0 = "rh
 static void advance_premac(Hier& H) {
     const int nga = H[0].ng_adv, nd = H[0].ndim;
     fill_patch_h(H, F_UTILDE, 0, nd, BCS_U, 0, 1, -1);
-    for (auto* c : H.L) {
-        set_val(*c, F_UFULL, 0.0, 0, 3, nga);
-        copy_fab(*c, F_UFULL, 0, F_W0CART, 0, nd, 0);
+    for (auto* c : H.L)
+        set_zeros(*c, {{F_UFULL, 0, 3, nga}, {F_UTRANS0, 0, 1, 1}, {F_UTRANS1, 0, 1, 1}, {F_UTRANS2, 0, 1, 1}});
+    if (H.n() == 1 && put1d_fills(H[0])) {  // w0_cart with its ghost cells, as w0_carts forms it
+        put1d_filled(H[0], {{F_UFULL, H[0].b1("w0"), nd - 1, nd, 1, BCS_U, 0}});
+    } else {
+        for (auto* c : H.L) copy_fab(*c, F_UFULL, 0, F_W0CART, 0, nd, 0);
+        fill_patch_h(H, F_UFULL, 0, nd, BCS_U, 0, 1, -1);
     }
-    fill_patch_h(H, F_UFULL, 0, nd, BCS_U, 0, 1, -1);
-    for (auto* c : H.L) {
-        add_fab(*c, F_UFULL, F_UTILDE, nd, nga);
-        for (int d = 0; d < 3; ++d) set_val(*c, F_UTRANS0 + d, 0.0, 0, 1, 1);
-    }
+    for (auto* c : H.L) add_fab(*c, F_UFULL, F_UTILDE, nd, nga);
     for (auto* c : H.L) make_utrans(*c);
     sync_faces_h(H, F_UTRANS0);
     make_vel_force_h(H);
@@ -544,8 +616,12 @@ static void advance_premac(Hier& H) {
 }
 
 // Maestro::ModifyScalForce (Source/MaestroForce.cpp:261-467)
-static void modify_scal_force_h(Hier& H, int comp, const char* s0_edge, int s0cart_fid, int fullform) {
-    if (!H[0].sph) put1d_h(H, F_S0ECART, s0_edge, 0, 1, 0, BCS_F, 0, 0, -1);  // planar only (:275-277)
+// s0: the base state put on the cells first, into s0cart_fid (null: it is there)
+static void modify_scal_force_h(Hier& H, int comp, const char* s0, const char* s0_edge, int s0cart_fid, int fullform) {
+    std::vector<Put1d> list;
+    if (s0) list.push_back({s0cart_fid, s0, 0, 1, 0, BCS_S, comp, 0, comp});
+    if (!H[0].sph) list.push_back({F_S0ECART, s0_edge, 0, 1, 0, BCS_F, 0, 0, -1});  // planar only (:275-277)
+    put1d_h(H, list);
     // spherical, uniform bins: div w0 on the cells (:283-305)
     if (H[0].sph && !H[0].geo.exact) put1d_h(H, F_DIVW0, "divw0", 0, 1, 0, BCS_U, 0, 0, -1);
     for (auto* c : H.L) modify_scal_force(*c, comp, s0cart_fid, fullform);
@@ -557,12 +633,13 @@ static void modify_scal_force_h(Hier& H, int comp, const char* s0_edge, int s0ca
 // p0_old, which_step 2 their old/new averages (:493-499)
 static void make_rhoh_force_h(Hier& H, int is_prediction, int add_thermal, int which_step) {
     const char* p0n = which_step == 1 ? "p0_old" : "p0_avg";
-    put1d_h(H, F_P0CART, p0n, 0, 1, 0, BCS_F, 0, 0, -1);
-    if (H[0].sph) make_s0mac_h(H, p0n, F_S0MAC0);  // p0mac (Source/MaestroForce.cpp:526-530)
-    put1d_h(H, F_PSICART, "psi", 0, 1, 0, BCS_F, 0, 0, -1);
-    put1d_h(H, F_RHO0CART, which_step == 1 ? "rho0_old" : "rho0_avg", 0, 1, 0, BCS_S, RHO, 0, RHO);
+    std::vector<Put1d> list{{F_P0CART, p0n, 0, 1, 0, BCS_F, 0, 0, -1},
+                            {F_PSICART, "psi", 0, 1, 0, BCS_F, 0, 0, -1},
+                            {F_RHO0CART, which_step == 1 ? "rho0_old" : "rho0_avg", 0, 1, 0, BCS_S, RHO, 0, RHO}};
     // the planar force's gravity (MakeGravCell); the spherical force does not read it
-    if (!H[0].sph) put1d_h(H, F_GRAVCART, "grav_cell", H[0].ndim - 1, H[0].ndim, 0, BCS_F, 0, 0, -1);
+    if (!H[0].sph) list.push_back({F_GRAVCART, "grav_cell", H[0].ndim - 1, H[0].ndim, 0, BCS_F, 0, 0, -1});
+    put1d_h(H, list);
+    if (H[0].sph) make_s0mac_h(H, p0n, F_S0MAC0);  // p0mac (Source/MaestroForce.cpp:526-530)
     for (auto* c : H.L) make_rhoh_force(*c, is_prediction, add_thermal);
     average_down_h(H, F_SCALFORCE, RHOH, 1);
     fill_patch_h(H, F_SCALFORCE, RHOH, 1, BCS_F, 0, 0, RHOH);
@@ -582,6 +659,22 @@ static void convert_rhox_to_x_h(Hier& H, int flag) {
     average_down_h(H, F_SOLD, FIRSTSPEC, ns);
     if (flag) fill_patch_h(H, F_SOLD, FIRSTSPEC, ns, BCS_F, 0, 0, FIRSTSPEC);
     else fill_patch_h(H, F_SOLD, FIRSTSPEC, ns, BCS_S, FIRSTSPEC, 0, FIRSTSPEC);
+}
+
+// ConvertRhoXToX with the density's PutInPertForm: before the prediction (flag) X = (rho X) / rho and
+// then rho' = rho - rho0; after it rho back and then rho X.  One planar level does both, and
+// fills both, in one pass.
+static void to_prediction_form_h(Hier& H, int flag, bool pert) {
+    if (pert && H.n() == 1 && !H[0].sph) {
+        Ctx& c = H[0];
+        convert_rhox_to_x(c, flag, FIRSTSPEC, c.nspec, c.b1("rho0_old"));
+        if (flag) fill_patch(c, F_SOLD, {FIRSTSPEC, c.nspec, BCS_F, 0}, {RHO, 1, BCS_F, 0});
+        else fill_patch(c, F_SOLD, {FIRSTSPEC, c.nspec, BCS_S, FIRSTSPEC}, {RHO, 1, BCS_S, RHO});
+        return;
+    }
+    if (flag) convert_rhox_to_x_h(H, 1);
+    if (pert) put_in_pert_form_h(H, "rho0_old", RHO, flag ? 0 : RHO, flag ? BCS_F : BCS_S, flag);
+    if (!flag) convert_rhox_to_x_h(H, 0);
 }
 
 // Maestro::UpdateScal (Source/MaestroAdvection.cpp:86-297): the update on every level, then
@@ -609,9 +702,8 @@ static void update_scal_sync_h(Hier& H, int start_comp) {
     } else {
         const int ns = H[0].nspec;
         average_down_h(H, F_SNEW, FIRSTSPEC, ns);
-        fill_patch_h(H, F_SNEW, FIRSTSPEC, ns, BCS_S, FIRSTSPEC, 0, FIRSTSPEC);
         average_down_h(H, F_SNEW, RHO, 1);
-        fill_patch_h(H, F_SNEW, RHO, 1, BCS_S, RHO, 0, RHO);
+        fill_patch_h(H, F_SNEW, {FIRSTSPEC, ns, BCS_S, FIRSTSPEC}, {RHO, 1, BCS_S, RHO});
     }
 }
 
@@ -671,8 +763,8 @@ static void density_advance_streamed(Hier& H, int which_step) {
     for (auto* c : H.L) set_val(*c, F_SCALFORCE, 0.0, 0, nscal, c->F[F_SCALFORCE].spec.ng);
     put1d_h(H, F_RHO0CART, "rho0_old", 0, 1, 0, BCS_S, RHO, 0, RHO);
     addw0_h(H, F_UMAC0, -1.0);
-    if (spt == 1) modify_scal_force_h(H, RHO, "rho0_edge_old", F_RHO0CART, 0);
-    else if (spt == 3) modify_scal_force_h(H, RHO, "rho0_edge_old", F_RHO0CART, 1);
+    if (spt == 1) modify_scal_force_h(H, RHO, nullptr, "rho0_edge_old", F_RHO0CART, 0);
+    else if (spt == 3) modify_scal_force_h(H, RHO, nullptr, "rho0_edge_old", F_RHO0CART, 1);
     addw0_h(H, F_UMAC0, 1.0);
     if (spt == 1 || spt == 3) convert_rhox_to_x_h(H, 1);
     if (spt == 1) put_in_pert_form_h(H, "rho0_old", RHO, 0, BCS_F, 1);
@@ -717,18 +809,16 @@ static void density_advance(Hier& H, int which_step, bool stream = false) {
     for (auto* c : H.L) set_val(*c, F_SCALFORCE, 0.0, 0, nscal, c->F[F_SCALFORCE].spec.ng);
     put1d_h(H, F_RHO0CART, "rho0_old", 0, 1, 0, BCS_S, RHO, 0, RHO);
     addw0_h(H, F_UMAC0, -1.0);
-    if (spt == 1) modify_scal_force_h(H, RHO, "rho0_edge_old", F_RHO0CART, 0);
-    else if (spt == 3) modify_scal_force_h(H, RHO, "rho0_edge_old", F_RHO0CART, 1);
+    if (spt == 1) modify_scal_force_h(H, RHO, nullptr, "rho0_edge_old", F_RHO0CART, 0);
+    else if (spt == 3) modify_scal_force_h(H, RHO, nullptr, "rho0_edge_old", F_RHO0CART, 1);
     addw0_h(H, F_UMAC0, 1.0);
-    if (spt == 1 || spt == 3) convert_rhox_to_x_h(H, 1);
-    if (spt == 1) put_in_pert_form_h(H, "rho0_old", RHO, 0, BCS_F, 1);
+    if (spt == 1 || spt == 3) to_prediction_form_h(H, 1, spt == 1);
     for (auto* c : H.L) make_edge_scal(*c, FIRSTSPEC, ns, BCS_S, spt == 2, 1);  // no force for X / rho X
-    if (spt == 1 || spt == 3)
-        for (auto* c : H.L) make_edge_scal(*c, RHO, 1, BCS_S, 0, 0);
+    if (spt == 1 || spt == 3)  // the same velocities: their coefficients are there
+        for (auto* c : H.L) make_edge_scal(*c, RHO, 1, BCS_S, 0, 0, 0, -1, false);
     else
         for (auto* c : H.L) sum_species_edges(*c);
-    if (spt == 1) put_in_pert_form_h(H, "rho0_old", RHO, RHO, BCS_S, 0);
-    if (spt == 1 || spt == 3) convert_rhox_to_x_h(H, 0);
+    if (spt == 1 || spt == 3) to_prediction_form_h(H, 0, spt == 1);
     const char* r0n = which_step == 1 ? "rho0_old" : "rho0_new";
     const char* r0en = which_step == 1 ? "rho0_edge_old" : "rho0_edge_new";
     if (H[0].sph) {  // rho0 on faces (Source/MaestroDensityAdvance.cpp:167-213)
@@ -792,8 +882,7 @@ static void enthalpy_advance(Hier& H, int which_step, bool stream = false) {
     addw0_h(H, F_UMAC0, -1.0);
     make_rhoh_force_h(H, 1, 1, 1);
     if (ept == 1) {
-        put1d_h(H, F_RHOH0CART, "rhoh0_old", 0, 1, 0, BCS_S, RHOH, 0, RHOH);
-        modify_scal_force_h(H, RHOH, "rhoh0_edge_old", F_RHOH0CART, 0);
+        modify_scal_force_h(H, RHOH, "rhoh0_old", "rhoh0_edge_old", F_RHOH0CART, 0);
     }
     if (ept == 2)  // the force of h: the (rho h) force over rho (:80-88)
         for (auto* c : H.L) h_force(*c);
@@ -1047,7 +1136,22 @@ static void stage_body(Hier& H, const std::vector<StageIO>& io) {
     for (int l = 0; l < H.n(); ++l) {
         Ctx& c = H[l];
         if (!c.dry) cudaMemsetAsync(c.d_flag, 0, sizeof(int), c.stream);
-        set_val(c, F_UTILDE, 0.0, 0, 3, c.ng_adv);
+        const int al = io[l].alias;
+        std::vector<ZeroJob> z{{F_UTILDE, 0, 3, c.ng_adv}, {F_THERMAL, 0, 1, 1}, {F_ETA, 0, 1, 0}};
+        if (!io[l].gpi) z.push_back({F_GPI, 0, 3, 0});
+        if (!(al & AL_SNEW)) z.push_back({F_SNEW, 0, c.nscal, c.ng_s});
+        for (int d = 0; d < 3; ++d) {
+            z.push_back({F_UMAC0 + d, 0, 1, 1});
+            // (Source/MaestroAdvance.cpp:190-191); streamed: the three slots; in a caller's FAB only
+            // Temp and Pi are not overwritten by the stage
+            const bool st = al & AL_STREAM;
+            for (int f : {F_SEDGE0 + d, F_SFLUX0 + d}) {
+                const bool own = al & (f < F_SFLUX0 ? AL_SEDGE : AL_SFLUX);
+                if (!st && own) z.push_back({f, TEMP, 2, 0});
+                else z.push_back({f, 0, st ? 3 : c.nscal, 0});
+            }
+        }
+        set_zeros(c, z);
         copy_fab(c, F_UTILDE, 0, F_USER + U_UOLD, 0, c.ndim, 0);
         if (!(io[l].alias & AL_SOLD)) copy_fab(c, F_SOLD, 0, F_USER + U_SOLD, 0, c.nscal, 0);
     }
@@ -1055,26 +1159,7 @@ static void stage_body(Hier& H, const std::vector<StageIO>& io) {
     for (int l = 0; l < H.n(); ++l) {
         Ctx& c = H[l];
         if (io[l].gpi) copy_fab(c, F_GPI, 0, F_USER + U_GPI, 0, c.ndim, 0);
-        else set_val(c, F_GPI, 0.0, 0, 3, 0);
-        set_val(c, F_THERMAL, 0.0, 0, 1, 1);
         if (io[l].thermal) copy_fab(c, F_THERMAL, 0, F_USER + U_THERMAL, 0, 1, 0);
-        const int al = io[l].alias;
-        if (!(al & AL_SNEW)) set_val(c, F_SNEW, 0.0, 0, c.nscal, c.ng_s);
-        for (int d = 0; d < 3; ++d) {
-            set_val(c, F_UMAC0 + d, 0.0, 0, 1, 1);
-            if (al & AL_STREAM) {  // the three slots
-                set_val(c, F_SEDGE0 + d, 0.0, 0, 3, 0);
-                set_val(c, F_SFLUX0 + d, 0.0, 0, 3, 0);
-                continue;
-            }
-            // (Source/MaestroAdvance.cpp:190-191); in a caller's FAB only Temp and Pi are not
-            // overwritten by the stage
-            if (al & AL_SEDGE) set_val(c, F_SEDGE0 + d, 0.0, TEMP, 2, 0);
-            else set_val(c, F_SEDGE0 + d, 0.0, 0, c.nscal, 0);
-            if (al & AL_SFLUX) set_val(c, F_SFLUX0 + d, 0.0, TEMP, 2, 0);
-            else set_val(c, F_SFLUX0 + d, 0.0, 0, c.nscal, 0);
-        }
-        set_val(c, F_ETA, 0.0, 0, 1, 0);
     }
     w0_carts(H);
     // STEP 3 and STEP 4 of Maestro::AdvanceTimeStep (Source/MaestroAdvance.cpp:359-548)
@@ -1327,6 +1412,7 @@ static int layout_level(Ctx& c, int nboxes, const madv_box* boxes, bool cover) {
         set_error("level 0 must cover the domain");
         return MADV_ERR_LAYOUT;
     }
+    c.covers = vol == dvol;
     c.nb = nboxes;
     try {
         for (int f = 0; f < NF_INTERNAL; ++f) {

@@ -105,7 +105,7 @@ struct CopyDesc {
     int lo[3];
     int n[3];
     int shift[3];
-    int pad;
+    int df;  // tables of several fields: which
     long start;
     PieceDiv dv;
 };
@@ -151,6 +151,7 @@ struct Ctx {
     int nspec = 0, nscal = 0, ng_s = 3, ng_adv = 3, nr = 0;
     bool per[3] = {false, false, false};
     std::vector<HBox> ba;
+    bool covers = false;  // the boxes cover the domain
     int nb = 0;
     bool have_layout = false, have_base = false;
     BCRecD bcs_s[MAX_SCAL], bcs_u[3], bcs_f[MAX_SCAL];
@@ -167,6 +168,7 @@ struct Ctx {
     FabView* dviews_alias = nullptr;
     FabView* hviews_alias = nullptr;
     std::map<std::array<int, 8>, RegionTable> regions;
+    std::map<std::vector<int>, RegionTable> unions;  // region_union
     std::map<std::array<int, 3>, CopyTable> copies;
     cudaStream_t stream = nullptr;
     int per_box = 0;      // launch mode: 0 batched, 1 one launch per box
@@ -258,6 +260,11 @@ struct Hier {
 const RegionTable& region(Ctx& c, int glo0, int glo1, int glo2, int ghi0, int ghi1, int ghi2,
                           int nodal = -1, int slab = -1);
 const CopyTable& copy_table(Ctx& c, int ng, int nodal);
+const CopyTable& copy_table_faces(Ctx& c, int ng);  // the three face directions' tables end to end
+// Regions (arguments of region()) laid end to end in one table, so that one launch covers all of
+// them; a piece's pad is the place of its region in the list.
+typedef std::array<int, 8> RegionKey;
+const RegionTable& region_union(Ctx& c, const std::vector<RegionKey>& parts);
 
 void set_error(const std::string& s);
 bool cuda_ok(cudaError_t e, const char* what);
@@ -289,6 +296,25 @@ void set_val(Ctx& c, int fid, double v, int c0, int nc, int ngrow);
 void copy_fab(Ctx& c, int dst, int dc0, int src, int sc0, int nc, int ngrow);
 void add_fab(Ctx& c, int dst, int src, int nc, int ngrow);
 void put1d(Ctx& c, int fid, const double* d_s0, int outcomp, int edge, int vec = 0);
+// FillPatch of two component ranges of a field on one level
+struct FillRange {
+    int c0, nc, which_bcs, bc_c0;
+};
+void fill_patch(Ctx& c, int fid, const FillRange& a, const FillRange& b);
+// setVal(0) of several fields
+struct ZeroJob {
+    int f, c0, nc, ng;
+};
+void set_zeros(Ctx& c, const std::vector<ZeroJob>& jobs);
+// Put1dArrayOnCart of several arrays with the ghost cells FillPatch gives them (a planar level
+// that covers the domain)
+struct Put1dJob {
+    int f;
+    const double* s0;
+    int outcomp, nc, edge, which_bcs, bc_c0;
+};
+bool put1d_fills(const Ctx& c);
+void put1d_filled(Ctx& c, const std::vector<Put1dJob>& jobs);
 void make_utrans(Ctx& c);
 // valid cells; face velocity fe .. fe+2; F_GRAVCART / F_RHO0CART filled by the caller
 void make_vel_force(Ctx& c, int fe = F_UTRANS0);
@@ -302,7 +328,8 @@ void edge_scal_setup(Ctx& c, int is_conservative);
 void modify_scal_force(Ctx& c, int comp, int s0cart_fid, int fullform);
 void make_rhoh_force(Ctx& c, int is_prediction, int add_thermal);
 void put_in_pert_form(Ctx& c, const double* d_s0, int comp, int flag);
-void convert_rhox_to_x(Ctx& c, int flag, int c0 = FIRSTSPEC, int nc = -1);  // nc -1: every species
+// s0: the density is put in perturbational form over it too (planar)
+void convert_rhox_to_x(Ctx& c, int flag, int c0 = FIRSTSPEC, int nc = -1, const double* s0 = nullptr);  // nc -1: every species
 // species c0 .. c0+nc-1 (nc -1: every species); slot >= 0: their edge state and flux in component
 // `slot` of F_SEDGE* / F_SFLUX* (one species per call), the Rho flux and etarhoflux accumulated
 void make_rhox_flux(Ctx& c, const double* r0_old, const double* r0e_old, const double* r0_new,

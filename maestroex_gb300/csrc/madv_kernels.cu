@@ -54,6 +54,34 @@ void add_fab(Ctx& c, int dst, int src, int nc, int ngrow) {
     launch(c, rg_grow(c, ngrow, nodal_of(c, dst)), 1, k_copy, c.V(), dst, 0, src, 0, nc, 1);
 }
 
+// setVal(0) of up to ZERO_JOBS fields in one launch (the stage's start clears 13; a small level's
+// launch takes 2.7 us, whatever it clears)
+static constexpr int ZERO_JOBS = 16;
+struct ZeroArgs {
+    int f[ZERO_JOBS], c0[ZERO_JOBS], nc[ZERO_JOBS];
+};
+__global__ void k_set_zeros(KARGS, const __grid_constant__ ZeroArgs z) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    const int q = R[e_].pad;
+    const FabView a = VW(z.f[q]);
+    for (int n = z.c0[q]; n < z.c0[q] + z.nc[q]; ++n) at(a, i, j, k, n) = 0.0;
+}
+
+void set_zeros(Ctx& c, const std::vector<ZeroJob>& jobs) {
+    for (size_t q0 = 0; q0 < jobs.size(); q0 += ZERO_JOBS) {
+        ZeroArgs z{};
+        std::vector<RegionKey> parts;
+        for (size_t q = q0; q < std::min(jobs.size(), q0 + ZERO_JOBS); ++q) {
+            const ZeroJob& w = jobs[q];
+            z.f[q - q0] = w.f;
+            z.c0[q - q0] = w.c0;
+            z.nc[q - q0] = w.nc;
+            parts.push_back({w.ng, w.ng, w.ng, w.ng, w.ng, w.ng, c.F[w.f].spec.nodal, -1});
+        }
+        launch(c, region_union(c, parts), 1, k_set_zeros, c.V(), z);
+    }
+}
+
 // Put1dArrayOnCart, planar (Source/MaestroFill3dData.cpp:79-93): valid cells only.
 __global__ void k_put1d(KARGS, int f, const double* __restrict__ s0, int outcomp, int edge) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
@@ -67,9 +95,98 @@ void put1d(Ctx& c, int fid, const double* d_s0, int outcomp, int edge, int vec) 
     launch(c, rg_grow(c, 0), 1, k_put1d, c.V(), fid, d_s0, outcomp, edge);
 }
 
+// One side's rule of phys_fill on its first ghost cell (first) or farther out, from A(q): the
+// value q cells inside the domain, which is ext cells long; refl: the cell's mirror image.
+template <typename A>
+__device__ __forceinline__ double phys_value(int t, bool first, int ext, int refl, A at_in) {
+    if (t == BC_FOEXTRAP || (t == BC_HOEXTRAP && !first)) return at_in(0);
+    if (t == BC_HOEXTRAP) {
+        if (ext >= 3) return 0.125 * (15. * at_in(0) - 10. * at_in(1) + 3. * at_in(2));
+        return half(3. * at_in(0) - at_in(1));
+    }
+    if (t == BC_REFLECT_EVEN) return at_in(refl);
+    if (t == BC_REFLECT_ODD) return -at_in(refl);
+    return 0.0;  // ext_dir of a velocity
+}
+
+// setVal(0), Put1dArrayOnCart and FillPatch of up to PUT1D_JOBS arrays in one launch on a planar
+// level that covers its domain: the field depends on the radial index alone, so every ghost
+// cell's value follows from its place -- wrapped along periodic directions, the boundary rules of
+// x, y, z in FillPatch's order elsewhere.  (Four launches an array otherwise, each 2.7 us on a
+// small level: the stage puts 16 arrays on the cells.)
+static constexpr int PUT1D_JOBS = 4;
+struct Put1dArgs {
+    struct {
+        const double* s0;
+        const BCRecD* bcs;
+        int f, outcomp, nc, edge;
+    } w[PUT1D_JOBS];
+    int lo[3], hi[3], per[3];
+};
+template <int ND>
+__global__ void k_put1d_filled(KARGS, const __grid_constant__ Put1dArgs a) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    const auto& w = a.w[R[e_].pad];
+    const FabView out = VW(w.f);
+    const int idx[3] = {i, j, k};
+    constexpr int RD = ND - 1;
+    for (int n = 0; n < w.nc; ++n) {
+        const BCRecD bc = w.bcs[n];
+        // the value over the radial index r at this (i, j): the array, then the rules across it
+        auto level = [&](int r) -> double {
+            double v = n != w.outcomp ? 0.0 : (w.edge ? half(w.s0[r] + w.s0[r + 1]) : w.s0[r]);
+#pragma unroll
+            for (int d = 0; d < RD; ++d) {
+                const int m = idx[d];
+                if (a.per[d] || (m >= a.lo[d] && m <= a.hi[d])) continue;
+                const bool below = m < a.lo[d];
+                const double g = v;
+                v = phys_value(below ? bc.lo[d] : bc.hi[d], m == (below ? a.lo[d] - 1 : a.hi[d] + 1),
+                               a.hi[d] - a.lo[d] + 1, 0, [&](int) { return g; });
+            }
+            return v;
+        };
+        const int m = idx[RD], lo = a.lo[RD], hi = a.hi[RD], ext = hi - lo + 1;
+        double v;
+        if (m >= lo && m <= hi) v = level(m);
+        else if (a.per[RD]) v = level(m < lo ? m + ext : m - ext);
+        else if (m < lo) v = phys_value(bc.lo[RD], m == lo - 1, ext, lo - 1 - m, [&](int q) { return level(lo + q); });
+        else v = phys_value(bc.hi[RD], m == hi + 1, ext, m - hi - 1, [&](int q) { return level(hi - q); });
+        at(out, i, j, k, n) = v;
+    }
+}
+
+// (A domain is at least 8 cells long, longer than any ghost layer and HOEXTRAP's three cells.)
+bool put1d_fills(const Ctx& c) { return !c.sph && c.covers && !c.per_box; }
+
+void put1d_filled(Ctx& c, const std::vector<Put1dJob>& jobs) {
+    for (size_t q0 = 0; q0 < jobs.size(); q0 += PUT1D_JOBS) {
+        Put1dArgs a{};
+        std::vector<RegionKey> parts;
+        for (size_t q = q0; q < std::min(jobs.size(), q0 + PUT1D_JOBS); ++q) {
+            const Put1dJob& w = jobs[q];
+            auto& o = a.w[q - q0];
+            o.s0 = w.s0;
+            o.bcs = bcs_dev(c, w.which_bcs) + w.bc_c0;
+            o.f = w.f;
+            o.outcomp = w.outcomp;
+            o.nc = w.nc;
+            o.edge = w.edge;
+            const int g = c.F[w.f].spec.ng;
+            parts.push_back({g, g, g, g, g, g, -1, -1});
+        }
+        for (int d = 0; d < 3; ++d) {
+            a.lo[d] = c.P.dom_lo[d];
+            a.hi[d] = c.P.dom_hi[d];
+            a.per[d] = c.per[d];
+        }
+        launch(c, region_union(c, parts), 1, c.ndim == 2 ? k_put1d_filled<2> : k_put1d_filled<3>, c.V(), a);
+    }
+}
+
 // ============================================================ ghost fills
 __global__ void k_fill_boundary(const CopyDesc* __restrict__ D, int nd, long total, const FabView* __restrict__ V,
-                                int nb, int f, int c0, int nc) {
+                                int nb, int f, int c0, int nc, int c1, int nc1) {
     MADV_LET_NEXT();
     const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= total) return;
@@ -77,83 +194,70 @@ __global__ void k_fill_boundary(const CopyDesc* __restrict__ D, int nd, long tot
     int i, j, k;
     piece_ijk(cd.lo, cd.n, cd.dv, gid - cd.start, i, j, k);
     MADV_WAIT();
-    const FabView dst = V[f * nb + cd.dst_b];
-    const FabView src = V[f * nb + cd.src_b];
-    for (int n = c0; n < c0 + nc; ++n)
+    const FabView dst = V[(f + cd.df) * nb + cd.dst_b];
+    const FabView src = V[(f + cd.df) * nb + cd.src_b];
+    for (int q = 0; q < nc + nc1; ++q) {
+        const int n = q < nc ? c0 + q : c1 + q - nc;
         at(dst, i, j, k, n) = at(src, i - cd.shift[0], j - cd.shift[1], k - cd.shift[2], n);
+    }
 }
 
-void fill_boundary(Ctx& c, int fid, int c0, int nc) {
-    const FieldSpec& s = c.F[fid].spec;
-    const CopyTable& ct = copy_table(c, s.ng, s.nodal);
+static void copy_pieces(Ctx& c, const CopyTable& ct, int fid, int c0, int nc, int c1, int nc1) {
     if (ct.total == 0 || c.dry) return;
     unsigned grid = (unsigned)((ct.total + TPB - 1) / TPB);
     launch_next(c, grid, TPB, k_fill_boundary, (const CopyDesc*)ct.d, (int)ct.h.size(), ct.total, c.V(), c.nb, fid,
-                c0, nc);
+                c0, nc, c1, nc1);
     c.launches++;
+}
+void fill_boundary(Ctx& c, int fid, int c0, int nc) {
+    const FieldSpec& s = c.F[fid].spec;
+    copy_pieces(c, copy_table(c, s.ng, s.nodal), fid, c0, nc, 0, 0);
 }
 
 // Physical-boundary fill of direction d (both sides) for a cell-centred field.  The
 // definitions of the BC types match the oracle's restatement of fab_filcc (foextrap,
 // hoextrap = quadratic face extrapolation in the first ghost, reflect_even/odd,
 // ext_dir = 0 for velocities).
-__global__ void k_phys_fill(KARGS, int f, int c0, int nc, const BCRecD* __restrict__ bcs, int bc_c0, int is_vel,
-                            int state_c0, int d, int domlo, int domhi) {
+// (Two component ranges, c0 .. with bcs and c1 .. with bcs1; the second may be empty.)
+__global__ void k_phys_fill(KARGS, int f, int c0, int nc, const BCRecD* __restrict__ bcs, int c1, int nc1,
+                            const BCRecD* __restrict__ bcs1, int d, int domlo, int domhi) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView q = VW(f);
-    const int idx[3] = {i, j, k};
-    const int m = idx[d];
-    const int side = m < domlo ? 0 : 1;
-    auto A = [&](int p, int n) -> double {
-        int i2 = i, j2 = j, k2 = k;
-        if (d == 0) i2 = p;
-        else if (d == 1) j2 = p;
-        else k2 = p;
-        return at(q, i2, j2, k2, n);
-    };
-    for (int n = c0; n < c0 + nc; ++n) {
-        const BCRecD bc = bcs[bc_c0 + n - c0];
-        const int t = side == 0 ? bc.lo[d] : bc.hi[d];
-        double v;
+    const int m = d == 0 ? i : (d == 1 ? j : k);
+    const bool below = m < domlo;
+    const int refl = below ? domlo - 1 - m : m - domhi - 1;
+    const long st = d == 0 ? 1 : (d == 1 ? q.sj : q.sk), in = below ? st : -st;
+    for (int p = 0; p < nc + nc1; ++p) {
+        const int n = p < nc ? c0 + p : c1 + p - nc;
+        const BCRecD& bc = p < nc ? bcs[p] : bcs1[p - nc];
+        const int t = below ? bc.lo[d] : bc.hi[d];
         if (t == BC_INT_DIR) continue;
-        if (t == BC_FOEXTRAP) {
-            v = A(side == 0 ? domlo : domhi, n);
-        } else if (t == BC_HOEXTRAP) {
-            if (side == 0) {
-                if (m < domlo - 1) v = A(domlo, n);
-                else if (domlo + 2 <= domhi) v = 0.125 * (15. * A(domlo, n) - 10. * A(domlo + 1, n) + 3. * A(domlo + 2, n));
-                else v = half(3. * A(domlo, n) - A(domlo + 1, n));
-            } else {
-                if (m > domhi + 1) v = A(domhi, n);
-                else if (domhi - 2 >= domlo) v = 0.125 * (15. * A(domhi, n) - 10. * A(domhi - 1, n) + 3. * A(domhi - 2, n));
-                else v = half(3. * A(domhi, n) - A(domhi - 1, n));
-            }
-        } else if (t == BC_REFLECT_EVEN) {
-            v = A(side == 0 ? 2 * domlo - 1 - m : 2 * domhi + 1 - m, n);
-        } else if (t == BC_REFLECT_ODD) {
-            v = -A(side == 0 ? 2 * domlo - 1 - m : 2 * domhi + 1 - m, n);
-        } else {  // ext_dir: zero for velocities and Pi; scalars are rejected on the host
-            v = 0.0;
-        }
-        (void)is_vel;
-        (void)state_c0;
-        at(q, i, j, k, n) = v;
+        double* const o = &at(q, i, j, k, n);
+        const double* const edge = o + (refl + 1) * in;  // the domain's cell next to the boundary
+        *o = phys_value(t, refl == 0, domhi - domlo + 1, refl, [&](int w) { return edge[w * in]; });
     }
 }
 
-void phys_fill(Ctx& c, int fid, int c0, int nc, const BCRecD* bcs_d, int bc_c0, int is_vel, int state_c0) {
+static void phys_ranges(Ctx& c, int fid, int c0, int nc, const BCRecD* bcs, int c1, int nc1, const BCRecD* bcs1) {
     const FieldSpec& s = c.F[fid].spec;
     for (int d = 0; d < 3; ++d) {
         if (c.per[d]) continue;
         const RegionTable& rt = region(c, s.ng, s.ng, s.ng, s.ng, s.ng, s.ng, s.nodal, d);
-        launch(c, rt, 1, k_phys_fill, c.V(), fid, c0, nc, bcs_d, bc_c0, is_vel, state_c0, d, c.P.dom_lo[d],
-               c.P.dom_hi[d]);
+        launch(c, rt, 1, k_phys_fill, c.V(), fid, c0, nc, bcs, c1, nc1, bcs1, d, c.P.dom_lo[d], c.P.dom_hi[d]);
     }
+}
+void phys_fill(Ctx& c, int fid, int c0, int nc, const BCRecD* bcs_d, int bc_c0, int, int) {
+    phys_ranges(c, fid, c0, nc, bcs_d + bc_c0, 0, 0, nullptr);
 }
 
 void fill_patch(Ctx& c, int fid, int c0, int nc, int which_bcs, int bc_c0, int is_vel, int state_c0) {
     fill_boundary(c, fid, c0, nc);
     phys_fill(c, fid, c0, nc, bcs_dev(c, which_bcs), bc_c0, is_vel, state_c0);
+}
+void fill_patch(Ctx& c, int fid, const FillRange& a, const FillRange& b) {
+    const FieldSpec& s = c.F[fid].spec;
+    copy_pieces(c, copy_table(c, s.ng, s.nodal), fid, a.c0, a.nc, b.c0, b.nc);
+    phys_ranges(c, fid, a.c0, a.nc, bcs_dev(c, a.which_bcs) + a.bc_c0, b.c0, b.nc, bcs_dev(c, b.which_bcs) + b.bc_c0);
 }
 
 // FillUmacGhost (Source/MaestroFillData.cpp:176-453): ghost faces behind physical
@@ -216,7 +320,7 @@ __global__ void k_umac_ghost(KARGS, int f0, int dd, int bclo, int bchi, int dlo,
 }
 
 void fill_face_ghosts(Ctx& c, int f0) {
-    for (int d = 0; d < 3; ++d) fill_boundary(c, f0 + d, 0, 1);
+    copy_pieces(c, copy_table_faces(c, c.F[f0].spec.ng), f0, 0, 1, 0, 0);
     for (int dd = 0; dd < 3; ++dd) {
         if (c.per[dd]) continue;
         const RegionTable& rt = region(c, 1, 1, 1, 1, 1, 1, dd);
@@ -258,12 +362,10 @@ __global__ void k_ppm_face(KARGS, int fs, int sc, int ff, int lo_ext, int hi_ext
 // formed once per velocity field and direction and shared by every traced component
 // (the reference forms them per component, cell and direction).
 // Face-centred velocity (the is_umac case): one (A, B) per D-face.
-template <int D>
-__global__ void k_trace_face(KARGS, int fu, int fout, double dt, RecipC rdx) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void trace_face(const FabView& u, const FabView& o, double dt, const RecipC& rdx, int i,
+                                           int j, int k) {
     double A, B;
-    trace_coeffs(at(VW(fu), i, j, k), dt, rdx, A, B);
-    const FabView o = VW(fout);
+    trace_coeffs(at(u, i, j, k), dt, rdx, A, B);
     at(o, i, j, k, 0) = A;
     at(o, i, j, k, 1) = B;
 }
@@ -396,14 +498,6 @@ void ppm_faces(Ctx& c, int d, int fs, int sc, int faces) {
     else one(std::integral_constant<int, 2>{});
 }
 
-// tracing coefficients of the face velocity fields umac0..2 (or utrans0..2)
-static void trace_coeffs_faces(Ctx& c, int fu0) {
-    // faces lo-1 .. hi+2 along d, cells lo-1 .. hi+1 across
-    launch(c, region(c, 1, 1, 1, 1, 1, 1, 0), 1, k_trace_face<0>, c.V(), fu0, F_TRA0, c.P.dt, make_recip(c.P.dx[0]));
-    launch(c, region(c, 1, 1, 1, 1, 1, 1, 1), 1, k_trace_face<1>, c.V(), fu0 + 1, F_TRA1, c.P.dt, make_recip(c.P.dx[1]));
-    launch(c, region(c, 1, 1, 1, 1, 1, 1, 2), 1, k_trace_face<2>, c.V(), fu0 + 2, F_TRA2, c.P.dt, make_recip(c.P.dx[2]));
-}
-
 static void slope_any(Ctx& c, int d, int fs, int sc, int fout, int oc, int ncomp, const BCRecD* bcs_d, int bc_c0) {
     const RegionTable& rc = rg_grow(c, 1);
     const int lo = c.P.dom_lo[d], hi = c.P.dom_hi[d], so = c.P.slope_order;
@@ -420,31 +514,79 @@ static void slope_any(Ctx& c, int d, int fs, int sc, int fout, int oc, int ncomp
 // dt/4.  These are the leading products of the reference's transverse expressions, e.g.
 // (dt6/hy)*(vmac(i,j+1,k)+vmac(i,j,k)) (Source/MaestroMakeEdgeScalars.cpp:920-927,
 // Source/MaestroVelPred.cpp:1166-1172), so forming them once keeps every result bitwise.
-__global__ void k_transverse_coeffs(KARGS, int fu0, double dt6h0, double dt6h1, double dt6h2, double dt4h0,
-                                    double dt4h1, double dt4h2) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+struct EdgeCoefs {
+    double dt;
+    RecipC r[3];
+    double dt6h[3], dt4h[3];
+};
+__device__ __forceinline__ void transverse_coeffs_cell(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+                                                       int fu0, const EdgeCoefs& e) {
     const FabView o = VW(F_TCOEF);
     const FabView u0 = VW(fu0), u1 = VW(fu0 + 1), u2 = VW(fu0 + 2);
     const double s0 = at(u0, i + 1, j, k) + at(u0, i, j, k);
     const double s1 = at(u1, i, j + 1, k) + at(u1, i, j, k);
     const double s2 = at(u2, i, j, k + 1) + at(u2, i, j, k);
-    at(o, i, j, k, 0) = dt6h0 * s0;
-    at(o, i, j, k, 1) = dt6h1 * s1;
-    at(o, i, j, k, 2) = dt6h2 * s2;
-    at(o, i, j, k, 3) = dt4h0 * s0;
-    at(o, i, j, k, 4) = dt4h1 * s1;
-    at(o, i, j, k, 5) = dt4h2 * s2;
+    at(o, i, j, k, 0) = e.dt6h[0] * s0;
+    at(o, i, j, k, 1) = e.dt6h[1] * s1;
+    at(o, i, j, k, 2) = e.dt6h[2] * s2;
+    at(o, i, j, k, 3) = e.dt4h[0] * s0;
+    at(o, i, j, k, 4) = e.dt4h[1] * s1;
+    at(o, i, j, k, 5) = e.dt4h[2] * s2;
+}
+// parts 0 .. 2: the tracing coefficients on the faces of a direction, 3: the transverse ones on
+// the cells (first: the first part of this launch's regions)
+__global__ void k_edge_coeffs(KARGS, int fu0, const __grid_constant__ EdgeCoefs e, int first) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    switch (first + R[e_].pad) {
+        case 0: trace_face(VW(fu0), VW(F_TRA0), e.dt, e.r[0], i, j, k); break;
+        case 1: trace_face(VW(fu0 + 1), VW(F_TRA1), e.dt, e.r[1], i, j, k); break;
+        case 2: trace_face(VW(fu0 + 2), VW(F_TRA2), e.dt, e.r[2], i, j, k); break;
+        default: transverse_coeffs_cell(V, nb, b, i, j, k, fu0, e);
+    }
 }
 
-static void transverse_coeffs(Ctx& c, int fu0) {
+static void edge_coeffs(Ctx& c, int fu0, bool trace, bool transverse) {
+    EdgeCoefs e{};
+    e.dt = c.P.dt;
     const double dt6 = c.P.dt / 6.0, dt4 = 0.25 * c.P.dt;
-    launch(c, rg_grow(c, 1), 1, k_transverse_coeffs, c.V(), fu0, dt6 / c.P.dx[0], dt6 / c.P.dx[1], dt6 / c.P.dx[2],
-           dt4 / c.P.dx[0], dt4 / c.P.dx[1], dt4 / c.P.dx[2]);
+    std::vector<RegionKey> parts;
+    for (int d = 0; d < c.ndim; ++d) {
+        e.r[d] = make_recip(c.P.dx[d]);
+        e.dt6h[d] = dt6 / c.P.dx[d];
+        e.dt4h[d] = dt4 / c.P.dx[d];
+        // faces lo-1 .. hi+2 along d, cells lo-1 .. hi+1 across
+        if (trace) parts.push_back({1, 1, 1, 1, 1, 1, d, -1});
+    }
+    if (transverse) parts.push_back({1, 1, 1, 1, 1, 1, -1, -1});
+    if (!parts.empty()) launch(c, region_union(c, parts), 1, k_edge_coeffs, c.V(), fu0, e, trace ? 0 : 3);
 }
 
-void edge_scal_coeffs(Ctx& c) {
-    trace_coeffs_faces(c, F_UMAC0);
-    transverse_coeffs(c, F_UMAC0);
+// tracing and transverse coefficients of the MAC velocities
+void edge_scal_coeffs(Ctx& c) { edge_coeffs(c, F_UMAC0, true, true); }
+
+// One launch over the faces of every direction (region_union's parts in the order of the
+// directions): a small level's launch takes 2.7 us, whatever it does.
+struct DirRules {
+    int bl[3], bh[3], dl[3], dh[3];  // boundary types and the domain of each direction
+    double h[3];
+};
+static DirRules phys_rules(const Ctx& c, double h0, double h1, double h2) {
+    DirRules p{};
+    for (int d = 0; d < 3; ++d) {
+        p.bl[d] = c.P.phys_bc_lo[d];
+        p.bh[d] = c.P.phys_bc_hi[d];
+        p.dl[d] = c.P.dom_lo[d];
+        p.dh[d] = c.P.dom_hi[d];
+    }
+    p.h[0] = h0;
+    p.h[1] = h1;
+    p.h[2] = h2;
+    return p;
+}
+#define RULES(D) p.bl[D], p.bh[D], p.dl[D], p.dh[D]
+static const RegionTable& rg_faces(Ctx& c) {
+    if (c.ndim == 2) return region_union(c, {{0, 0, 0, 0, 0, 0, 0, -1}, {0, 0, 0, 0, 0, 0, 1, -1}});
+    return region_union(c, {{0, 0, 0, 0, 0, 0, 0, -1}, {0, 0, 0, 0, 0, 0, 1, -1}, {0, 0, 0, 0, 0, 0, 2, -1}});
 }
 
 // ============================================================ MakeUtrans
@@ -453,9 +595,9 @@ void edge_scal_coeffs(Ctx& c) {
 // utilde component D along D (ufull tracing) is the same sweep VelPred needs, so it is
 // stored where VelPred reads it (F_IPC0+D / F_IMC0+D, comp D) and not repeated there.
 template <int D>
-__global__ void k_utrans(KARGS, int ppm_type, double dt2dx, int bclo, int bchi, int domlo, int domhi, double rel_eps,
-                         int sph) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void utrans_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int ppm_type, double dt2dx, int bclo, int bchi, int domlo, int domhi, double rel_eps,
+    int sph) {
     constexpr int di = D == 0, dj = D == 1, dk = D == 2;
     const int I = D == 0 ? i : (D == 1 ? j : k);
     const FabView ut = VW(F_UTILDE);
@@ -463,8 +605,8 @@ __global__ void k_utrans(KARGS, int ppm_type, double dt2dx, int bclo, int bchi, 
     if (ppm_type == 0) {
         const FabView uf = VW(F_UFULL);
         const FabView sl = VW(F_SLOPE);
-        l = at(ut, i - di, j - dj, k - dk, D) + (0.5 - dt2dx * mx(0.0, at(uf, i - di, j - dj, k - dk, D))) * at(sl, i - di, j - dj, k - dk, 0);
-        r = at(ut, i, j, k, D) - (0.5 + dt2dx * mn(0.0, at(uf, i, j, k, D))) * at(sl, i, j, k, 0);
+        l = at(ut, i - di, j - dj, k - dk, D) + (0.5 - dt2dx * mx(0.0, at(uf, i - di, j - dj, k - dk, D))) * at(sl, i - di, j - dj, k - dk, D);
+        r = at(ut, i, j, k, D) - (0.5 + dt2dx * mn(0.0, at(uf, i, j, k, D))) * at(sl, i, j, k, D);
     } else {
         l = at(VW(F_IPC0 + D), i - di, j - dj, k - dk, D);
         r = at(VW(F_IMC0 + D), i, j, k, D);
@@ -499,6 +641,15 @@ __global__ void k_utrans(KARGS, int ppm_type, double dt2dx, int bclo, int bchi, 
     at(VW(F_UTRANS0 + D), i, j, k) = v;
 }
 
+__global__ void k_utrans(KARGS, int ppm_type, const __grid_constant__ DirRules p, double rel_eps, int sph) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    switch (R[e_].pad) {
+        case 0: utrans_face<0>(V, nb, b, i, j, k, ppm_type, p.h[0], RULES(0), rel_eps, sph); break;
+        case 1: utrans_face<1>(V, nb, b, i, j, k, ppm_type, p.h[1], RULES(1), rel_eps, sph); break;
+        default: utrans_face<2>(V, nb, b, i, j, k, ppm_type, p.h[2], RULES(2), rel_eps, sph);
+    }
+}
+
 void make_utrans(Ctx& c) {
     if (c.ndim == 2) return make_utrans_2d_entry(c);
     const double dt2 = 0.5 * c.P.dt;
@@ -509,20 +660,12 @@ void make_utrans(Ctx& c) {
     // others by vel_pred
     const bool march = ppm_marches(c);
     if (march) ppm_march_comps(c, 7, F_UTILDE, 0, 3, c.bcs_u, F_UFULL, 0, F_IPC0, F_IMC0);
-    for (int d = 0; d < 3; ++d) {
-        if (c.P.ppm_type == 0) {
-            slope_any(c, d, F_UTILDE, d, F_SLOPE, 0, 1, bcs_dev(c, BCS_U), d);
-        } else if (!march) {
-            ppm_any(c, d, F_UTILDE, d, c.bcs_u[d], F_UFULL, d, 0, F_IPC0 + d, F_IMC0 + d);
-        }
-        const RegionTable& rt = rg_grow(c, 0, d);
-        const double dt2dx = dt2 / c.P.dx[d];
-        const int bl = c.P.phys_bc_lo[d], bh = c.P.phys_bc_hi[d], dl = c.P.dom_lo[d], dh = c.P.dom_hi[d];
-        const int sph = c.sph;
-        if (d == 0) launch(c, rt, 1, k_utrans<0>, c.V(), c.P.ppm_type, dt2dx, bl, bh, dl, dh, c.P.rel_eps, sph);
-        else if (d == 1) launch(c, rt, 1, k_utrans<1>, c.V(), c.P.ppm_type, dt2dx, bl, bh, dl, dh, c.P.rel_eps, sph);
-        else launch(c, rt, 1, k_utrans<2>, c.V(), c.P.ppm_type, dt2dx, bl, bh, dl, dh, c.P.rel_eps, sph);
+    for (int d = 0; d < 3 && !march; ++d) {
+        if (c.P.ppm_type == 0) slope_any(c, d, F_UTILDE, d, F_SLOPE, d, 1, bcs_dev(c, BCS_U), d);
+        else ppm_any(c, d, F_UTILDE, d, c.bcs_u[d], F_UFULL, d, 0, F_IPC0 + d, F_IMC0 + d);
     }
+    launch(c, rg_faces(c), 1, k_utrans, c.V(), c.P.ppm_type,
+           phys_rules(c, dt2 / c.P.dx[0], dt2 / c.P.dx[1], dt2 / c.P.dx[2]), c.P.rel_eps, (int)c.sph);
 }
 
 // ============================================================ MakeVelForce
@@ -556,9 +699,9 @@ void make_vel_force(Ctx& c, int fe) {
 // VelPredInterface, 3-D (Source/MaestroVelPred.cpp:735-1128): predictor states of all
 // three velocity components on D-faces, and their upwind values.
 template <int D>
-__global__ void k_vp_interface(KARGS, int ppm_type, double dt2, double hd, int bclo, int bchi, int domlo, int domhi,
-                               long long epsb) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void vp_interface_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int ppm_type, double dt2, double hd, int bclo, int bchi, int domlo, int domhi,
+    long long epsb) {
     constexpr int di = D == 0, dj = D == 1, dk = D == 2;
     const int I = D == 0 ? i : (D == 1 ? j : k);
     const int il = i - di, jl = j - dj, kl = k - dk;
@@ -638,8 +781,8 @@ __global__ void k_vp_interface(KARGS, int ppm_type, double dt2, double hd, int b
 // VelPredTransverse (Source/MaestroVelPred.cpp:1130-1595): component C on D-faces
 // corrected in the third direction T.  F_TCOEF comp T holds (dt6/h_T)*(trans_T sum).
 template <int C, int D>
-__global__ void k_vp_transverse(KARGS, int bclo, int bchi, int domlo, int domhi, long long epsb) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void vp_transverse_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int bclo, int bchi, int domlo, int domhi, long long epsb) {
     constexpr int T = 3 - C - D;
     constexpr int di = D == 0, dj = D == 1, dk = D == 2;
     constexpr int ti = T == 0, tj = T == 1, tk = T == 2;
@@ -672,9 +815,9 @@ __global__ void k_vp_transverse(KARGS, int bclo, int bchi, int domlo, int domhi,
 // VelPredVelocities (Source/MaestroVelPred.cpp:1597-1915).  F_TCOEF comps 3..5 hold
 // (dt4/h_t)*(trans_t sum).
 template <int D>
-__global__ void k_vp_velocities(KARGS, double dt2, int bclo, int bchi, int domlo, int domhi, double rel_eps, int sph,
-                                int ptf) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void vp_velocities_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    double dt2, int bclo, int bchi, int domlo, int domhi, double rel_eps, int sph,
+    int ptf) {
     constexpr int di = D == 0, dj = D == 1, dk = D == 2;
     constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
     constexpr int a1i = T1 == 0, a1j = T1 == 1, a1k = T1 == 2;
@@ -726,30 +869,33 @@ __global__ void k_vp_velocities(KARGS, double dt2, int bclo, int bchi, int domlo
     at(VW(F_UMAC0 + D), i, j, k) = v;
 }
 
-template <int C, int D>
-static void vp_transverse_launch(Ctx& c) {
-    int glo[3] = {0, 0, 0}, ghi[3] = {0, 0, 0};
-    glo[C] = 1;
-    ghi[C] = 1;
-    ghi[D] = 1;
-    const RegionTable& rt = region(c, glo[0], glo[1], glo[2], ghi[0], ghi[1], ghi[2], -1);
-    launch(c, rt, 1, k_vp_transverse<C, D>, c.V(), c.P.phys_bc_lo[D], c.P.phys_bc_hi[D], c.P.dom_lo[D],
-           c.P.dom_hi[D], dbits_host(c.P.rel_eps));
+__global__ void k_vp_interface(KARGS, int ppm_type, double dt2, const __grid_constant__ DirRules p, long long epsb) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    switch (R[e_].pad) {
+        case 0: vp_interface_face<0>(V, nb, b, i, j, k, ppm_type, dt2, p.h[0], RULES(0), epsb); break;
+        case 1: vp_interface_face<1>(V, nb, b, i, j, k, ppm_type, dt2, p.h[1], RULES(1), epsb); break;
+        default: vp_interface_face<2>(V, nb, b, i, j, k, ppm_type, dt2, p.h[2], RULES(2), epsb);
+    }
 }
-
-template <int D>
-static void vp_interface_launch(Ctx& c) {
-    int glo[3] = {1, 1, 1};
-    glo[D] = 0;
-    const RegionTable& rt = region(c, glo[0], glo[1], glo[2], 1, 1, 1, -1);
-    launch(c, rt, 1, k_vp_interface<D>, c.V(), c.P.ppm_type, 0.5 * c.P.dt, c.P.dx[D], c.P.phys_bc_lo[D],
-           c.P.phys_bc_hi[D], c.P.dom_lo[D], c.P.dom_hi[D], dbits_host(c.P.rel_eps));
+// parts: (C, D) = (0, 1), (0, 2), (1, 0), (1, 2), (2, 0), (2, 1)
+__global__ void k_vp_transverse(KARGS, const __grid_constant__ DirRules p, long long epsb) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    switch (R[e_].pad) {
+        case 0: vp_transverse_face<0, 1>(V, nb, b, i, j, k, RULES(1), epsb); break;
+        case 1: vp_transverse_face<0, 2>(V, nb, b, i, j, k, RULES(2), epsb); break;
+        case 2: vp_transverse_face<1, 0>(V, nb, b, i, j, k, RULES(0), epsb); break;
+        case 3: vp_transverse_face<1, 2>(V, nb, b, i, j, k, RULES(2), epsb); break;
+        case 4: vp_transverse_face<2, 0>(V, nb, b, i, j, k, RULES(0), epsb); break;
+        default: vp_transverse_face<2, 1>(V, nb, b, i, j, k, RULES(1), epsb);
+    }
 }
-
-template <int D>
-static void vp_velocities_launch(Ctx& c) {
-    launch(c, rg_grow(c, 0, D), 1, k_vp_velocities<D>, c.V(), 0.5 * c.P.dt, c.P.phys_bc_lo[D], c.P.phys_bc_hi[D],
-           c.P.dom_lo[D], c.P.dom_hi[D], c.P.rel_eps, (int)c.sph, c.P.ppm_trace_forces);
+__global__ void k_vp_velocities(KARGS, double dt2, const __grid_constant__ DirRules p, double rel_eps, int sph, int ptf) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    switch (R[e_].pad) {
+        case 0: vp_velocities_face<0>(V, nb, b, i, j, k, dt2, RULES(0), rel_eps, sph, ptf); break;
+        case 1: vp_velocities_face<1>(V, nb, b, i, j, k, dt2, RULES(1), rel_eps, sph, ptf); break;
+        default: vp_velocities_face<2>(V, nb, b, i, j, k, dt2, RULES(2), rel_eps, sph, ptf);
+    }
 }
 
 void vel_pred(Ctx& c) {
@@ -769,19 +915,22 @@ void vel_pred(Ctx& c) {
         if (c.P.ppm_trace_forces)
             for (int d = 0; d < 3; ++d) ppm_any(c, d, F_VELFORCE, d, c.bcs_u[d], F_UFULL, d, 0, F_IPF, F_IMF);
     }
-    vp_interface_launch<0>(c);
-    vp_interface_launch<1>(c);
-    vp_interface_launch<2>(c);
-    transverse_coeffs(c, F_UTRANS0);
-    vp_transverse_launch<0, 1>(c);
-    vp_transverse_launch<0, 2>(c);
-    vp_transverse_launch<1, 0>(c);
-    vp_transverse_launch<1, 2>(c);
-    vp_transverse_launch<2, 0>(c);
-    vp_transverse_launch<2, 1>(c);
-    vp_velocities_launch<0>(c);
-    vp_velocities_launch<1>(c);
-    vp_velocities_launch<2>(c);
+    const DirRules p = phys_rules(c, c.P.dx[0], c.P.dx[1], c.P.dx[2]);
+    const long long eb = dbits_host(c.P.rel_eps);
+    launch(c, region_union(c, {{0, 1, 1, 1, 1, 1, -1, -1}, {1, 0, 1, 1, 1, 1, -1, -1}, {1, 1, 0, 1, 1, 1, -1, -1}}), 1,
+           k_vp_interface, c.V(), c.P.ppm_type, 0.5 * c.P.dt, p, eb);
+    edge_coeffs(c, F_UTRANS0, false, true);
+    std::vector<RegionKey> parts;  // grown along C, one more face along D
+    for (int C = 0; C < 3; ++C)
+        for (int D = 0; D < 3; ++D) {
+            if (D == C) continue;
+            RegionKey r{0, 0, 0, 0, 0, 0, -1, -1};
+            r[C] = 1;
+            r[3 + C] = r[3 + D] = 1;
+            parts.push_back(r);
+        }
+    launch(c, region_union(c, parts), 1, k_vp_transverse, c.V(), p, eb);
+    launch(c, rg_faces(c), 1, k_vp_velocities, c.V(), 0.5 * c.P.dt, p, c.P.rel_eps, (int)c.sph, c.P.ppm_trace_forces);
 }
 
 // ============================================================ MakeEdgeScal
@@ -1047,17 +1196,16 @@ static void es_edges_launch(Ctx& c, int comp, const BCRecD& bc, int is_cons, int
 
 // velocity-only quantities shared by every component of a MakeEdgeScal call
 void edge_scal_setup(Ctx& c, int is_cons) {
-    if (is_cons) launch(c, rg_grow(c, 1), 1, k_divu, c.V(), make_recip(c.P.dx[0]));
-    if (c.P.ppm_type != 0) trace_coeffs_faces(c, F_UMAC0);
-    if (!is_cons) transverse_coeffs(c, F_UMAC0);
+    if (is_cons && c.ndim == 3) launch(c, rg_grow(c, 1), 1, k_divu, c.V(), make_recip(c.P.dx[0]));
+    edge_coeffs(c, F_UMAC0, c.P.ppm_type != 0, !is_cons && c.ndim == 3);
 }
 
 // force_zero: the components' force is identically zero (DensityAdvance species)
 void make_edge_scal(Ctx& c, int start_comp, int num_comp, int which_bcs, int is_cons, int force_zero, int is_vel,
                     int slot, bool setup) {
+    if (setup) edge_scal_setup(c, is_cons);
     if (c.ndim == 2) return make_edge_scal_2d_entry(c, start_comp, num_comp, which_bcs, is_cons);
     const BCRecD* bh = bcs_host(c, which_bcs);
-    if (setup) edge_scal_setup(c, is_cons);
     // component streams: every other component on the side stream, in its own scratch
     // (components are independent: each reads the state, the velocities and the shared
     // coefficients formed above, and writes only its scratch and its edge state)
@@ -1199,21 +1347,26 @@ void put_in_pert_form(Ctx& c, const double* d_s0, int comp, int flag) {
 }
 
 // ConvertRhoXToX (Source/MaestroConvert.cpp:64-91), valid region
-__global__ void k_rhox_to_x(KARGS, int c0, int nc, int flag) {
+// (s0: with PutInPertForm of the density, after the conversion to X or before the one back; rd:
+// the radial direction)
+__global__ void k_rhox_to_x(KARGS, int c0, int nc, int flag, const double* __restrict__ s0, int rd) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView s = VW(F_SOLD);
-    const double rho = at(s, i, j, k, RHO);
+    double rho = at(s, i, j, k, RHO);
+    const double base = s0 ? s0[rd == 2 ? k : j] : 0.0;
     if (flag) {
         // every species over the same rho: its reciprocal once, then 4 FP64 instructions each
         const RecipV r = recip_v(rho);
         for (int comp = c0; comp < c0 + nc; ++comp) at(s, i, j, k, comp) = div_v(at(s, i, j, k, comp), r);
+        if (s0) at(s, i, j, k, RHO) = rho - base;
     } else {
+        if (s0) at(s, i, j, k, RHO) = rho = rho + base;
         for (int comp = c0; comp < c0 + nc; ++comp) at(s, i, j, k, comp) = at(s, i, j, k, comp) * rho;
     }
 }
 
-void convert_rhox_to_x(Ctx& c, int flag, int c0, int nc) {
-    launch(c, rg_grow(c, 0), 1, k_rhox_to_x, c.V(), c0, nc < 0 ? c.nspec : nc, flag);
+void convert_rhox_to_x(Ctx& c, int flag, int c0, int nc, const double* s0) {
+    launch(c, rg_grow(c, 0), 1, k_rhox_to_x, c.V(), c0, nc < 0 ? c.nspec : nc, flag, s0, c.ndim - 1);
 }
 
 // ============================================================ fluxes
@@ -1222,10 +1375,10 @@ void convert_rhox_to_x(Ctx& c, int flag, int c0, int nc) {
 // component `slot`.  The Rho flux (the species fluxes summed in order from 0) and etarhoflux
 // carry over between calls, so species streamed one call at a time sum in the same order.
 template <int D>
-__global__ void k_rhox_flux(KARGS, int c0, int nc, int nspec, int slot, int spt, int do_eta,
-                            const double* __restrict__ r0o, const double* __restrict__ r0n,
-                            const double* __restrict__ w0, const double* __restrict__ r0pe) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void rhox_flux_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int c0, int nc, int nspec, int slot, int spt, int do_eta,
+    const double* __restrict__ r0o, const double* __restrict__ r0n,
+    const double* __restrict__ w0, const double* __restrict__ r0pe) {
     const FabView fl = VW(F_SFLUX0 + D), e = VW(F_SEDGE0 + D);
     const double u = at(VW(F_UMAC0 + D), i, j, k);
     double frho = c0 == FIRSTSPEC ? 0.0 : at(fl, i, j, k, RHO);
@@ -1249,6 +1402,18 @@ __global__ void k_rhox_flux(KARGS, int c0, int nc, int nspec, int slot, int spt,
     if (D == 2 && do_eta) at(VW(F_ETA), i, j, k) = eta;
 }
 
+__global__ void k_rhox_flux(KARGS, int c0, int nc, int nspec, int slot, int spt, int do_eta,
+                            const double* __restrict__ r0o, const double* __restrict__ r0n,
+                            const double* __restrict__ r0eo, const double* __restrict__ r0en,
+                            const double* __restrict__ w0, const double* __restrict__ r0pe) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    switch (R[e_].pad) {
+        case 0: rhox_flux_face<0>(V, nb, b, i, j, k, c0, nc, nspec, slot, spt, 0, r0o, r0n, w0, r0pe); break;
+        case 1: rhox_flux_face<1>(V, nb, b, i, j, k, c0, nc, nspec, slot, spt, 0, r0o, r0n, w0, r0pe); break;
+        default: rhox_flux_face<2>(V, nb, b, i, j, k, c0, nc, nspec, slot, spt, do_eta, r0eo, r0en, w0, r0pe);
+    }
+}
+
 void make_rhox_flux(Ctx& c, const double* r0_old, const double* r0e_old, const double* r0_new, const double* r0e_new,
                     int c0, int nc, int slot) {
     if (nc < 0) nc = c.nspec;
@@ -1258,18 +1423,16 @@ void make_rhox_flux(Ctx& c, const double* r0_old, const double* r0e_old, const d
     const double* w0 = c.b1("w0");
     const double* rpe = c.b1("rho0_predicted_edge");
     const int ns = c.nspec, spt = c.P.species_pred_type;
-    launch(c, rg_grow(c, 0, 0), 1, k_rhox_flux<0>, c.V(), c0, nc, ns, slot, spt, 0, r0_old, r0_new, w0, rpe);
-    launch(c, rg_grow(c, 0, 1), 1, k_rhox_flux<1>, c.V(), c0, nc, ns, slot, spt, 0, r0_old, r0_new, w0, rpe);
-    launch(c, rg_grow(c, 0, 2), 1, k_rhox_flux<2>, c.V(), c0, nc, ns, slot, spt, do_eta, r0e_old, r0e_new, w0, rpe);
+    launch(c, rg_faces(c), 1, k_rhox_flux, c.V(), c0, nc, ns, slot, spt, do_eta, r0_old, r0_new, r0e_old, r0e_new, w0, rpe);
 }
 
 // MakeRhoHFlux, planar 3-D (Source/MaestroMakeFlux.cpp:673-786)
 // enthalpy_pred_type 2 (the edge state is h, :673-786 have_h): (rho0 edge + rho') h with
 // species_pred_type 1 (ra, rb: rho0 on the faces' radial positions), rho h otherwise
 template <int D>
-__global__ void k_rhoh_flux(KARGS, int ept, const double* __restrict__ a, const double* __restrict__ bb, int spt,
-                            const double* __restrict__ ra, const double* __restrict__ rb) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void rhoh_flux_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int ept, const double* __restrict__ a, const double* __restrict__ bb, int spt,
+    const double* __restrict__ ra, const double* __restrict__ rb) {
     const FabView e = VW(F_SEDGE0 + D);
     const double u = at(VW(F_UMAC0 + D), i, j, k);
     double f;
@@ -1289,15 +1452,27 @@ __global__ void k_rhoh_flux(KARGS, int ept, const double* __restrict__ a, const 
     at(VW(F_SFLUX0 + D), i, j, k, RHOH) = f;
 }
 
+struct RhohBase {
+    const double *cell[4], *edge[4];  // rhoh0 old and new, rho0 old and new: on the cells' and edges' radii
+};
+__global__ void k_rhoh_flux(KARGS, int ept, int spt, RhohBase q) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    const auto &c = q.cell, &e = q.edge;
+    switch (R[e_].pad) {
+        case 0: rhoh_flux_face<0>(V, nb, b, i, j, k, ept, c[0], c[1], spt, c[2], c[3]); break;
+        case 1: rhoh_flux_face<1>(V, nb, b, i, j, k, ept, c[0], c[1], spt, c[2], c[3]); break;
+        default: rhoh_flux_face<2>(V, nb, b, i, j, k, ept, e[0], e[1], spt, e[2], e[3]);
+    }
+}
+
 void make_rhoh_flux(Ctx& c, const double* rh0_old, const double* rh0e_old, const double* rh0_new,
                     const double* rh0e_new, const double* r0_old, const double* r0e_old, const double* r0_new,
                     const double* r0e_new) {
     if (c.sph) return make_rhoh_flux_sph(c);
     if (c.ndim == 2) return make_rhoh_flux_2d(c, rh0_old, rh0e_old, rh0_new, rh0e_new, r0_old, r0e_old, r0_new, r0e_new);
     const int ept = c.P.enthalpy_pred_type, spt = c.P.species_pred_type;
-    launch(c, rg_grow(c, 0, 0), 1, k_rhoh_flux<0>, c.V(), ept, rh0_old, rh0_new, spt, r0_old, r0_new);
-    launch(c, rg_grow(c, 0, 1), 1, k_rhoh_flux<1>, c.V(), ept, rh0_old, rh0_new, spt, r0_old, r0_new);
-    launch(c, rg_grow(c, 0, 2), 1, k_rhoh_flux<2>, c.V(), ept, rh0e_old, rh0e_new, spt, r0e_old, r0e_new);
+    const RhohBase q{{rh0_old, rh0_new, r0_old, r0_new}, {rh0e_old, rh0e_new, r0e_old, r0e_new}};
+    launch(c, rg_faces(c), 1, k_rhoh_flux, c.V(), ept, spt, q);
 }
 
 // Maestro::ConvertRhoHToH on the valid region (Source/MaestroConvert.cpp:93-105): flag,
@@ -1577,15 +1752,15 @@ __global__ void k_addw0_2d(KARGS, int f, const double* __restrict__ w0, double m
 
 // MakeUtrans, 2-D y faces (Source/MaestroMakeUtrans.cpp:161-266): the lo-side wall case
 // sets vry = 0 twice and leaves vly; the solve tests v + w0_cart.
-__global__ void k_utrans_2dy(KARGS, int ppm_type, double dt2dy, int bclo, int bchi, int domlo, int domhi,
-                             double rel_eps) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void utrans_2dy_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int ppm_type, double dt2dy, int bclo, int bchi, int domlo, int domhi,
+    double rel_eps) {
     const FabView ut = VW(F_UTILDE);
     double l, r;
     if (ppm_type == 0) {
         const FabView uf = VW(F_UFULL), sl = VW(F_SLOPE);
-        l = at(ut, i, j - 1, k, 1) + (0.5 - dt2dy * mx(0.0, at(uf, i, j - 1, k, 1))) * at(sl, i, j - 1, k, 0);
-        r = at(ut, i, j, k, 1) - (0.5 + dt2dy * mn(0.0, at(uf, i, j, k, 1))) * at(sl, i, j, k, 0);
+        l = at(ut, i, j - 1, k, 1) + (0.5 - dt2dy * mx(0.0, at(uf, i, j - 1, k, 1))) * at(sl, i, j - 1, k, 1);
+        r = at(ut, i, j, k, 1) - (0.5 + dt2dy * mn(0.0, at(uf, i, j, k, 1))) * at(sl, i, j, k, 1);
     } else {
         l = at(VW(F_IPC0 + 1), i, j - 1, k, 1);
         r = at(VW(F_IMC0 + 1), i, j, k, 1);
@@ -1611,20 +1786,26 @@ __global__ void k_utrans_2dy(KARGS, int ppm_type, double dt2dy, int bclo, int bc
     at(VW(F_UTRANS1), i, j, k) = test ? 0.0 : v;
 }
 
+__global__ void k_utrans_2d(KARGS, int ppm_type, const __grid_constant__ DirRules p, double rel_eps) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    if (R[e_].pad == 0) utrans_face<0>(V, nb, b, i, j, k, ppm_type, p.h[0], RULES(0), rel_eps, 0);
+    else utrans_2dy_face(V, nb, b, i, j, k, ppm_type, p.h[1], RULES(1), rel_eps);
+}
+
 static void make_utrans_2d(Ctx& c) {
     const double dt2 = 0.5 * c.P.dt;
     if (c.P.ppm_type != 0)
         launch(c, rg2(c, 1), 1, k_trace_cell, c.V(), F_UFULL, c.P.dt, make_recip(c.P.dx[0]),
                make_recip(c.P.dx[1]), make_recip(c.P.dx[2]));
-    for (int d = 0; d < 2; ++d) {
-        if (c.P.ppm_type == 0) slope_any(c, d, F_UTILDE, d, F_SLOPE, 0, 1, bcs_dev(c, BCS_U), d);
+    // marched: every sweep of the velocity at once, as in 3-D
+    const bool march = ppm_marches(c);
+    if (march) ppm_march_comps(c, 3, F_UTILDE, 0, 2, c.bcs_u, F_UFULL, 0, F_IPC0, F_IMC0);
+    for (int d = 0; d < 2 && !march; ++d) {
+        if (c.P.ppm_type == 0) slope_any(c, d, F_UTILDE, d, F_SLOPE, d, 1, bcs_dev(c, BCS_U), d);
         else ppm_any(c, d, F_UTILDE, d, c.bcs_u[d], F_UFULL, d, 0, F_IPC0 + d, F_IMC0 + d);
-        const RegionTable& rt = rg2(c, 0, d);
-        const double dt2dx = dt2 / c.P.dx[d];
-        const int bl = c.P.phys_bc_lo[d], bh = c.P.phys_bc_hi[d], dl = c.P.dom_lo[d], dh = c.P.dom_hi[d];
-        if (d == 0) launch(c, rt, 1, k_utrans<0>, c.V(), c.P.ppm_type, dt2dx, bl, bh, dl, dh, c.P.rel_eps, 0);
-        else launch(c, rt, 1, k_utrans_2dy, c.V(), c.P.ppm_type, dt2dx, bl, bh, dl, dh, c.P.rel_eps);
     }
+    launch(c, rg_faces(c), 1, k_utrans_2d, c.V(), c.P.ppm_type, phys_rules(c, dt2 / c.P.dx[0], dt2 / c.P.dx[1], 0.0),
+           c.P.rel_eps);
 }
 
 // MakeVelForce, planar 2-D (Source/MaestroForce.cpp:100-137)
@@ -1647,9 +1828,9 @@ __global__ void k_vel_force_2d(KARGS, double cutoff_rho, int domhi, double dy) {
 // VelPredInterface, 2-D (Source/MaestroVelPred.cpp:296-537).  D = 0: ulx/urx/uimhx into
 // F_SL0/F_SR0/F_SIMH0; D = 1: uly/ury/uimhy into F_SL1/F_SR1/F_SIMH1.
 template <int D>
-__global__ void k_vp_interface_2d(KARGS, int ppm_type, double dt2h, int bclo, int bchi, int domlo, int domhi,
-                                  double rel_eps) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void vp_interface_2d_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int ppm_type, double dt2h, int bclo, int bchi, int domlo, int domhi,
+    double rel_eps) {
     constexpr int di = D == 0, dj = D == 1;
     constexpr int T = 1 - D;  // the transverse component upwinded into uimh
     const int I = D == 0 ? i : j;
@@ -1737,9 +1918,9 @@ __global__ void k_vp_interface_2d(KARGS, int ppm_type, double dt2h, int bclo, in
 
 // VelPredVelocities, 2-D (Source/MaestroVelPred.cpp:539-727)
 template <int D>
-__global__ void k_vp_velocities_2d(KARGS, double dt2, double dt4h, int bclo, int bchi, int domlo, int domhi,
-                                   double rel_eps) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void vp_velocities_2d_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    double dt2, double dt4h, int bclo, int bchi, int domlo, int domhi,
+    double rel_eps) {
     constexpr int di = D == 0, dj = D == 1;
     constexpr int T = 1 - D;
     constexpr int ti = T == 0, tj = T == 1;
@@ -1784,37 +1965,42 @@ __global__ void k_vp_velocities_2d(KARGS, double dt2, double dt4h, int bclo, int
     at(VW(F_UMAC0 + D), i, j, k) = v;
 }
 
+__global__ void k_vp_interface_2d(KARGS, int ppm_type, const __grid_constant__ DirRules p, double rel_eps) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    if (R[e_].pad == 0) vp_interface_2d_face<0>(V, nb, b, i, j, k, ppm_type, p.h[0], RULES(0), rel_eps);
+    else vp_interface_2d_face<1>(V, nb, b, i, j, k, ppm_type, p.h[1], RULES(1), rel_eps);
+}
+__global__ void k_vp_velocities_2d(KARGS, double dt2, const __grid_constant__ DirRules p, double rel_eps) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    if (R[e_].pad == 0) vp_velocities_2d_face<0>(V, nb, b, i, j, k, dt2, p.h[1], RULES(0), rel_eps);
+    else vp_velocities_2d_face<1>(V, nb, b, i, j, k, dt2, p.h[0], RULES(1), rel_eps);
+}
+// the faces of both directions inside the cells grown by one (growLo(obx, d, -1))
+static const RegionTable& rg2_inner_faces(Ctx& c) {
+    return region_union(c, {{0, 1, 0, 1, 1, 0, -1, -1}, {1, 0, 0, 1, 1, 0, -1, -1}});
+}
+
 static void vel_pred_2d(Ctx& c) {
     if (c.P.ppm_type == 0) {
         slope_any(c, 0, F_UTILDE, 0, F_IPC0, 0, 2, bcs_dev(c, BCS_U), 0);  // slopex -> Ipu
         slope_any(c, 1, F_UTILDE, 0, F_IMC1, 0, 2, bcs_dev(c, BCS_U), 0);  // slopey -> Imv
-    } else {
-        // component d along d was traced by make_utrans (same inputs)
+    } else if (!ppm_marches(c)) {
+        // component d along d (marched: every sweep) was traced by make_utrans (same inputs)
         ppm_any(c, 1, F_UTILDE, 0, c.bcs_u[0], F_UFULL, 1, 0, F_IPC0, F_IMC0);
         ppm_any(c, 0, F_UTILDE, 1, c.bcs_u[1], F_UFULL, 0, 0, F_IPC0 + 1, F_IMC0 + 1);
     }
     const double dt2 = 0.5 * c.P.dt, dt4 = 0.25 * c.P.dt;
-    for (int d = 0; d < 2; ++d) {
-        const RegionTable& rm = region(c, d == 0 ? 0 : 1, d == 1 ? 0 : 1, 0, 1, 1, 0, -1);  // growLo(obx, d, -1)
-        const int bl = c.P.phys_bc_lo[d], bh = c.P.phys_bc_hi[d], dl = c.P.dom_lo[d], dh = c.P.dom_hi[d];
-        if (d == 0)
-            launch(c, rm, 1, k_vp_interface_2d<0>, c.V(), c.P.ppm_type, dt2 / c.P.dx[0], bl, bh, dl, dh, c.P.rel_eps);
-        else
-            launch(c, rm, 1, k_vp_interface_2d<1>, c.V(), c.P.ppm_type, dt2 / c.P.dx[1], bl, bh, dl, dh, c.P.rel_eps);
-    }
-    for (int d = 0; d < 2; ++d) {
-        const int bl = c.P.phys_bc_lo[d], bh = c.P.phys_bc_hi[d], dl = c.P.dom_lo[d], dh = c.P.dom_hi[d];
-        const double dt4h = dt4 / c.P.dx[1 - d];
-        if (d == 0) launch(c, rg2(c, 0, 0), 1, k_vp_velocities_2d<0>, c.V(), dt2, dt4h, bl, bh, dl, dh, c.P.rel_eps);
-        else launch(c, rg2(c, 0, 1), 1, k_vp_velocities_2d<1>, c.V(), dt2, dt4h, bl, bh, dl, dh, c.P.rel_eps);
-    }
+    launch(c, rg2_inner_faces(c), 1, k_vp_interface_2d, c.V(), c.P.ppm_type,
+           phys_rules(c, dt2 / c.P.dx[0], dt2 / c.P.dx[1], 0.0), c.P.rel_eps);
+    launch(c, rg_faces(c), 1, k_vp_velocities_2d, c.V(), dt2, phys_rules(c, dt4 / c.P.dx[0], dt4 / c.P.dx[1], 0.0),
+           c.P.rel_eps);
 }
 
 // MakeEdgeScalPredictor, 2-D (Source/MaestroMakeEdgeScalars.cpp:306-452)
 template <int D>
-__global__ void k_es_predictor_2d(KARGS, int comp, int ppm_type, double dt2, double hd, int bclo, int bchi, int domlo,
-                                  int domhi, double rel_eps) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void es_predictor_2d_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int comp, int q, int ppm_type, double dt2, double hd, int bclo, int bchi, int domlo,
+    int domhi, double rel_eps) {
     constexpr int di = D == 0, dj = D == 1;
     const int I = D == 0 ? i : j;
     const FabView s = VW(F_SOLD), ud = VW(F_UMAC0 + D);
@@ -1825,8 +2011,8 @@ __global__ void k_es_predictor_2d(KARGS, int comp, int ppm_type, double dt2, dou
         l = at(s, i - di, j - dj, k, comp) + (0.5 - dt2 * u / hd) * at(sl, i - di, j - dj, k, D);
         r = at(s, i, j, k, comp) - (0.5 + dt2 * u / hd) * at(sl, i, j, k, D);
     } else {
-        l = at(VW(F_IPC0), i - di, j - dj, k, D);
-        r = at(VW(F_IMC0), i, j, k, D);
+        l = at(VW(F_IPC0 + q), i - di, j - dj, k, D);
+        r = at(VW(F_IMC0 + q), i, j, k, D);
     }
     if (I == domlo) {
         if (bclo == BC_EXT_DIR) {
@@ -1845,17 +2031,17 @@ __global__ void k_es_predictor_2d(KARGS, int comp, int ppm_type, double dt2, dou
             l = r = 0.0;
         }
     }
-    at(VW(F_SL0 + D), i, j, k) = l;
-    at(VW(F_SR0 + D), i, j, k) = r;
+    at(VW(F_SL0 + D), i, j, k, q) = l;
+    at(VW(F_SR0 + D), i, j, k, q) = r;
     double sm = (u > 0.0) ? l : r;
-    at(VW(F_SIMH0 + D), i, j, k) = (fabs(u) > rel_eps) ? sm : half(l + r);
+    at(VW(F_SIMH0 + D), i, j, k, q) = (fabs(u) > rel_eps) ? sm : half(l + r);
 }
 
 // MakeEdgeScalEdges, 2-D (Source/MaestroMakeEdgeScalars.cpp:454-644)
 template <int D>
-__global__ void k_es_edges_2d(KARGS, int comp, int is_cons, double dt2, double dt4, double hd, double ht, int bclo,
-                              int bchi, int domlo, int domhi, double rel_eps) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void es_edges_2d_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int comp, int q, int is_cons, double dt2, double dt4, double hd, double ht, int bclo,
+    int bchi, int domlo, int domhi, double rel_eps) {
     constexpr int di = D == 0, dj = D == 1;
     constexpr int T = 1 - D;
     constexpr int ti = T == 0, tj = T == 1;
@@ -1864,18 +2050,18 @@ __global__ void k_es_edges_2d(KARGS, int comp, int is_cons, double dt2, double d
     const FabView s = VW(F_SOLD), ud = VW(F_UMAC0 + D), ut = VW(F_UMAC0 + T), st = VW(F_SIMH0 + T);
     const FabView f = VW(F_SCALFORCE);
     const double fl = at(f, il, jl, k, comp), fr = at(f, i, j, k, comp);
-    const double l = at(VW(F_SL0 + D), i, j, k), r = at(VW(F_SR0 + D), i, j, k);
+    const double l = at(VW(F_SL0 + D), i, j, k, q), r = at(VW(F_SR0 + D), i, j, k, q);
     double lq, rq;
     if (is_cons) {
-        lq = l - (dt2 / ht) * (at(st, il + ti, jl + tj, k) * at(ut, il + ti, jl + tj, k) - at(st, il, jl, k) * at(ut, il, jl, k)) -
+        lq = l - (dt2 / ht) * (at(st, il + ti, jl + tj, k, q) * at(ut, il + ti, jl + tj, k) - at(st, il, jl, k, q) * at(ut, il, jl, k)) -
              (dt2 / hd) * at(s, il, jl, k, comp) * (at(ud, i, j, k) - at(ud, il, jl, k)) + dt2 * fl;
-        rq = r - (dt2 / ht) * (at(st, i + ti, j + tj, k) * at(ut, i + ti, j + tj, k) - at(st, i, j, k) * at(ut, i, j, k)) -
+        rq = r - (dt2 / ht) * (at(st, i + ti, j + tj, k, q) * at(ut, i + ti, j + tj, k) - at(st, i, j, k, q) * at(ut, i, j, k)) -
              (dt2 / hd) * at(s, i, j, k, comp) * (at(ud, i + di, j + dj, k) - at(ud, i, j, k)) + dt2 * fr;
     } else {
         lq = l - (dt4 / ht) * (at(ut, il + ti, jl + tj, k) + at(ut, il, jl, k)) *
-                     (at(st, il + ti, jl + tj, k) - at(st, il, jl, k)) +
+                     (at(st, il + ti, jl + tj, k, q) - at(st, il, jl, k, q)) +
              dt2 * fl;
-        rq = r - (dt4 / ht) * (at(ut, i + ti, j + tj, k) + at(ut, i, j, k)) * (at(st, i + ti, j + tj, k) - at(st, i, j, k)) +
+        rq = r - (dt4 / ht) * (at(ut, i + ti, j + tj, k) + at(ut, i, j, k)) * (at(st, i + ti, j + tj, k, q) - at(st, i, j, k, q)) +
              dt2 * fr;
     }
     const double u = at(ud, i, j, k);
@@ -1893,39 +2079,58 @@ __global__ void k_es_edges_2d(KARGS, int comp, int is_cons, double dt2, double d
     at(VW(F_SEDGE0 + D), i, j, k, comp) = v;
 }
 
+// the boundary rules of up to three components of a launch
+struct Es2dRules {
+    int lo[3][2], hi[3][2];
+};
+__global__ void k_es_predictor_2d(KARGS, int comp0, unsigned nq, int ppm_type, double dt2, const __grid_constant__ DirRules p,
+                                  const __grid_constant__ Es2dRules bc, double rel_eps) {
+    const unsigned bx = blockIdx.x / nq, q = blockIdx.x - bx * nq;
+    MADV_ELEMENT_OF(bx, R, ne, g0, g1, b, i, j, k);
+    if (R[e_].pad == 0)
+        es_predictor_2d_face<0>(V, nb, b, i, j, k, comp0 + q, q, ppm_type, dt2, p.h[0], bc.lo[q][0], bc.hi[q][0], p.dl[0],
+                                p.dh[0], rel_eps);
+    else
+        es_predictor_2d_face<1>(V, nb, b, i, j, k, comp0 + q, q, ppm_type, dt2, p.h[1], bc.lo[q][1], bc.hi[q][1], p.dl[1],
+                                p.dh[1], rel_eps);
+}
+__global__ void k_es_edges_2d(KARGS, int comp0, unsigned nq, int is_cons, double dt2, double dt4,
+                              const __grid_constant__ DirRules p, const __grid_constant__ Es2dRules bc, double rel_eps) {
+    const unsigned bx = blockIdx.x / nq, q = blockIdx.x - bx * nq;
+    MADV_ELEMENT_OF(bx, R, ne, g0, g1, b, i, j, k);
+    if (R[e_].pad == 0)
+        es_edges_2d_face<0>(V, nb, b, i, j, k, comp0 + q, q, is_cons, dt2, dt4, p.h[0], p.h[1], bc.lo[q][0], bc.hi[q][0],
+                            p.dl[0], p.dh[0], rel_eps);
+    else
+        es_edges_2d_face<1>(V, nb, b, i, j, k, comp0 + q, q, is_cons, dt2, dt4, p.h[1], p.h[0], bc.lo[q][1], bc.hi[q][1],
+                            p.dl[1], p.dh[1], rel_eps);
+}
+
+// marched PPM: up to three components a launch, each with its own Ip / Im and its own component of
+// the face states
 static void make_edge_scal_2d(Ctx& c, int start_comp, int num_comp, int which_bcs, int is_cons) {
     const BCRecD* bh = bcs_host(c, which_bcs);
     const double dt2 = 0.5 * c.P.dt, dt4 = 0.25 * c.P.dt;
-    if (c.P.ppm_type != 0) {
-        launch(c, region(c, 1, 1, 0, 1, 1, 0, 0), 1, k_trace_face<0>, c.V(), F_UMAC0, F_TRA0, c.P.dt, make_recip(c.P.dx[0]));
-        launch(c, region(c, 1, 1, 0, 1, 1, 0, 1), 1, k_trace_face<1>, c.V(), F_UMAC1, F_TRA1, c.P.dt, make_recip(c.P.dx[1]));
-    }
-    for (int comp = start_comp; comp < start_comp + num_comp; ++comp) {
-        const BCRecD& bc = bh[comp];
+    const DirRules p = phys_rules(c, c.P.dx[0], c.P.dx[1], 0.0);
+    const int batch = ppm_marches(c) ? 3 : 1;
+    for (int comp = start_comp; comp < start_comp + num_comp; comp += batch) {
+        const int nq = std::min(batch, start_comp + num_comp - comp);
         if (c.P.ppm_type == 0) {
             for (int d = 0; d < 2; ++d) slope_any(c, d, F_SOLD, comp, F_SLOPE, d, 1, bcs_dev(c, which_bcs), comp);
+        } else if (ppm_marches(c)) {
+            ppm_march_comps(c, 3, F_SOLD, comp, nq, bh + comp, F_UMAC0, 1, F_IPC0, F_IMC0);
         } else {
-            for (int d = 0; d < 2; ++d) ppm_any(c, d, F_SOLD, comp, bc, F_UMAC0 + d, 0, 1, F_IPC0, F_IMC0);
+            for (int d = 0; d < 2; ++d) ppm_any(c, d, F_SOLD, comp, bh[comp], F_UMAC0 + d, 0, 1, F_IPC0, F_IMC0);
         }
-        for (int d = 0; d < 2; ++d) {
-            const RegionTable& rm = region(c, d == 0 ? 0 : 1, d == 1 ? 0 : 1, 0, 1, 1, 0, -1);
-            const int dl = c.P.dom_lo[d], dh = c.P.dom_hi[d];
-            if (d == 0)
-                launch(c, rm, 1, k_es_predictor_2d<0>, c.V(), comp, c.P.ppm_type, dt2, c.P.dx[0], bc.lo[0], bc.hi[0], dl,
-                       dh, c.P.rel_eps);
-            else
-                launch(c, rm, 1, k_es_predictor_2d<1>, c.V(), comp, c.P.ppm_type, dt2, c.P.dx[1], bc.lo[1], bc.hi[1], dl,
-                       dh, c.P.rel_eps);
-        }
-        for (int d = 0; d < 2; ++d) {
-            const int dl = c.P.dom_lo[d], dh = c.P.dom_hi[d];
-            if (d == 0)
-                launch(c, rg2(c, 0, 0), 1, k_es_edges_2d<0>, c.V(), comp, is_cons, dt2, dt4, c.P.dx[0], c.P.dx[1],
-                       bc.lo[0], bc.hi[0], dl, dh, c.P.rel_eps);
-            else
-                launch(c, rg2(c, 0, 1), 1, k_es_edges_2d<1>, c.V(), comp, is_cons, dt2, dt4, c.P.dx[1], c.P.dx[0],
-                       bc.lo[1], bc.hi[1], dl, dh, c.P.rel_eps);
-        }
+        Es2dRules bc{};
+        for (int q = 0; q < nq; ++q)
+            for (int d = 0; d < 2; ++d) {
+                bc.lo[q][d] = bh[comp + q].lo[d];
+                bc.hi[q][d] = bh[comp + q].hi[d];
+            }
+        launch(c, rg2_inner_faces(c), nq, k_es_predictor_2d, c.V(), comp, (unsigned)nq, c.P.ppm_type, dt2, p, bc,
+               c.P.rel_eps);
+        launch(c, rg_faces(c), nq, k_es_edges_2d, c.V(), comp, (unsigned)nq, is_cons, dt2, dt4, p, bc, c.P.rel_eps);
     }
 }
 
@@ -1972,10 +2177,10 @@ __global__ void k_pert_2d(KARGS, int comp, const double* __restrict__ s0, int fl
 
 // MakeRhoXFlux, 2-D (Source/MaestroMakeFlux.cpp:101-182)
 template <int D>
-__global__ void k_rhox_flux_2d(KARGS, int nspec, int spt, int do_eta, const double* __restrict__ r0o,
-                               const double* __restrict__ r0n, const double* __restrict__ w0,
-                               const double* __restrict__ r0pe) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void rhox_flux_2d_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int nspec, int spt, int do_eta, const double* __restrict__ r0o,
+    const double* __restrict__ r0n, const double* __restrict__ w0,
+    const double* __restrict__ r0pe) {
     const FabView fl = VW(F_SFLUX0 + D), e = VW(F_SEDGE0 + D);
     const double u = at(VW(F_UMAC0 + D), i, j, k);
     double frho = 0.0, eta = D == 1 && do_eta ? at(VW(F_ETA), i, j, k) : 0.0;
@@ -1998,9 +2203,9 @@ __global__ void k_rhox_flux_2d(KARGS, int nspec, int spt, int do_eta, const doub
 
 // MakeRhoHFlux, 2-D (Source/MaestroMakeFlux.cpp:597-662)
 template <int D>
-__global__ void k_rhoh_flux_2d(KARGS, int ept, const double* __restrict__ a, const double* __restrict__ bb, int spt,
-                               const double* __restrict__ ra, const double* __restrict__ rb) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+__device__ __forceinline__ void rhoh_flux_2d_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
+    int ept, const double* __restrict__ a, const double* __restrict__ bb, int spt,
+    const double* __restrict__ ra, const double* __restrict__ rb) {
     const FabView e = VW(F_SEDGE0 + D);
     const double u = at(VW(F_UMAC0 + D), i, j, k);
     double f;
@@ -2018,6 +2223,21 @@ __global__ void k_rhoh_flux_2d(KARGS, int ept, const double* __restrict__ a, con
         f = D == 0 ? u * (rhoh0_edge + at(e, i, j, k, RHOH)) : u * (at(e, i, j, k, RHOH) + rhoh0_edge);
     }
     at(VW(F_SFLUX0 + D), i, j, k, RHOH) = f;
+}
+
+__global__ void k_rhox_flux_2d(KARGS, int nspec, int spt, int do_eta, const double* __restrict__ r0o,
+                               const double* __restrict__ r0n, const double* __restrict__ r0eo,
+                               const double* __restrict__ r0en, const double* __restrict__ w0,
+                               const double* __restrict__ r0pe) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    if (R[e_].pad == 0) rhox_flux_2d_face<0>(V, nb, b, i, j, k, nspec, spt, 0, r0o, r0n, w0, r0pe);
+    else rhox_flux_2d_face<1>(V, nb, b, i, j, k, nspec, spt, do_eta, r0eo, r0en, w0, r0pe);
+}
+__global__ void k_rhoh_flux_2d(KARGS, int ept, int spt, RhohBase q) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    const auto &c = q.cell, &e = q.edge;
+    if (R[e_].pad == 0) rhoh_flux_2d_face<0>(V, nb, b, i, j, k, ept, c[0], c[1], spt, c[2], c[3]);
+    else rhoh_flux_2d_face<1>(V, nb, b, i, j, k, ept, e[0], e[1], spt, e[2], e[3]);
 }
 
 // UpdateScal, 2-D (Source/MaestroAdvection.cpp:117-251)
@@ -2097,16 +2317,15 @@ void make_rhox_flux_2d(Ctx& c, const double* r0_old, const double* r0e_old, cons
     const int do_eta = c.P.evolve_base_state && !c.P.use_exact_base_state;
     const double* w0 = c.b1("w0");
     const double* rpe = c.b1("rho0_predicted_edge");
-    launch(c, rg2(c, 0, 0), 1, k_rhox_flux_2d<0>, c.V(), c.nspec, c.P.species_pred_type, 0, r0_old, r0_new, w0, rpe);
-    launch(c, rg2(c, 0, 1), 1, k_rhox_flux_2d<1>, c.V(), c.nspec, c.P.species_pred_type, do_eta, r0e_old, r0e_new,
-           w0, rpe);
+    launch(c, rg_faces(c), 1, k_rhox_flux_2d, c.V(), c.nspec, c.P.species_pred_type, do_eta, r0_old, r0_new, r0e_old,
+           r0e_new, w0, rpe);
 }
 void make_rhoh_flux_2d(Ctx& c, const double* rh0_old, const double* rh0e_old, const double* rh0_new,
                        const double* rh0e_new, const double* r0_old, const double* r0e_old, const double* r0_new,
                        const double* r0e_new) {
     const int ept = c.P.enthalpy_pred_type, spt = c.P.species_pred_type;
-    launch(c, rg2(c, 0, 0), 1, k_rhoh_flux_2d<0>, c.V(), ept, rh0_old, rh0_new, spt, r0_old, r0_new);
-    launch(c, rg2(c, 0, 1), 1, k_rhoh_flux_2d<1>, c.V(), ept, rh0e_old, rh0e_new, spt, r0e_old, r0e_new);
+    const RhohBase q{{rh0_old, rh0_new, r0_old, r0_new}, {rh0e_old, rh0e_new, r0e_old, r0e_new}};
+    launch(c, rg_faces(c), 1, k_rhoh_flux_2d, c.V(), ept, spt, q);
 }
 void sum_species_edges_2d(Ctx& c) {
     launch(c, rg2(c, 0, 0), 1, k_sum_species<0>, c.V(), c.nspec);
@@ -2130,7 +2349,8 @@ void vel_pred_prep(Ctx& c) {
     const RegionTable& rt = c.ndim == 2 ? rg2(c, 1) : rg_grow(c, 1);
     launch(c, rt, 1, k_trace_cell, c.V(), F_UFULL, c.P.dt, make_recip(c.P.dx[0]),
                make_recip(c.P.dx[1]), make_recip(c.P.dx[2]));
-    if (c.ndim == 3 && ppm_marches(c)) return ppm_march_comps(c, 7, F_UTILDE, 0, 3, c.bcs_u, F_UFULL, 0, F_IPC0, F_IMC0);
+    if (ppm_marches(c))
+        return ppm_march_comps(c, c.ndim == 2 ? 3 : 7, F_UTILDE, 0, c.ndim, c.bcs_u, F_UFULL, 0, F_IPC0, F_IMC0);
     for (int d = 0; d < c.ndim; ++d) ppm_any(c, d, F_UTILDE, d, c.bcs_u[d], F_UFULL, d, 0, F_IPC0 + d, F_IMC0 + d);
 }
 void vel_pred_2d_entry(Ctx& c) { vel_pred_2d(c); }
