@@ -233,7 +233,12 @@ __device__ __forceinline__ double div_c(double a, const RecipC& r) {
     int hi, lo;
     dsplit(a, hi, lo);
     const unsigned ex = ((unsigned)hi >> 20) & 0x7ff;
-    if (ex < 64 || ex >= 2000) return a / r.y;
+    if (ex < 64 || ex >= 2000) {
+        // Zeros are common (still fluid, equal neighbours) and cost no division: one lane's took its
+        // warp's 20 FP64 instructions, 21 instead of 5 for a tracing coefficient.
+        if ((((unsigned)hi << 1) | (unsigned)lo) == 0 && dhigh(r.y) > 0) return a;
+        return a / r.y;
+    }
     if (r.nbad != 0) {
         if (r.nbad < 0) return div_corrected(a, r);
         const unsigned l = (unsigned)lo;
@@ -260,7 +265,10 @@ __device__ __forceinline__ RecipV recip_v(double y) {
 }
 __device__ __forceinline__ double div_v(double a, const RecipV& v) {
     const unsigned ex = ((unsigned)dhigh(a) >> 20) & 0x7ff;
-    if (!v.ok || ex < 323 || ex >= 1723) return a / v.r.y;  // |a| outside 2^-700 .. 2^700
+    if (!v.ok || ex < 323 || ex >= 1723) {  // |a| outside 2^-700 .. 2^700
+        if (v.ok && !nz(a)) return dflip(a, dhigh(v.r.y) < 0);  // a species the cell has none of
+        return a / v.r.y;
+    }
     return div_corrected(a, v.r);
 }
 

@@ -123,36 +123,51 @@ struct Put1dArgs {
     } w[PUT1D_JOBS];
     int lo[3], hi[3], per[3];
 };
+// the value of component n behind a boundary
+template <int ND>
+__device__ __noinline__ double put1d_behind(const Put1dArgs& a, int job, int n, int i, int j, int k) {
+    const auto& w = a.w[job];
+    const int idx[3] = {i, j, k};
+    constexpr int RD = ND - 1;
+    const BCRecD bc = w.bcs[n];
+    // the value over the radial index r at this (i, j): the array, then the rules across it
+    auto level = [&](int r) -> double {
+        double v = n != w.outcomp ? 0.0 : (w.edge ? half(w.s0[r] + w.s0[r + 1]) : w.s0[r]);
+        for (int d = 0; d < RD; ++d) {
+            const int m = idx[d];
+            if (a.per[d] || (m >= a.lo[d] && m <= a.hi[d])) continue;
+            const bool below = m < a.lo[d];
+            const double g = v;
+            v = phys_value(below ? bc.lo[d] : bc.hi[d], m == (below ? a.lo[d] - 1 : a.hi[d] + 1),
+                           a.hi[d] - a.lo[d] + 1, 0, [&](int) { return g; });
+        }
+        return v;
+    };
+    const int m = idx[RD], lo = a.lo[RD], hi = a.hi[RD], ext = hi - lo + 1;
+    if (m >= lo && m <= hi) return level(m);
+    if (a.per[RD]) return level(m < lo ? m + ext : m - ext);
+    if (m < lo) return phys_value(bc.lo[RD], m == lo - 1, ext, lo - 1 - m, [&](int q) { return level(lo + q); });
+    return phys_value(bc.hi[RD], m == hi + 1, ext, m - hi - 1, [&](int q) { return level(hi - q); });
+}
 template <int ND>
 __global__ void k_put1d_filled(KARGS, const __grid_constant__ Put1dArgs a) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    const auto& w = a.w[R[e_].pad];
+    const int job = R[e_].pad;
+    const auto& w = a.w[job];
     const FabView out = VW(w.f);
-    const int idx[3] = {i, j, k};
     constexpr int RD = ND - 1;
-    for (int n = 0; n < w.nc; ++n) {
-        const BCRecD bc = w.bcs[n];
-        // the value over the radial index r at this (i, j): the array, then the rules across it
-        auto level = [&](int r) -> double {
-            double v = n != w.outcomp ? 0.0 : (w.edge ? half(w.s0[r] + w.s0[r + 1]) : w.s0[r]);
+    const int idx[3] = {i, j, k};
+    bool plain = true;
 #pragma unroll
-            for (int d = 0; d < RD; ++d) {
-                const int m = idx[d];
-                if (a.per[d] || (m >= a.lo[d] && m <= a.hi[d])) continue;
-                const bool below = m < a.lo[d];
-                const double g = v;
-                v = phys_value(below ? bc.lo[d] : bc.hi[d], m == (below ? a.lo[d] - 1 : a.hi[d] + 1),
-                               a.hi[d] - a.lo[d] + 1, 0, [&](int) { return g; });
-            }
-            return v;
-        };
-        const int m = idx[RD], lo = a.lo[RD], hi = a.hi[RD], ext = hi - lo + 1;
-        double v;
-        if (m >= lo && m <= hi) v = level(m);
-        else if (a.per[RD]) v = level(m < lo ? m + ext : m - ext);
-        else if (m < lo) v = phys_value(bc.lo[RD], m == lo - 1, ext, lo - 1 - m, [&](int q) { return level(lo + q); });
-        else v = phys_value(bc.hi[RD], m == hi + 1, ext, m - hi - 1, [&](int q) { return level(hi - q); });
-        at(out, i, j, k, n) = v;
+    for (int d = 0; d < ND; ++d) plain = plain && (a.per[d] || (idx[d] >= a.lo[d] && idx[d] <= a.hi[d]));
+    if (plain) {
+        int r = idx[RD];
+        const int ext = a.hi[RD] - a.lo[RD] + 1;
+        r += r < a.lo[RD] ? ext : (r > a.hi[RD] ? -ext : 0);
+        const double v = w.edge ? half(w.s0[r] + w.s0[r + 1]) : w.s0[r];
+        for (int n = 0; n < w.nc; ++n) at(out, i, j, k, n) = n == w.outcomp ? v : 0.0;
+    } else {
+        for (int n = 0; n < w.nc; ++n) at(out, i, j, k, n) = put1d_behind<ND>(a, job, n, i, j, k);
     }
 }
 
@@ -265,7 +280,6 @@ void fill_patch(Ctx& c, int fid, const FillRange& a, const FillRange& b) {
 __global__ void k_umac_ghost(KARGS, int f0, int dd, int bclo, int bchi, int dlo, int dhi) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const int I = dd == 0 ? i : (dd == 1 ? j : k);
-    if (I != dlo - 1 && I != dhi + 2) return;
     const int di = dd == 0, dj = dd == 1, dk = dd == 2;
     const FabView q[3] = {VW(f0), VW(f0 + 1), VW(f0 + 2)};
     if (I == dlo - 1) {
@@ -319,11 +333,32 @@ __global__ void k_umac_ghost(KARGS, int f0, int dd, int bclo, int bchi, int dlo,
     }
 }
 
+// The planes dlo - 1 and dhi + 2 of the boxes' dd-faces grown by one
+static const RegionTable& ghost_planes(Ctx& c, int dd) {
+    const std::array<int, 8> key{1002, dd, 0, 0, 0, 0, 0, 0};
+    auto it = c.regions.find(key);
+    if (it != c.regions.end()) return it->second;
+    const std::vector<RegionBox> grown = region(c, 1, 1, 1, 1, 1, 1, dd).h;
+    RegionTable& t = c.regions[key];
+    for (const RegionBox& g : grown)
+        for (int I : {c.P.dom_lo[dd] - 1, c.P.dom_hi[dd] + 2}) {
+            if (I < g.lo[dd] || I >= g.lo[dd] + g.n[dd]) continue;
+            RegionBox r = g;
+            r.lo[dd] = I;
+            r.n[dd] = 1;
+            r.start = t.total;
+            t.total += (long)r.n[0] * r.n[1] * r.n[2];
+            t.h.push_back(r);
+        }
+    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    return t;
+}
+
 void fill_face_ghosts(Ctx& c, int f0) {
     copy_pieces(c, copy_table_faces(c, c.F[f0].spec.ng), f0, 0, 1, 0, 0);
     for (int dd = 0; dd < 3; ++dd) {
         if (c.per[dd]) continue;
-        const RegionTable& rt = region(c, 1, 1, 1, 1, 1, 1, dd);
+        const RegionTable& rt = ghost_planes(c, dd);
         launch(c, rt, 1, k_umac_ghost, c.V(), f0, dd, c.P.phys_bc_lo[dd], c.P.phys_bc_hi[dd], c.P.dom_lo[dd],
                c.P.dom_hi[dd]);
     }
@@ -676,8 +711,9 @@ __global__ void k_vel_force(KARGS, double cutoff_rho, int domhi, RecipC r2dz, in
     const double r = at(rho, i, j, k, RHO);
     double rhopert = r - at(VW(F_RHO0CART), i, j, k);
     if (r < cutoff_rho) rhopert = 0.0;
-    for (int dim = 0; dim < 2; ++dim) at(vf, i, j, k, dim) = -at(gpi, i, j, k, dim) / r;
-    double f2 = (rhopert * at(VW(F_GRAVCART), i, j, k, 2) - at(gpi, i, j, k, 2)) / r - at(VW(F_W0FCART), i, j, k, 2);
+    const RecipV rr = recip_v(r);  // three quotients by the density: 10 + 3 x 4 FP64 instructions, not 3 x 10
+    for (int dim = 0; dim < 2; ++dim) at(vf, i, j, k, dim) = div_v(-at(gpi, i, j, k, dim), rr);
+    double f2 = div_v(rhopert * at(VW(F_GRAVCART), i, j, k, 2) - at(gpi, i, j, k, 2), rr) - at(VW(F_W0FCART), i, j, k, 2);
     if (k <= -1 || k >= domhi) {
     } else {
         const FabView we = VW(fe + 2), w0 = VW(F_W0CART);
@@ -1382,15 +1418,16 @@ __device__ __forceinline__ void rhox_flux_face(const FabView* __restrict__ V, in
     const FabView fl = VW(F_SFLUX0 + D), e = VW(F_SEDGE0 + D);
     const double u = at(VW(F_UMAC0 + D), i, j, k);
     double frho = c0 == FIRSTSPEC ? 0.0 : at(fl, i, j, k, RHO);
+    // the species' common factor, u times the edge density, once: it took two of five FP64
+    // instructions of each species (the compiler cannot hoist what the stores below might change)
+    double m = u;
+    if (spt == 1) m = u * (half(r0o[k] + r0n[k]) + at(e, i, j, k, RHO));
+    else if (spt != 2) m = u * at(e, i, j, k, RHO);
     // etarhoflux is accumulated into species by species, as the reference does (:170-178)
     double eta = D == 2 && do_eta ? at(VW(F_ETA), i, j, k) : 0.0;
     for (int comp = c0; comp < c0 + nc; ++comp) {
         const int ec = slot >= 0 ? slot : comp;
-        const double rho0_edge = half(r0o[k] + r0n[k]);
-        double f = 0.0;
-        if (spt == 1) f = u * (rho0_edge + at(e, i, j, k, RHO)) * at(e, i, j, k, ec);
-        else if (spt == 2) f = u * at(e, i, j, k, ec);
-        else f = u * at(e, i, j, k, RHO) * at(e, i, j, k, ec);
+        const double f = m * at(e, i, j, k, ec);
         at(fl, i, j, k, ec) = f;
         if (D == 2 && do_eta) {
             eta += f;
@@ -1566,9 +1603,11 @@ __device__ __forceinline__ void rhox_fix_cell(const FabView* __restrict__ V, int
                 double sumX = 0.0;
                 for (int c2 = FIRSTSPEC; c2 < FIRSTSPEC + nspec; ++c2)
                     if (c2 != comp && at(sn, i, j, k, c2) >= 0.0) sumX += at(sn, i, j, k, c2);
+                // every species over the same sum: its reciprocal once, then 4 FP64 instructions each
+                const RecipV rs = recip_v(sumX);
                 for (int c2 = FIRSTSPEC; c2 < FIRSTSPEC + nspec; ++c2)
                     if (c2 != comp && at(sn, i, j, k, c2) >= 0.0) {
-                        const double frac = at(sn, i, j, k, c2) / sumX;
+                        const double frac = div_v(at(sn, i, j, k, c2), rs);
                         at(sn, i, j, k, c2) -= frac * delta;
                     }
                 at(sn, i, j, k, comp) = 0.0;
@@ -2268,9 +2307,11 @@ __global__ void k_update_rhox_2d(KARGS, int nspec, double dt, double dx0, double
                 double sumX = 0.0;
                 for (int c2 = FIRSTSPEC; c2 < FIRSTSPEC + nspec; ++c2)
                     if (c2 != comp && at(sn, i, j, k, c2) >= 0.0) sumX += at(sn, i, j, k, c2);
+                // every species over the same sum: its reciprocal once, then 4 FP64 instructions each
+                const RecipV rs = recip_v(sumX);
                 for (int c2 = FIRSTSPEC; c2 < FIRSTSPEC + nspec; ++c2)
                     if (c2 != comp && at(sn, i, j, k, c2) >= 0.0) {
-                        const double frac = at(sn, i, j, k, c2) / sumX;
+                        const double frac = div_v(at(sn, i, j, k, c2), rs);
                         at(sn, i, j, k, c2) -= frac * delta;
                     }
                 at(sn, i, j, k, comp) = 0.0;

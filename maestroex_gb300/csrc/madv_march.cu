@@ -498,37 +498,44 @@ __global__ void __launch_bounds__(256) k_es_trans(KARGS, int comp0, unsigned nq,
     else es_trans<2, CONS>(V, nb, b, i, j, k, k1, bi, bj, bk0, bk1, comp0 + q, q, rules, epsb);
 }
 
-// Edge states of D-faces (MakeEdgeScalEdges, Source/MaestroMakeEdgeScalars.cpp:1361-1667).
+// Edge states of D-faces (MakeEdgeScalEdges, Source/MaestroMakeEdgeScalars.cpp:1361-1667): what the
+// faces of a column read, with pointers at the cell above the face.
 template <int D, bool CONS>
-__device__ __forceinline__ void es_edge(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int k1, int comp,
-                                        int oc0, int q, const EsRules& rules, int force_zero, int ptf, double dt2,
-                                        long long epsb, const EsCons& ec) {
-    constexpr int A = D == 0 ? 1 : 0, B = D == 2 ? 1 : 2;
-    constexpr int di = D == 0, dj = D == 1, dk = D == 2;
-    const EsBox x = es_box(V, nb, b);
-    const FabView uv = VW(F_UMAC0 + D), e = VW(F_SEDGE0 + D), f = VW(F_SCALFORCE);
-    const double* pu = &at(uv, i, j, k);
-    const long uk = uv.sk;
-    const long o = x.off(i, j, k), s = x.s<D>(), sa = x.s<A>(), sb = x.s<B>();
-    const double *ip = VW(F_IPC0 + q).p + o + D * x.sn, *im = VW(F_IMC0 + q).p + o + D * x.sn;
-    const double *ta = x.tc + o + (3 + A) * x.sn, *tb = x.tc + o + (3 + B) * x.sn;
-    const double *qa = VW(trans_field(A, B)).p + o + q * x.sn, *qb = VW(trans_field(B, A)).p + o + q * x.sn;
-    double* out = &at(e, i, j, k, oc0 + q);
-    // force: the field's, or (traced) Ip of the cell below, Im of the one above
-    const long fs = ptf ? s : (di ? 1 : (dj ? f.sj : f.sk)), fk = ptf ? x.s2 : f.sk;
-    const double *fp = nullptr, *fm = nullptr;
-    if (!force_zero) {
-        fp = ptf ? VW(F_IPF).p + o + D * x.sn : &at(f, i, j, k, comp);
-        fm = ptf ? VW(F_IMF).p + o + D * x.sn : fp;
+struct EsFace {
+    static constexpr int A = D == 0 ? 1 : 0, B = D == 2 ? 1 : 2;
+    static constexpr int di = D == 0, dj = D == 1, dk = D == 2;
+    const double *ip, *im, *ta, *tb, *qa, *qb, *fp, *fm;
+    long s, sa, sb, s2, fs, fk;
+    __device__ __forceinline__ EsFace(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int comp, int q,
+                                      int force_zero, int ptf) {
+        const EsBox x = es_box(V, nb, b);
+        const long o = x.off(i, j, k);
+        s = x.s<D>(), sa = x.s<A>(), sb = x.s<B>(), s2 = x.s2;
+        ip = VW(F_IPC0 + q).p + o + D * x.sn, im = VW(F_IMC0 + q).p + o + D * x.sn;
+        ta = x.tc + o + (3 + A) * x.sn, tb = x.tc + o + (3 + B) * x.sn;
+        qa = VW(trans_field(A, B)).p + o + q * x.sn, qb = VW(trans_field(B, A)).p + o + q * x.sn;
+        // force: the field's, or (traced) Ip of the cell below, Im of the one above
+        const FabView f = VW(F_SCALFORCE);
+        fs = ptf ? s : (di ? 1 : (dj ? f.sj : f.sk)), fk = ptf ? x.s2 : f.sk;
+        fp = fm = nullptr;
+        if (!force_zero) {
+            fp = ptf ? VW(F_IPF).p + o + D * x.sn : &at(f, i, j, k, comp);
+            fm = ptf ? VW(F_IMF).p + o + D * x.sn : fp;
+        }
     }
-    // the corrected state of the cell below the face, or above
-    auto state = [&](bool below, unsigned code) {
-        const long c = below ? -s : 0;
+    // the corrected state of the cell below the face, or above (CLAMP: and clamped at a boundary)
+    template <bool CLAMP>
+    __device__ __forceinline__ double state(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int comp,
+                                            bool below, int force_zero, double dt2, const EsCons& ec) const {
+        long c = below ? -s : 0;
+        // (kept from the compiler: folded into an address, the -1 of D = 0 came out wrong for the
+        // second state of a tie with u < 0)
+        asm("" : "+l"(c));
         double v = (below ? ip : im)[c];
-        if (code == FR_CLAMP) v = clamp_out(v, below);
+        if (CLAMP) v = clamp_out(v, below);
         if (CONS) {
             const int m = below ? -1 : 0, ci = i + m * di, cj = j + m * dj, ck = k + m * dk;
-            const FabView ua = VW(F_UMAC0 + A), ub = VW(F_UMAC0 + B), sv = VW(F_SOLD);
+            const FabView ua = VW(F_UMAC0 + A), ub = VW(F_UMAC0 + B), uv = VW(F_UMAC0 + D), sv = VW(F_SOLD);
             const double a0 = at(ua, ci, cj, ck), a1 = at(ua, ci + (A == 0), cj + (A == 1), ck + (A == 2));
             const double b0 = at(ub, ci, cj, ck), b1 = at(ub, ci + (B == 0), cj + (B == 1), ck + (B == 2));
             const double d0 = at(uv, ci, cj, ck), d1 = at(uv, ci + di, cj + dj, ck + dk);
@@ -538,29 +545,58 @@ __device__ __forceinline__ void es_edge(const FabView* __restrict__ V, int nb, i
             v = v - ta[c] * (qa[c + sa] - qa[c]) - tb[c] * (qb[c + sb] - qb[c]);
         }
         if (!force_zero) v = v + dt2 * (below ? fp[-fs] : fm[0]);
-        if (code == FR_CLAMP) v = clamp_out(v, below);
+        if (CLAMP) v = clamp_out(v, below);
         return v;
-    };
+    }
+};
+
+// a boundary face's state by its rule.  A call of its own: inlined, the clamps' four FP64
+// comparisons ran on every face, where an interior one needs 6 FP64 instructions (8 with a force).
+template <int D, bool CONS>
+__device__ __noinline__ double es_edge_bnd(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int comp, int q,
+                                           unsigned rule, int force_zero, int ptf, double dt2, const EsCons& ec) {
+    const unsigned code = rule & 7;
+    const bool below = rule & 8;
+    if (code == FR_ZERO) return 0.0;
+    if (code == FR_GHOST) return *es_ghost(V, nb, b, i, j, k, D, below ? 0 : -1, comp);
+    const EsFace<D, CONS> x(V, nb, b, i, j, k, comp, q, force_zero, ptf);
+    return code == FR_CLAMP ? x.template state<true>(V, nb, b, i, j, k, comp, below, force_zero, dt2, ec)
+                            : x.template state<false>(V, nb, b, i, j, k, comp, below, force_zero, dt2, ec);
+}
+
+template <int D, bool CONS>
+__device__ __forceinline__ void es_edge(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int k1, int comp,
+                                        int oc0, int q, const EsRules& rules, int force_zero, int ptf, double dt2,
+                                        long long epsb, const EsCons& ec) {
+    EsFace<D, CONS> x(V, nb, b, i, j, k, comp, q, force_zero, ptf);
+    const FabView uv = VW(F_UMAC0 + D), e = VW(F_SEDGE0 + D);
+    const double* pu = &at(uv, i, j, k);
+    const long uk = uv.sk;
+    double* out = &at(e, i, j, k, oc0 + q);
     double u = *pu;
     for (; k < k1; ++k) {
         double un = 0;
         if (k + 1 < k1) un = pu[uk];
-        const bool left = dhigh(u) >= 0;
         const int side = face_side<D>(rules, D == 0 ? i : (D == 1 ? j : k));
-        const unsigned r = side ? face_rule<D>(rules, q, side) : 0, code = r & 7;
-        const bool first = code ? (r & 8) != 0 : left;
-        double v = state(first, code);
-        if (dmag(u) <= epsb && !code) v = half(v + state(!left, 0));  // the mean of both sides
-        if (code == FR_ZERO) v = 0.0;
-        else if (code == FR_GHOST) v = *es_ghost(V, nb, b, i, j, k, D, r & 8 ? 0 : -1, comp);
+        const unsigned r = side ? face_rule<D>(rules, q, side) : 0;
+        double v;
+        if (r) {
+            v = es_edge_bnd<D, CONS>(V, nb, b, i, j, k, comp, q, r, force_zero, ptf, dt2, ec);
+        } else {
+            const bool left = dhigh(u) >= 0;
+            v = x.template state<false>(V, nb, b, i, j, k, comp, left, force_zero, dt2, ec);
+            if (dmag(u) <= epsb)  // the mean of both sides
+                v = half(v + x.template state<false>(V, nb, b, i, j, k, comp, !left, force_zero, dt2, ec));
+        }
         *out = v;
         u = un;
-        pu += uk, ip += x.s2, im += x.s2, ta += x.s2, tb += x.s2, qa += x.s2, qb += x.s2, fp += fk, fm += fk;
+        pu += uk, x.ip += x.s2, x.im += x.s2, x.ta += x.s2, x.tb += x.s2, x.qa += x.s2, x.qb += x.s2;
+        x.fp += x.fk, x.fm += x.fk;
         out += e.sk;
     }
 }
 template <bool CONS>
-__global__ void __launch_bounds__(256) k_es_edge(KARGS, int comp0, int oc0, unsigned nq, EsRules rules, int force_zero,
+__global__ void __launch_bounds__(256, CONS ? 2 : 4) k_es_edge(KARGS, int comp0, int oc0, unsigned nq, EsRules rules, int force_zero,
                                                   int ptf, double dt2, long long epsb, EsCons ec) {
     MADV_ES_COLUMN();
     if (dir == 0) es_edge<0, CONS>(V, nb, b, i, j, k, k1, comp0 + q, oc0, q, rules, force_zero, ptf, dt2, epsb, ec);
@@ -571,7 +607,7 @@ __global__ void __launch_bounds__(256) k_es_edge(KARGS, int comp0, int oc0, unsi
 // Regions of the three directions one after the other (pad = D): the faces (nodal) or cells of
 // direction D, grown by g across it, in z columns of at most ES_LEN cells -- shorter where the
 // level has too few of them to fill the chip (about 2^19 threads).
-constexpr long ES_LEN = 8;
+constexpr long ES_LEN = 16;
 static const RegionTable& dirs_region(Ctx& c, bool nodal, int g) {
     const std::array<int, 8> key{1001, nodal, g, 0, 0, 0, 0, 0};
     auto it = c.regions.find(key);

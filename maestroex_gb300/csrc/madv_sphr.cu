@@ -293,8 +293,9 @@ __global__ void k_vel_force_sph(KARGS, double cutoff_rho, SphGeo g, int fe) {
     const double r = at(VW(F_SOLD), i, j, k, RHO);
     double rhopert = r - at(VW(F_RHO0CART), i, j, k);
     if (r < cutoff_rho) rhopert = 0.0;
+    const RecipV rr = recip_v(r);
     for (int dim = 0; dim < 3; ++dim)
-        at(vf, i, j, k, dim) = (rhopert * at(grav, i, j, k, dim) - at(gpi, i, j, k, dim)) / r - at(w0f, i, j, k, dim);
+        at(vf, i, j, k, dim) = div_v(rhopert * at(grav, i, j, k, dim) - at(gpi, i, j, k, dim), rr) - at(w0f, i, j, k, dim);
     const FabView ue = VW(fe), ve = VW(fe + 1), we = VW(fe + 2);
     const double ut_dot_er = half(at(ue, i, j, k) + at(ue, i + 1, j, k)) * nrm[0] +
                              half(at(ve, i, j, k) + at(ve, i, j + 1, k)) * nrm[1] +
