@@ -43,16 +43,34 @@ __device__ __forceinline__ bool ppm2_face_out(double se, double a, double b) {
     const long long ks = dkey(se), ka = dkey(a), kb = dkey(b);
     return (ks > ka && ks > kb) || (ks < ka && ks < kb);
 }
+// Colella's limited curvature max(min(a, 1.25 min of the signed curvatures), 0), a >= 0, as
+// mx(mn(..), 0) of FP64 comparisons gives it.  Finite ones: the smallest positive curvature by its
+// bit pattern (x -> RN(1.25 x) keeps the order), 0 where one is not positive -- one FP64
+// instruction instead of six or eight.
+__device__ __forceinline__ bool all_finite(double a, double b, double c) {
+    return max(max(dmag(a), dmag(b)), dmag(c)) < 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ double limited_curvature(double a, double fl, double fr) {
+    const double C = 1.25;
+    if (!all_finite(a, fl, fr)) return mx(mn(C * fl, mn(C * fr, a)), 0.0);
+    const long long m = min(dbits(fl), dbits(fr));
+    if (m <= 0) {
+        // the comparisons' zero: -0 where the first of the smallest is one
+        const bool mz = !nz(fl) ? dbits(fl) < 0 : dbits(fr) < 0;
+        return lt0(fl) || lt0(fr) || !mz ? 0.0 : -0.0;
+    }
+    return __longlong_as_double(min(dbits(C * __longlong_as_double(m)), dbits(a)));
+}
+
 // the limited value of one that does
 template <typename SF>
 __device__ __forceinline__ double ppm2_face_limit(SF S, int m, double se, const RecipC& r6) {
-    const double C = 1.25;
     if (prod_gt0(se - S(m - 1), se - S(m))) {
         double D2 = 3.0 * (S(m - 1) - twice(se) + S(m));
         double D2L = S(m - 2) - twice(S(m - 1)) + S(m);
         double D2R = S(m - 1) - twice(S(m)) + S(m + 1);
         const bool neg = dhigh(D2) < 0;  // sgn = copysign(1, D2): sgn * x is x or -x
-        double D2LIM = dflip(mx(mn(C * dflip(D2L, neg), mn(C * dflip(D2R, neg), dabs(D2))), 0.0), neg);
+        double D2LIM = dflip(limited_curvature(dabs(D2), dflip(D2L, neg), dflip(D2R, neg)), neg);
         se = half(S(m - 1) + S(m)) - div_6(D2LIM, r6);
     }
     return se;
@@ -173,7 +191,6 @@ __device__ __forceinline__ void ppm_cell_any(SF S, FF F, RF FR, int I, int lo_ex
             }
         }
     } else {
-        const double C = 1.25;
         double sedgel = Fc(-1), sedge = Fc(0), sedger = Fc(1), sedgerr = Fc(2);
         if (D == 0 && hi_ext && I == domhi - 1) sedgerr = FR(2);
         if (lo_ext && I == domlo) {
@@ -208,11 +225,20 @@ __device__ __forceinline__ void ppm_cell_any(SF S, FF F, RF FR, int I, int lo_ex
                 double D2R = s0 - twice(S(1)) + S(2);
                 double D2C = S(-1) - twice(s0) + S(1);
                 const bool neg = dhigh(D2) < 0;  // sgn = copysign(1, D2)
-                double D2LIM = mx(mn(dabs(D2), mn(C * dflip(D2L, neg), mn(C * dflip(D2R, neg), C * dflip(D2C, neg)))), 0.0);
+                const double fl = dflip(D2L, neg), fr = dflip(D2R, neg), fc = dflip(D2C, neg), a = dabs(D2);
+                const double C = 1.25;
+                double D2LIM;
+                if (all_finite(fl, fr, fc) && dmag(a) < 0x7ff0000000000000LL) {
+                    const long long m = min(min(dbits(fl), dbits(fr)), dbits(fc));
+                    D2LIM = m <= 0 ? 0.0 : __longlong_as_double(min(dbits(C * __longlong_as_double(m)), dbits(a)));
+                } else {
+                    D2LIM = mx(mn(a, mn(C * fl, mn(C * fr, C * fc))), 0.0);
+                }
                 if (nz(D2LIM) || !finite2(alpham, alphap)) {
-                    double D2ABS = mx(dabs(D2), 1.e-10);
-                    alpham = alpham * D2LIM / D2ABS;
-                    alphap = alphap * D2LIM / D2ABS;
+                    // one divisor: its reciprocal, then 4 FP64 instructions a quotient
+                    const RecipV r = recip_v(mx(a, 1.e-10));
+                    alpham = div_v(alpham * D2LIM, r);
+                    alphap = div_v(alphap * D2LIM, r);
                 } else {  // a finite alpha times 0 over a positive number: the zero of its sign
                     alpham = dsigned(0.0, alpham);
                     alphap = dsigned(0.0, alphap);
