@@ -548,7 +548,9 @@ static void put1d_h(Hier& H, int fid, const char* s0, int outcomp, int nc, int e
     put1d_h(H, {{fid, s0, outcomp, nc, edge, which_bcs, bc_c0, is_vel, state_c0}});
 }
 // Maestro::Addw0 (Source/MaestroFill3dData.cpp:357-462)
-static void addw0_h(Hier& H, int f0, double mult) {
+// fills: how often sync_faces_h has filled the ghost faces since their faces were formed
+static void addw0_h(Hier& H, int f0, double mult, int fills = 0) {
+    if (fills >= 2 && H.n() == 1 && addw0_fills(H[0])) return addw0_filled(H[0], f0, mult);
     for (auto* c : H.L) addw0(*c, f0, mult);
     sync_faces_h(H, f0);
 }
@@ -756,16 +758,16 @@ static void flux_sync_one_h(Hier& H, int comp, int slot) {
 //   back before the species do (converting X back to rho X reads the full density);
 // * the closing pass (density from the species' changes, floor, negative-species fix) and
 //   the reflux follow the last species, as in UpdateScal.
-static void density_advance_streamed(Hier& H, int which_step) {
+static void density_advance_streamed(Hier& H, int which_step, int fills) {
     constexpr int SLOT = 2;
     const int spt = H[0].P.species_pred_type;
     const int ns = H[0].nspec, nscal = H[0].nscal;
     for (auto* c : H.L) set_val(*c, F_SCALFORCE, 0.0, 0, nscal, c->F[F_SCALFORCE].spec.ng);
     put1d_h(H, F_RHO0CART, "rho0_old", 0, 1, 0, BCS_S, RHO, 0, RHO);
-    addw0_h(H, F_UMAC0, -1.0);
+    addw0_h(H, F_UMAC0, -1.0, fills);
     if (spt == 1) modify_scal_force_h(H, RHO, nullptr, "rho0_edge_old", F_RHO0CART, 0);
     else if (spt == 3) modify_scal_force_h(H, RHO, nullptr, "rho0_edge_old", F_RHO0CART, 1);
-    addw0_h(H, F_UMAC0, 1.0);
+    addw0_h(H, F_UMAC0, 1.0, fills + 1);
     if (spt == 1 || spt == 3) convert_rhox_to_x_h(H, 1);
     if (spt == 1) put_in_pert_form_h(H, "rho0_old", RHO, 0, BCS_F, 1);
     const int cons = spt == 2;  // the species' form; rho's edge state is advective
@@ -802,16 +804,17 @@ static void density_advance_streamed(Hier& H, int which_step) {
 
 // Maestro::DensityAdvance (Source/MaestroDensityAdvance.cpp:6-243); which_step 2 passes the
 // new base state to the fluxes (:186-219)
-static void density_advance(Hier& H, int which_step, bool stream = false) {
-    if (stream) return density_advance_streamed(H, which_step);
+// (fills: of the MAC velocities' ghost faces, see addw0_h)
+static void density_advance(Hier& H, int which_step, bool stream = false, int fills = 0) {
+    if (stream) return density_advance_streamed(H, which_step, fills);
     const int spt = H[0].P.species_pred_type;
     const int ns = H[0].nspec, nscal = H[0].nscal;
     for (auto* c : H.L) set_val(*c, F_SCALFORCE, 0.0, 0, nscal, c->F[F_SCALFORCE].spec.ng);
     put1d_h(H, F_RHO0CART, "rho0_old", 0, 1, 0, BCS_S, RHO, 0, RHO);
-    addw0_h(H, F_UMAC0, -1.0);
+    addw0_h(H, F_UMAC0, -1.0, fills);
     if (spt == 1) modify_scal_force_h(H, RHO, nullptr, "rho0_edge_old", F_RHO0CART, 0);
     else if (spt == 3) modify_scal_force_h(H, RHO, nullptr, "rho0_edge_old", F_RHO0CART, 1);
-    addw0_h(H, F_UMAC0, 1.0);
+    addw0_h(H, F_UMAC0, 1.0, fills + 1);
     if (spt == 1 || spt == 3) to_prediction_form_h(H, 1, spt == 1);
     for (auto* c : H.L) make_edge_scal(*c, FIRSTSPEC, ns, BCS_S, spt == 2, 1);  // no force for X / rho X
     if (spt == 1 || spt == 3)  // the same velocities: their coefficients are there
@@ -872,21 +875,21 @@ static void rhoh_flux_h(Hier& H, int which_step) {
                        c->b1("rho0_edge_old"), c->b1(r0n), c->b1(r0en));
 }
 
-static void enthalpy_advance(Hier& H, int which_step, bool stream = false) {
+static void enthalpy_advance(Hier& H, int which_step, bool stream = false, int fills = 0) {
     const int ept = H[0].P.enthalpy_pred_type;
     const int nscal = H[0].nscal;
     // predict_h: (rho h) -> h (Source/MaestroEnthalpyAdvance.cpp:40-43)
     if (ept == 2) convert_rhoh_to_h_h(H, 1);
     // scal_force.setVal(0) (Source/MaestroEnthalpyAdvance.cpp:51); the enthalpy half reads RhoH only
     for (auto* c : H.L) set_val(*c, F_SCALFORCE, 0.0, RHOH, 1, c->F[F_SCALFORCE].spec.ng);
-    addw0_h(H, F_UMAC0, -1.0);
+    addw0_h(H, F_UMAC0, -1.0, fills);
     make_rhoh_force_h(H, 1, 1, 1);
     if (ept == 1) {
         modify_scal_force_h(H, RHOH, "rhoh0_old", "rhoh0_edge_old", F_RHOH0CART, 0);
     }
     if (ept == 2)  // the force of h: the (rho h) force over rho (:80-88)
         for (auto* c : H.L) h_force(*c);
-    addw0_h(H, F_UMAC0, 1.0);
+    addw0_h(H, F_UMAC0, 1.0, fills + 1);
     if (ept == 1) put_in_pert_form_h(H, "rhoh0_old", RHOH, 0, BCS_F, 1);
     for (auto* c : H.L) make_edge_scal(*c, RHOH, 1, BCS_S, ept == 0, 0);
     if (ept == 1) put_in_pert_form_h(H, "rhoh0_old", RHOH, RHOH, BCS_S, 0);
@@ -894,9 +897,9 @@ static void enthalpy_advance(Hier& H, int which_step, bool stream = false) {
     rhoh_flux_h(H, which_step);
     flux_sync_h(H, RHOH, 1, stream);
     for (auto* c : H.L) set_val(*c, F_SCALFORCE, 0.0, RHOH, 1, c->F[F_SCALFORCE].spec.ng);
-    addw0_h(H, F_UMAC0, -1.0);
+    addw0_h(H, F_UMAC0, -1.0, fills + 2);
     make_rhoh_force_h(H, 0, 0, which_step);
-    addw0_h(H, F_UMAC0, 1.0);
+    addw0_h(H, F_UMAC0, 1.0, fills + 3);
     update_scal_h(H, RHOH);
 }
 
@@ -1166,11 +1169,11 @@ static void stage_body(Hier& H, const std::vector<StageIO>& io) {
     const bool stream = io[0].stream;
     advance_premac(H);
     addw0_h(H, F_UMAC0, 1.0);
-    density_advance(H, 1, stream);
-    addw0_h(H, F_UMAC0, -1.0);
-    addw0_h(H, F_UMAC0, 1.0);
-    enthalpy_advance(H, 1, stream);
-    addw0_h(H, F_UMAC0, -1.0);
+    density_advance(H, 1, stream, 1);
+    addw0_h(H, F_UMAC0, -1.0, 3);
+    addw0_h(H, F_UMAC0, 1.0, 4);
+    enthalpy_advance(H, 1, stream, 5);
+    addw0_h(H, F_UMAC0, -1.0, 9);
     // outputs (valid region)
     for (int l = 0; l < H.n(); ++l) {
         Ctx& c = H[l];
@@ -2355,14 +2358,14 @@ int madv_velocity_advance(madv_ctx* h, const madv_multifab* uold, const madv_mul
         // MakeVelForce(vel_force, umac, sold, rho0_old, grav_cell_old, w0_force_cart, 1)
         copy_fab(c, F_SOLD, RHO, F_USER + U_SOLD, RHO, 1, 0);
         make_vel_force_h(H, F_UMAC0, "rho0_old");
-        addw0_h(H, F_UMAC0, 1.0);
+        addw0_h(H, F_UMAC0, 1.0, 1);
         // MakeEdgeScal(uold, uedge, umac, vel_force, true, bcs_u, AMREX_SPACEDIM, 0, 0, AMREX_SPACEDIM, false)
         copy_fab(c, F_SOLD, 0, F_USER + U_UOLD, 0, 3, 0);
         fill_patch_h(H, F_SOLD, 0, 3, BCS_U, 0, 1, -1);
         copy_fab(c, F_SCALFORCE, 0, F_VELFORCE, 0, 3, c.F[F_VELFORCE].spec.ng);
         for (int d = 0; d < 3; ++d) set_val(c, F_SEDGE0 + d, 0.0, 0, 3, 0);
         make_edge_scal(c, 0, 3, BCS_U, 0, 0, 1);
-        addw0_h(H, F_UMAC0, -1.0);
+        addw0_h(H, F_UMAC0, -1.0, 2);
         // MakeVelForce(vel_force, umac, rhohalf, rho0_nph, grav_cell_nph, w0_force_cart, 1)
         copy_fab(c, F_SOLD, RHO, F_USER + U_RHOHALF, 0, 1, 0);
         make_vel_force_h(H, F_UMAC0, "rho0_avg");

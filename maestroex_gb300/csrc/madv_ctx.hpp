@@ -292,6 +292,8 @@ int mac_project_two_levels(Ctx& c, Ctx& f, int srhs, int srho, int sphi, const d
                            const double* b1, const double* b1e, double tol_rel, int max_iter, int* iters_out,
                            double* ratio_out);
 void addw0(Ctx& c, int f0, double mult);
+bool addw0_fills(const Ctx& c);
+void addw0_filled(Ctx& c, int f0, double mult);  // Addw0 on filled faces, their ghost faces included
 void set_val(Ctx& c, int fid, double v, int c0, int nc, int ngrow);
 void copy_fab(Ctx& c, int dst, int dc0, int src, int sc0, int nc, int ngrow);
 void add_fab(Ctx& c, int dst, int src, int nc, int ngrow);

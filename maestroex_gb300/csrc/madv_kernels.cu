@@ -20,8 +20,34 @@
 #include "madv_launch.cuh"
 #include "madv_ppm.cuh"
 #include "madv_slope.cuh"
+#include <climits>
 
 namespace madv {
+
+// One launch over the faces of every direction (region_union's parts in the order of the
+// directions): a small level's launch takes 2.7 us, whatever it does.
+struct DirRules {
+    int bl[3], bh[3], dl[3], dh[3];  // boundary types and the domain of each direction
+    double h[3];
+};
+static DirRules phys_rules(const Ctx& c, double h0, double h1, double h2) {
+    DirRules p{};
+    for (int d = 0; d < 3; ++d) {
+        p.bl[d] = c.P.phys_bc_lo[d];
+        p.bh[d] = c.P.phys_bc_hi[d];
+        p.dl[d] = c.P.dom_lo[d];
+        p.dh[d] = c.P.dom_hi[d];
+    }
+    p.h[0] = h0;
+    p.h[1] = h1;
+    p.h[2] = h2;
+    return p;
+}
+#define RULES(D) p.bl[D], p.bh[D], p.dl[D], p.dh[D]
+static const RegionTable& rg_faces(Ctx& c) {
+    if (c.ndim == 2) return region_union(c, {{0, 0, 0, 0, 0, 0, 0, -1}, {0, 0, 0, 0, 0, 0, 1, -1}});
+    return region_union(c, {{0, 0, 0, 0, 0, 0, 0, -1}, {0, 0, 0, 0, 0, 0, 1, -1}, {0, 0, 0, 0, 0, 0, 2, -1}});
+}
 
 // ============================================================ elementwise utilities
 __global__ void k_set_val(KARGS, int f, double v, int c0, int nc) {
@@ -253,8 +279,97 @@ __global__ void k_phys_fill(KARGS, int f, int c0, int nc, const BCRecD* __restri
     }
 }
 
+// Every non-periodic direction at once (two or three of them): a ghost cell's value is the rule of
+// the last direction it lies outside in over values that are the rule of the one before, and so
+// on, as the sweeps x, y, z give it; only cells inside the domain along those directions are
+// read.  One launch for three (the full star's stage fills 37 times).
+struct PhysBox {
+    int lo[3], hi[3], per[3];
+};
+template <int D>
+__device__ __noinline__ double phys_corner(const FabView& q, const PhysBox& x, const BCRecD& bc, int i, int j, int k, int n) {
+    const int m = D == 0 ? i : (D == 1 ? j : k);
+    auto below_d = [&](int i2, int j2, int k2) -> double {
+        if constexpr (D == 0) return at(q, i2, j2, k2, n);
+        else return phys_corner<D - 1>(q, x, bc, i2, j2, k2, n);
+    };
+    const bool lo = m < x.lo[D];
+    const int t = lo ? bc.lo[D] : bc.hi[D];
+    if (x.per[D] || (m >= x.lo[D] && m <= x.hi[D]) || t == BC_INT_DIR) return below_d(i, j, k);
+    const int refl = lo ? x.lo[D] - 1 - m : m - x.hi[D] - 1;
+    return phys_value(t, refl == 0, x.hi[D] - x.lo[D] + 1, refl, [&](int w) {
+        const int p = lo ? x.lo[D] + w : x.hi[D] - w;
+        return below_d(D == 0 ? p : i, D == 1 ? p : j, D == 2 ? p : k);
+    });
+}
+__global__ void k_phys_fill_all(KARGS, int f, int c0, int nc, const BCRecD* __restrict__ bcs, int c1, int nc1,
+                                const BCRecD* __restrict__ bcs1, const __grid_constant__ PhysBox x) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    const FabView q = VW(f);
+    const int idx[3] = {i, j, k};
+    int out = 0, d = 0;  // directions the cell lies outside in, and the last of them
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+        if (!x.per[e] && (idx[e] < x.lo[e] || idx[e] > x.hi[e])) ++out, d = e;
+    const int m = idx[d], domlo = x.lo[d], domhi = x.hi[d];
+    const bool below = m < domlo;
+    const int refl = below ? domlo - 1 - m : m - domhi - 1;
+    const long st = d == 0 ? 1 : (d == 1 ? q.sj : q.sk), in = below ? st : -st;
+    for (int p = 0; p < nc + nc1; ++p) {
+        const int n = p < nc ? c0 + p : c1 + p - nc;
+        const BCRecD& bc = p < nc ? bcs[p] : bcs1[p - nc];
+        double* const o = &at(q, i, j, k, n);
+        if (out > 1) {
+            *o = phys_corner<2>(q, x, bc, i, j, k, n);
+            continue;
+        }
+        const int t = below ? bc.lo[d] : bc.hi[d];
+        if (t == BC_INT_DIR) continue;
+        const double* const edge = o + (refl + 1) * in;
+        *o = phys_value(t, refl == 0, domhi - domlo + 1, refl, [&](int w) { return edge[w * in]; });
+    }
+}
+// the cells within ng of the boxes that lie outside the domain in a non-periodic direction
+static const RegionTable& outside_cells(Ctx& c, int ng) {
+    const std::array<int, 8> key{1003, ng, 0, 0, 0, 0, 0, 0};
+    auto it = c.regions.find(key);
+    if (it != c.regions.end()) return it->second;
+    const std::vector<RegionBox> grown = rg_grow(c, ng).h;
+    RegionTable& t = c.regions[key];
+    for (const RegionBox& g : grown) {
+        RegionBox rest = g;  // z slabs (full x, y), then y slabs of the rest, then x slabs
+        for (int d = 2; d >= 0; --d) {
+            if (c.per[d]) continue;
+            const int lo = std::max(rest.lo[d], c.P.dom_lo[d]), hi = std::min(rest.lo[d] + rest.n[d] - 1, c.P.dom_hi[d]);
+            for (int side = 0; side < 2; ++side) {
+                RegionBox r = rest;
+                r.lo[d] = side ? hi + 1 : rest.lo[d];
+                r.n[d] = side ? rest.lo[d] + rest.n[d] - 1 - hi : lo - rest.lo[d];
+                if (r.n[d] <= 0) continue;
+                r.start = t.total;
+                t.total += (long)r.n[0] * r.n[1] * r.n[2];
+                t.h.push_back(r);
+            }
+            rest.lo[d] = lo;
+            rest.n[d] = hi - lo + 1;
+        }
+    }
+    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    return t;
+}
+
 static void phys_ranges(Ctx& c, int fid, int c0, int nc, const BCRecD* bcs, int c1, int nc1, const BCRecD* bcs1) {
     const FieldSpec& s = c.F[fid].spec;
+    if (s.nodal < 0 && !c.per[0] + !c.per[1] + !c.per[2] > 1) {
+        PhysBox x{};
+        for (int d = 0; d < 3; ++d) {
+            x.lo[d] = c.P.dom_lo[d];
+            x.hi[d] = c.P.dom_hi[d];
+            x.per[d] = c.per[d];
+        }
+        launch(c, outside_cells(c, s.ng), 1, k_phys_fill_all, c.V(), fid, c0, nc, bcs, c1, nc1, bcs1, x);
+        return;
+    }
     for (int d = 0; d < 3; ++d) {
         if (c.per[d]) continue;
         const RegionTable& rt = region(c, s.ng, s.ng, s.ng, s.ng, s.ng, s.ng, s.nodal, d);
@@ -374,6 +489,48 @@ void addw0(Ctx& c, int f0, double mult) {
     if (c.sph) return addw0_sph(c, f0, mult);
     if (c.ndim == 2) return addw0_2d(c, f0, mult);
     launch(c, region(c, 1, 1, 0, 1, 1, 0, 2), 1, k_addw0, c.V(), f0 + 2, (const double*)c.b1("w0"), mult);
+}
+
+// Addw0 on face velocities whose ghost faces are filled (fill_face_ghosts), ghost faces included: the
+// radial faces change by their own level's w0, so a ghost face changes as the face that fills
+// it does -- its periodic or neighbouring box's image at the same level, or by FillUmacGhost's
+// rule -- and the fill need not run again.  One launch for three, eight times a stage.  (Bitwise: a
+// copy plus w0 is the copy of the sum.  Filled twice: on the domain's edges the first fill's x
+// planes read what its y and z planes set, so that the ghost faces there settle with the second.)
+template <int ND>
+__global__ void k_addw0_filled(KARGS, int f, const double* __restrict__ w0, double mult,
+                               const __grid_constant__ DirRules p) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    constexpr int RD = ND - 1;
+    const int idx[3] = {i, j, k};
+    const int r = idx[RD], lo = p.dl[RD], hi = p.dh[RD] + 1;
+    // FillUmacGhost's planes across stop short of the box's last radial ghost face
+    const bool last = r == R[e_].lo[RD] + R[e_].n[RD] - 1 && r <= hi;
+#pragma unroll
+    for (int d = 0; d < RD; ++d) {
+        if (idx[d] >= p.dl[d] && idx[d] <= p.dh[d]) continue;
+        const int t = idx[d] < p.dl[d] ? p.bl[d] : p.bh[d];
+        if (last || t == PB_INFLOW || t == PB_SLIPWALL || t == PB_NOSLIPWALL) return;  // stays as it is, or zero
+    }
+    double& v = at(VW(f), i, j, k);
+    if (r >= lo && r <= hi) {
+        v += mult * w0[r];
+        return;
+    }
+    const bool below = r < lo;
+    const int t = below ? p.bl[RD] : p.bh[RD];
+    if (t == PB_INFLOW || t == PB_OUTFLOW) v += mult * w0[below ? lo : hi];
+    else if (t == PB_SYMMETRY) v = dflip(dflip(v) + mult * w0[below ? lo + 1 : hi - 1]);
+}
+
+bool addw0_fills(const Ctx& c) { return !c.sph && !c.per_box && !c.per[c.ndim - 1]; }
+void addw0_filled(Ctx& c, int f0, double mult) {
+    const int rd = c.ndim - 1;
+    DirRules p = phys_rules(c, 0, 0, 0);
+    for (int d = 0; d < rd; ++d)
+        if (c.per[d]) p.dl[d] = INT_MIN, p.dh[d] = INT_MAX;
+    launch(c, region(c, 1, 1, 1, 1, 1, 1, rd), 1, c.ndim == 2 ? k_addw0_filled<2> : k_addw0_filled<3>, c.V(), f0 + rd,
+           (const double*)c.b1("w0"), mult, p);
 }
 
 // ============================================================ PPM
@@ -598,31 +755,6 @@ static void edge_coeffs(Ctx& c, int fu0, bool trace, bool transverse) {
 
 // tracing and transverse coefficients of the MAC velocities
 void edge_scal_coeffs(Ctx& c) { edge_coeffs(c, F_UMAC0, true, true); }
-
-// One launch over the faces of every direction (region_union's parts in the order of the
-// directions): a small level's launch takes 2.7 us, whatever it does.
-struct DirRules {
-    int bl[3], bh[3], dl[3], dh[3];  // boundary types and the domain of each direction
-    double h[3];
-};
-static DirRules phys_rules(const Ctx& c, double h0, double h1, double h2) {
-    DirRules p{};
-    for (int d = 0; d < 3; ++d) {
-        p.bl[d] = c.P.phys_bc_lo[d];
-        p.bh[d] = c.P.phys_bc_hi[d];
-        p.dl[d] = c.P.dom_lo[d];
-        p.dh[d] = c.P.dom_hi[d];
-    }
-    p.h[0] = h0;
-    p.h[1] = h1;
-    p.h[2] = h2;
-    return p;
-}
-#define RULES(D) p.bl[D], p.bh[D], p.dl[D], p.dh[D]
-static const RegionTable& rg_faces(Ctx& c) {
-    if (c.ndim == 2) return region_union(c, {{0, 0, 0, 0, 0, 0, 0, -1}, {0, 0, 0, 0, 0, 0, 1, -1}});
-    return region_union(c, {{0, 0, 0, 0, 0, 0, 0, -1}, {0, 0, 0, 0, 0, 0, 1, -1}, {0, 0, 0, 0, 0, 0, 2, -1}});
-}
 
 // ============================================================ MakeUtrans
 // Face kernel of Maestro::MakeUtrans, 3-D (Source/MaestroMakeUtrans.cpp:304-387, 419-502,
