@@ -762,7 +762,10 @@ static void density_advance_streamed(Hier& H, int which_step, int fills) {
     constexpr int SLOT = 2;
     const int spt = H[0].P.species_pred_type;
     const int ns = H[0].nspec, nscal = H[0].nscal;
-    for (auto* c : H.L) set_val(*c, F_SCALFORCE, 0.0, 0, nscal, c->F[F_SCALFORCE].spec.ng);
+    // one planar level: species_step below; it and the species' edge states read no force
+    const bool fused = H.n() == 1 && !H[0].sph;
+    for (auto* c : H.L)
+        set_val(*c, F_SCALFORCE, 0.0, fused ? RHO : 0, fused ? 1 : nscal, c->F[F_SCALFORCE].spec.ng);
     put1d_h(H, F_RHO0CART, "rho0_old", 0, 1, 0, BCS_S, RHO, 0, RHO);
     addw0_h(H, F_UMAC0, -1.0, fills);
     if (spt == 1) modify_scal_force_h(H, RHO, nullptr, "rho0_edge_old", F_RHO0CART, 0);
@@ -781,9 +784,17 @@ static void density_advance_streamed(Hier& H, int which_step, int fills) {
         make_s0mac_h(H, "rho0_old", F_S0MAC0);
         make_s0mac_h(H, r0n, F_S0MACB0);
     }
+    // (the Rho flux, which only the levels' synchronisation reads, is not formed)
+    if (fused) species_factor(H[0], SLOT, H[0].b1("rho0_old"), H[0].b1("rho0_edge_old"), H[0].b1(r0n), H[0].b1(r0en));
     for (int n = 0; n < ns; ++n) {
         const int comp = FIRSTSPEC + n;
         for (auto* c : H.L) make_edge_scal(*c, comp, 1, BCS_S, cons, 1, 0, SLOT, false);  // no force for X / rho X
+        if (fused) {
+            if (spt == 2) sum_species_edge_step(H[0], SLOT, n == 0);
+            species_step(H[0], comp, SLOT, SLOT, spt != 2);
+            if (spt != 2) fill_patch_h(H, F_SOLD, comp, 1, BCS_S, comp, 0, comp);
+            continue;
+        }
         if (spt == 2)
             for (auto* c : H.L) sum_species_edge_step(*c, SLOT, n == 0);
         if (spt == 1 || spt == 3) {  // X -> rho X (Maestro::ConvertRhoXToX, flag false)

@@ -350,6 +350,11 @@ void update_scal(Ctx& c, int start_comp);
 // UpdateScal of the species split for streaming: one species from its flux in F_SFLUX* comp
 // `slot`, then the density, floor and negative-species pass over all of them
 void update_species(Ctx& c, int comp, int slot);
+// streamed species on one planar level: the fluxes' common factor, and one species' conversion back,
+// fluxes and update (edge states in component ec, the factor in component fc of F_SFLUX*)
+void species_factor(Ctx& c, int fc, const double* r0_old, const double* r0e_old, const double* r0_new,
+                    const double* r0e_new);
+void species_step(Ctx& c, int comp, int ec, int fc, int conv);
 void update_rhox_fix(Ctx& c);
 void update_vel(Ctx& c, int fu, int fsponge);  // UpdateVel into F_SNEW comps 0-2; fsponge -1: no sponge
 // EstDt maxima of a level into c.d_red[0..6] (spdx, spdy, spdz, spdr, fx, fy, fz as bit patterns)

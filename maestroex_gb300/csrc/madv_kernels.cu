@@ -1754,6 +1754,72 @@ __global__ void k_update_rhox(KARGS, int nspec, double dt, RecipC r0, RecipC r1,
     rhox_fix_cell(V, nb, b, nspec, half_cutoff, i, j, k);
 }
 
+// Streamed species on one planar level: the factor that their fluxes share (u times the edge
+// density), in component fc of F_SFLUX*
+template <int D>
+__device__ __forceinline__ void species_factor(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int fc,
+                                               int spt, const double* __restrict__ r0o, const double* __restrict__ r0n) {
+    const double u = at(VW(F_UMAC0 + D), i, j, k);
+    double m = u;
+    if (spt == 1) m = u * (half(r0o[k] + r0n[k]) + at(VW(F_SEDGE0 + D), i, j, k, RHO));
+    else if (spt != 2) m = u * at(VW(F_SEDGE0 + D), i, j, k, RHO);
+    at(VW(F_SFLUX0 + D), i, j, k, fc) = m;
+}
+__global__ void k_species_factor(KARGS, int fc, int spt, const double* __restrict__ r0o, const double* __restrict__ r0n,
+                                 const double* __restrict__ r0eo, const double* __restrict__ r0en) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    switch (R[e_].pad) {
+        case 0: species_factor<0>(V, nb, b, i, j, k, fc, spt, r0o, r0n); break;
+        case 1: species_factor<1>(V, nb, b, i, j, k, fc, spt, r0o, r0n); break;
+        default: species_factor<2>(V, nb, b, i, j, k, fc, spt, r0eo, r0en);
+    }
+}
+// and one species from its edge states (component ec): X back to rho X (conv), its fluxes through the
+// cell's faces, etarhoflux, and the update -- no force: the species have none.  Nobody else reads
+// a streamed species' fluxes on one level, so they are not stored: 10 fields through memory for
+// the 27 of a conversion, a flux and an update kernel, and 21 FP64 instructions for 30 though each
+// flux is formed in both of its cells.
+__global__ void k_species_step(KARGS, int comp, int ec, int fc, int conv, int do_eta, int last, double dt, RecipC r0,
+                               RecipC r1, RecipC r2, const double* __restrict__ w0, const double* __restrict__ r0pe) {
+    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    const FabView so = VW(F_SOLD), mx_ = VW(F_SFLUX0), my = VW(F_SFLUX1), mz = VW(F_SFLUX2), ex = VW(F_SEDGE0),
+                  ey = VW(F_SEDGE1), ez = VW(F_SEDGE2);
+    const double fx0 = at(mx_, i, j, k, fc) * at(ex, i, j, k, ec), fx1 = at(mx_, i + 1, j, k, fc) * at(ex, i + 1, j, k, ec);
+    const double fy0 = at(my, i, j, k, fc) * at(ey, i, j, k, ec), fy1 = at(my, i, j + 1, k, fc) * at(ey, i, j + 1, k, ec);
+    const double fz0 = at(mz, i, j, k, fc) * at(ez, i, j, k, ec), fz1 = at(mz, i, j, k + 1, fc) * at(ez, i, j, k + 1, ec);
+    double x = at(so, i, j, k, comp);
+    if (conv) {
+        x = x * at(so, i, j, k, RHO);
+        at(so, i, j, k, comp) = x;
+    }
+    double divterm = div_c(fx1 - fx0, r0);
+    divterm += div_c(fy1 - fy0, r1);
+    divterm += div_c(fz1 - fz0, r2);
+    at(VW(F_SNEW), i, j, k, comp) = x + dt * (-divterm + 0.0);
+    if (do_eta) {  // the cell's low face; the box's last cell its high face too
+        const FabView eta = VW(F_ETA);
+        double v = at(eta, i, j, k) + fz0;
+        if (last) v -= w0[k] * r0pe[k];
+        at(eta, i, j, k) = v;
+        if (k == R[e_].lo[2] + R[e_].n[2] - 1) {
+            v = at(eta, i, j, k + 1) + fz1;
+            if (last) v -= w0[k + 1] * r0pe[k + 1];
+            at(eta, i, j, k + 1) = v;
+        }
+    }
+}
+
+void species_factor(Ctx& c, int fc, const double* r0_old, const double* r0e_old, const double* r0_new,
+                    const double* r0e_new) {
+    launch(c, rg_faces(c), 1, k_species_factor, c.V(), fc, c.P.species_pred_type, r0_old, r0_new, r0e_old, r0e_new);
+}
+void species_step(Ctx& c, int comp, int ec, int fc, int conv) {
+    const int do_eta = c.P.evolve_base_state && !c.P.use_exact_base_state;
+    launch(c, rg_grow(c, 0), 1, k_species_step, c.V(), comp, ec, fc, conv, do_eta, (int)(comp == FIRSTSPEC + c.nspec - 1),
+           c.P.dt, make_recip(c.P.dx[0]), make_recip(c.P.dx[1]), make_recip(c.P.dx[2]), (const double*)c.b1("w0"),
+           (const double*)c.b1("rho0_predicted_edge"));
+}
+
 __global__ void k_update_species(KARGS, int comp, int fc, double dt, RecipC r0, RecipC r1, RecipC r2) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     update_species_cell(V, nb, b, comp, fc, dt, r0, r1, r2, i, j, k);
