@@ -584,14 +584,15 @@ static void w0_carts(Hier& H) {
 
 // Maestro::MakeVelForce, planar (Source/MaestroForce.cpp:6-259)
 // fe: the face velocity of the utilde force term (utrans in AdvancePremac, umac in
-// VelocityAdvance); rho0: the base-state density of the buoyancy
-static void make_vel_force_h(Hier& H, int fe = F_UTRANS0, const char* rho0 = "rho0_old") {
+// VelocityAdvance); rho0: the base-state density of the buoyancy; component crho of field
+// frho: the density
+static void make_vel_force_h(Hier& H, int fe = F_UTRANS0, const char* rho0 = "rho0_old", int frho = F_SOLD, int crho = RHO) {
     const int nd = H[0].ndim;
     // spherical, uniform bins: dw0/dr on the cells (Source/MaestroForce.cpp:36-52)
     if (H[0].sph && !H[0].geo.exact) put1d_h(H, F_GRADW0, "gradw0", 0, 1, 0, BCS_U, 0, 1, -1);
     put1d_h(H, {{F_GRAVCART, "grav_cell", nd - 1, nd, 0, BCS_F, 0, 0, -1},
                 {F_RHO0CART, rho0, 0, 1, 0, BCS_S, RHO, 0, RHO}});
-    for (auto* c : H.L) make_vel_force(*c, fe);
+    for (auto* c : H.L) make_vel_force(*c, fe, frho, crho);
     average_down_h(H, F_VELFORCE, 0, nd);
     fill_patch_h(H, F_VELFORCE, 0, nd, BCS_U, 0, 1, -1);
 }
@@ -600,9 +601,13 @@ static void make_vel_force_h(Hier& H, int fe = F_UTRANS0, const char* rho0 = "rh
 static void advance_premac(Hier& H) {
     const int nga = H[0].ng_adv, nd = H[0].ndim;
     fill_patch_h(H, F_UTILDE, 0, nd, BCS_U, 0, 1, -1);
-    for (auto* c : H.L)
-        set_zeros(*c, {{F_UFULL, 0, 3, nga}, {F_UTRANS0, 0, 1, 1}, {F_UTRANS1, 0, 1, 1}, {F_UTRANS2, 0, 1, 1}});
-    if (H.n() == 1 && put1d_fills(H[0])) {  // w0_cart with its ghost cells, as w0_carts forms it
+    const bool w0_fills = H.n() == 1 && put1d_fills(H[0]);
+    for (auto* c : H.L) {
+        std::vector<ZeroJob> z{{F_UTRANS0, 0, 1, 1}, {F_UTRANS1, 0, 1, 1}, {F_UTRANS2, 0, 1, 1}};
+        if (nd == 2 || !w0_fills) z.push_back({F_UFULL, 0, 3, nga});
+        set_zeros(*c, z);
+    }
+    if (w0_fills) {  // w0_cart with its ghost cells, as w0_carts forms it
         put1d_filled(H[0], {{F_UFULL, H[0].b1("w0"), nd - 1, nd, 1, BCS_U, 0}});
     } else {
         for (auto* c : H.L) copy_fab(*c, F_UFULL, 0, F_W0CART, 0, nd, 0);
@@ -682,8 +687,8 @@ static void to_prediction_form_h(Hier& H, int flag, bool pert) {
 // Maestro::UpdateScal (Source/MaestroAdvection.cpp:86-297): the update on every level, then
 // the levels' synchronisation
 static void update_scal_sync_h(Hier& H, int start_comp);
-static void update_scal_h(Hier& H, int start_comp) {
-    for (auto* c : H.L) update_scal(*c, start_comp);
+static void update_scal_h(Hier& H, int start_comp, bool no_force = false) {
+    for (auto* c : H.L) update_scal(*c, start_comp, no_force);
     update_scal_sync_h(H, start_comp);
 }
 static void update_scal_sync_h(Hier& H, int start_comp) {
@@ -820,7 +825,10 @@ static void density_advance(Hier& H, int which_step, bool stream = false, int fi
     if (stream) return density_advance_streamed(H, which_step, fills);
     const int spt = H[0].P.species_pred_type;
     const int ns = H[0].nspec, nscal = H[0].nscal;
-    for (auto* c : H.L) set_val(*c, F_SCALFORCE, 0.0, 0, nscal, c->F[F_SCALFORCE].spec.ng);
+    // the species have no force: 3-D edge states and updates do not read it (the adjoint keeps it)
+    const bool no_force = H[0].ndim == 3 && !H[0].edge_tape_begin;
+    for (auto* c : H.L)
+        set_val(*c, F_SCALFORCE, 0.0, no_force ? RHO : 0, no_force ? 1 : nscal, c->F[F_SCALFORCE].spec.ng);
     put1d_h(H, F_RHO0CART, "rho0_old", 0, 1, 0, BCS_S, RHO, 0, RHO);
     addw0_h(H, F_UMAC0, -1.0, fills);
     if (spt == 1) modify_scal_force_h(H, RHO, nullptr, "rho0_edge_old", F_RHO0CART, 0);
@@ -844,7 +852,7 @@ static void density_advance(Hier& H, int which_step, bool stream = false, int fi
     // scal_force.setVal(0) before UpdateScal (Source/MaestroDensityAdvance.cpp:229-231): of
     // the components read from here on, only Rho has been written since the zeroing above
     for (auto* c : H.L) set_val(*c, F_SCALFORCE, 0.0, RHO, 1, c->F[F_SCALFORCE].spec.ng);
-    update_scal_h(H, FIRSTSPEC);
+    update_scal_h(H, FIRSTSPEC, no_force);
 }
 
 // Maestro::EnthalpyAdvance (Source/MaestroEnthalpyAdvance.cpp:6-352); which_step 2 averages
@@ -1083,6 +1091,56 @@ static FabView* alias_fields(Ctx& c, StageIO& io) {
     return base;
 }
 
+// For the rest of the call field f stands for the FABs of view table row `row` (a user slot or another
+// field): no copy in or out.  Any FAB that bind() accepts can stand in for a field that is only
+// read, or only written on the valid region.
+struct InPlace {
+    Ctx& c;
+    FabView* const base;
+    InPlace(Ctx& ctx, const std::vector<std::pair<int, int>>& list) : c(ctx), base(ctx.dviews) {
+        if (list.empty()) return;
+        const size_t nv = (size_t)NF_TOTAL * c.nb;
+        if (!c.dviews_alias) {
+            if (!cuda_ok(cudaMalloc(&c.dviews_alias, sizeof(FabView) * nv), "cudaMalloc(views)") ||
+                !cuda_ok(cudaMallocHost(&c.hviews_alias, sizeof(FabView) * nv), "cudaMallocHost(views)"))
+                throw Fail{MADV_ERR_CUDA};
+        }
+        std::memcpy(c.hviews_alias, c.hviews_pinned, sizeof(FabView) * nv);
+        for (const auto& [f, row] : list)
+            std::memcpy(c.hviews_alias + (size_t)f * c.nb, c.hviews_pinned + (size_t)row * c.nb, sizeof(FabView) * c.nb);
+        if (!cuda_ok(cudaMemcpyAsync(c.dviews_alias, c.hviews_alias, sizeof(FabView) * nv, cudaMemcpyHostToDevice, c.stream),
+                     "cudaMemcpyAsync(views)"))
+            throw Fail{MADV_ERR_CUDA};
+        c.dviews = c.dviews_alias;
+    }
+    ~InPlace() { c.dviews = base; }
+    InPlace(const InPlace&) = delete;
+};
+// No FAB of the outputs shares memory with another one: what is written early is not read later
+static bool apart(const std::vector<const madv_multifab*>& out, const std::vector<const madv_multifab*>& in) {
+    struct Seg {
+        uintptr_t a, b;
+        bool out;
+    };
+    std::vector<Seg> v;
+    for (const auto* list : {&out, &in})
+        for (const madv_multifab* m : *list)
+            for (int q = 0; m && q < m->nfab; ++q) {
+                const madv_fab& f = m->fab[q];
+                size_t n = sizeof(double) * (size_t)f.ncomp;
+                for (int e = 0; e < 3; ++e) n *= (size_t)(f.hi[e] - f.lo[e] + 1);
+                v.push_back({(uintptr_t)f.p, (uintptr_t)f.p + n, list == &out});
+            }
+    std::sort(v.begin(), v.end(), [](const Seg& x, const Seg& y) { return x.a < y.a; });
+    uintptr_t end_out = 0, end_any = 0;
+    for (const Seg& s : v) {
+        if (s.a < (s.out ? end_any : end_out)) return false;
+        end_any = std::max(end_any, s.b);
+        if (s.out) end_out = std::max(end_out, s.b);
+    }
+    return true;
+}
+
 // The per-component scratch of MakeEdgeScal (3-D): what one component's chain writes
 // before its edge state (PPM, slopes, predictor, transverse states, traced force)
 static const int SIDE_SCRATCH[] = {F_DSVL, F_FACE0, F_FACE1, F_FACE2, F_IPC0, F_IMC0, F_SLOPE, F_SL0, F_SL1,
@@ -1151,7 +1209,9 @@ static void stage_body(Hier& H, const std::vector<StageIO>& io) {
         Ctx& c = H[l];
         if (!c.dry) cudaMemsetAsync(c.d_flag, 0, sizeof(int), c.stream);
         const int al = io[l].alias;
-        std::vector<ZeroJob> z{{F_UTILDE, 0, 3, c.ng_adv}, {F_THERMAL, 0, 1, 1}, {F_ETA, 0, 1, 0}};
+        std::vector<ZeroJob> z{{F_THERMAL, 0, 1, 1}, {F_ETA, 0, 1, 0}};
+        // (3-D level 0: the copy and FillPatch write every cell of it)
+        if (c.ndim == 2 || !put1d_fills(c)) z.push_back({F_UTILDE, 0, 3, c.ng_adv});
         if (!io[l].gpi) z.push_back({F_GPI, 0, 3, 0});
         if (!(al & AL_SNEW)) z.push_back({F_SNEW, 0, c.nscal, c.ng_s});
         for (int d = 0; d < 3; ++d) {
@@ -2224,6 +2284,17 @@ int madv_make_edge_scal(madv_ctx* h, const madv_multifab* state, const madv_mult
                 (rc = bind(c, U_SEDGE0 + d, &sedge[d], start_scomp + num_comp, d, 0)))
                 return rc;
         if ((rc = upload_user_views(c))) return rc;
+        // in the caller's FABs: eight copies were 18% of a call of one component
+        if (apart({sedge, sedge + 1, sedge + 2}, {state, force, umac, umac + 1, umac + 2})) {
+            std::vector<std::pair<int, int>> in{{F_SOLD, F_USER + U_SOLD}, {F_SCALFORCE, F_USER + U_FORCE}};
+            for (int d = 0; d < 3; ++d) {
+                in.push_back({F_UMAC0 + d, F_USER + U_UMAC0 + d});
+                in.push_back({F_SEDGE0 + d, F_USER + U_SEDGE0 + d});
+            }
+            InPlace views(c, in);
+            make_edge_scal(c, start_scomp, num_comp, BCS_S, is_conservative != 0, 0);
+            return finish(H);
+        }
         copy_fab(c, F_SOLD, start_scomp, F_USER + U_SOLD, start_scomp, num_comp, c.ng_s);
         copy_fab(c, F_SCALFORCE, start_scomp, F_USER + U_FORCE, start_scomp, num_comp, c.F[F_SCALFORCE].spec.ng);
         for (int d = 0; d < 3; ++d) copy_fab(c, F_UMAC0 + d, 0, F_USER + U_UMAC0 + d, 0, 1, 1);
@@ -2359,32 +2430,32 @@ int madv_velocity_advance(madv_ctx* h, const madv_multifab* uold, const madv_mul
             if (uedge && (rc = bind(c, U_UEDGE0 + d, &uedge[d], 3, d, 0))) return rc;
         }
         if ((rc = upload_user_views(c))) return rc;
-        copy_fab(c, F_GPI, 0, F_USER + U_GPI, 0, 3, 0);
-        for (int d = 0; d < 3; ++d) {
-            set_val(c, F_UMAC0 + d, 0.0, 0, 1, 1);
-            copy_fab(c, F_UMAC0 + d, 0, F_USER + U_UMAC0 + d, 0, 1, 0);
-        }
+        // in the caller's FABs: grad pi, and the edge states where nothing read later lies in them; the
+        // edge states' force is the velocity force
+        std::vector<std::pair<int, int>> in{{F_GPI, F_USER + U_GPI}, {F_SCALFORCE, F_VELFORCE}};
+        const bool own_edges =
+            uedge && apart({uedge, uedge + 1, uedge + 2}, {uold, rhohalf, gpi, sponge, unew, sold, umac, umac + 1, umac + 2});
+        for (int d = 0; d < 3 && own_edges; ++d) in.push_back({F_SEDGE0 + d, F_USER + U_UEDGE0 + d});
+        InPlace views(c, in);
+        set_zeros(c, {{F_UMAC0, 0, 1, 1}, {F_UMAC1, 0, 1, 1}, {F_UMAC2, 0, 1, 1}});
+        for (int d = 0; d < 3; ++d) copy_fab(c, F_UMAC0 + d, 0, F_USER + U_UMAC0 + d, 0, 1, 0);
         sync_faces_h(H, F_UMAC0);  // the ghost faces as MacProj leaves them (FillUmacGhost)
         w0_carts(H);
         // MakeVelForce(vel_force, umac, sold, rho0_old, grav_cell_old, w0_force_cart, 1)
-        copy_fab(c, F_SOLD, RHO, F_USER + U_SOLD, RHO, 1, 0);
-        make_vel_force_h(H, F_UMAC0, "rho0_old");
+        make_vel_force_h(H, F_UMAC0, "rho0_old", F_USER + U_SOLD, RHO);
         addw0_h(H, F_UMAC0, 1.0, 1);
         // MakeEdgeScal(uold, uedge, umac, vel_force, true, bcs_u, AMREX_SPACEDIM, 0, 0, AMREX_SPACEDIM, false)
         copy_fab(c, F_SOLD, 0, F_USER + U_UOLD, 0, 3, 0);
         fill_patch_h(H, F_SOLD, 0, 3, BCS_U, 0, 1, -1);
-        copy_fab(c, F_SCALFORCE, 0, F_VELFORCE, 0, 3, c.F[F_VELFORCE].spec.ng);
-        for (int d = 0; d < 3; ++d) set_val(c, F_SEDGE0 + d, 0.0, 0, 3, 0);
         make_edge_scal(c, 0, 3, BCS_U, 0, 0, 1);
         addw0_h(H, F_UMAC0, -1.0, 2);
         // MakeVelForce(vel_force, umac, rhohalf, rho0_nph, grav_cell_nph, w0_force_cart, 1)
-        copy_fab(c, F_SOLD, RHO, F_USER + U_RHOHALF, 0, 1, 0);
-        make_vel_force_h(H, F_UMAC0, "rho0_avg");
+        make_vel_force_h(H, F_UMAC0, "rho0_avg", F_USER + U_RHOHALF, 0);
         update_vel(c, F_USER + U_UOLD, sponge ? F_USER + U_SPONGE : -1);
         average_down_h(H, F_SNEW, 0, 3);
         fill_patch_h(H, F_SNEW, 0, 3, BCS_U, 0, 1, -1);
         copy_fab(c, F_USER + U_SNEW, 0, F_SNEW, 0, 3, held_ghosts(c, unew, -1, c.ng_s));
-        if (uedge)
+        if (uedge && !own_edges)
             for (int d = 0; d < 3; ++d) copy_fab(c, F_USER + U_UEDGE0 + d, 0, F_SEDGE0 + d, 0, 3, 0);
         return finish(H);
     } catch (const Fail& f) {

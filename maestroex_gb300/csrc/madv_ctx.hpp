@@ -319,7 +319,7 @@ bool put1d_fills(const Ctx& c);
 void put1d_filled(Ctx& c, const std::vector<Put1dJob>& jobs);
 void make_utrans(Ctx& c);
 // valid cells; face velocity fe .. fe+2; F_GRAVCART / F_RHO0CART filled by the caller
-void make_vel_force(Ctx& c, int fe = F_UTRANS0);
+void make_vel_force(Ctx& c, int fe = F_UTRANS0, int frho = F_SOLD, int crho = RHO);
 void vel_pred(Ctx& c);
 void vel_pred_prep(Ctx& c);  // the MakeUtrans work VelPred reuses, for a VelPred call on its own
 // slot >= 0: the edge state of every component goes to component `slot` of F_SEDGE* (species
@@ -346,7 +346,7 @@ void sum_species_edges(Ctx& c);
 int ppm_box_run(const madv_params& P, const madv_box* bx, const madv_fab* s, int comp, const madv_fab* u,
                 const madv_fab* v, const madv_fab* w, int is_umac, const int* bc, const madv_fab* Ip,
                 const madv_fab* Im, cudaStream_t st, long& launches);
-void update_scal(Ctx& c, int start_comp);
+void update_scal(Ctx& c, int start_comp, bool no_force = false);  // no_force: the species' force is zero
 // UpdateScal of the species split for streaming: one species from its flux in F_SFLUX* comp
 // `slot`, then the density, floor and negative-species pass over all of them
 void update_species(Ctx& c, int comp, int slot);
@@ -366,7 +366,7 @@ void make_w0mac(Ctx& c);
 void make_s0mac_faces(Ctx& c, int dst0);  // faces of F_S0CART2 into dst0 .. dst0 + 2
 void make_s0mac_interp(Ctx& c, const double* d_s0, int dst0);  // s0mac_interp_type 2, 3 (uniform bins)
 void addw0_sph(Ctx& c, int f0, double mult);
-void make_vel_force_sph(Ctx& c, int fe);
+void make_vel_force_sph(Ctx& c, int fe, int frho, int crho);
 void modify_scal_force_sph(Ctx& c, int comp, int s0cart_fid, int fullform);
 void make_rhoh_force_sph(Ctx& c, int is_prediction, int add_thermal);
 void put_in_pert_form_sph(Ctx& c, const double* d_s0, int comp, int flag);

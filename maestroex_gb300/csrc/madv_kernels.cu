@@ -837,10 +837,10 @@ void make_utrans(Ctx& c) {
 
 // ============================================================ MakeVelForce
 // Maestro::MakeVelForce, planar (Source/MaestroForce.cpp:100-126)
-__global__ void k_vel_force(KARGS, double cutoff_rho, int domhi, RecipC r2dz, int fe) {
+__global__ void k_vel_force(KARGS, double cutoff_rho, int domhi, RecipC r2dz, int fe, int frho, int crho) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    const FabView gpi = VW(F_GPI), rho = VW(F_SOLD), vf = VW(F_VELFORCE);
-    const double r = at(rho, i, j, k, RHO);
+    const FabView gpi = VW(F_GPI), rho = VW(frho), vf = VW(F_VELFORCE);
+    const double r = at(rho, i, j, k, crho);
     double rhopert = r - at(VW(F_RHO0CART), i, j, k);
     if (r < cutoff_rho) rhopert = 0.0;
     const RecipV rr = recip_v(r);  // three quotients by the density: 10 + 3 x 4 FP64 instructions, not 3 x 10
@@ -855,12 +855,13 @@ __global__ void k_vel_force(KARGS, double cutoff_rho, int domhi, RecipC r2dz, in
 }
 
 // valid cells of one level; F_GRAVCART and F_RHO0CART are filled by the caller
-void make_vel_force(Ctx& c, int fe) {
-    if (c.sph) return make_vel_force_sph(c, fe);
+void make_vel_force(Ctx& c, int fe, int frho, int crho) {
+    if (c.sph) return make_vel_force_sph(c, fe, frho, crho);
     if (c.ndim == 2) return make_vel_force_2d(c);
-    set_val(c, F_VELFORCE, 0.0, 0, 3, c.F[F_VELFORCE].spec.ng);
+    // (level 0: this kernel and FillPatch write every cell)
+    if (!put1d_fills(c)) set_val(c, F_VELFORCE, 0.0, 0, 3, c.F[F_VELFORCE].spec.ng);
     launch(c, rg_grow(c, 0), 1, k_vel_force, c.V(), c.P.buoyancy_cutoff_factor * c.P.base_cutoff_density,
-           c.P.dom_hi[2], make_recip(2.0 * c.P.dx[2]), fe);
+           c.P.dom_hi[2], make_recip(2.0 * c.P.dx[2]), fe, frho, crho);
 }
 
 // ============================================================ VelPred
@@ -1704,13 +1705,13 @@ void sum_species_edges(Ctx& c) {
 // the new (rho X) of one species from its flux in component fc of F_SFLUX*
 __device__ __forceinline__ void update_species_cell(const FabView* __restrict__ V, int nb, int b, int comp, int fc,
                                                     double dt, const RecipC& r0, const RecipC& r1, const RecipC& r2,
-                                                    int i, int j, int k) {
+                                                    int i, int j, int k, bool no_force = false) {
     const FabView so = VW(F_SOLD), sn = VW(F_SNEW), fx = VW(F_SFLUX0), fy = VW(F_SFLUX1), fz = VW(F_SFLUX2),
                   fo = VW(F_SCALFORCE);
     double divterm = div_c(at(fx, i + 1, j, k, fc) - at(fx, i, j, k, fc), r0);
     divterm += div_c(at(fy, i, j + 1, k, fc) - at(fy, i, j, k, fc), r1);
     divterm += div_c(at(fz, i, j, k + 1, fc) - at(fz, i, j, k, fc), r2);
-    at(sn, i, j, k, comp) = at(so, i, j, k, comp) + dt * (-divterm + at(fo, i, j, k, comp));
+    at(sn, i, j, k, comp) = at(so, i, j, k, comp) + dt * (-divterm + (no_force ? 0.0 : at(fo, i, j, k, comp)));
 }
 
 // rho from the species' changes, the density floor and the negative-species fix
@@ -1748,9 +1749,10 @@ __device__ __forceinline__ void rhox_fix_cell(const FabView* __restrict__ V, int
     }
 }
 
-__global__ void k_update_rhox(KARGS, int nspec, double dt, RecipC r0, RecipC r1, RecipC r2, double half_cutoff) {
+__global__ void k_update_rhox(KARGS, int nspec, double dt, RecipC r0, RecipC r1, RecipC r2, double half_cutoff,
+                              int no_force) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    for (int n = 0; n < nspec; ++n) update_species_cell(V, nb, b, FIRSTSPEC + n, FIRSTSPEC + n, dt, r0, r1, r2, i, j, k);
+    for (int n = 0; n < nspec; ++n) update_species_cell(V, nb, b, FIRSTSPEC + n, FIRSTSPEC + n, dt, r0, r1, r2, i, j, k, no_force);
     rhox_fix_cell(V, nb, b, nspec, half_cutoff, i, j, k);
 }
 
@@ -1942,7 +1944,7 @@ void dt_maxima(Ctx& c) {
     launch(c, rg_grow(c, 0), 1, k_dt_maxima, c.V(), (int)c.sph, c.ndim, w0m, c.d_red);
 }
 
-void update_scal(Ctx& c, int start_comp) {
+void update_scal(Ctx& c, int start_comp, bool no_force) {
     if (c.ndim == 2) return update_scal_2d(c, start_comp);
     const RegionTable& rt = rg_grow(c, 0);
     if (start_comp == RHOH) {
@@ -1950,7 +1952,7 @@ void update_scal(Ctx& c, int start_comp) {
                make_recip(c.P.dx[2]), c.P.do_eos_h_above_cutoff, c.P.base_cutoff_density, c.d_flag);
     } else {
         launch(c, rt, 1, k_update_rhox, c.V(), c.nspec, c.P.dt, make_recip(c.P.dx[0]), make_recip(c.P.dx[1]),
-               make_recip(c.P.dx[2]), 0.5 * c.P.base_cutoff_density);
+               make_recip(c.P.dx[2]), 0.5 * c.P.base_cutoff_density, (int)no_force);
     }
 }
 

@@ -282,7 +282,7 @@ void addw0_sph(Ctx& c, int f0, double mult) {
 // MakeVelForce, spherical (Source/MaestroForce.cpp:151-252; MakeNormal :1190-1227).  gradw0:
 // dw0/dr of the uniform bins on the cells (F_GRADW0); the exact base state has gradw0 = 0
 // (:30-41), so the utilde term subtracts Ut.e_r * 0 * e_r.
-__global__ void k_vel_force_sph(KARGS, double cutoff_rho, SphGeo g, int fe) {
+__global__ void k_vel_force_sph(KARGS, double cutoff_rho, SphGeo g, int fe, int frho, int crho) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const double gradw0 = g.exact ? 0.0 : at(VW(F_GRADW0), i, j, k);
     double x, y, z;
@@ -290,7 +290,7 @@ __global__ void k_vel_force_sph(KARGS, double cutoff_rho, SphGeo g, int fe) {
     const double inv_radius = 1.0 / sqrt(x * x + y * y + z * z);
     const double nrm[3] = {x * inv_radius, y * inv_radius, z * inv_radius};
     const FabView gpi = VW(F_GPI), vf = VW(F_VELFORCE), grav = VW(F_GRAVCART), w0f = VW(F_W0FCART);
-    const double r = at(VW(F_SOLD), i, j, k, RHO);
+    const double r = at(VW(frho), i, j, k, crho);
     double rhopert = r - at(VW(F_RHO0CART), i, j, k);
     if (r < cutoff_rho) rhopert = 0.0;
     const RecipV rr = recip_v(r);
@@ -303,10 +303,10 @@ __global__ void k_vel_force_sph(KARGS, double cutoff_rho, SphGeo g, int fe) {
     for (int dim = 0; dim < 3; ++dim) at(vf, i, j, k, dim) -= ut_dot_er * gradw0 * nrm[dim];
 }
 
-void make_vel_force_sph(Ctx& c, int fe) {
+void make_vel_force_sph(Ctx& c, int fe, int frho, int crho) {
     set_val(c, F_VELFORCE, 0.0, 0, 3, c.F[F_VELFORCE].spec.ng);
     launch(c, rg_grow(c, 0), 1, k_vel_force_sph, c.V(), c.P.buoyancy_cutoff_factor * c.P.base_cutoff_density, c.geo,
-           fe);
+           fe, frho, crho);
 }
 
 // ModifyScalForce, spherical (Source/MaestroForce.cpp:335-412); divu_cart is Put1dArrayOnCart
