@@ -124,13 +124,28 @@ __device__ __forceinline__ void region_ijk(const RegionBox& r, long l, int& i, i
 // MADV_ELEMENT_OF: the element of block bx (kernels that put components into the block index).
 #define MADV_ELEMENT(R, ne, g0, g1, b, i, j, k) MADV_ELEMENT_OF(blockIdx.x, R, ne, g0, g1, b, i, j, k)
 #define MADV_ELEMENT_OF(bx, R, ne, g0, g1, b, i, j, k)                     \
+    MADV_PIECE(bx, R, ne, g0, g1, b, i, j, k);                            \
+    MADV_WAIT()
+// (what a kernel needs of its piece is read before the wait: part_ is the piece's pad)
+#define MADV_PIECE(bx, R, ne, g0, g1, b, i, j, k)                          \
     MADV_LET_NEXT();                                                      \
     const long gid_ = (g0) + (long)(bx) * blockDim.x + threadIdx.x;        \
     if (gid_ >= (g1)) return;                                             \
     const int e_ = find_box((R), (ne), gid_);                             \
     const int b = (R)[e_].b;                                              \
+    [[maybe_unused]] const int part_ = (R)[e_].pad;                        \
     int i, j, k;                                                          \
-    region_ijk((R)[e_], gid_ - (R)[e_].start, i, j, k);                   \
+    region_ijk((R)[e_], gid_ - (R)[e_].start, i, j, k)
+
+// The cells (i, j, k .. k1 - 1) of a thread of a column region (region_columns); COL = false: of a
+// region as it is, one cell
+#define MADV_COLUMN(COL, R, ne, g0, g1, b, i, j, k, k1)                    \
+    MADV_PIECE(blockIdx.x, R, ne, g0, g1, b, i, j, k);                     \
+    const int klo_ = (R)[e_].lo[2];                                       \
+    const int len_ = (COL) ? (R)[e_].len : 1;                              \
+    const int kend_ = klo_ + ((COL) ? (R)[e_].ext : (R)[e_].n[2]);         \
+    if (COL) k = klo_ + (k - klo_) * len_;                                 \
+    const int k1 = (COL) ? min(k + len_, kend_) : k + 1;                   \
     MADV_WAIT()
 
 // amrex::min / amrex::max (std::min / std::max semantics).  (An integer-key form measured

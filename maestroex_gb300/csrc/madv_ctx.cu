@@ -105,6 +105,30 @@ const RegionTable& region_union(Ctx& c, const std::vector<RegionKey>& parts) {
     return t;
 }
 
+const RegionTable& region_columns(Ctx& c, const std::vector<RegionKey>& parts) {
+    std::vector<int> key{-1};  // (a union's key is made of whole RegionKeys)
+    for (const RegionKey& p : parts) key.insert(key.end(), p.begin(), p.end());
+    auto it = c.unions.find(key);
+    if (it != c.unions.end()) return it->second;
+    const RegionTable& u = region_union(c, parts);
+    const int len = (int)std::min(8L, u.total >> 19);
+    if (len <= 1) return u;
+    const std::vector<RegionBox> h = u.h;
+    RegionTable& t = c.unions[key];
+    t.columns = true;
+    for (RegionBox r : h) {
+        r.ext = r.n[2];
+        const int nch = (r.ext + len - 1) / len;
+        r.len = (r.ext + nch - 1) / nch;
+        r.n[2] = (r.ext + r.len - 1) / r.len;
+        r.start = t.total;
+        t.total += (long)r.n[0] * r.n[1] * r.n[2];
+        t.h.push_back(r);
+    }
+    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    return t;
+}
+
 // a minus b as up to six disjoint boxes appended to out
 static void box_minus(const HBox& a, const HBox& b, std::vector<HBox>& out) {
     for (int d = 0; d < 3; ++d)

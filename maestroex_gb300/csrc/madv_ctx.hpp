@@ -98,6 +98,7 @@ struct RegionTable {
     RegionBox* d = nullptr;
     std::vector<RegionBox> h;  // region pieces (one per box, two for boundary slabs)
     long total = 0;
+    bool columns = false;  // of region_columns, with more than one cell a thread
 };
 
 struct CopyDesc {
@@ -265,6 +266,11 @@ const CopyTable& copy_table_faces(Ctx& c, int ng);  // the three face directions
 // them; a piece's pad is the place of its region in the list.
 typedef std::array<int, 8> RegionKey;
 const RegionTable& region_union(Ctx& c, const std::vector<RegionKey>& parts);
+// The same in z columns of up to 8 cells, for kernels that do little per cell: finding a cell's place
+// costs some 60 instructions, and a store-only kernel ran at 1.5 TB/s.  Columns are shorter where
+// the regions have too few cells to fill the chip (about 2^19 threads); columns of one cell are the
+// union itself, whose kernels run without the loop (it cost a 32^3 stage 1%).
+const RegionTable& region_columns(Ctx& c, const std::vector<RegionKey>& parts);
 
 void set_error(const std::string& s);
 bool cuda_ok(cudaError_t e, const char* what);

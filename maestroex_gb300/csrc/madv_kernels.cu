@@ -50,22 +50,31 @@ static const RegionTable& rg_faces(Ctx& c) {
 }
 
 // ============================================================ elementwise utilities
+template <bool COL>
 __global__ void k_set_val(KARGS, int f, double v, int c0, int nc) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    MADV_COLUMN(COL, R, ne, g0, g1, b, i, j, k, k1);
     const FabView a = VW(f);
-    for (int n = c0; n < c0 + nc; ++n) at(a, i, j, k, n) = v;
+    for (int n = c0; n < c0 + nc; ++n)
+        for (int q = k; q < k1; ++q) at(a, i, j, q, n) = v;
 }
+
+static const RegionTable& rg_columns(Ctx& c, int g, int nodal) { return region_columns(c, {{g, g, g, g, g, g, nodal, -1}}); }
 
 void set_val(Ctx& c, int fid, double v, int c0, int nc, int ngrow) {
-    launch(c, rg_grow(c, ngrow, c.F[fid].spec.nodal), 1, k_set_val, c.V(), fid, v, c0, nc);
+    const RegionTable& rt = rg_columns(c, ngrow, c.F[fid].spec.nodal);
+    launch(c, rt, 1, rt.columns ? k_set_val<true> : k_set_val<false>, c.V(), fid, v, c0, nc);
 }
 
+template <bool COL>
 __global__ void k_copy(KARGS, int fd, int dc0, int fs, int sc0, int nc, int add) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    MADV_COLUMN(COL, R, ne, g0, g1, b, i, j, k, k1);
     const FabView d = VW(fd), s = VW(fs);
     for (int n = 0; n < nc; ++n) {
-        if (add) at(d, i, j, k, dc0 + n) += at(s, i, j, k, sc0 + n);
-        else at(d, i, j, k, dc0 + n) = at(s, i, j, k, sc0 + n);
+        for (int q = k; q < k1; ++q) {
+            const double v = at(s, i, j, q, sc0 + n);
+            if (add) at(d, i, j, q, dc0 + n) += v;
+            else at(d, i, j, q, dc0 + n) = v;
+        }
     }
 }
 
@@ -73,11 +82,13 @@ static int nodal_of(const Ctx& c, int fid) { return fid < NF_INTERNAL ? c.F[fid]
 
 void copy_fab(Ctx& c, int dst, int dc0, int src, int sc0, int nc, int ngrow) {
     int nd = dst < NF_INTERNAL ? nodal_of(c, dst) : nodal_of(c, src);
-    launch(c, rg_grow(c, ngrow, nd), 1, k_copy, c.V(), dst, dc0, src, sc0, nc, 0);
+    const RegionTable& rt = rg_columns(c, ngrow, nd);
+    launch(c, rt, 1, rt.columns ? k_copy<true> : k_copy<false>, c.V(), dst, dc0, src, sc0, nc, 0);
 }
 
 void add_fab(Ctx& c, int dst, int src, int nc, int ngrow) {
-    launch(c, rg_grow(c, ngrow, nodal_of(c, dst)), 1, k_copy, c.V(), dst, 0, src, 0, nc, 1);
+    const RegionTable& rt = rg_columns(c, ngrow, nodal_of(c, dst));
+    launch(c, rt, 1, rt.columns ? k_copy<true> : k_copy<false>, c.V(), dst, 0, src, 0, nc, 1);
 }
 
 // setVal(0) of up to ZERO_JOBS fields in one launch (the stage's start clears 13; a small level's
@@ -86,11 +97,13 @@ static constexpr int ZERO_JOBS = 16;
 struct ZeroArgs {
     int f[ZERO_JOBS], c0[ZERO_JOBS], nc[ZERO_JOBS];
 };
+template <bool COL>
 __global__ void k_set_zeros(KARGS, const __grid_constant__ ZeroArgs z) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    const int q = R[e_].pad;
+    MADV_COLUMN(COL, R, ne, g0, g1, b, i, j, k, k1);
+    const int q = part_;
     const FabView a = VW(z.f[q]);
-    for (int n = z.c0[q]; n < z.c0[q] + z.nc[q]; ++n) at(a, i, j, k, n) = 0.0;
+    for (int n = z.c0[q]; n < z.c0[q] + z.nc[q]; ++n)
+        for (int p = k; p < k1; ++p) at(a, i, j, p, n) = 0.0;
 }
 
 void set_zeros(Ctx& c, const std::vector<ZeroJob>& jobs) {
@@ -104,7 +117,8 @@ void set_zeros(Ctx& c, const std::vector<ZeroJob>& jobs) {
             z.nc[q - q0] = w.nc;
             parts.push_back({w.ng, w.ng, w.ng, w.ng, w.ng, w.ng, c.F[w.f].spec.nodal, -1});
         }
-        launch(c, region_union(c, parts), 1, k_set_zeros, c.V(), z);
+        const RegionTable& rt = region_columns(c, parts);
+        launch(c, rt, 1, rt.columns ? k_set_zeros<true> : k_set_zeros<false>, c.V(), z);
     }
 }
 
@@ -175,25 +189,32 @@ __device__ __noinline__ double put1d_behind(const Put1dArgs& a, int job, int n, 
     if (m < lo) return phys_value(bc.lo[RD], m == lo - 1, ext, lo - 1 - m, [&](int q) { return level(lo + q); });
     return phys_value(bc.hi[RD], m == hi + 1, ext, m - hi - 1, [&](int q) { return level(hi - q); });
 }
-template <int ND>
+template <int ND, bool COL>
 __global__ void k_put1d_filled(KARGS, const __grid_constant__ Put1dArgs a) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    const int job = R[e_].pad;
+    MADV_COLUMN(COL, R, ne, g0, g1, b, i, j, k, k1);
+    const int job = part_;
     const auto& w = a.w[job];
     const FabView out = VW(w.f);
     constexpr int RD = ND - 1;
-    const int idx[3] = {i, j, k};
-    bool plain = true;
+    const double* const s0 = w.s0;
+    const int edge = w.edge, nc = w.nc, oc = w.outcomp;
+    bool across = true;  // inside the domain or periodic across the radial direction
+    {
+        const int idx[2] = {i, j};
 #pragma unroll
-    for (int d = 0; d < ND; ++d) plain = plain && (a.per[d] || (idx[d] >= a.lo[d] && idx[d] <= a.hi[d]));
-    if (plain) {
-        int r = idx[RD];
-        const int ext = a.hi[RD] - a.lo[RD] + 1;
-        r += r < a.lo[RD] ? ext : (r > a.hi[RD] ? -ext : 0);
-        const double v = w.edge ? half(w.s0[r] + w.s0[r + 1]) : w.s0[r];
-        for (int n = 0; n < w.nc; ++n) at(out, i, j, k, n) = n == w.outcomp ? v : 0.0;
-    } else {
-        for (int n = 0; n < w.nc; ++n) at(out, i, j, k, n) = put1d_behind<ND>(a, job, n, i, j, k);
+        for (int d = 0; d < RD; ++d) across = across && (a.per[d] || (idx[d] >= a.lo[d] && idx[d] <= a.hi[d]));
+    }
+    const int lo = a.lo[RD], hi = a.hi[RD], ext = hi - lo + 1;
+    for (int q = k; q < k1; ++q) {
+        int r = RD == 2 ? q : j;
+        const bool behind = r < lo || r > hi;
+        if (across && (!behind || a.per[RD])) {
+            r += r < lo ? ext : (r > hi ? -ext : 0);
+            const double v = edge ? half(s0[r] + s0[r + 1]) : s0[r];
+            for (int n = 0; n < nc; ++n) at(out, i, j, q, n) = n == oc ? v : 0.0;
+        } else {
+            for (int n = 0; n < nc; ++n) at(out, i, j, q, n) = put1d_behind<ND>(a, job, n, i, j, q);
+        }
     }
 }
 
@@ -221,7 +242,9 @@ void put1d_filled(Ctx& c, const std::vector<Put1dJob>& jobs) {
             a.hi[d] = c.P.dom_hi[d];
             a.per[d] = c.per[d];
         }
-        launch(c, region_union(c, parts), 1, c.ndim == 2 ? k_put1d_filled<2> : k_put1d_filled<3>, c.V(), a);
+        const RegionTable& rt = region_columns(c, parts);
+        auto k3 = rt.columns ? k_put1d_filled<3, true> : k_put1d_filled<3, false>;
+        launch(c, rt, 1, c.ndim == 2 ? k_put1d_filled<2, false> : k3, c.V(), a);
     }
 }
 
@@ -497,30 +520,36 @@ void addw0(Ctx& c, int f0, double mult) {
 // rule -- and the fill need not run again.  One launch for three, eight times a stage.  (Bitwise: a
 // copy plus w0 is the copy of the sum.  Filled twice: on the domain's edges the first fill's x
 // planes read what its y and z planes set, so that the ghost faces there settle with the second.)
-template <int ND>
+template <int ND, bool COL>
 __global__ void k_addw0_filled(KARGS, int f, const double* __restrict__ w0, double mult,
                                const __grid_constant__ DirRules p) {
-    MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
+    MADV_COLUMN(COL, R, ne, g0, g1, b, i, j, k, k1);
     constexpr int RD = ND - 1;
-    const int idx[3] = {i, j, k};
-    const int r = idx[RD], lo = p.dl[RD], hi = p.dh[RD] + 1;
-    // FillUmacGhost's planes across stop short of the box's last radial ghost face
-    const bool last = r == R[e_].lo[RD] + R[e_].n[RD] - 1 && r <= hi;
+    const int idx[2] = {i, j}, lo = p.dl[RD], hi = p.dh[RD] + 1;
+    bool outside = false;
 #pragma unroll
     for (int d = 0; d < RD; ++d) {
         if (idx[d] >= p.dl[d] && idx[d] <= p.dh[d]) continue;
         const int t = idx[d] < p.dl[d] ? p.bl[d] : p.bh[d];
-        if (last || t == PB_INFLOW || t == PB_SLIPWALL || t == PB_NOSLIPWALL) return;  // stays as it is, or zero
+        if (t == PB_INFLOW || t == PB_SLIPWALL || t == PB_NOSLIPWALL) return;  // stays zero
+        outside = true;
     }
-    double& v = at(VW(f), i, j, k);
-    if (r >= lo && r <= hi) {
-        v += mult * w0[r];
-        return;
+    // FillUmacGhost's planes across stop short of the box's last radial ghost face
+    const int last = RD == 2 ? kend_ - 1 : R[e_].lo[1] + R[e_].n[1] - 1;
+    const FabView u = VW(f);
+    for (int q = k; q < k1; ++q) {
+        const int r = RD == 2 ? q : j;
+        if (outside && r == last && r <= hi) continue;
+        double& v = at(u, i, j, q);
+        if (r >= lo && r <= hi) {
+            v += mult * w0[r];
+            continue;
+        }
+        const bool below = r < lo;
+        const int t = below ? p.bl[RD] : p.bh[RD];
+        if (t == PB_INFLOW || t == PB_OUTFLOW) v += mult * w0[below ? lo : hi];
+        else if (t == PB_SYMMETRY) v = dflip(dflip(v) + mult * w0[below ? lo + 1 : hi - 1]);
     }
-    const bool below = r < lo;
-    const int t = below ? p.bl[RD] : p.bh[RD];
-    if (t == PB_INFLOW || t == PB_OUTFLOW) v += mult * w0[below ? lo : hi];
-    else if (t == PB_SYMMETRY) v = dflip(dflip(v) + mult * w0[below ? lo + 1 : hi - 1]);
 }
 
 bool addw0_fills(const Ctx& c) { return !c.sph && !c.per_box && !c.per[c.ndim - 1]; }
@@ -529,7 +558,11 @@ void addw0_filled(Ctx& c, int f0, double mult) {
     DirRules p = phys_rules(c, 0, 0, 0);
     for (int d = 0; d < rd; ++d)
         if (c.per[d]) p.dl[d] = INT_MIN, p.dh[d] = INT_MAX;
-    launch(c, region(c, 1, 1, 1, 1, 1, 1, rd), 1, c.ndim == 2 ? k_addw0_filled<2> : k_addw0_filled<3>, c.V(), f0 + rd,
+    if (c.ndim == 2)
+        return launch(c, region(c, 1, 1, 1, 1, 1, 1, rd), 1, k_addw0_filled<2, false>, c.V(), f0 + rd,
+                      (const double*)c.b1("w0"), mult, p);
+    const RegionTable& rt = rg_columns(c, 1, rd);
+    launch(c, rt, 1, rt.columns ? k_addw0_filled<3, true> : k_addw0_filled<3, false>, c.V(), f0 + rd,
            (const double*)c.b1("w0"), mult, p);
 }
 
@@ -729,7 +762,7 @@ __device__ __forceinline__ void transverse_coeffs_cell(const FabView* __restrict
 // the cells (first: the first part of this launch's regions)
 __global__ void k_edge_coeffs(KARGS, int fu0, const __grid_constant__ EdgeCoefs e, int first) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    switch (first + R[e_].pad) {
+    switch (first + part_) {
         case 0: trace_face(VW(fu0), VW(F_TRA0), e.dt, e.r[0], i, j, k); break;
         case 1: trace_face(VW(fu0 + 1), VW(F_TRA1), e.dt, e.r[1], i, j, k); break;
         case 2: trace_face(VW(fu0 + 2), VW(F_TRA2), e.dt, e.r[2], i, j, k); break;
@@ -810,7 +843,7 @@ __device__ __forceinline__ void utrans_face(const FabView* __restrict__ V, int n
 
 __global__ void k_utrans(KARGS, int ppm_type, const __grid_constant__ DirRules p, double rel_eps, int sph) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    switch (R[e_].pad) {
+    switch (part_) {
         case 0: utrans_face<0>(V, nb, b, i, j, k, ppm_type, p.h[0], RULES(0), rel_eps, sph); break;
         case 1: utrans_face<1>(V, nb, b, i, j, k, ppm_type, p.h[1], RULES(1), rel_eps, sph); break;
         default: utrans_face<2>(V, nb, b, i, j, k, ppm_type, p.h[2], RULES(2), rel_eps, sph);
@@ -1040,7 +1073,7 @@ __device__ __forceinline__ void vp_velocities_face(const FabView* __restrict__ V
 
 __global__ void k_vp_interface(KARGS, int ppm_type, double dt2, const __grid_constant__ DirRules p, long long epsb) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    switch (R[e_].pad) {
+    switch (part_) {
         case 0: vp_interface_face<0>(V, nb, b, i, j, k, ppm_type, dt2, p.h[0], RULES(0), epsb); break;
         case 1: vp_interface_face<1>(V, nb, b, i, j, k, ppm_type, dt2, p.h[1], RULES(1), epsb); break;
         default: vp_interface_face<2>(V, nb, b, i, j, k, ppm_type, dt2, p.h[2], RULES(2), epsb);
@@ -1049,7 +1082,7 @@ __global__ void k_vp_interface(KARGS, int ppm_type, double dt2, const __grid_con
 // parts: (C, D) = (0, 1), (0, 2), (1, 0), (1, 2), (2, 0), (2, 1)
 __global__ void k_vp_transverse(KARGS, const __grid_constant__ DirRules p, long long epsb) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    switch (R[e_].pad) {
+    switch (part_) {
         case 0: vp_transverse_face<0, 1>(V, nb, b, i, j, k, RULES(1), epsb); break;
         case 1: vp_transverse_face<0, 2>(V, nb, b, i, j, k, RULES(2), epsb); break;
         case 2: vp_transverse_face<1, 0>(V, nb, b, i, j, k, RULES(0), epsb); break;
@@ -1060,7 +1093,7 @@ __global__ void k_vp_transverse(KARGS, const __grid_constant__ DirRules p, long 
 }
 __global__ void k_vp_velocities(KARGS, double dt2, const __grid_constant__ DirRules p, double rel_eps, int sph, int ptf) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    switch (R[e_].pad) {
+    switch (part_) {
         case 0: vp_velocities_face<0>(V, nb, b, i, j, k, dt2, RULES(0), rel_eps, sph, ptf); break;
         case 1: vp_velocities_face<1>(V, nb, b, i, j, k, dt2, RULES(1), rel_eps, sph, ptf); break;
         default: vp_velocities_face<2>(V, nb, b, i, j, k, dt2, RULES(2), rel_eps, sph, ptf);
@@ -1577,7 +1610,7 @@ __global__ void k_rhox_flux(KARGS, int c0, int nc, int nspec, int slot, int spt,
                             const double* __restrict__ r0eo, const double* __restrict__ r0en,
                             const double* __restrict__ w0, const double* __restrict__ r0pe) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    switch (R[e_].pad) {
+    switch (part_) {
         case 0: rhox_flux_face<0>(V, nb, b, i, j, k, c0, nc, nspec, slot, spt, 0, r0o, r0n, w0, r0pe); break;
         case 1: rhox_flux_face<1>(V, nb, b, i, j, k, c0, nc, nspec, slot, spt, 0, r0o, r0n, w0, r0pe); break;
         default: rhox_flux_face<2>(V, nb, b, i, j, k, c0, nc, nspec, slot, spt, do_eta, r0eo, r0en, w0, r0pe);
@@ -1628,7 +1661,7 @@ struct RhohBase {
 __global__ void k_rhoh_flux(KARGS, int ept, int spt, RhohBase q) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const auto &c = q.cell, &e = q.edge;
-    switch (R[e_].pad) {
+    switch (part_) {
         case 0: rhoh_flux_face<0>(V, nb, b, i, j, k, ept, c[0], c[1], spt, c[2], c[3]); break;
         case 1: rhoh_flux_face<1>(V, nb, b, i, j, k, ept, c[0], c[1], spt, c[2], c[3]); break;
         default: rhoh_flux_face<2>(V, nb, b, i, j, k, ept, e[0], e[1], spt, e[2], e[3]);
@@ -1770,7 +1803,7 @@ __device__ __forceinline__ void species_factor(const FabView* __restrict__ V, in
 __global__ void k_species_factor(KARGS, int fc, int spt, const double* __restrict__ r0o, const double* __restrict__ r0n,
                                  const double* __restrict__ r0eo, const double* __restrict__ r0en) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    switch (R[e_].pad) {
+    switch (part_) {
         case 0: species_factor<0>(V, nb, b, i, j, k, fc, spt, r0o, r0n); break;
         case 1: species_factor<1>(V, nb, b, i, j, k, fc, spt, r0o, r0n); break;
         default: species_factor<2>(V, nb, b, i, j, k, fc, spt, r0eo, r0en);
@@ -2027,7 +2060,7 @@ __device__ __forceinline__ void utrans_2dy_face(const FabView* __restrict__ V, i
 
 __global__ void k_utrans_2d(KARGS, int ppm_type, const __grid_constant__ DirRules p, double rel_eps) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    if (R[e_].pad == 0) utrans_face<0>(V, nb, b, i, j, k, ppm_type, p.h[0], RULES(0), rel_eps, 0);
+    if (part_ == 0) utrans_face<0>(V, nb, b, i, j, k, ppm_type, p.h[0], RULES(0), rel_eps, 0);
     else utrans_2dy_face(V, nb, b, i, j, k, ppm_type, p.h[1], RULES(1), rel_eps);
 }
 
@@ -2206,12 +2239,12 @@ __device__ __forceinline__ void vp_velocities_2d_face(const FabView* __restrict_
 
 __global__ void k_vp_interface_2d(KARGS, int ppm_type, const __grid_constant__ DirRules p, double rel_eps) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    if (R[e_].pad == 0) vp_interface_2d_face<0>(V, nb, b, i, j, k, ppm_type, p.h[0], RULES(0), rel_eps);
+    if (part_ == 0) vp_interface_2d_face<0>(V, nb, b, i, j, k, ppm_type, p.h[0], RULES(0), rel_eps);
     else vp_interface_2d_face<1>(V, nb, b, i, j, k, ppm_type, p.h[1], RULES(1), rel_eps);
 }
 __global__ void k_vp_velocities_2d(KARGS, double dt2, const __grid_constant__ DirRules p, double rel_eps) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    if (R[e_].pad == 0) vp_velocities_2d_face<0>(V, nb, b, i, j, k, dt2, p.h[1], RULES(0), rel_eps);
+    if (part_ == 0) vp_velocities_2d_face<0>(V, nb, b, i, j, k, dt2, p.h[1], RULES(0), rel_eps);
     else vp_velocities_2d_face<1>(V, nb, b, i, j, k, dt2, p.h[0], RULES(1), rel_eps);
 }
 // the faces of both directions inside the cells grown by one (growLo(obx, d, -1))
@@ -2326,7 +2359,7 @@ __global__ void k_es_predictor_2d(KARGS, int comp0, unsigned nq, int ppm_type, d
                                   const __grid_constant__ Es2dRules bc, double rel_eps) {
     const unsigned bx = blockIdx.x / nq, q = blockIdx.x - bx * nq;
     MADV_ELEMENT_OF(bx, R, ne, g0, g1, b, i, j, k);
-    if (R[e_].pad == 0)
+    if (part_ == 0)
         es_predictor_2d_face<0>(V, nb, b, i, j, k, comp0 + q, q, ppm_type, dt2, p.h[0], bc.lo[q][0], bc.hi[q][0], p.dl[0],
                                 p.dh[0], rel_eps);
     else
@@ -2337,7 +2370,7 @@ __global__ void k_es_edges_2d(KARGS, int comp0, unsigned nq, int is_cons, double
                               const __grid_constant__ DirRules p, const __grid_constant__ Es2dRules bc, double rel_eps) {
     const unsigned bx = blockIdx.x / nq, q = blockIdx.x - bx * nq;
     MADV_ELEMENT_OF(bx, R, ne, g0, g1, b, i, j, k);
-    if (R[e_].pad == 0)
+    if (part_ == 0)
         es_edges_2d_face<0>(V, nb, b, i, j, k, comp0 + q, q, is_cons, dt2, dt4, p.h[0], p.h[1], bc.lo[q][0], bc.hi[q][0],
                             p.dl[0], p.dh[0], rel_eps);
     else
@@ -2469,13 +2502,13 @@ __global__ void k_rhox_flux_2d(KARGS, int nspec, int spt, int do_eta, const doub
                                const double* __restrict__ r0en, const double* __restrict__ w0,
                                const double* __restrict__ r0pe) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
-    if (R[e_].pad == 0) rhox_flux_2d_face<0>(V, nb, b, i, j, k, nspec, spt, 0, r0o, r0n, w0, r0pe);
+    if (part_ == 0) rhox_flux_2d_face<0>(V, nb, b, i, j, k, nspec, spt, 0, r0o, r0n, w0, r0pe);
     else rhox_flux_2d_face<1>(V, nb, b, i, j, k, nspec, spt, do_eta, r0eo, r0en, w0, r0pe);
 }
 __global__ void k_rhoh_flux_2d(KARGS, int ept, int spt, RhohBase q) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const auto &c = q.cell, &e = q.edge;
-    if (R[e_].pad == 0) rhoh_flux_2d_face<0>(V, nb, b, i, j, k, ept, c[0], c[1], spt, c[2], c[3]);
+    if (part_ == 0) rhoh_flux_2d_face<0>(V, nb, b, i, j, k, ept, c[0], c[1], spt, c[2], c[3]);
     else rhoh_flux_2d_face<1>(V, nb, b, i, j, k, ept, e[0], e[1], spt, e[2], e[3]);
 }
 

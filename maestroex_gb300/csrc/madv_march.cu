@@ -379,11 +379,12 @@ __device__ __forceinline__ int trans_field(int a, int b) {
 // prologue of the three kernels: component q, direction dir, cells (i, j, k .. k1 - 1)
 #define MADV_ES_COLUMN()                                                    \
     const unsigned bx_ = blockIdx.x / nq, q = blockIdx.x - bx_ * nq;        \
-    MADV_ELEMENT_OF(bx_, R, ne, g0, g1, b, i, j, k);                        \
+    MADV_PIECE(bx_, R, ne, g0, g1, b, i, j, k);                             \
     const RegionBox& r = R[e_];                                             \
-    const int dir = r.pad, len = r.len, klo = r.lo[2];                      \
+    const int dir = part_, len = r.len, klo = r.lo[2], ext = r.ext;         \
     k = klo + (k - klo) * len;                                              \
-    const int k1 = min(k + len, klo + r.ext)
+    const int k1 = min(k + len, klo + ext);                                 \
+    MADV_WAIT()
 
 // The conservative form's factors: dt/3/h_T, dt/2/h_T, dt/3
 struct EsCons {
@@ -492,7 +493,7 @@ __global__ void __launch_bounds__(256) k_es_trans(KARGS, int comp0, unsigned nq,
     MADV_ES_COLUMN();
     // the region is grown by one across the direction: its inner cells lie in the box
     const bool bi = i > r.lo[0] && i < r.lo[0] + r.n[0] - 1, bj = j > r.lo[1] && j < r.lo[1] + r.n[1] - 1;
-    const int bk0 = klo + 1, bk1 = klo + r.ext - 2;
+    const int bk0 = klo + 1, bk1 = klo + ext - 2;
     if (dir == 0) es_trans<0, CONS>(V, nb, b, i, j, k, k1, bi, bj, bk0, bk1, comp0 + q, q, rules, epsb);
     else if (dir == 1) es_trans<1, CONS>(V, nb, b, i, j, k, k1, bi, bj, bk0, bk1, comp0 + q, q, rules, epsb);
     else es_trans<2, CONS>(V, nb, b, i, j, k, k1, bi, bj, bk0, bk1, comp0 + q, q, rules, epsb);
