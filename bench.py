@@ -31,25 +31,24 @@ HBM_PEAK_FALLBACK = 6792.7
 
 # Per-cell work of the kernels that bound the stage, counted by ncu on one batched stage of
 # 128^3 cells in 8 boxes of 64^3, NumSpec 13, ppm_type 1 (the counts per valid cell do not
-# depend on how many 64^3 boxes there are; summaries under profiles/):
-#   fp64: FP64 warp instructions (smsp__inst_executed_pipe_fp64.sum) per valid cell, one launch
-#   dram: DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per valid cell, one launch
+# depend on how many 64^3 boxes there are; summaries under profiles/).  Means over the stage's
+# launches of the kernel: MakeEdgeScal's take up to three components each, 15 in 7 launches.
+#   fp64: FP64 warp instructions (smsp__inst_executed_pipe_fp64.sum) per valid cell and launch
+#   dram: DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per valid cell and launch
 KERNEL_WORK = {
-    "k_ppm_cell<0,1,1>": {"fp64": 0.6582, "dram": 50.7},
-    "k_ppm_cell<1,1,1>": {"fp64": 0.6467, "dram": 51.3},
-    "k_ppm_cell<2,1,1>": {"fp64": 0.6482, "dram": 51.9},
-    "k_ppm_cell<0,1,0>": {"fp64": 0.7034, "dram": 50.4},
-    "k_ppm_cell<1,1,0>": {"fp64": 0.6736, "dram": 50.8},
-    "k_ppm_cell<2,1,0>": {"fp64": 0.6502, "dram": 50.9},
-    "k_update_rhox": {"fp64": 9.0, "dram": 675.0},
-    "k_ppm_face<0,1>": {"fp64": 0.4189, "dram": 18.4},
-    "k_ppm_face<1,1>": {"fp64": 0.4188, "dram": 19.0},
-    "k_ppm_face<2,1>": {"fp64": 0.4287, "dram": 19.0},
-    "k_es_edges<0,0,1>": {"fp64": 0.4433, "dram": 62.4},
-    "k_es_edges<1,0,1>": {"fp64": 0.4191, "dram": 63.7},
-    "k_es_edges<2,0,1>": {"fp64": 0.3989, "dram": 64.0},
+    "k_ppm_march<1,1>": {"fp64": 1.6770, "dram": 67.0},
+    "k_ppm_march<2,1>": {"fp64": 1.6975, "dram": 68.5},
+    "k_ppm_march<1,0>": {"fp64": 2.4055, "dram": 88.3},
+    "k_ppm_march<2,0>": {"fp64": 2.3840, "dram": 90.1},
+    "k_ppm_rows<1>": {"fp64": 1.9011, "dram": 65.5},
+    "k_ppm_rows<0>": {"fp64": 2.6385, "dram": 86.0},
+    "k_es_edge<0>": {"fp64": 1.7656, "dram": 349.1},
+    "k_es_trans<0>": {"fp64": 0.8664, "dram": 334.5},
+    "k_es_cinc<0>": {"fp64": 0.5709, "dram": 196.6},
+    "k_update_rhox": {"fp64": 6.5625, "dram": 565.3},
+    "k_rhox_flux": {"fp64": 3.9990, "dram": 701.6},
 }
-STAGE_FP64_PER_CELL = 146.50  # FP64 warp instructions per valid cell, whole stage
+STAGE_FP64_PER_CELL = 91.06  # FP64 warp instructions per valid cell, whole stage
 
 
 def jsonable(o):
@@ -70,7 +69,7 @@ def measured_peaks():
 
 
 def demangle(name):
-    """Short form of a madv kernel symbol: _ZN4madv10k_ppm_cellILi1ELi1ELi1EEEv... -> k_ppm_cell<1,1,1>."""
+    """Short form of a madv kernel symbol: _ZN4madv11k_ppm_marchILi1ELi1EEEv... -> k_ppm_march<1,1>."""
     import re
     m = re.match(r"_ZN4madv(\d+)", name)
     if not m:
@@ -942,7 +941,7 @@ def main():
     ap.add_argument("--profile-once", action="store_true",
                     help="run one batched stage and exit (the command ncu captures)")
     ap.add_argument("--staged-ppm", type=int, default=-1, choices=[-1, 0, 1],
-                    help="PPM form of the headline stage: 1 staged sweeps, 0 three launches, -1 the library default")
+                    help="PPM form of the headline stage: 1 staged sweeps, 0 marched, -1 the library default")
     ap.add_argument("--component-streams", type=int, default=-1, choices=[-1, 0, 1],
                     help="headline and AMR stages: 1 MakeEdgeScal components alternate between two streams, "
                          "0 one stream, -1 the library default")

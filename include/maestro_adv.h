@@ -388,8 +388,8 @@ int madv_profile_report(madv_ctx* ctx, char* buf, int len);
  * No counterpart in the reference. */
 int madv_autotune_trial(madv_ctx* ctx, int threads);
 /* The PPM form, tuned the same way per level: for each form f in [0, MADV_AUTOTUNE_PPM_FORMS):
- * madv_autotune_ppm_trial(ctx, f); run the stage.  Form 0 is the three-launch PPM (slopes,
- * interfaces, cell limiter); forms 1-4 the staged sweep kernel with tile shapes (across x;
+ * madv_autotune_ppm_trial(ctx, f); run the stage.  Form 0 is the marched PPM (columns in
+ * registers); forms 1-4 the staged sweep kernel with tile shapes (across x;
  * across y and z) 4x2; 32x2, 8x2; 32x1, 2x2; 16x2 and 4x4; 16x4.  finish keeps the form
  * whose PPM kernels took the least time on each level ("L<level> ppm_form" in the table).
  * Results do not depend on the form. */
@@ -401,10 +401,9 @@ int madv_autotune_apply(madv_ctx* ctx, const char* json);
 /* Implementation options of a context (no counterpart in the reference; results never
  * depend on them):
  *   "staged_ppm"      1: each PPM direction runs as one kernel over tiles of whole pencils
- *                     staged in shared memory by bulk copies; 0 (default): three launches
- *                     (slopes, interface values, cell limiter) through global memory, which
- *                     measure faster on GB300 (the stage is FP64-issue bound, and the fused
- *                     kernel's registers and shared memory cut its occupancy).
+ *                     staged in shared memory by bulk copies; 0 (default): columns marched in
+ *                     registers, which measure faster on GB300 (the stage is FP64-issue bound,
+ *                     and the staged kernel's registers and shared memory cut its occupancy).
  *   "sweep_tile_Da", "sweep_tile_Db" (D = 0, 1, 2): cells of a staged tile across
  *                     direction D, in the first / second transverse direction (x before y
  *                     before z); defaults 4 x 2 for D = 0 and 32 x 2 for D = 1, 2.
@@ -413,7 +412,7 @@ int madv_autotune_apply(madv_ctx* ctx, const char* json);
  *                     the caller's stream and a second one, which works in its own copy of
  *                     the per-component scratch (allocated at first use: about 46 doubles per
  *                     cell); 0 (default): one stream -- the stage is FP64-issue bound and
- *                     the overlap measures 0.5% on GB300.
+ *                     the overlap measures nothing at 256^3 and 3% at 128^3 on GB300.
  *   "es_inline"       1 (default): in 3-D, MakeEdgeScal forms only the side of each face that
  *                     the wind comes from, transverse states included, in per-direction
  *                     kernels that store three fields a component; 0: the predictor,

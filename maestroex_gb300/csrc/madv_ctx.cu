@@ -2721,8 +2721,7 @@ int madv_ppm(madv_ctx* h, const madv_box* bx, const madv_fab* s, int comp, const
 }
 
 // ------------------------------------------------------------------ launch-shape autotuner
-// The PPM forms the autotuner tries per level: three launches (slopes, interfaces, cell
-// limiter), or the staged sweep kernel with a tile shape across x (D = 0) and across y / z.
+// The PPM forms the autotuner tries per level: the marched sweeps (madv_march.cu), or the staged sweep kernel with a tile shape across x (D = 0) and across y / z.
 struct PpmForm {
     int staged;
     int x_a, x_b, yz_a, yz_b;

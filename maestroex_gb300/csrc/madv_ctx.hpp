@@ -196,7 +196,7 @@ struct Ctx {
     int tpb_trial = 0;
     // PPM form trials of the autotuner (madv_autotune_ppm_trial): the candidate being timed
     // (-1: none), the PPM kernels' device time per candidate, and the per-kernel cache of
-    // "is a PPM kernel" (k_dsvl, k_ppm_face, k_ppm_cell, k_ppm_sweep)
+    // "is a PPM kernel" (marched, staged, or of the separate launches)
     int ppm_trial = -1;
     std::map<int, double> ppm_tune_ms;
     std::map<const void*, bool> is_ppm_fn;

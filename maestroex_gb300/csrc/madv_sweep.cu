@@ -10,7 +10,7 @@
 // repeated between tiles.  The slopes and interface values then live in shared memory
 // only; the kernel writes just Ip / Im.  The arithmetic is the element functions of
 // madv_ppm.cuh, applied to shared-memory views, so results are bitwise those of the
-// three-launch form (k_dsvl, k_ppm_face, k_ppm_cell).
+// marched form and of k_dsvl, k_ppm_face, k_ppm_cell.
 //
 // Rows whose addresses or lengths do not meet the bulk copy's 16-byte rules (odd FAB
 // extents) are staged with ordinary loads instead.  The mbarrier wait is bounded: after
@@ -310,7 +310,7 @@ static void sweep_launch(Ctx& c, const SweepPlan& pl, int fs, int sc, int fu, in
 }
 
 // The fused sweep of direction D for component sc of field fs (Ip / Im into comps D of
-// fip / fim); false when the caller should use the three-launch form (2-D, or the adjoint
+// fip / fim); false when the caller should use another form (2-D, or the adjoint
 // keeping the interface values on its tape).
 bool ppm_sweep(Ctx& c, int D, int fs, int sc, int fu, int uc, int umac, int fip, int fim, int lo_ext, int hi_ext) {
     if (!c.staged_ppm || c.ndim != 3 || c.edge_tape_begin || c.P.ppm_type == 0) return false;

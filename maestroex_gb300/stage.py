@@ -328,7 +328,7 @@ class ScalarAdvectionStage:
     def autotune(self, run_batched, candidates=(32, 64, 128, 256, 512), ppm_forms=range(5)):
         """Launch-shape autotuner (madv_autotune_*): run_batched() runs the caller's stage once
         in MODE_BATCHED; it is timed per kernel for every candidate block size, and the fastest
-        per (level, kernel) is applied; then per level the fastest PPM form (three launches or
+        per (level, kernel) is applied; then per level the fastest PPM form (marched or
         the staged sweep with one of its tile shapes) among ppm_forms.  Returns the chosen
         table (dict)."""
         import json
