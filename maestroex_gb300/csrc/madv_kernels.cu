@@ -2081,18 +2081,19 @@ static void make_utrans_2d(Ctx& c) {
 }
 
 // MakeVelForce, planar 2-D (Source/MaestroForce.cpp:100-137)
-__global__ void k_vel_force_2d(KARGS, double cutoff_rho, int domhi, double dy) {
+__global__ void k_vel_force_2d(KARGS, double cutoff_rho, int domhi, RecipC r2dy) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView gpi = VW(F_GPI), rho = VW(F_SOLD), vf = VW(F_VELFORCE);
     const double r = at(rho, i, j, k, RHO);
     double rhopert = r - at(VW(F_RHO0CART), i, j, k);
     if (r < cutoff_rho) rhopert = 0.0;
-    at(vf, i, j, k, 0) = -at(gpi, i, j, k, 0) / r;
-    double f1 = (rhopert * at(VW(F_GRAVCART), i, j, k, 1) - at(gpi, i, j, k, 1)) / r - at(VW(F_W0FCART), i, j, k, 1);
+    const RecipV rr = recip_v(r);
+    at(vf, i, j, k, 0) = div_v(-at(gpi, i, j, k, 0), rr);
+    double f1 = div_v(rhopert * at(VW(F_GRAVCART), i, j, k, 1) - at(gpi, i, j, k, 1), rr) - at(VW(F_W0FCART), i, j, k, 1);
     if (j <= -1 || j >= domhi) {
     } else {
         const FabView ve = VW(F_UTRANS1), w0 = VW(F_W0CART);
-        f1 -= (at(ve, i, j + 1, k) + at(ve, i, j, k)) * (at(w0, i, j + 1, k, 1) - at(w0, i, j, k, 1)) / (2.0 * dy);
+        f1 -= div_c((at(ve, i, j + 1, k) + at(ve, i, j, k)) * (at(w0, i, j + 1, k, 1) - at(w0, i, j, k, 1)), r2dy);
     }
     at(vf, i, j, k, 1) = f1;
 }
@@ -2312,7 +2313,7 @@ __device__ __forceinline__ void es_predictor_2d_face(const FabView* __restrict__
 // MakeEdgeScalEdges, 2-D (Source/MaestroMakeEdgeScalars.cpp:454-644)
 template <int D>
 __device__ __forceinline__ void es_edges_2d_face(const FabView* __restrict__ V, int nb, int b, int i, int j, int k,
-    int comp, int q, int is_cons, double dt2, double dt4, double hd, double ht, int bclo,
+    int comp, int q, int is_cons, double dt2, double dt4ht, double dt2hd, double dt2ht, int bclo,
     int bchi, int domlo, int domhi, double rel_eps) {
     constexpr int di = D == 0, dj = D == 1;
     constexpr int T = 1 - D;
@@ -2325,15 +2326,15 @@ __device__ __forceinline__ void es_edges_2d_face(const FabView* __restrict__ V, 
     const double l = at(VW(F_SL0 + D), i, j, k, q), r = at(VW(F_SR0 + D), i, j, k, q);
     double lq, rq;
     if (is_cons) {
-        lq = l - (dt2 / ht) * (at(st, il + ti, jl + tj, k, q) * at(ut, il + ti, jl + tj, k) - at(st, il, jl, k, q) * at(ut, il, jl, k)) -
-             (dt2 / hd) * at(s, il, jl, k, comp) * (at(ud, i, j, k) - at(ud, il, jl, k)) + dt2 * fl;
-        rq = r - (dt2 / ht) * (at(st, i + ti, j + tj, k, q) * at(ut, i + ti, j + tj, k) - at(st, i, j, k, q) * at(ut, i, j, k)) -
-             (dt2 / hd) * at(s, i, j, k, comp) * (at(ud, i + di, j + dj, k) - at(ud, i, j, k)) + dt2 * fr;
+        lq = l - dt2ht * (at(st, il + ti, jl + tj, k, q) * at(ut, il + ti, jl + tj, k) - at(st, il, jl, k, q) * at(ut, il, jl, k)) -
+             dt2hd * at(s, il, jl, k, comp) * (at(ud, i, j, k) - at(ud, il, jl, k)) + dt2 * fl;
+        rq = r - dt2ht * (at(st, i + ti, j + tj, k, q) * at(ut, i + ti, j + tj, k) - at(st, i, j, k, q) * at(ut, i, j, k)) -
+             dt2hd * at(s, i, j, k, comp) * (at(ud, i + di, j + dj, k) - at(ud, i, j, k)) + dt2 * fr;
     } else {
-        lq = l - (dt4 / ht) * (at(ut, il + ti, jl + tj, k) + at(ut, il, jl, k)) *
+        lq = l - dt4ht * (at(ut, il + ti, jl + tj, k) + at(ut, il, jl, k)) *
                      (at(st, il + ti, jl + tj, k, q) - at(st, il, jl, k, q)) +
              dt2 * fl;
-        rq = r - (dt4 / ht) * (at(ut, i + ti, j + tj, k) + at(ut, i, j, k)) * (at(st, i + ti, j + tj, k, q) - at(st, i, j, k, q)) +
+        rq = r - dt4ht * (at(ut, i + ti, j + tj, k) + at(ut, i, j, k)) * (at(st, i + ti, j + tj, k, q) - at(st, i, j, k, q)) +
              dt2 * fr;
     }
     const double u = at(ud, i, j, k);
@@ -2351,9 +2352,10 @@ __device__ __forceinline__ void es_edges_2d_face(const FabView* __restrict__ V, 
     at(VW(F_SEDGE0 + D), i, j, k, comp) = v;
 }
 
-// the boundary rules of up to three components of a launch
+// the boundary rules of up to three components of a launch; dt / 4 and dt / 2 over the cell sizes
 struct Es2dRules {
     int lo[3][2], hi[3][2];
+    double dt4h[2], dt2h[2];
 };
 __global__ void k_es_predictor_2d(KARGS, int comp0, unsigned nq, int ppm_type, double dt2, const __grid_constant__ DirRules p,
                                   const __grid_constant__ Es2dRules bc, double rel_eps) {
@@ -2366,16 +2368,16 @@ __global__ void k_es_predictor_2d(KARGS, int comp0, unsigned nq, int ppm_type, d
         es_predictor_2d_face<1>(V, nb, b, i, j, k, comp0 + q, q, ppm_type, dt2, p.h[1], bc.lo[q][1], bc.hi[q][1], p.dl[1],
                                 p.dh[1], rel_eps);
 }
-__global__ void k_es_edges_2d(KARGS, int comp0, unsigned nq, int is_cons, double dt2, double dt4,
+__global__ void k_es_edges_2d(KARGS, int comp0, unsigned nq, int is_cons, double dt2,
                               const __grid_constant__ DirRules p, const __grid_constant__ Es2dRules bc, double rel_eps) {
     const unsigned bx = blockIdx.x / nq, q = blockIdx.x - bx * nq;
     MADV_ELEMENT_OF(bx, R, ne, g0, g1, b, i, j, k);
     if (part_ == 0)
-        es_edges_2d_face<0>(V, nb, b, i, j, k, comp0 + q, q, is_cons, dt2, dt4, p.h[0], p.h[1], bc.lo[q][0], bc.hi[q][0],
-                            p.dl[0], p.dh[0], rel_eps);
+        es_edges_2d_face<0>(V, nb, b, i, j, k, comp0 + q, q, is_cons, dt2, bc.dt4h[1], bc.dt2h[0], bc.dt2h[1], bc.lo[q][0],
+                            bc.hi[q][0], p.dl[0], p.dh[0], rel_eps);
     else
-        es_edges_2d_face<1>(V, nb, b, i, j, k, comp0 + q, q, is_cons, dt2, dt4, p.h[1], p.h[0], bc.lo[q][1], bc.hi[q][1],
-                            p.dl[1], p.dh[1], rel_eps);
+        es_edges_2d_face<1>(V, nb, b, i, j, k, comp0 + q, q, is_cons, dt2, bc.dt4h[0], bc.dt2h[1], bc.dt2h[0], bc.lo[q][1],
+                            bc.hi[q][1], p.dl[1], p.dh[1], rel_eps);
 }
 
 // marched PPM: up to three components a launch, each with its own Ip / Im and its own component of
@@ -2395,6 +2397,10 @@ static void make_edge_scal_2d(Ctx& c, int start_comp, int num_comp, int which_bc
             for (int d = 0; d < 2; ++d) ppm_any(c, d, F_SOLD, comp, bh[comp], F_UMAC0 + d, 0, 1, F_IPC0, F_IMC0);
         }
         Es2dRules bc{};
+        for (int d = 0; d < 2; ++d) {
+            bc.dt4h[d] = dt4 / c.P.dx[d];
+            bc.dt2h[d] = dt2 / c.P.dx[d];
+        }
         for (int q = 0; q < nq; ++q)
             for (int d = 0; d < 2; ++d) {
                 bc.lo[q][d] = bh[comp + q].lo[d];
@@ -2402,36 +2408,37 @@ static void make_edge_scal_2d(Ctx& c, int start_comp, int num_comp, int which_bc
             }
         launch(c, rg2_inner_faces(c), nq, k_es_predictor_2d, c.V(), comp, (unsigned)nq, c.P.ppm_type, dt2, p, bc,
                c.P.rel_eps);
-        launch(c, rg_faces(c), nq, k_es_edges_2d, c.V(), comp, (unsigned)nq, is_cons, dt2, dt4, p, bc, c.P.rel_eps);
+        launch(c, rg_faces(c), nq, k_es_edges_2d, c.V(), comp, (unsigned)nq, is_cons, dt2, p, bc, c.P.rel_eps);
     }
 }
 
 // ModifyScalForce, planar 2-D (Source/MaestroForce.cpp:419-447)
-__global__ void k_modify_scal_force_2d(KARGS, int comp, int s0cart, int fullform, double dx0, double dx1) {
+__global__ void k_modify_scal_force_2d(KARGS, int comp, int s0cart, int fullform, RecipC r0, RecipC r1) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView um = VW(F_UMAC0), vm = VW(F_UMAC1), s0a = VW(s0cart), s0e = VW(F_S0ECART), w0a = VW(F_W0CART);
     const double scal = at(VW(F_SOLD), i, j, k, comp);
-    double divu = (at(um, i + 1, j, k) - at(um, i, j, k)) / dx0 + (at(vm, i, j + 1, k) - at(vm, i, j, k)) / dx1;
-    divu += (at(w0a, i, j + 1, k, 1) - at(w0a, i, j, k, 1)) / dx1;
+    const double du = at(um, i + 1, j, k) - at(um, i, j, k);
+    double divu = div_c(du, r0) + div_c(at(vm, i, j + 1, k) - at(vm, i, j, k), r1);
+    divu += div_c(at(w0a, i, j + 1, k, 1) - at(w0a, i, j, k, 1), r1);
     double& force = at(VW(F_SCALFORCE), i, j, k, comp);
     if (fullform == 1) {
         force -= scal * divu;
     } else {
         const double s0 = at(s0a, i, j, k);
-        const double divs0u = s0 * (at(um, i + 1, j, k) - at(um, i, j, k)) / dx0 +
-                              (at(vm, i, j + 1, k) * at(s0e, i, j + 1, k) - at(vm, i, j, k) * at(s0e, i, j, k)) / dx1;
+        const double divs0u = div_c(s0 * du, r0) +
+                              div_c(at(vm, i, j + 1, k) * at(s0e, i, j + 1, k) - at(vm, i, j, k) * at(s0e, i, j, k), r1);
         force += -(scal - s0) * divu - divs0u;
     }
 }
 
 // MakeRhoHForce, planar 2-D (Source/MaestroForce.cpp:586-603)
-__global__ void k_rhoh_force_2d(KARGS, int cutoff, int domhi, double dy, int psi_in, int add_thermal) {
+__global__ void k_rhoh_force_2d(KARGS, int cutoff, int domhi, RecipC ry, int psi_in, int add_thermal) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView p0c = VW(F_P0CART);
     double gradp0;
     if (j < cutoff) gradp0 = at(VW(F_RHO0CART), i, j, k) * at(VW(F_GRAVCART), i, j, k, 1);
-    else if (j == domhi) gradp0 = (at(p0c, i, j, k) - at(p0c, i, j - 1, k)) / dy;
-    else gradp0 = (at(p0c, i, j + 1, k) - at(p0c, i, j, k)) / dy;
+    else if (j == domhi) gradp0 = div_c(at(p0c, i, j, k) - at(p0c, i, j - 1, k), ry);
+    else gradp0 = div_c(at(p0c, i, j + 1, k) - at(p0c, i, j, k), ry);
     const FabView vm = VW(F_UMAC1);
     const double veladv = half(at(vm, i, j, k) + at(vm, i, j + 1, k));
     double f = veladv * gradp0;
@@ -2513,13 +2520,13 @@ __global__ void k_rhoh_flux_2d(KARGS, int ept, int spt, RhohBase q) {
 }
 
 // UpdateScal, 2-D (Source/MaestroAdvection.cpp:117-251)
-__global__ void k_update_rhox_2d(KARGS, int nspec, double dt, double dx0, double dx1, double half_cutoff) {
+__global__ void k_update_rhox_2d(KARGS, int nspec, double dt, RecipC r0, RecipC r1, double half_cutoff) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView so = VW(F_SOLD), sn = VW(F_SNEW), fx = VW(F_SFLUX0), fy = VW(F_SFLUX1), fo = VW(F_SCALFORCE);
     for (int n = 0; n < nspec; ++n) {
         const int comp = FIRSTSPEC + n;
-        double divterm = (at(fx, i + 1, j, k, comp) - at(fx, i, j, k, comp)) / dx0;
-        divterm += (at(fy, i, j + 1, k, comp) - at(fy, i, j, k, comp)) / dx1;
+        double divterm = div_c(at(fx, i + 1, j, k, comp) - at(fx, i, j, k, comp), r0);
+        divterm += div_c(at(fy, i, j + 1, k, comp) - at(fy, i, j, k, comp), r1);
         at(sn, i, j, k, comp) = at(so, i, j, k, comp) + dt * (-divterm + at(fo, i, j, k, comp));
     }
     double rho = at(so, i, j, k, RHO);
@@ -2553,11 +2560,11 @@ __global__ void k_update_rhox_2d(KARGS, int nspec, double dt, double dx0, double
     }
 }
 
-__global__ void k_update_rhoh_2d(KARGS, double dt, double dx0, double dx1, int eos_check, double cutoff, int* flag) {
+__global__ void k_update_rhoh_2d(KARGS, double dt, RecipC r0, RecipC r1, int eos_check, double cutoff, int* flag) {
     MADV_ELEMENT(R, ne, g0, g1, b, i, j, k);
     const FabView so = VW(F_SOLD), sn = VW(F_SNEW), fx = VW(F_SFLUX0), fy = VW(F_SFLUX1), fo = VW(F_SCALFORCE);
-    const double divterm = ((at(fx, i + 1, j, k, RHOH) - at(fx, i, j, k, RHOH)) / dx0 +
-                            (at(fy, i, j + 1, k, RHOH) - at(fy, i, j, k, RHOH)) / dx1);
+    const double divterm = div_c(at(fx, i + 1, j, k, RHOH) - at(fx, i, j, k, RHOH), r0) +
+                           div_c(at(fy, i, j + 1, k, RHOH) - at(fy, i, j, k, RHOH), r1);
     at(sn, i, j, k, RHOH) = at(so, i, j, k, RHOH) + dt * (-divterm + at(fo, i, j, k, RHOH));
     if (eos_check && at(sn, i, j, k, RHO) <= cutoff) atomicOr(flag, 1);
 }
@@ -2572,15 +2579,16 @@ void addw0_2d(Ctx& c, int f0, double mult) {
 void make_vel_force_2d(Ctx& c) {
     set_val(c, F_VELFORCE, 0.0, 0, 2, 1);
     launch(c, rg2(c, 0), 1, k_vel_force_2d, c.V(), c.P.buoyancy_cutoff_factor * c.P.base_cutoff_density,
-           c.P.dom_hi[1], c.P.dx[1]);
+           c.P.dom_hi[1], make_recip(2.0 * c.P.dx[1]));
 }
 void modify_scal_force_2d(Ctx& c, int comp, int s0cart_fid, int fullform) {
-    launch(c, rg2(c, 0), 1, k_modify_scal_force_2d, c.V(), comp, s0cart_fid, fullform, c.P.dx[0], c.P.dx[1]);
+    launch(c, rg2(c, 0), 1, k_modify_scal_force_2d, c.V(), comp, s0cart_fid, fullform, make_recip(c.P.dx[0]),
+           make_recip(c.P.dx[1]));
 }
 void make_rhoh_force_2d(Ctx& c, int is_prediction, int add_thermal) {
     const int ept = c.P.enthalpy_pred_type;
     const int psi_in = (is_prediction == 1 && ept == 2) || (is_prediction == 1 && ept == 0) || (is_prediction == 0);
-    launch(c, rg2(c, 0), 1, k_rhoh_force_2d, c.V(), c.P.base_cutoff_density_coord, c.P.dom_hi[1], c.P.dx[1], psi_in,
+    launch(c, rg2(c, 0), 1, k_rhoh_force_2d, c.V(), c.P.base_cutoff_density_coord, c.P.dom_hi[1], make_recip(c.P.dx[1]), psi_in,
            add_thermal);
 }
 void put_in_pert_form_2d(Ctx& c, const double* d_s0, int comp, int flag) {
@@ -2608,10 +2616,11 @@ void sum_species_edges_2d(Ctx& c) {
 void update_scal_2d(Ctx& c, int start_comp) {
     const RegionTable& rt = rg2(c, 0);
     if (start_comp == RHOH)
-        launch(c, rt, 1, k_update_rhoh_2d, c.V(), c.P.dt, c.P.dx[0], c.P.dx[1], c.P.do_eos_h_above_cutoff,
+        launch(c, rt, 1, k_update_rhoh_2d, c.V(), c.P.dt, make_recip(c.P.dx[0]), make_recip(c.P.dx[1]), c.P.do_eos_h_above_cutoff,
                c.P.base_cutoff_density, c.d_flag);
     else
-        launch(c, rt, 1, k_update_rhox_2d, c.V(), c.nspec, c.P.dt, c.P.dx[0], c.P.dx[1], 0.5 * c.P.base_cutoff_density);
+        launch(c, rt, 1, k_update_rhox_2d, c.V(), c.nspec, c.P.dt, make_recip(c.P.dx[0]), make_recip(c.P.dx[1]),
+               0.5 * c.P.base_cutoff_density);
 }
 void make_utrans_2d_entry(Ctx& c) { make_utrans_2d(c); }
 
