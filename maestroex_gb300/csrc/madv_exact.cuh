@@ -94,6 +94,8 @@ __host__ inline long long dbits_host(double x) {
 __device__ __forceinline__ bool gt0(double x) { return dbits(x) > 0; }
 // x < 0.0 (-0 is not below 0): the pattern of -x is positive
 __device__ __forceinline__ bool lt0(double x) { return dbits(dflip(x)) > 0; }
+// x is NaN (a quiet one, as every FP64 instruction returns)
+__device__ __forceinline__ bool is_nan(double x) { return (dhigh(x) & 0x7fffffff) > 0x7ff00000; }
 // |x| > 0.0
 __device__ __forceinline__ bool nz(double x) { return dmag(x) != 0; }
 // x > t, with tb = bits(t), t >= +0

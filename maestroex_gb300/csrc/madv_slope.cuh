@@ -47,15 +47,18 @@ __device__ __forceinline__ double limited_slope(SF S, int I, int bclo, int bchi,
         }
     } else if (slope_order == 4) {
         // dcen, dmin, dpls of the three cells and their limited slopes dxl, dxr; the
-        // differences are formed once, the limits on the integer pipe (vl_slope)
+        // differences are formed once, the limits on the integer pipe (vl_slope).  A NaN among the
+        // cells makes a difference NaN: the comparisons then give slope 0 where the product of
+        // two differences is NaN, and pass a NaN ds on.
         const double e0 = S(-1) - S(-2), e1 = S(0) - S(-1), e2 = S(1) - S(0), e3 = S(2) - S(1);
-        double dxl = vl_slope(S(0) - S(-2), e0, e1), dxr = vl_slope(S(2) - S(0), e2, e3);
+        const bool n0 = is_nan(e0), n1 = is_nan(e1), n2 = is_nan(e2), n3 = is_nan(e3);
+        double dxl = n0 || n1 ? 0.0 : vl_slope(S(0) - S(-2), e0, e1), dxr = n2 || n3 ? 0.0 : vl_slope(S(2) - S(0), e2, e3);
         const double dcen = half(S(1) - S(-1));
         double dmin = twice(e1), dpls = twice(e2);
-        const double dlim = prod_gt0(dpls, dmin) ? __longlong_as_double(min(dmag(dmin), dmag(dpls))) : 0.0;
+        const double dlim = !n1 && !n2 && prod_gt0(dpls, dmin) ? __longlong_as_double(min(dmag(dmin), dmag(dpls))) : 0.0;
         double ds = 4.0 / 3.0 * dcen - div_6(dxr + dxl, r6);
         auto limited = [&](double v) {  // copysign(1, dcen) * min(|v|, dlim)
-            return dsigned(__longlong_as_double(min(dmag(v), dmag(dlim))), dcen);
+            return is_nan(v) ? v : dsigned(__longlong_as_double(min(dmag(v), dmag(dlim))), dcen);
         };
         out = limited(ds);
         // the x sweep tests the centred dlim where y and z test the one-sided slim
