@@ -38,10 +38,11 @@ __device__ __forceinline__ double ppm2_face_raw(SF S, int m) {
 }
 // Whether it may lie outside its two cells a, b.  reference: (se - s(m-1)) * (s(m) - se) < 0, i.e.
 // the product of (se - s(m-1)) and -(s(m) - se) = se - s(m) (exact) is positive.  The
-// differences have the sign of the comparison (on integer keys, no FP64 instruction).
+// differences have the sign of the comparison (on integer keys, no FP64 instruction) unless se
+// is infinite or NaN, whose differences may be NaN: ppm2_face_limit decides on those.
 __device__ __forceinline__ bool ppm2_face_out(double se, double a, double b) {
     const long long ks = dkey(se), ka = dkey(a), kb = dkey(b);
-    return (ks > ka && ks > kb) || (ks < ka && ks < kb);
+    return (ks > ka && ks > kb) || (ks < ka && ks < kb) || (dhigh(se) & 0x7ff00000) == 0x7ff00000;
 }
 // Colella's limited curvature max(min(a, 1.25 min of the signed curvatures), 0), a >= 0, as
 // mx(mn(..), 0) of FP64 comparisons gives it.  Finite ones: the smallest positive curvature by its
@@ -216,7 +217,9 @@ __device__ __forceinline__ void ppm_cell_any(SF S, FF F, RF FR, int I, int lo_ex
                 double dafacep = sedgerr - sedger;
                 double dabarm = s0 - S(-1);
                 double dabarp = S(1) - s0;
-                const bool face = min(dmag(dafacem), dmag(dafacep)) >= min(dmag(dabarm), dmag(dabarp));
+                // (the minimum of a pair is NaN where its first value is, and no minimum compares then)
+                const bool face = !is_nan(dafacem) && !is_nan(dabarm) &&
+                                  min(dmag(dafacem), dmag(dafacep)) >= min(dmag(dabarm), dmag(dabarp));
                 extremum = !prod_gt0(face ? dafacem : dabarm, face ? dafacep : dabarp);
             }
             if (extremum) {

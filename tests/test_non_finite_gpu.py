@@ -7,9 +7,10 @@ import torch
 import pyoracle
 from maestroex_gb300 import configs
 from maestroex_gb300.params import FIRSTSPEC, INTERIOR
-from maestroex_gb300.stage import MultiFab, make_stage
+from maestroex_gb300.stage import MultiFab, ScalarAdvectionStage, make_stage
 from members import MemberInputs, zeros_like
 from test_members_gpu import to_mf
+from test_ppm_box_gpu import ppm_case
 
 pytestmark = pytest.mark.gpu
 
@@ -46,3 +47,29 @@ def test_limited_slopes(cons, order, special):
             c = slice(FIRSTSPEC, FIRSTSPEC + 4)
             assert np.array_equal(f.cpu().numpy()[c], r[c], equal_nan=True), d
     st.close()
+
+
+@pytest.mark.parametrize("umac", [0, 1])
+@pytest.mark.parametrize("D", range(3))
+@pytest.mark.parametrize("special", [np.nan, np.inf])
+def test_fourth_order_limiter(umac, D, special):
+    """ppm_type 2 next to planes of NaN (the cell that has one as the outermost of its stencil,
+    three cells below it) and of infinities (every cell)."""
+    bx, bc = (0, 0, 0, 33, 33, 33), (0,) * 6
+    p, s, s_lo, vel, vel_lo = ppm_case(2, umac, bc, 77 + D, bx, ndom=40)
+    planes = [slice(None)] * 3
+    planes[2 - D] = slice(4, None, 9)
+    s[1][tuple(planes)] = special
+    ref = pyoracle.ppm(p, bx, s, s_lo, 1, vel, vel_lo, umac, bc)
+    st = ScalarAdvectionStage(p)
+    out = [torch.zeros((3, 34, 34, 34), dtype=torch.float64, device="cuda") for _ in range(2)]
+    st.ppm(bx, torch.from_numpy(s).cuda(), s_lo, 1, [torch.from_numpy(v).cuda() for v in vel], vel_lo, umac, bc, *out)
+    torch.cuda.synchronize()
+    st.close()
+    if np.isnan(special):
+        planes[2 - D] = slice(4 + s_lo[D] + 3, None, 9)
+    else:
+        planes[2 - D] = slice(None)
+    for a, r in zip(out, ref):
+        a, r = a[D].cpu().numpy()[tuple(planes)], r[D][tuple(planes)]
+        assert np.isfinite(r).any() and np.array_equal(a, r, equal_nan=True)
