@@ -196,6 +196,9 @@ __global__ void k_mg_smooth(MGGrid g, MGBC bc, int color) {
     mg_smooth_cell(g, bc, 2 * i + ((j + k + color) & 1), j, k);
 }
 
+// the bit pattern of |x| for a maximum of such: 0 where x is NaN, which fmax ignores
+__device__ __forceinline__ long long mg_mag(double x) { return is_nan(x) ? 0 : dmag(x); }
+
 // max |rhs - A phi| (bit pattern of a non-negative double)
 __global__ void k_mg_resid_max(MGGrid g, MGBC bc, unsigned long long* out_max) {
     MADV_LET_NEXT();
@@ -206,7 +209,7 @@ __global__ void k_mg_resid_max(MGGrid g, MGBC bc, unsigned long long* out_max) {
     for (int c = (int)(blockIdx.x * blockDim.x + threadIdx.x); c < n; c += gridDim.x * blockDim.x) {
         int i, j, k;
         piece_ijk(lo, g.n, g.dv, c, i, j, k);
-        m = max(m, dmag(mg_resid_cell(g, bc, i, j, k)));
+        m = max(m, mg_mag(mg_resid_cell(g, bc, i, j, k)));
     }
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0 && m) atomicMax(out_max, (unsigned long long)m);
@@ -383,7 +386,7 @@ __global__ void k_mg_norms(const double* __restrict__ x, long n, unsigned long l
     long long m = 0;
     double s = 0.0;
     for (long c = (long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long)gridDim.x * blockDim.x) {
-        m = max(m, dmag(x[c]));
+        m = max(m, mg_mag(x[c]));
         if (part) s += x[c];
     }
     for (int o = 16; o > 0; o >>= 1) {

@@ -1,12 +1,13 @@
 """Infinities and NaNs in the state, where a limiter's comparisons decide what becomes of them:
-against the oracle, whose limiters are the reference's expressions, bit for bit (a NaN is a NaN)."""
+against the oracle, whose limiters are the reference's expressions, bit for bit (a NaN is a NaN);
+and in the right-hand side of the MAC projection."""
 import numpy as np
 import pytest
 import torch
 
 import pyoracle
-from maestroex_gb300 import configs
-from maestroex_gb300.params import FIRSTSPEC, INTERIOR
+from maestroex_gb300 import capi, configs
+from maestroex_gb300.params import FIRSTSPEC, INTERIOR, OUTFLOW
 from maestroex_gb300.stage import MultiFab, ScalarAdvectionStage, make_stage
 from members import MemberInputs, zeros_like
 from test_members_gpu import to_mf
@@ -73,3 +74,32 @@ def test_fourth_order_limiter(umac, D, special):
     for a, r in zip(out, ref):
         a, r = a[D].cpu().numpy()[tuple(planes)], r[D][tuple(planes)]
         assert np.isfinite(r).any() and np.array_equal(a, r, equal_nan=True)
+
+
+@pytest.mark.parametrize("side,special,cycles", [(INTERIOR, np.nan, 0), (INTERIOR, np.inf, 0), (OUTFLOW, np.nan, 1)])
+def test_mac_projection_stops(side, special, cycles):
+    """The stopping test's maximum passes NaNs over: none left to reduce ends the cycles."""
+    cfg = configs.planar_config(n=(32, 32, 48), nspec=2, ppm_type=1, max_grid=16, bc_lo=(INTERIOR,) * 2 + (side,),
+                                bc_hi=(INTERIOR,) * 2 + (side,), w0_amp=0.0)
+    st, q = make_stage(cfg), mac_inputs(cfg, special)
+    assert st.mac_project(*q, np.full(48, 1.0e6), max_iter=20)[0] == cycles
+    st.close()
+
+
+@pytest.mark.parametrize("exact", [True, False])
+def test_spherical_mac_projection_refuses_a_nan(exact):
+    cfg = configs.spherical_config(n=32, nspec=2, ppm_type=1, max_grid=16, exact=exact)
+    st, q = make_stage(cfg), mac_inputs(cfg, np.nan)
+    with pytest.raises(capi.MadvError) as e:
+        st.mac_project(*q, cfg["rho0_old"], max_iter=20)
+    assert e.value.code == -7  # MADV_ERR_NOCONV
+    st.close()
+
+
+def mac_inputs(cfg, special):
+    """umac, macrhs with one special cell, rho"""
+    b = cfg["boxes"]
+    rhs = MultiFab(b, 1, 0)
+    rhs.data.normal_(generator=torch.Generator(device="cuda").manual_seed(4))
+    rhs.fabs[0][0, 3, 4, 5] = special
+    return [MultiFab(b, 1, 1, nodal=d, fill=1.0e3) for d in range(3)], rhs, MultiFab(b, 1, 0).from_domain(cfg["sold"][:1])
