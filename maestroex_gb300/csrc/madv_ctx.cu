@@ -1447,10 +1447,15 @@ static int init_level(Ctx& c, const madv_params& p, int lev) {
     return MADV_OK;
 }
 
-static void destroy_level(Ctx& c) {
-    free_layout(c);
+static void free_radial(Ctx& c) {
     for (auto& kv : c.d1) cudaFree(kv.second);
     c.d1.clear();
+    c.h1.clear();
+}
+
+static void destroy_level(Ctx& c) {
+    free_layout(c);
+    free_radial(c);
     for (auto e : c.ev_pool) cudaEventDestroy(e);
     c.ev_pool.clear();
     if (c.side) cudaStreamDestroy(c.side);
@@ -1753,7 +1758,9 @@ int madv_set_layout_levels(madv_ctx* h, int nlev, const int* nboxes, const madv_
         // (Source/MaestroSetup.cpp:60-96, Source/BaseStateGeometry.cpp:86-104)
         const Ctx& fl = H[nlev - 1];
         for (auto* c : H.L) {
+            const int nr = c->nr;
             sph_radial_grid(*c, fl.P.dx[0], fl.P.dom_hi[0] - fl.P.dom_lo[0] + 1);
+            if (c->nr != nr) free_radial(*c);  // its arrays are as long as the grid
             c->have_base = false;
         }
     }
