@@ -2525,8 +2525,10 @@ int madv_mac_project(madv_ctx* h, const madv_multifab* umac, const madv_multifab
             double*& d = c.d1["beta0_mac"];
             const std::vector<double> v = radial_table(c, b);
             if (!d && !cuda_ok(cudaMalloc(&d, sizeof(double) * radial_table_max(c)), "cudaMalloc(beta0)")) return MADV_ERR_CUDA;
+            // (the source is this block's: the copy ends here)
             if (!cuda_ok(cudaMemcpyAsync(d, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice, c.stream),
-                         "cudaMemcpyAsync(beta0)"))
+                         "cudaMemcpyAsync(beta0)") ||
+                !cuda_ok(cudaStreamSynchronize(c.stream), "cudaStreamSynchronize(beta0)"))
                 return MADV_ERR_CUDA;
             make_s0mac_h(H, "beta0_mac", F_S0MAC0);
         }
