@@ -338,6 +338,15 @@ __device__ __forceinline__ EsBox es_box(const FabView* __restrict__ V, int nb, i
     return EsBox{p.p, p.sj, p.sk, p.sn, p.lo0, p.lo1, p.lo2};
 }
 
+// The offset of one of a face's two cells: lo (below) or o.  Opaque to the compiler: the offset -1 of
+// D = 0 where u < 0, folded into the address arithmetic by nvcc 13.0.88, read the wrong cell (the
+// second state of a tie with u in [-rel_eps, 0), 2-way select of -1 and 0 on the sign of u).
+__device__ __forceinline__ long side_offset(bool below, long lo, long o) {
+    long c = below ? lo : o;
+    asm("" : "+l"(c));
+    return c;
+}
+
 // v less the transverse correction of the cell at o (components sn apart)
 template <bool CONS>
 __device__ __forceinline__ double es_less(double v, const double* c, long o, long sn) {
@@ -354,7 +363,7 @@ __device__ __noinline__ double es_bnd(const double* ip, const double* im, const 
     const bool below = rule & 8;
     if (code == FR_ZERO) return 0.0;
     if (code == FR_GHOST) return *ghost;
-    const long oc = below ? lo : o;
+    const long oc = side_offset(below, lo, o);
     double v = (below ? ip : im)[oc];
     if (code == FR_CLAMP) v = clamp_out(v, below);
     if (inc) {
@@ -463,7 +472,7 @@ __device__ __forceinline__ void es_trans(const FabView* __restrict__ V, int nb, 
         double un = 0;
         if (k + 1 < k1) un = pu[uk];
         const bool left = dhigh(u) >= 0;
-        const long oc = left ? -s : 0;
+        const long oc = side_offset(left, -s, 0);
         const double base = (left ? ip : im)[oc];
         double vb = 0.0, vc = 0.0;
         if (wantB) vb = es_less<CONS>(base, cb, oc, x.sn);
@@ -528,10 +537,7 @@ struct EsFace {
     template <bool CLAMP>
     __device__ __forceinline__ double state(const FabView* __restrict__ V, int nb, int b, int i, int j, int k, int comp,
                                             bool below, int force_zero, double dt2, const EsCons& ec) const {
-        long c = below ? -s : 0;
-        // (kept from the compiler: folded into an address, the -1 of D = 0 came out wrong for the
-        // second state of a tie with u < 0)
-        asm("" : "+l"(c));
+        const long c = side_offset(below, -s, 0);
         double v = (below ? ip : im)[c];
         if (CLAMP) v = clamp_out(v, below);
         if (CONS) {
@@ -592,7 +598,7 @@ __device__ __forceinline__ void es_edge(const FabView* __restrict__ V, int nb, i
         *out = v;
         u = un;
         pu += uk, x.ip += x.s2, x.im += x.s2, x.ta += x.s2, x.tb += x.s2, x.qa += x.s2, x.qb += x.s2;
-        x.fp += x.fk, x.fm += x.fk;
+        if (!force_zero) x.fp += x.fk, x.fm += x.fk;  // (null otherwise)
         out += e.sk;
     }
 }
