@@ -15,7 +15,10 @@
 //    at most a few X solve, found once from the residues of X modulo Y (multiplication by an
 //    arbitrary-precision constant: N. Brisebarre, J.-M. Muller, IEEE Trans. Comput. 57(2),
 //    2008); the significands that do round wrongly are kept (none where Y ends in two zero
-//    bits) and take the IEEE division, as do zeros and |a| outside [2^-959, 2^977).
+//    bits) and take the IEEE division, as do zeros, |a| outside [2^-959, 2^977) and those whose
+//    quotient is outside [2^-960, 2^1020): below, a*zl loses bits as a subnormal number (of a
+//    significand next to a boundary and y near 2^27 the quotient came out wrong for |a| < 2^-940);
+//    above, the two products can be infinities of opposite sign.
 //    Cost: 1 DMUL + 1 DFMA.
 //    By 6 there are none: with a = A 2^e the quotient is A/3 2^(e-1), and a third of an integer
 //    is never closer than 1/6 ulp to a rounding boundary.
@@ -173,7 +176,8 @@ __device__ __forceinline__ bool prod_gt0(double x, double y) {
 struct RecipC {
     double y, zh, zl;
     unsigned bad[4];  // low words of the significands that the two-step quotient misrounds
-    int nbad;         // -1: more than 4 (or y not normal), the quotient is corrected
+    int nbad;         // -1: more than 4, the quotient is corrected
+    unsigned exlo, exn;  // exponent fields of a that are divided so: exn from exlo (0: y not normal)
 };
 
 // The integer significands X in [2^52, 2^53) whose quotient by Y (the same range) comes within
@@ -205,12 +209,14 @@ __host__ inline RecipC make_recip(double y) {
     const double e = __builtin_fma(-r.zh, y, 1.0);
     r.zl = e / y;
     r.nbad = 0;
+    r.exlo = r.exn = 0;
+    for (unsigned& q : r.bad) q = 0;
     const long long b = dbits_host(y);
     const int ex = (int)(b >> 52) & 0x7ff;
-    if (ex < 64 || ex > 1983) {  // the reciprocal's words could under- or overflow
-        r.nbad = -1;
-        return r;
-    }
+    if (ex < 64 || ex > 1983) return r;  // the reciprocal's words could under- or overflow
+    const int lo = ex > 1024 ? ex - 960 : 64, hi = ex < 980 ? ex + 1020 : 2000;
+    r.exlo = (unsigned)lo;
+    r.exn = (unsigned)(hi - lo);
     unsigned long long X[16];
     const int n = hard_significands((unsigned long long)(b & 0x000fffffffffffffLL) | (1ULL << 52), X);
     for (int q = 0; q < n; ++q) {
@@ -235,7 +241,7 @@ __device__ __forceinline__ double div_c(double a, const RecipC& r) {
     int hi, lo;
     dsplit(a, hi, lo);
     const unsigned ex = ((unsigned)hi >> 20) & 0x7ff;
-    if (ex < 64 || ex >= 2000) {
+    if (ex - r.exlo >= r.exn) {
         // Zeros are common (still fluid, equal neighbours) and cost no division: one lane's took its
         // warp's 20 FP64 instructions, 21 instead of 5 for a tracing coefficient.
         if ((((unsigned)hi << 1) | (unsigned)lo) == 0 && dhigh(r.y) > 0) return a;

@@ -95,7 +95,7 @@ __global__ void k_selftest(unsigned long long n, unsigned long long seed, RecipC
         // the significands next to a rounding boundary of the quotient, and one off them
         if (hx.n && kind == 4) {
             unsigned long long X = hx.x[(h >> 40) % hx.n] + ((h >> 50) & 1 ? 0 : (h >> 51) % 3 - 1);
-            a = __longlong_as_double((long long)((X & 0x000fffffffffffffULL) | ((100 + (h >> 20) % 1800) << 52)));
+            a = __longlong_as_double((long long)((X & 0x000fffffffffffffULL) | ((60 + (h >> 20) % 1950) << 52)));
             if (h & 32) a = -a;
         }
         const double q = div_c(a, r);
