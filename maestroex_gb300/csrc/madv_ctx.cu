@@ -1355,7 +1355,8 @@ int Ctx::tpb_of(const void* fn) {
     int t = tpb_trial;
     if (!t) {
         auto it = tpb_choice.find(fn);
-        t = it == tpb_choice.end() ? 256 : it->second;
+        t = it == tpb_choice.end() ? 256 : it->second / 32 * 32;  // whole warps, whatever a table says
+        if (t < 32) t = 32;
     }
     return t > maxt ? maxt : t;
 }
