@@ -194,7 +194,7 @@ static const RegionTable& shell_table(Ctx& c, int ng, int nodal) {
         }
     }
     t.total = start;
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -232,7 +232,7 @@ static const RegionTable& down_table(Ctx& cf, const Ctx& cc, int nodal) {
         }
     }
     t.total = start;
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(cf, t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -279,7 +279,7 @@ static const RegionTable& coarse_shell_table(Ctx& cf, int ng) {
                 push(lo, hi);
             }
     }
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(cf, t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -463,7 +463,7 @@ static const RegionTable& reg_table(Ctx& cf, int o) {
         t.h.push_back(r);
     }
     t.total = start;
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(cf, t.h, t.total, REGION_HINT);
     return t;
 }
 

@@ -77,7 +77,7 @@ const RegionTable& region(Ctx& c, int glo0, int glo1, int glo2, int ghi0, int gh
         }
     }
     t.total = start;
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -101,7 +101,7 @@ const RegionTable& region_union(Ctx& c, const std::vector<RegionKey>& parts) {
     RegionTable& t = c.unions[key];
     t.h = h;
     t.total = total;
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -125,7 +125,7 @@ const RegionTable& region_columns(Ctx& c, const std::vector<RegionKey>& parts) {
         t.total += (long)r.n[0] * r.n[1] * r.n[2];
         t.h.push_back(r);
     }
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -232,7 +232,7 @@ const CopyTable& copy_table(Ctx& c, int ng, int nodal) {
         }
     }
     t.total = start;
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, COPY_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, COPY_HINT);
     return t;
 }
 
@@ -254,7 +254,7 @@ const CopyTable& copy_table_faces(Ctx& c, int ng) {
     CopyTable& t = c.copies[key];
     t.h = h;
     t.total = total;
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, COPY_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, COPY_HINT);
     return t;
 }
 

@@ -117,32 +117,6 @@ struct CopyTable {
     long total = 0;
 };
 
-// The pieces of a table on the device, as find_piece reads them: extents' reciprocals set, one
-// more piece that starts at the total, then the piece of every (1 << sh)th element.
-template <typename Piece>
-Piece* upload_pieces(std::vector<Piece>& h, long total, int sh) {
-    for (Piece& p : h) p.dv = piece_div(p.n);
-    const size_t nh = (size_t)(total >> sh) + 1, bytes = sizeof(Piece) * (h.size() + 1);
-    std::vector<char> buf(bytes + sizeof(int) * nh);
-    Piece end{};
-    end.start = total;
-    memcpy(buf.data(), h.data(), sizeof(Piece) * h.size());
-    memcpy(buf.data() + sizeof(Piece) * h.size(), &end, sizeof(Piece));
-    int* hint = reinterpret_cast<int*>(buf.data() + bytes);
-    size_t e = 0;
-    for (size_t q = 0; q < nh; ++q) {
-        while (e + 1 < h.size() && h[e + 1].start <= (long)(q << sh)) ++e;
-        hint[q] = (int)e;
-    }
-    Piece* d = nullptr;
-    if (cudaMalloc(&d, buf.size()) != cudaSuccess) throw Fail{MADV_ERR_CUDA};
-    if (cudaMemcpy(d, buf.data(), buf.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaFree(d);
-        throw Fail{MADV_ERR_CUDA};
-    }
-    return d;
-}
-
 struct Ctx {
     madv_params P{};  // dx, domain and base_cutoff_density_coord are this level's
     int lev = 0;
@@ -253,6 +227,35 @@ struct Hier {
     int n() const { return (int)L.size(); }
     Ctx& operator[](int l) const { return *L[l]; }
 };
+
+// The pieces of a table on the device, as find_piece reads them: extents' reciprocals set, one
+// more piece that starts at the total, then the piece of every (1 << sh)th element.
+template <typename Piece>
+Piece* upload_pieces(const Ctx& c, std::vector<Piece>& h, long total, int sh) {
+    for (Piece& p : h) p.dv = piece_div(p.n);
+    const size_t nh = (size_t)(total >> sh) + 1, bytes = sizeof(Piece) * (h.size() + 1);
+    std::vector<char> buf(bytes + sizeof(int) * nh);
+    Piece end{};
+    end.start = total;
+    memcpy(buf.data(), h.data(), sizeof(Piece) * h.size());
+    memcpy(buf.data() + sizeof(Piece) * h.size(), &end, sizeof(Piece));
+    int* hint = reinterpret_cast<int*>(buf.data() + bytes);
+    size_t e = 0;
+    for (size_t q = 0; q < nh; ++q) {
+        while (e + 1 < h.size() && h[e + 1].start <= (long)(q << sh)) ++e;
+        hint[q] = (int)e;
+    }
+    Piece* d = nullptr;
+    if (cudaMalloc(&d, buf.size()) != cudaSuccess) throw Fail{MADV_ERR_CUDA};
+    // The copy is the default stream's, and may still be on its way when it returns; a stream of the
+    // caller's does not wait for it, and the kernels read a table before MADV_WAIT.
+    if (cudaMemcpy(d, buf.data(), buf.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+        ((c.stream || c.comp_streams) && cudaStreamSynchronize(nullptr) != cudaSuccess)) {
+        cudaFree(d);
+        throw Fail{MADV_ERR_CUDA};
+    }
+    return d;
+}
 
 // Region of each box: the valid cell box grown by glo (low side) / ghi (high side), with
 // `nodal` marking a face-centred index space (hi[nodal] + 1 before growing).

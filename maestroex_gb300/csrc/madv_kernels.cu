@@ -377,7 +377,7 @@ static const RegionTable& outside_cells(Ctx& c, int ng) {
             rest.n[d] = hi - lo + 1;
         }
     }
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -488,7 +488,7 @@ static const RegionTable& ghost_planes(Ctx& c, int dd) {
             t.total += (long)r.n[0] * r.n[1] * r.n[2];
             t.h.push_back(r);
         }
-    if (!t.h.empty()) t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
     return t;
 }
 

@@ -181,7 +181,7 @@ static const RegionTable& march_region(Ctx& c, int D) {
         t.total += (long)r.n[0] * r.n[1] * r.n[2];
         t.h.push_back(r);
     }
-    t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
     return t;
 }
 
@@ -644,7 +644,7 @@ static const RegionTable& dirs_region(Ctx& c, bool nodal, int g) {
             t.total += (long)r.n[0] * r.n[1] * r.n[2];
             t.h.push_back(r);
         }
-    t.d = upload_pieces(t.h, t.total, REGION_HINT);
+    t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
     return t;
 }
 
