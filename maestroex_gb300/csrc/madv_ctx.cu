@@ -2093,7 +2093,7 @@ static int begin_call(madv_ctx* h, void* stream, Hier& H, bool levels = false) {
     if (rc) return rc;
     set_mode(H, (cudaStream_t)stream, 0, false);
     reset_launches(H);
-    cudaMemsetAsync(h->c.d_flag, 0, sizeof(int), h->c.stream);
+    for (auto* c : H.L) cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->stream);  // finish reads every level's
     return MADV_OK;
 }
 
