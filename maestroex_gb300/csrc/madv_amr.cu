@@ -154,7 +154,7 @@ static const RegionTable& shell_table(Ctx& c, int ng, int nodal) {
     std::array<int, 4> key{0, ng, nodal, 0};
     auto it = c.amr_tables.find(key);
     if (it != c.amr_tables.end()) return it->second;
-    RegionTable& t = c.amr_tables[key];
+    RegionTable t;
     long start = 0;
     auto push = [&](int b, const int lo[3], const int hi[3]) {
         RegionBox r{};
@@ -195,7 +195,7 @@ static const RegionTable& shell_table(Ctx& c, int ng, int nodal) {
     }
     t.total = start;
     if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
-    return t;
+    return c.amr_tables[key] = std::move(t);
 }
 
 // Coarse cells (nodal = -1) or coarse d-faces under each fine box, split by the coarse box
@@ -205,7 +205,7 @@ static const RegionTable& down_table(Ctx& cf, const Ctx& cc, int nodal) {
     std::array<int, 4> key{1, nodal, 0, 0};
     auto it = cf.amr_tables.find(key);
     if (it != cf.amr_tables.end()) return it->second;
-    RegionTable& t = cf.amr_tables[key];
+    RegionTable t;
     long start = 0;
     for (int fb = 0; fb < cf.nb; ++fb) {
         int clo[3], chi[3];
@@ -233,7 +233,7 @@ static const RegionTable& down_table(Ctx& cf, const Ctx& cc, int nodal) {
     }
     t.total = start;
     if (!t.h.empty()) t.d = upload_pieces(cf, t.h, t.total, REGION_HINT);
-    return t;
+    return cf.amr_tables[key] = std::move(t);
 }
 
 // The coarse cells under the ghost cells (ng deep) of the fine boxes; pad, ext, len: the fine
@@ -242,7 +242,7 @@ static const RegionTable& coarse_shell_table(Ctx& cf, int ng) {
     std::array<int, 4> key{3, ng, 0, 0};
     auto it = cf.amr_tables.find(key);
     if (it != cf.amr_tables.end()) return it->second;
-    RegionTable& t = cf.amr_tables[key];
+    RegionTable t;
     for (int b = 0; b < cf.nb; ++b) {
         HBox g, v;  // with the ghost cells and without
         for (int d = 0; d < 3; ++d) {
@@ -280,7 +280,7 @@ static const RegionTable& coarse_shell_table(Ctx& cf, int ng) {
             }
     }
     if (!t.h.empty()) t.d = upload_pieces(cf, t.h, t.total, REGION_HINT);
-    return t;
+    return cf.amr_tables[key] = std::move(t);
 }
 
 // ------------------------------------------------------------------ kernels
@@ -444,7 +444,7 @@ static const RegionTable& reg_table(Ctx& cf, int o) {
     std::array<int, 4> key{2, o, 0, 0};
     auto it = cf.amr_tables.find(key);
     if (it != cf.amr_tables.end()) return it->second;
-    RegionTable& t = cf.amr_tables[key];
+    RegionTable t;
     const int D = o % 3, side = o / 3;
     long start = 0;
     for (int fb = 0; fb < cf.nb; ++fb) {
@@ -464,7 +464,7 @@ static const RegionTable& reg_table(Ctx& cf, int o) {
     }
     t.total = start;
     if (!t.h.empty()) t.d = upload_pieces(cf, t.h, t.total, REGION_HINT);
-    return t;
+    return cf.amr_tables[key] = std::move(t);
 }
 
 // register storage of a fine level: [orientation][face][component], allocated on first use

@@ -38,7 +38,7 @@ const RegionTable& region(Ctx& c, int glo0, int glo1, int glo2, int ghi0, int gh
     std::array<int, 8> key{glo0, glo1, glo2, ghi0, ghi1, ghi2, nodal, slab};
     auto it = c.regions.find(key);
     if (it != c.regions.end()) return it->second;
-    RegionTable& t = c.regions[key];
+    RegionTable t;
     const int glo[3] = {glo0, glo1, glo2}, ghi[3] = {ghi0, ghi1, ghi2};
     long start = 0;
     auto push = [&](int b, const int lo[3], const int hi[3]) {
@@ -78,7 +78,7 @@ const RegionTable& region(Ctx& c, int glo0, int glo1, int glo2, int ghi0, int gh
     }
     t.total = start;
     if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
-    return t;
+    return c.regions[key] = std::move(t);
 }
 
 const RegionTable& region_union(Ctx& c, const std::vector<RegionKey>& parts) {
@@ -98,11 +98,11 @@ const RegionTable& region_union(Ctx& c, const std::vector<RegionKey>& parts) {
         }
         total += r.total;
     }
-    RegionTable& t = c.unions[key];
+    RegionTable t;
     t.h = h;
     t.total = total;
     if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
-    return t;
+    return c.unions[key] = std::move(t);
 }
 
 const RegionTable& region_columns(Ctx& c, const std::vector<RegionKey>& parts) {
@@ -114,7 +114,7 @@ const RegionTable& region_columns(Ctx& c, const std::vector<RegionKey>& parts) {
     const int len = (int)std::min(8L, u.total >> 19);
     if (len <= 1) return u;
     const std::vector<RegionBox> h = u.h;
-    RegionTable& t = c.unions[key];
+    RegionTable t;
     t.columns = true;
     for (RegionBox r : h) {
         r.ext = r.n[2];
@@ -126,7 +126,7 @@ const RegionTable& region_columns(Ctx& c, const std::vector<RegionKey>& parts) {
         t.h.push_back(r);
     }
     if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
-    return t;
+    return c.unions[key] = std::move(t);
 }
 
 // a minus b as up to six disjoint boxes appended to out
@@ -163,7 +163,7 @@ const CopyTable& copy_table(Ctx& c, int ng, int nodal) {
     std::array<int, 3> key{ng, nodal, 0};
     auto it = c.copies.find(key);
     if (it != c.copies.end()) return it->second;
-    CopyTable& t = c.copies[key];
+    CopyTable t;
     int len[3];
     for (int d = 0; d < 3; ++d) len[d] = c.P.dom_hi[d] - c.P.dom_lo[d] + 1;
     long start = 0;
@@ -233,7 +233,7 @@ const CopyTable& copy_table(Ctx& c, int ng, int nodal) {
     }
     t.total = start;
     if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, COPY_HINT);
-    return t;
+    return c.copies[key] = std::move(t);
 }
 
 const CopyTable& copy_table_faces(Ctx& c, int ng) {
@@ -251,11 +251,11 @@ const CopyTable& copy_table_faces(Ctx& c, int ng) {
         }
         total += one.total;
     }
-    CopyTable& t = c.copies[key];
+    CopyTable t;
     t.h = h;
     t.total = total;
     if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, COPY_HINT);
-    return t;
+    return c.copies[key] = std::move(t);
 }
 
 // ------------------------------------------------------------------ setup helpers

@@ -7,6 +7,7 @@
 #include <functional>
 #include <map>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/maestro_adv.h"

@@ -358,7 +358,7 @@ static const RegionTable& outside_cells(Ctx& c, int ng) {
     auto it = c.regions.find(key);
     if (it != c.regions.end()) return it->second;
     const std::vector<RegionBox> grown = rg_grow(c, ng).h;
-    RegionTable& t = c.regions[key];
+    RegionTable t;
     for (const RegionBox& g : grown) {
         RegionBox rest = g;  // z slabs (full x, y), then y slabs of the rest, then x slabs
         for (int d = 2; d >= 0; --d) {
@@ -378,7 +378,7 @@ static const RegionTable& outside_cells(Ctx& c, int ng) {
         }
     }
     if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
-    return t;
+    return c.regions[key] = std::move(t);
 }
 
 static void phys_ranges(Ctx& c, int fid, int c0, int nc, const BCRecD* bcs, int c1, int nc1, const BCRecD* bcs1) {
@@ -477,7 +477,7 @@ static const RegionTable& ghost_planes(Ctx& c, int dd) {
     auto it = c.regions.find(key);
     if (it != c.regions.end()) return it->second;
     const std::vector<RegionBox> grown = region(c, 1, 1, 1, 1, 1, 1, dd).h;
-    RegionTable& t = c.regions[key];
+    RegionTable t;
     for (const RegionBox& g : grown)
         for (int I : {c.P.dom_lo[dd] - 1, c.P.dom_hi[dd] + 2}) {
             if (I < g.lo[dd] || I >= g.lo[dd] + g.n[dd]) continue;
@@ -489,7 +489,7 @@ static const RegionTable& ghost_planes(Ctx& c, int dd) {
             t.h.push_back(r);
         }
     if (!t.h.empty()) t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
-    return t;
+    return c.regions[key] = std::move(t);
 }
 
 void fill_face_ghosts(Ctx& c, int f0) {

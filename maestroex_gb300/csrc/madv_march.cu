@@ -158,7 +158,7 @@ static const RegionTable& march_region(Ctx& c, int D) {
     const std::array<int, 8> key{1000, D, c.P.ppm_type, 0, 0, 0, 0, 0};
     auto it = c.regions.find(key);
     if (it != c.regions.end()) return it->second;
-    RegionTable& t = c.regions[key];
+    RegionTable t;
     const int len = march_len(c);
     for (int b = 0; b < c.nb; ++b) {
         RegionBox r{};
@@ -182,7 +182,7 @@ static const RegionTable& march_region(Ctx& c, int D) {
         t.h.push_back(r);
     }
     t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
-    return t;
+    return c.regions[key] = std::move(t);
 }
 
 template <int D, int PPMT, int UMAC>
@@ -622,7 +622,7 @@ static const RegionTable& dirs_region(Ctx& c, bool nodal, int g) {
     const std::array<int, 8> key{1001, nodal, g, 0, 0, 0, 0, 0};
     auto it = c.regions.find(key);
     if (it != c.regions.end()) return it->second;
-    RegionTable& t = c.regions[key];
+    RegionTable t;
     long cells = 0;
     for (const HBox& v : c.ba) cells += (long)(v.hi[0] - v.lo[0] + 1) * (v.hi[1] - v.lo[1] + 1) * (v.hi[2] - v.lo[2] + 1);
     const int len = (int)std::min(ES_LEN, std::max(1L, 3 * cells >> 19));
@@ -645,7 +645,7 @@ static const RegionTable& dirs_region(Ctx& c, bool nodal, int g) {
             t.h.push_back(r);
         }
     t.d = upload_pieces(c, t.h, t.total, REGION_HINT);
-    return t;
+    return c.regions[key] = std::move(t);
 }
 
 // Edge states of components comp0 .. comp0 + nq - 1 (nq <= 3; conservative form: 1) of F_SOLD, 3-D,
