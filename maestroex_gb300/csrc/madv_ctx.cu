@@ -2141,6 +2141,7 @@ int madv_addw0(madv_ctx* h, const madv_multifab* umac, double mult, void* stream
             if ((rc = bind(c, U_UMAC0 + d, &umac[d], 1, d, 1))) return rc;
         if ((rc = upload_user_views(c))) return rc;
         for (int d = 0; d < c.ndim; ++d) copy_fab(c, F_UMAC0 + d, 0, F_USER + U_UMAC0 + d, 0, 1, 1);
+        if (c.sph) w0_carts(H);  // w0mac of this base state
         addw0_h(H, F_UMAC0, mult);
         for (int d = 0; d < c.ndim; ++d) copy_fab(c, F_USER + U_UMAC0 + d, 0, F_UMAC0 + d, 0, 1, 1);
         return finish(H);
