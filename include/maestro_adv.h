@@ -321,9 +321,10 @@ int madv_ppm(madv_ctx* ctx, const madv_box* bx, const madv_fab* s, int comp, con
  * cudaMalloc where they run PPM -- e.g. an AMReX application whose arena already holds most
  * of the GPU's memory, or code that must avoid the implicit device synchronisation of
  * cudaMalloc and cudaFree.  No counterpart in the reference.  Same arguments and results as
- * madv_ppm, with the parameters taken from `params` instead of a context.  A box whose
- * intermediates would take more than MADV_PPM_NOALLOC_MAX_DOUBLES doubles (larger than
- * 66 x 66 x 66 cells) is rejected with MADV_ERR_LAYOUT. */
+ * madv_ppm, with the parameters taken from `params` instead of a context.  A box larger than
+ * 66 x 66 x 66 cells is rejected with MADV_ERR_LAYOUT: the limit of an earlier form that kept
+ * MADV_PPM_NOALLOC_MAX_DOUBLES doubles of intermediates in a static array, kept for its
+ * callers; nothing is held any more, and madv_ppm takes any size. */
 #define MADV_PPM_NOALLOC_MAX_DOUBLES 1184832
 int madv_ppm_noalloc(const madv_params* params, const madv_box* bx, const madv_fab* s, int comp,
                      const madv_fab* u, const madv_fab* v, const madv_fab* w, int is_umac,
@@ -384,7 +385,8 @@ int madv_profile_report(madv_ctx* ctx, char* buf, int len);
  *     madv_autotune_finish(ctx, json, len);
  * finish picks the fastest candidate per (level, kernel), applies it to later launches and
  * graphs, and writes the table {"L<level> <kernel symbol>": threads, ...} (a cache for
- * madv_autotune_apply in a later run).  Kernels are clamped to the block size they can take.
+ * madv_autotune_apply in a later run).  Kernels are clamped to the block size they can take,
+ * and a table's sizes are brought down to whole warps (at least one).
  * No counterpart in the reference. */
 int madv_autotune_trial(madv_ctx* ctx, int threads);
 /* The PPM form, tuned the same way per level: for each form f in [0, MADV_AUTOTUNE_PPM_FORMS):

@@ -918,7 +918,7 @@ __global__ void k_adj_pert(KARGS, int comp, const double* __restrict__ s0a, cons
     }
 }
 
-// Transverse coefficients transposed (k_transverse_coeffs: per cell c and direction t,
+// Transverse coefficients transposed (transverse_coeffs_cell: per cell c and direction t,
 // dt6/h_t (u_t(c+e_t) + u_t(c)) and dt4/h_t (...)), gathered per t-face from the two
 // cells that read it: the adjoints of F_TCOEF are in A_ATCOEF, the face-velocity adjoint
 // is added to slot ts + T.

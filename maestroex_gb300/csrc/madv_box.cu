@@ -6,7 +6,8 @@
 // the level kernels (madv_march.cuh: columns marched along y and z, rows by shuffles, ppm_type
 // 2's limited cells listed) with the tracing coefficients formed where they are used.  No
 // scratch.  Twelve dependent launches with every intermediate in memory spent their time
-// between launches: 63 us a call for a 34^3 box, 27 us now with the caller's side of it.
+// between launches: 63 us a call for a 34^3 box, 28 us now (17 us on the device, the rest the
+// caller's side and the launch).
 #include "madv_ctx.hpp"
 #include "madv_exact.cuh"
 #include "madv_launch.cuh"

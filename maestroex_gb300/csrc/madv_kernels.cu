@@ -5,11 +5,15 @@
 // the reference expression for expression (same operands, same order, IEEE binary64,
 // no FMA contraction: the library is built with --fmad=false), so results match the
 // reference algorithm bit for bit.  What changes is the amount of FP64 work: GB300 issues
-// FP64 at a small fraction of its FP32 rate, so every intermediate of the stage is
-// computed once and stored, where the reference recomputes it:
-//   * PPM: the limited interface value of each face is computed once per face (the
-//     reference evaluates four van Leer slopes and two interface values per cell and
-//     direction, and in MakeUtrans sweeps all three directions where one is used);
+// FP64 at a small fraction of its FP32 rate, so an intermediate is formed once where the
+// reference recomputes it, and kept where that costs least:
+//   * PPM and the edge states of 3-D scalars run in madv_march.cu, which passes slopes and interface
+//     values on in registers; the separate kernels here (k_dsvl, k_ppm_face, k_ppm_cell, the
+//     predictor, transverse and edge kernels) store them, for the adjoint's taped forward,
+//     es_inline = 0 and sweeps too long for the staged form;
+//   * MakeUtrans' sweeps of the velocity are VelPred's, made once;
+//   * what depends on the velocity alone (tracing and transverse coefficients) is stored once
+//     for all components;
 //   * constant quotients such as (dt/6)/dy are formed once on the host, where the
 //     reference forms them per element (same IEEE operations, same values).
 #include <cstdio>
@@ -2005,7 +2009,7 @@ void update_rhox_fix(Ctx& c) {
 // have k = 0 only, two velocity components.  Regions of a 2-D context never grow in z.
 // PPM, the limited slopes, the fills and the x-face transverse velocity are the 3-D
 // kernels run in x and y; the kernels below restate the 2-D branches of the reference
-// (their expressions and quirks differ from 3-D), with plain IEEE division.
+// (their expressions and quirks differ from 3-D).
 namespace madv {
 
 static const RegionTable& rg2(Ctx& c, int g, int nodal = -1) { return region(c, g, g, 0, g, g, 0, nodal); }

@@ -1,16 +1,17 @@
 // PPM and the scalar edge states with the intermediates of a direction in registers.
 //
 // What bounds it: FP64 issue.  One FP64 warp instruction takes the issue slots of about 64
-// others on GB300 (1.68 FP64 lanes a clock and SM measured), so the FP64 instructions of the method are
+// others on GB300 (2 FP64 lanes a clock and SM), so the FP64 instructions of the method are
 // the floor, and every launch that stores an intermediate adds an index computation, its
 // loads and its latency.  Three launches a direction (slopes, interfaces, cells) and twelve
 // for the corner coupling of one component become six for up to three components:
 //   k_ppm_march<D>  y and z: a thread marches along D over a chunk of a column, lanes along x.
 //                   Every difference, slope and interface value is formed once and passed on
-//                   in registers: 20 FP64 instructions a cell (ppm_type 1) against 23 in three
-//                   launches, one load of the state instead of nine.
+//                   in registers: 23 FP64 instructions a cell (ppm_type 1, counted) against 41 in
+//                   three launches, one load of the state instead of nine.
 //   k_ppm_rows      x: lanes along the row, slopes and interface values passed to the
-//                   neighbour lane by shuffles, the warps overlapping by 2 lanes.  A march across lanes would read 32 rows at once.
+//                   neighbour lane by shuffles, the warps overlapping by 2 lanes.  A march
+//                   across lanes would read 32 rows at once.
 //   k_ppm_march2, k_ppm_rows2  the same for ppm_type 2, the limited faces and cells listed and
 //                   finished 32 at a time (madv_march.cuh): three components at 128^3 0.26 ms a
 //                   direction, 0.47 ms with the limiter in place (the velocity's sweeps 0.43

@@ -9,15 +9,15 @@
 // shared memory, so this entry point holds no memory of its own and calls on different
 // streams do not meet.
 //
-// The size limit is the entry point's contract: a box up to 66 x 66 x 66 cells (a 64^3 box
-// grown by one cell, the box the reference passes to PPM) is accepted, a box whose
-// intermediates would exceed MADV_PPM_NOALLOC_MAX_DOUBLES doubles is rejected with
-// MADV_ERR_LAYOUT before anything runs.
+// The size limit is kept for its callers' sake alone: it was that of a static array of
+// MADV_PPM_NOALLOC_MAX_DOUBLES doubles of intermediates, which is gone.  A box up to 66 x 66 x 66
+// cells (a 64^3 box grown by one cell, the box the reference passes to PPM) is accepted, a
+// larger one is rejected with MADV_ERR_LAYOUT before anything runs, as before.
 #include "madv_ctx.hpp"
 
 using namespace madv;
 
-// Doubles of one direction's intermediates: interface values (n_d + 4 faces), van Leer slopes
+// The limit's measure: doubles of one direction's interface values (n_d + 4 faces), van Leer slopes
 // (n_d + 2 cells) and two tracing coefficients (n_d + 1 faces), the worst of the three.
 static long intermediates(const int n[3]) {
     long worst = 0;
